@@ -55,10 +55,11 @@ struct Timeout : std::runtime_error {
     using std::runtime_error::runtime_error;
 };
 
-// after a call's kernels have finished: did a TMA wait of the L_p pass give up?
+// after a call's kernels have finished: did a bounded wait of the L_p pass or of the sweeps give up?
 static void check_device_waits() {
-    if (lp_take_wait_timeouts())
-        throw Timeout("a TMA load of the L_p product's FFT grid did not arrive within its wait limit");
+    const bool lp = lp_take_wait_timeouts() != 0, sweep = sweep_take_wait_timeouts() != 0;
+    if (lp) throw Timeout("a TMA load of the L_p product's FFT grid did not arrive within its wait limit");
+    if (sweep) throw Timeout("a wait inside the preconditioner's triangular sweeps ran out");
 }
 
 // Device allocations owned by an object, freed together.
@@ -215,11 +216,14 @@ struct Workspace {
     // inner (precision R) per slot
     void *V = nullptr, *w = nullptr, *z = nullptr, *T = nullptr, *zfac = nullptr, *yfac = nullptr, *uvec = nullptr,
          *sd = nullptr, *vcur = nullptr;
+    // the FP32 sweeps: solutions interleaved by column group (zfac, uvec likewise), and the tiles' counters
+    c32* yint = nullptr;
+    int* cnt = nullptr;
     c64* partial = nullptr;
     // precision 3: the FP32 inner solve's preconditioner applied in FP64 (input, output and the sweeps' vectors)
     c64 *pr64 = nullptr, *pz64 = nullptr, *zfac64 = nullptr, *yfac64 = nullptr, *uvec64 = nullptr, *sd64 = nullptr;
     GmresState st{};
-    int *slot_col = nullptr, *slot_op = nullptr, *g_ptr = nullptr, *g_slot = nullptr, *g_op = nullptr, *col_op = nullptr;
+    int *slot_col = nullptr, *slot_op = nullptr, *g_ptr = nullptr, *g_slot = nullptr, *g_op = nullptr, *g_pair = nullptr, *col_op = nullptr;
     int* slot_pc = nullptr;      // each slot's factorisation (the preconditioner's tables, panels and pivots)
     int* act = nullptr;
     int* act_host = nullptr;
@@ -244,6 +248,8 @@ struct gt_geometry {
     Geo geo{};
     Orient o[2]{};
     Fronts F{};
+    SweepPlan sweep{};
+    std::vector<int> sweep_level_f, sweep_level_b;   // the plan's tasks up to the end of each level (backward: root first)
     Pool pool;
     std::vector<int64_t> level_ptr;
     std::vector<int> level_maxnf, level_maxnown;
@@ -311,9 +317,9 @@ struct gt_operators {
     c32* tab32 = nullptr;        // the admittance table rounded to FP32 (the FP32 preconditioner's stencils)
     // per front P = [Linv_own; -L_bnd Linv_own] (nf x nown) and the pivot reciprocals dinv ([op][nfac])
     c64* panel64 = nullptr;      // column-major per front (forward solves)
-    c32* panel32 = nullptr;
     c64* panel64_rm = nullptr;   // row-major copies (backward solves)
-    c32* panel32_rm = nullptr;
+    c32* panel32 = nullptr;      // the FP32 sweeps' forward and backward tiles (sweep.cu)
+    c32* panel32_b = nullptr;
     c64* dinv64 = nullptr;
     c32* dinv32 = nullptr;
     std::vector<int> own;        // the operator whose frequency each factorisation was made at
@@ -364,18 +370,9 @@ template <> const c64* tw0_of<double>(const Orient& o) { return o.tw0_64; }
 template <typename R> static const cx<R>* tw1_of(const Orient& o);
 template <> const c32* tw1_of<float>(const Orient& o) { return o.tw1_32; }
 template <> const c64* tw1_of<double>(const Orient& o) { return o.tw1_64; }
-template <typename R> static const cx<R>* panel_of(const gt_operators* ops);
-template <> const c32* panel_of<float>(const gt_operators* ops) { return ops->panel32; }
-template <> const c64* panel_of<double>(const gt_operators* ops) { return ops->panel64; }
-template <typename R> static const cx<R>* panel_rm_of(const gt_operators* ops);
-template <> const c32* panel_rm_of<float>(const gt_operators* ops) { return ops->panel32_rm; }
-template <> const c64* panel_rm_of<double>(const gt_operators* ops) { return ops->panel64_rm; }
 template <typename R> static const cx<R>* tab_of(const gt_operators* ops);
 template <> const c32* tab_of<float>(const gt_operators* ops) { return ops->tab32; }
 template <> const c64* tab_of<double>(const gt_operators* ops) { return ops->tab; }
-template <typename R> static const cx<R>* dinv_of(const gt_operators* ops);
-template <> const c32* dinv_of<float>(const gt_operators* ops) { return ops->dinv32; }
-template <> const c64* dinv_of<double>(const gt_operators* ops) { return ops->dinv64; }
 template <typename R> static const cx<R>* low_w_of(const gt_operators* ops);
 template <> const c32* low_w_of<float>(const gt_operators* ops) { return ops->low_w32; }
 template <> const c64* low_w_of<double>(const gt_operators* ops) { return ops->low_w64; }
@@ -518,72 +515,101 @@ static void matvec(gt_geometry* G, gt_operators* ops, const cx<R>* x, const cx<R
     }
 }
 
-// out = M^-1 r for nslot slots whose vectors are ldr apart (inputs) and ldo apart (outputs)
-template <typename R>
-static void precond(gt_geometry* G, gt_operators* ops, const cx<R>* r, int64_t ldr, cx<R>* out, int64_t ldo, int nslot,
-                    const int* slot_op, const Groups& grp, int gmax, cx<R>* zfac, cx<R>* yfac, cx<R>* uvec, cx<R>* sd,
-                    cudaStream_t st,
-                    const int* col_list = nullptr) {
+// the FP32 sweeps over all groups: one launch, or, with the profiler's level timing, one per elimination level
+static void sweep32(gt_geometry* G, const gt_operators* ops, const Groups& grp, const c32* s, c32* z, c32* y, c32* u, c32* sd,
+                    int* cnt, int nslot, cudaStream_t st) {
     Profiler* P = &G->prof;
-    if (!panel_of<R>(ops) || !panel_rm_of<R>(ops))
-        throw Invalid("these operators keep their FP32 panels only (GT_OPS_FP32_PANELS): no FP64 preconditioner");
-    const double es = sizeof(cx<R>), n = (double)G->geo.n, nfac = (double)G->F.nfac;
-    const double nodes = (double)G->geo.S * G->geo.nx * G->geo.ny, nXYC = (double)(G->geo.off_b - G->geo.off_x);
-    // the factor's panels are read once per column group in each direction
-    const double panel = (double)grp.ngroup * es * G->F.panel_total;
-    {
-        Scope s(P, "pc_node", st, nslot * es * (nXYC + nodes + nfac));
-        launch_pc_node<R>(G->geo, r, ldr, yfac, nslot, slot_op, tab_of<R>(ops), col_list, st);
+    const double es = sizeof(c32), panel = (double)grp.ngroup * es * G->F.panel_total, nfac = (double)G->F.nfac;
+    auto run = [&](int t0, int t1) {
+        launch_sweep(G->sweep, G->F, ops->panel32, ops->panel32_b, ops->dinv32, s, z, y, u, sd, grp, cnt, t0, t1, st);
+    };
+    const int nt = G->sweep.nft + G->sweep.nbt;
+    if (!P->on || !P->levels) {
+        Scope sc(P, "fwdbwd_f32", st, 2 * panel + nslot * es * (4 * nfac + 2.0 * G->F.vec_total));
+        run(0, nt);
+        return;
     }
-    const cx<R>* pan = panel_of<R>(ops);
     const int nlev = (int)G->level_ptr.size() - 1;
-    const int nsub = P->levels ? 1 : std::min(gt_geometry::NSUB, grp.ngroup);
+    for (int dir = 0; dir < 2; ++dir) {
+        Scope sc(P, dir ? "bwd_f32" : "fwd_f32", st, panel + nslot * es * (dir ? 2 * nfac : 2 * nfac + 2.0 * G->F.vec_total));
+        for (int q = 0; q < nlev; ++q) {
+            const std::vector<int>& end = dir ? G->sweep_level_b : G->sweep_level_f;
+            const int h = dir ? nlev - 1 - q : q;
+            Scope sl(P, ((dir ? "bwd_f32.L" : "fwd_f32.L") + std::to_string(h)).c_str(), st, grp.ngroup * es * G->level_panel[h]);
+            GT_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int), st));
+            run(q ? end[q - 1] : (dir ? G->sweep.nft : 0), end[q]);
+        }
+    }
+}
+
+// the FP64 sweeps, level by level; independent column groups on streams of their own
+static void sweep64(gt_geometry* G, const gt_operators* ops, const Groups& grp, int gmax, c64* s, c64* z, c64* u, c64* sd,
+                    int nslot, cudaStream_t st) {
+    Profiler* P = &G->prof;
+    const double es = sizeof(c64), panel = (double)grp.ngroup * es * G->F.panel_total, nfac = (double)G->F.nfac;
+    const int nlev = (int)G->level_ptr.size() - 1;
+    auto fwd = [&](int h, const Groups& g, cudaStream_t sk) {
+        launch_fwd_level<double>(G->F, G->d_order + G->level_ptr[h], (int)(G->level_ptr[h + 1] - G->level_ptr[h]),
+                                 G->level_maxnf[h], G->level_maxnown[h], ops->panel64, ops->dinv64, s, z, u, s, g, gmax, sk);
+    };
+    auto bwd = [&](int h, const Groups& g, cudaStream_t sk) {
+        launch_bwd_level<double>(G->F, G->d_order + G->level_ptr[h], (int)(G->level_ptr[h + 1] - G->level_ptr[h]),
+                                 G->level_maxnf[h], G->level_maxnown[h], ops->panel64_rm, z, s, sd, g, gmax, sk);
+    };
+    const bool levels = P->on && P->levels;
+    const int nsub = levels ? 1 : std::min(gt_geometry::NSUB, grp.ngroup);
     if (nsub > 1) {
         // forward and backward sweeps per stream, each on a share of the column groups
-        Scope s(P, sizeof(R) == 4 ? "fwdbwd_f32" : "fwdbwd_f64", st,
-                2 * panel + nslot * es * (4 * nfac + 2.0 * G->F.vec_total));
+        Scope sc(P, "fwdbwd_f64", st, 2 * panel + nslot * es * (4 * nfac + 2.0 * G->F.vec_total));
         G->make_streams();
         GT_CUDA(cudaEventRecord(G->fork, st));
         for (int k = 0; k < nsub; ++k) {
             cudaStream_t sk = G->sub[k];
             GT_CUDA(cudaStreamWaitEvent(sk, G->fork, 0));
             const int g0 = (int)((int64_t)k * grp.ngroup / nsub), g1 = (int)((int64_t)(k + 1) * grp.ngroup / nsub);
-            const Groups gk{g1 - g0, grp.gptr + g0, grp.gslot, grp.op + g0};
-            for (int h = 0; h < nlev; ++h) {
-                const int nf = (int)(G->level_ptr[h + 1] - G->level_ptr[h]);
-                launch_fwd_level<R>(G->F, G->d_order + G->level_ptr[h], nf, G->level_maxnf[h], G->level_maxnown[h],
-                                    pan, dinv_of<R>(ops), yfac, zfac, uvec, yfac, gk, gmax, sk);
-            }
-            for (int h = nlev - 1; h >= 0; --h) {
-                const int nf = (int)(G->level_ptr[h + 1] - G->level_ptr[h]);
-                launch_bwd_level<R>(G->F, G->d_order + G->level_ptr[h], nf, G->level_maxnf[h], G->level_maxnown[h],
-                                    panel_rm_of<R>(ops), zfac, yfac, sd, gk, gmax, sk);
-            }
+            const Groups gk{g1 - g0, grp.gptr + g0, grp.gslot, grp.op + g0, grp.pair0 + g0};
+            for (int h = 0; h < nlev; ++h) fwd(h, gk, sk);
+            for (int h = nlev - 1; h >= 0; --h) bwd(h, gk, sk);
             GT_CUDA(cudaEventRecord(G->join[k], sk));
             GT_CUDA(cudaStreamWaitEvent(st, G->join[k], 0));
         }
-    } else {
+        return;
+    }
     {
-        Scope s(P, sizeof(R) == 4 ? "fwd_f32" : "fwd_f64", st, panel + nslot * es * (2 * nfac + 2.0 * G->F.vec_total));
+        Scope sc(P, "fwd_f64", st, panel + nslot * es * (2 * nfac + 2.0 * G->F.vec_total));
         for (int h = 0; h < nlev; ++h) {
-            int nf = (int)(G->level_ptr[h + 1] - G->level_ptr[h]);
-            Scope sl(P->levels ? P : nullptr, (std::string(sizeof(R) == 4 ? "fwd_f32.L" : "fwd_f64.L") +
-                                               std::to_string(h)).c_str(), st, grp.ngroup * es * G->level_panel[h]);
-            launch_fwd_level<R>(G->F, G->d_order + G->level_ptr[h], nf, G->level_maxnf[h], G->level_maxnown[h], pan,
-                                dinv_of<R>(ops), yfac, zfac, uvec, yfac, grp, gmax, st);
+            Scope sl(levels ? P : nullptr, ("fwd_f64.L" + std::to_string(h)).c_str(), st, grp.ngroup * es * G->level_panel[h]);
+            fwd(h, grp, st);
         }
     }
     {
-        Scope s(P, sizeof(R) == 4 ? "bwd_f32" : "bwd_f64", st, panel + nslot * es * 2 * nfac);
+        Scope sc(P, "bwd_f64", st, panel + nslot * es * 2 * nfac);
         for (int h = nlev - 1; h >= 0; --h) {
-            int nf = (int)(G->level_ptr[h + 1] - G->level_ptr[h]);
-            Scope sl(P->levels ? P : nullptr, (std::string(sizeof(R) == 4 ? "bwd_f32.L" : "bwd_f64.L") +
-                                               std::to_string(h)).c_str(), st, grp.ngroup * es * G->level_panel[h]);
-            launch_bwd_level<R>(G->F, G->d_order + G->level_ptr[h], nf, G->level_maxnf[h], G->level_maxnown[h],
-                                panel_rm_of<R>(ops), zfac, yfac, sd, grp, gmax, st);
+            Scope sl(levels ? P : nullptr, ("bwd_f64.L" + std::to_string(h)).c_str(), st, grp.ngroup * es * G->level_panel[h]);
+            bwd(h, grp, st);
         }
     }
+}
+
+// out = M^-1 r for nslot slots whose vectors are ldr apart (inputs) and ldo apart (outputs).  yint and cnt are the FP32
+// sweeps' (null in FP64)
+template <typename R>
+static void precond(gt_geometry* G, gt_operators* ops, const cx<R>* r, int64_t ldr, cx<R>* out, int64_t ldo, int nslot,
+                    const int* slot_op, const Groups& grp, int gmax, cx<R>* zfac, cx<R>* yfac, cx<R>* uvec, cx<R>* sd,
+                    c32* yint, int* cnt, cudaStream_t st, const int* col_list = nullptr) {
+    constexpr bool f32 = sizeof(R) == 4;
+    Profiler* P = &G->prof;
+    if (!f32 && (!ops->panel64 || !ops->panel64_rm))
+        throw Invalid("these operators keep their FP32 panels only (GT_OPS_FP32_PANELS): no FP64 preconditioner");
+    const double es = sizeof(cx<R>), n = (double)G->geo.n, nfac = (double)G->F.nfac;
+    const double nodes = (double)G->geo.S * G->geo.nx * G->geo.ny, nXYC = (double)(G->geo.off_b - G->geo.off_x);
+    {
+        Scope s(P, "pc_node", st, nslot * es * (nXYC + nodes + nfac));
+        launch_pc_node<R>(G->geo, r, ldr, yfac, nslot, slot_op, tab_of<R>(ops), col_list, f32 ? cnt : nullptr,
+                          f32 ? sweep_counters(G->F.nfront, grp.ngroup) : 0, st);
     }
+    if constexpr (f32) sweep32(G, ops, grp, yfac, zfac, yint, uvec, sd, cnt, nslot, st);
+    else sweep64(G, ops, grp, gmax, yfac, zfac, uvec, sd, nslot, st);
     if (ops->nlow) {
         // the derived stack's added branches: y -= W Minv U^T y (the coefficients in zfac, free after the sweeps)
         Scope s(P, "lowrank", st, nslot * es * (double)G->F.nnode * (ops->nlow + 2));
@@ -596,11 +622,12 @@ static void precond(gt_geometry* G, gt_operators* ops, const cx<R>* r, int64_t l
     }
 }
 
-// The triangular sweeps stage, per block, a front's rows for every column of a group in shared memory: the own
+// The FP64 triangular sweeps stage, per block, a front's rows for every column of a group in shared memory: the own
 // and boundary rows of the forward assembly (max_nown + max_nf), the own rows plus up to 17 x 32 rows of tiles
 // and partial sums of the forward products (max_nown + 544), the front's rows plus up to 16 x 32 partial sums of
 // the backward products (max_nf + 512).  The widest group of 8, 4, 2 or 1 columns whose staging fits a block's
-// 227 KB is taken (narrower groups read the panel once per fewer columns); 0 when not even one column fits.
+// 227 KB is taken (narrower groups read the panel once per fewer columns); 0 when not even one column fits.  The FP32
+// sweeps stream a front's rows through fixed stages: 8 columns for any front.
 static int group_width(const gt_geometry* G, size_t elem) {
     size_t nown = 1;
     for (int v : G->level_maxnown) nown = std::max(nown, (size_t)v);
@@ -609,7 +636,7 @@ static int group_width(const gt_geometry* G, size_t elem) {
     const char* cap_env = std::getenv("GT_GROUP_WIDTH");       // a lower cap, for tests of the narrow groups
     const int cap = cap_env ? std::atoi(cap_env) : 8;
     for (int gc : {8, 4, 2, 1})
-        if (gc <= cap && (size_t)gc * rows * elem <= 227 * 1024) return gc;
+        if (gc <= cap && (elem == sizeof(c32) || (size_t)gc * rows * elem <= 227 * 1024)) return gc;
     return 0;
 }
 
@@ -623,10 +650,11 @@ static int group_max(const gt_geometry* G, size_t elem) {
 
 
 // the listed slots (sorted by operator) -> groups of <= gmax slots sharing one operator:
-// group g holds gslot[gptr[g] .. gptr[g+1])
+// group g holds gslot[gptr[g] .. gptr[g+1]); pair0[g]: the column pairs before it in the FP32 sweeps' vectors
 static void make_groups(const std::vector<int>& slots, const std::vector<int>& slot_op, int gmax, std::vector<int>& gptr,
-                        std::vector<int>& gslot, std::vector<int>& op) {
+                        std::vector<int>& gslot, std::vector<int>& op, std::vector<int>& pair0) {
     gptr.assign(1, 0);
+    pair0.assign(1, 0);
     gslot.clear();
     op.clear();
     int n = (int)slots.size();
@@ -636,6 +664,7 @@ static void make_groups(const std::vector<int>& slots, const std::vector<int>& s
         for (int q = s; q < e; ++q) gslot.push_back(slots[q]);
         gptr.push_back((int)gslot.size());
         op.push_back(slot_op[slots[s]]);
+        pair0.push_back(pair0.back() + (e - s <= 2 ? 1 : e - s <= 4 ? 2 : 4));
         s = e;
     }
 }
@@ -645,42 +674,50 @@ static void make_groups(const std::vector<int>& slots, const std::vector<int>& s
 template <typename R>
 static void lowrank_w(gt_geometry* G, const gt_operators* base, int nf, int k, const int* ends, cx<R>* w,
                       cudaStream_t st) {
+    constexpr bool f32 = sizeof(R) == 4;
     const int64_t nnode = G->F.nnode, nfac = G->F.nfac, ntot = (int64_t)nf * k;
     const int gmax = group_max(G, sizeof(cx<R>));
-    const int bc = (int)std::min<int64_t>(ntot, 64);
+    const int bc = (int)std::min<int64_t>(ntot, 64), wide = f32 ? 2 * bc : bc;
     Pool tmp;
     cx<R>* sv = tmp.alloc<cx<R>>((size_t)bc * nfac);
-    cx<R>* zv = tmp.alloc<cx<R>>((size_t)bc * nfac);
-    cx<R>* uv = tmp.alloc<cx<R>>((size_t)bc * std::max<int64_t>(G->F.vec_total, 1));
+    cx<R>* zv = tmp.alloc<cx<R>>((size_t)wide * nfac);
+    cx<R>* uv = tmp.alloc<cx<R>>((size_t)wide * std::max<int64_t>(G->F.vec_total, 1));
+    c32* yv = f32 ? tmp.alloc<c32>((size_t)wide * nfac) : nullptr;
+    int* cnt = f32 ? tmp.alloc<int>(sweep_counters(G->F.nfront, bc)) : nullptr;
     int* d_gptr = tmp.alloc<int>(bc + 1);
     int* d_gslot = tmp.alloc<int>(bc);
     int* d_gop = tmp.alloc<int>(bc);
-    const int nlev = (int)G->level_ptr.size() - 1;
+    int* d_gpair = tmp.alloc<int>(bc + 1);
     for (int64_t c0 = 0; c0 < ntot; c0 += bc) {
         const int nc = (int)std::min<int64_t>(bc, ntot - c0);
         cx<R>* wout = w + c0 * nnode;
         GT_CUDA(cudaMemsetAsync(sv, 0, (size_t)nc * nfac * sizeof(cx<R>), st));
         GT_CUDA(cudaMemsetAsync(wout, 0, (size_t)nc * nnode * sizeof(cx<R>), st));
         launch_lowrank_rhs<R>(sv, nfac, (int)c0, nc, k, ends, G->geo.perm, st);
-        std::vector<int> slots(nc), sfact(nc), gptr, gslot, gop;
+        std::vector<int> slots(nc), sfact(nc), gptr, gslot, gop, gpair;
         for (int q = 0; q < nc; ++q) {
             slots[q] = q;
             sfact[q] = (int)((c0 + q) / k);
         }
-        make_groups(slots, sfact, gmax, gptr, gslot, gop);
+        make_groups(slots, sfact, gmax, gptr, gslot, gop, gpair);
         GT_CUDA(cudaMemcpy(d_gptr, gptr.data(), gptr.size() * sizeof(int), cudaMemcpyHostToDevice));
         GT_CUDA(cudaMemcpy(d_gslot, gslot.data(), gslot.size() * sizeof(int), cudaMemcpyHostToDevice));
         GT_CUDA(cudaMemcpy(d_gop, gop.data(), gop.size() * sizeof(int), cudaMemcpyHostToDevice));
-        const Groups grp{(int)gop.size(), d_gptr, d_gslot, d_gop};
-        for (int h = 0; h < nlev; ++h) {
-            const int nfl = (int)(G->level_ptr[h + 1] - G->level_ptr[h]);
-            launch_fwd_level<R>(G->F, G->d_order + G->level_ptr[h], nfl, G->level_maxnf[h], G->level_maxnown[h],
-                                panel_of<R>(base), dinv_of<R>(base), sv, zv, uv, sv, grp, gmax, st);
-        }
-        for (int h = nlev - 1; h >= 0; --h) {
-            const int nfl = (int)(G->level_ptr[h + 1] - G->level_ptr[h]);
-            launch_bwd_level<R>(G->F, G->d_order + G->level_ptr[h], nfl, G->level_maxnf[h], G->level_maxnown[h],
-                                panel_rm_of<R>(base), zv, sv, wout, grp, gmax, st);
+        GT_CUDA(cudaMemcpy(d_gpair, gpair.data(), gpair.size() * sizeof(int), cudaMemcpyHostToDevice));
+        const Groups grp{(int)gop.size(), d_gptr, d_gslot, d_gop, d_gpair};
+        if constexpr (f32) {
+            GT_CUDA(cudaMemsetAsync(cnt, 0, sweep_counters(G->F.nfront, grp.ngroup) * sizeof(int), st));
+            launch_sweep(G->sweep, G->F, base->panel32, base->panel32_b, base->dinv32, sv, zv, yv, uv, wout, grp, cnt, 0,
+                         G->sweep.nft + G->sweep.nbt, st);
+        } else {
+            const int nlev = (int)G->level_ptr.size() - 1;
+            for (int h = 0; h < nlev; ++h)
+                launch_fwd_level<R>(G->F, G->d_order + G->level_ptr[h], (int)(G->level_ptr[h + 1] - G->level_ptr[h]),
+                                    G->level_maxnf[h], G->level_maxnown[h], base->panel64, base->dinv64, sv, zv, uv, sv, grp,
+                                    gmax, st);
+            for (int h = nlev - 1; h >= 0; --h)
+                launch_bwd_level<R>(G->F, G->d_order + G->level_ptr[h], (int)(G->level_ptr[h + 1] - G->level_ptr[h]),
+                                    G->level_maxnf[h], G->level_maxnown[h], base->panel64_rm, zv, sv, wout, grp, gmax, st);
         }
         GT_CUDA(cudaStreamSynchronize(st));   // the group tables are reused by the next batch
     }
@@ -735,9 +772,15 @@ static void fill_ws(Workspace& W, gt_geometry* G, int ncol, int m, int prec, int
     W.w = p.alloc<unsigned char>((size_t)ncol * n * es);
     W.z = p.alloc<unsigned char>((size_t)ncol * n * es);
     W.T = p.alloc<unsigned char>((size_t)ncol * G->maxT * es);
-    W.zfac = p.alloc<unsigned char>((size_t)ncol * G->F.nfac * es);
+    // the FP32 sweeps' interleaved vectors: whole pairs of columns per group, at most two columns for each
+    const size_t wide = (size_t)(prec == 1 ? 1 : 2) * ncol;
+    W.zfac = p.alloc<unsigned char>(wide * G->F.nfac * es);
     W.yfac = p.alloc<unsigned char>((size_t)ncol * G->F.nfac * es);
-    W.uvec = p.alloc<unsigned char>((size_t)ncol * std::max<int64_t>(G->F.vec_total, 1) * es);
+    W.uvec = p.alloc<unsigned char>(wide * std::max<int64_t>(G->F.vec_total, 1) * es);
+    if (prec != 1) {
+        W.yint = p.alloc<c32>(wide * G->F.nfac);
+        W.cnt = p.alloc<int>(sweep_counters(G->F.nfront, ncol));
+    }
     // node-ordered s / y of the preconditioner: entries of nodes that are not kept stay zero
     W.sd = p.alloc<unsigned char>((size_t)ncol * G->F.nnode * es);
     if (!dry) GT_CUDA(cudaMemsetAsync(W.sd, 0, (size_t)ncol * G->F.nnode * es, st));
@@ -777,6 +820,7 @@ static void fill_ws(Workspace& W, gt_geometry* G, int ncol, int m, int prec, int
     W.g_ptr = p.alloc<int>(ncol + 1);
     W.g_slot = p.alloc<int>(ncol);
     W.g_op = p.alloc<int>(ncol);
+    W.g_pair = p.alloc<int>(ncol + 1);
     W.act = p.alloc<int>(ncol);
     if (!dry) GT_CUDA(cudaMallocHost(&W.act_host, ncol * sizeof(int)));
     W.gP = p.alloc<c64>((size_t)kmax * ncol * n);
@@ -850,21 +894,22 @@ static int solve_impl(gt_geometry* G, gt_operators* ops, int ncol, const int* h_
             if (pc64) {
                 launch_recast<double, float>(W.pr64, n, rin, ldr, list, n, nsl, st);
                 precond<double>(G, ops, W.pr64, n, W.pz64, n, nsl, W.slot_pc, g, gmax, W.zfac64, W.yfac64, W.uvec64,
-                                W.sd64, st, list);
+                                W.sd64, nullptr, nullptr, st, list);
                 launch_recast<float, double>(out, n, W.pz64, n, list, n, nsl, st);
                 return;
             }
         }
-        precond<R>(G, ops, rin, ldr, out, n, nsl, W.slot_pc, g, gmax, zfac, yfac, uvec, sd, st, list);
+        precond<R>(G, ops, rin, ldr, out, n, nsl, W.slot_pc, g, gmax, zfac, yfac, uvec, sd, W.yint, W.cnt, st, list);
     };
-    std::vector<int> slot_col, slot_op, slot_pc, gptr, gslot, gop, act;
+    std::vector<int> slot_col, slot_op, slot_pc, gptr, gslot, gop, gpair, act;
     auto upload_groups = [&](const std::vector<int>& slots) {
-        make_groups(slots, slot_pc, gmax, gptr, gslot, gop);
+        make_groups(slots, slot_pc, gmax, gptr, gslot, gop, gpair);
         GT_CUDA(cudaMemcpyAsync(W.act, slots.data(), slots.size() * sizeof(int), cudaMemcpyHostToDevice, st));
         GT_CUDA(cudaMemcpyAsync(W.g_ptr, gptr.data(), gptr.size() * sizeof(int), cudaMemcpyHostToDevice, st));
         GT_CUDA(cudaMemcpyAsync(W.g_slot, gslot.data(), gslot.size() * sizeof(int), cudaMemcpyHostToDevice, st));
         GT_CUDA(cudaMemcpyAsync(W.g_op, gop.data(), gop.size() * sizeof(int), cudaMemcpyHostToDevice, st));
-        return Groups{(int)gop.size(), W.g_ptr, W.g_slot, W.g_op};
+        GT_CUDA(cudaMemcpyAsync(W.g_pair, gpair.data(), gpair.size() * sizeof(int), cudaMemcpyHostToDevice, st));
+        return Groups{(int)gop.size(), W.g_ptr, W.g_slot, W.g_op, W.g_pair};
     };
     const int K = std::max(1, o.outer_k);
     const int64_t ldk = (int64_t)ncol * n;          // between GCR directions
@@ -1413,6 +1458,26 @@ int gt_geometry_create(const gt_geometry_desc* d, gt_geometry** out) {
         G->nbig = (int)big.size();
         G->d_bigfronts = p.upload(big.data(), big.size());
     }
+    {
+        const SweepPlanHost H = make_sweep_plan(nf, d->n_levels, d->level_ptr, d->front_order, d->own_start, d->nown, d->nbnd,
+                                                d->bnd_ptr, d->bnd_idx, d->child_ptr, d->child_idx, d->cmap_ptr, d->cmap_idx,
+                                                d->vec_off);
+        SweepPlan& W = G->sweep;
+        W.nft = H.nft;
+        W.nbt = H.nbt;
+        W.nsrc = H.nsrc;
+        W.src_rows = H.src_rows;
+        W.ptotal = H.ptotal;
+        W.tasks = p.upload(H.tasks.data(), H.tasks.size());
+        W.src = p.upload(H.src.data(), H.src.size());
+        W.bidx = p.upload(H.bidx.data(), H.bidx.size());
+        W.hf = p.upload(H.hf.data(), H.hf.size());
+        W.hb = p.upload(H.hb.data(), H.hb.size());
+        W.offf = p.upload(H.offf.data(), H.offf.size());
+        W.offb = p.upload(H.offb.data(), H.offb.size());
+        G->sweep_level_f = H.level_f;
+        G->sweep_level_b = H.level_b;
+    }
     if (d->n_lowrank < 0 || d->n_lowrank > d->n_branches || d->n_lowrank > LOWRANK_MAX)
         throw Invalid("n_lowrank must be in 0 .. min(n_branches, 64)");
     G->n_lowrank = d->n_lowrank;
@@ -1556,8 +1621,8 @@ int gt_operators_create_ex(gt_geometry* G, int32_t n_ops, const double* omega, c
     int* status = tmp.alloc<int>(1);
     GT_CUDA(cudaMemsetAsync(status, 0, sizeof(int), st));
     O->panel64 = (keep64 ? p : tmp).alloc<c64>((size_t)n_ops * F.panel_total);
-    O->panel32 = p.alloc<c32>((size_t)n_ops * F.panel_total);
-    O->panel32_rm = p.alloc<c32>((size_t)n_ops * F.panel_total);
+    O->panel32 = p.alloc<c32>((size_t)n_ops * G->sweep.ptotal);
+    O->panel32_b = p.alloc<c32>((size_t)n_ops * G->sweep.ptotal);
     O->panel64_rm = keep64 ? p.alloc<c64>((size_t)n_ops * F.panel_total) : nullptr;
     O->dinv64 = p.alloc<c64>((size_t)n_ops * F.nfac);
     O->dinv32 = p.alloc<c32>((size_t)n_ops * F.nfac);
@@ -1596,7 +1661,7 @@ int gt_operators_create_ex(gt_geometry* G, int32_t n_ops, const double* omega, c
     }
     {
         Scope sc(P, "factor_convert", st);
-        launch_panel_convert(F, O->panel64, O->panel32, O->panel32_rm, O->panel64_rm, O->dinv64, O->dinv32, n_ops,
+        launch_panel_convert(F, G->sweep, O->panel64, O->panel32, O->panel32_b, O->panel64_rm, O->dinv64, O->dinv32, n_ops,
                              G->tiled_nf, st);
     }
     int h_status = 0;
@@ -1661,7 +1726,7 @@ int gt_operators_derive(gt_geometry* G, const gt_operators* base, int32_t n_ops,
     O->panel64 = base->panel64;
     O->panel32 = base->panel32;
     O->panel64_rm = base->panel64_rm;
-    O->panel32_rm = base->panel32_rm;
+    O->panel32_b = base->panel32_b;
     O->dinv64 = base->dinv64;
     O->dinv32 = base->dinv32;
     O->nlow = k;
@@ -1896,20 +1961,24 @@ int gt_apply(gt_geometry* G, gt_operators* ops, int32_t kind, int32_t precision,
             cx<R>* T = tmp.alloc<cx<R>>((size_t)n_cols * G->maxT);
             matvec<R>(G, ops, xi, nullptr, yo, n, n_cols, d_op, kind == 0 ? 0 : 2, T, st);
         } else {
-            std::vector<int> gptr, gslot, gop, all(n_cols);
+            std::vector<int> gptr, gslot, gop, gpair, all(n_cols);
             for (int c = 0; c < n_cols; ++c) all[c] = c;
             const int gmax = group_max(G, sizeof(cx<R>));
-            make_groups(all, h_pc, gmax, gptr, gslot, gop);
+            make_groups(all, h_pc, gmax, gptr, gslot, gop, gpair);
             int* g0 = tmp.upload(gptr.data(), gptr.size());
             int* g1 = tmp.upload(gslot.data(), gslot.size());
             int* g2 = tmp.upload(gop.data(), gop.size());
-            Groups grp{(int)gop.size(), g0, g1, g2};
-            cx<R>* zf = tmp.alloc<cx<R>>((size_t)n_cols * G->F.nfac);
+            Groups grp{(int)gop.size(), g0, g1, g2, tmp.upload(gpair.data(), gpair.size())};
+            constexpr bool f32 = sizeof(R) == 4;
+            const size_t wide = (size_t)(f32 ? 2 : 1) * n_cols;
+            cx<R>* zf = tmp.alloc<cx<R>>(wide * G->F.nfac);
             cx<R>* yf = tmp.alloc<cx<R>>((size_t)n_cols * G->F.nfac);
-            cx<R>* uv = tmp.alloc<cx<R>>((size_t)n_cols * std::max<int64_t>(G->F.vec_total, 1));
+            cx<R>* uv = tmp.alloc<cx<R>>(wide * std::max<int64_t>(G->F.vec_total, 1));
+            c32* yi = f32 ? tmp.alloc<c32>(wide * G->F.nfac) : nullptr;
+            int* cnt = f32 ? tmp.alloc<int>(sweep_counters(G->F.nfront, n_cols)) : nullptr;
             cx<R>* sdv = tmp.alloc<cx<R>>((size_t)n_cols * G->F.nnode);
             GT_CUDA(cudaMemsetAsync(sdv, 0, (size_t)n_cols * G->F.nnode * sizeof(cx<R>), st));
-            precond<R>(G, ops, xi, n, yo, n, n_cols, d_pc, grp, gmax, zf, yf, uv, sdv, st);
+            precond<R>(G, ops, xi, n, yo, n, n_cols, d_pc, grp, gmax, zf, yf, uv, sdv, yi, cnt, st);
         }
         if constexpr (sizeof(R) == 4) {
             std::vector<c32> h32((size_t)n_cols * n);

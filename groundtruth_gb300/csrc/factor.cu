@@ -531,10 +531,10 @@ void launch_invert_tiled(const Fronts& F, const int64_t* front_list, int nfront,
 }
 
 // Finish the solve panels: the own block gets its inverse below an explicit unit diagonal (moved from the
-// upper triangle, which becomes zero; the pivots go to dinv as 1/D), and the FP32 column-major, FP32 / FP64
-// row-major copies are written.
+// upper triangle, which becomes zero; the pivots go to dinv as 1/D), and the copies the sweeps read are written: the
+// FP32 forward and backward tiles (sweep.cu) and the FP64 row-major panel.
 // r64 (the FP64 row-major copy) may be null: operators that keep their FP32 panels only
-__global__ void panel_convert_kernel(Fronts F, c64* __restrict__ p64, c32* __restrict__ p32, c32* __restrict__ r32,
+__global__ void panel_convert_kernel(Fronts F, SweepPlan S, c64* __restrict__ p64, c32* __restrict__ pf, c32* __restrict__ pb,
                                      c64* __restrict__ r64, c64* __restrict__ d64, c32* __restrict__ d32, int tiled_nf) {
     const int f = blockIdx.x;
     const int op = blockIdx.y;
@@ -542,12 +542,29 @@ __global__ void panel_convert_kernel(Fronts F, c64* __restrict__ p64, c32* __res
     const bool in_place = nf >= tiled_nf;                       // the blocked inversion: X below the diagonal
     const int64_t base = (int64_t)op * F.panel_total + F.panel_off[f];
     const int64_t dbase = (int64_t)op * F.nfac + F.own_start[f];
+    const int H = S.hf[f], C = S.hb[f];
+    c32* tf = pf + (int64_t)op * S.ptotal + S.offf[f];
+    c32* tb = pb + (int64_t)op * S.ptotal + S.offb[f];
+    // element (i, k) into its forward tile (rows gH .., inner k < min(nown, (g + 1) H)) and its backward one (columns
+    // tC .., inner i >= tC)
+    auto put = [&](int i, int k, c32 v) {
+        const int g = i / H;
+        if (k < min(nown, (g + 1) * H)) {
+            const int m = min(g, nown / H), h = min(H, nf - g * H);
+            tf[(int64_t)H * H * m * (m + 1) / 2 + (int64_t)H * nown * (g - m) + (int64_t)k * ((h + 1) & ~1) + (i - g * H)] = v;
+        }
+        const int t = k / C;
+        if (i >= t * C) {
+            const int h = min(C, nown - t * C);
+            tb[(int64_t)C * ((int64_t)t * nf - (int64_t)C * t * (t - 1) / 2) + (int64_t)(i - t * C) * ((h + 1) & ~1) +
+               (k - t * C)] = v;
+        }
+    };
     for (int64_t q = threadIdx.x; q < (int64_t)nf * nown; q += blockDim.x) {
         int k = int(q / nf), i = int(q - (int64_t)k * nf);      // column-major element (i, k)
         if (i < k) {                                             // the upper triangle: zero
             if (in_place) {
-                p32[base + q] = zero<float>();
-                r32[base + (int64_t)i * nown + k] = zero<float>();
+                put(i, k, zero<float>());
                 if (r64) r64[base + (int64_t)i * nown + k] = zero<double>();
             }
             continue;                                            // (else with its partner below)
@@ -565,19 +582,17 @@ __global__ void panel_convert_kernel(Fronts F, c64* __restrict__ p64, c32* __res
             v = p64[base + qt];
             p64[base + q] = v;
             p64[base + qt] = zero<double>();
-            p32[base + qt] = zero<float>();
-            r32[base + (int64_t)k * nown + i] = zero<float>();
+            put(k, i, zero<float>());
             if (r64) r64[base + (int64_t)k * nown + i] = zero<double>();
         }
-        p32[base + q] = cvt<float>(v);
-        r32[base + (int64_t)i * nown + k] = cvt<float>(v);
+        put(i, k, cvt<float>(v));
         if (r64) r64[base + (int64_t)i * nown + k] = v;
     }
 }
 
-void launch_panel_convert(const Fronts& F, c64* p64, c32* p32, c32* r32, c64* r64, c64* d64, c32* d32, int nops,
+void launch_panel_convert(const Fronts& F, const SweepPlan& S, c64* p64, c32* pf, c32* pb, c64* r64, c64* d64, c32* d32, int nops,
                           int tiled_nf, cudaStream_t st) {
-    panel_convert_kernel<<<dim3(F.nfront, nops), 256, 0, st>>>(F, p64, p32, r32, r64, d64, d32, tiled_nf);
+    panel_convert_kernel<<<dim3(F.nfront, nops), 256, 0, st>>>(F, S, p64, pf, pb, r64, d64, d32, tiled_nf);
     GT_LAUNCH_CHECK();
 }
 
@@ -1005,9 +1020,7 @@ void launch_bwd_level(const Fronts& F, const int64_t* front_list, int nf_level, 
     }
 }
 
-template void launch_fwd_level<float>(const Fronts&, const int64_t*, int, int, int, const c32*, const c32*, const c32*, c32*, c32*, c32*, const Groups&, int, cudaStream_t);
 template void launch_fwd_level<double>(const Fronts&, const int64_t*, int, int, int, const c64*, const c64*, const c64*, c64*, c64*, c64*, const Groups&, int, cudaStream_t);
-template void launch_bwd_level<float>(const Fronts&, const int64_t*, int, int, int, const c32*, const c32*, c32*, c32*, const Groups&, int, cudaStream_t);
 template void launch_bwd_level<double>(const Fronts&, const int64_t*, int, int, int, const c64*, const c64*, c64*, c64*, const Groups&, int, cudaStream_t);
 
 }  // namespace gt

@@ -2,6 +2,8 @@
 #pragma once
 #include "common.cuh"
 
+#include <vector>
+
 namespace gt {
 
 // The geometry as the kernels see it (device pointers, sizes).
@@ -95,9 +97,10 @@ void launch_tail(const Geo& g, const cx<R>* x, const cx<R>* rhs, cx<R>* out, int
 
 // preconditioner: s = r_V - Ar^T D^-1 r_1 into factor order (sd [col][nfac]); then, with y in node order in
 // sd [col][S*nx*ny] (zero at nodes that are not kept), out = [D^-1 (r_1 + Ar y); y]
+// (cnt: ncnt counters of the sweep that follows, cleared by the way)
 template <typename R>
 void launch_pc_node(const Geo& g, const cx<R>* r, int64_t ld, cx<R>* sd, int ncol, const int* col_op,
-                    const cx<R>* tab, const int* col_list, cudaStream_t st);
+                    const cx<R>* tab, const int* col_list, int* cnt, int64_t ncnt, cudaStream_t st);
 template <typename R>
 void launch_pc_strip(const Geo& g, const cx<R>* r, int64_t ldr, const cx<R>* sd, cx<R>* out, int64_t ldo, int ncol,
                      const int* col_op, const cx<R>* tab, const int* col_list, cudaStream_t st);
@@ -161,18 +164,60 @@ void launch_bnd_inv(const Fronts& F, c64* panel, int max_nbnd, int nops, int til
 // or more, and panel_convert takes their inverse in place
 void launch_invert_tiled(const Fronts& F, const int64_t* front_list, int nfront, int max_nf, int max_nown, c64* panel,
                          int nops, cudaStream_t st);
-// the solve panels: own blocks get a unit diagonal and zeros above it (pivot reciprocals to d64 / d32,
-// [op][nfac]); FP32 column-major, FP32 and FP64 row-major copies
-void launch_panel_convert(const Fronts& F, c64* p64, c32* p32, c32* r32, c64* r64, c64* d64, c32* d32, int nops, int tiled_nf,
-                          cudaStream_t st);
-
-// triangular solves, per level; groups of columns sharing an operator
+// triangular solves; groups of columns sharing an operator
 struct Groups {
     int ngroup;
     const int* gptr;       // group g: columns gslot[gptr[g] .. gptr[g+1])
     const int* gslot;
     const int* op;
+    const int* pair0;      // column pairs before group g in the sweeps' interleaved vectors: 1, 2 or 4 pairs a group
 };
+
+// --- FP32 sweeps in one launch (sweep.cu)
+struct alignas(16) SwTask {
+    int r0, h;             // outputs r0 .. r0 + h: rows of the front (forward) or own columns (backward)
+    int k0, k1;            // inner indices: own columns (forward), front rows (backward)
+    int dep, need;         // counter to wait on and the finished tiles it has to show
+    int sig;               // counter to raise when done
+    int nown, own0, voff;  // the front's own count, first factor index and place among the update vectors
+    int64_t goff;          // forward: the front's first row in the source table; backward: its first boundary entry
+    int64_t off;           // first panel entry
+};
+struct SweepPlanHost {
+    std::vector<SwTask> tasks;          // forward, leaves to root, then backward, root to leaves
+    int nft = 0, nbt = 0, nsrc = 0;
+    int64_t src_rows = 0, ptotal = 0;
+    std::vector<int> src, bidx;
+    std::vector<int> hf, hb;            // outputs per tile of each front
+    std::vector<int64_t> offf, offb;    // first entry of each front's tiles
+    std::vector<int> level_f, level_b;  // tasks up to the end of each level, in the order they run
+};
+struct SweepPlan {
+    const SwTask* tasks;
+    int nft, nbt, nsrc;
+    int64_t src_rows, ptotal;
+    const int* src;
+    const int* bidx;
+    const int *hf, *hb;
+    const int64_t *offf, *offb;
+};
+SweepPlanHost make_sweep_plan(int nfront, int nlev, const int64_t* level_ptr, const int64_t* order, const int64_t* own_start,
+                              const int64_t* nown, const int64_t* nbnd, const int64_t* bnd_ptr, const int64_t* bnd_idx,
+                              const int64_t* child_ptr, const int64_t* child_idx, const int64_t* cmap_ptr,
+                              const int64_t* cmap_idx, const int64_t* vec_off);
+// tasks t0 .. t1 of the plan for every column group; cnt: sweep_counters ints, zero before the first launch of a sweep and
+// the first of them (the ticket counter) before each.
+// s: [slot][nfac]; z, y, u: interleaved by group (2 columns a pair, pair0 pairs before a group); sd: [slot][nnode]
+inline int64_t sweep_counters(int nfront, int ngroup) { return 1 + 3 * (int64_t)nfront * ngroup; }
+void launch_sweep(const SweepPlan& S, const Fronts& F, const c32* pf, const c32* pb, const c32* dinv, const c32* s, c32* z,
+                  c32* y, c32* u, c32* sd, const Groups& G, int* cnt, int t0, int t1, cudaStream_t st);
+// waits of the sweep that gave up since the last call (and clears the count); read once the kernels are done
+unsigned int sweep_take_wait_timeouts();
+// the solve panels: own blocks get a unit diagonal and zeros above it (pivot reciprocals to d64 / d32,
+// [op][nfac]); the FP32 sweeps' forward and backward tiles (pf, pb) and the FP64 row-major copy
+void launch_panel_convert(const Fronts& F, const SweepPlan& S, c64* p64, c32* pf, c32* pb, c64* r64, c64* d64, c32* d32, int nops,
+                          int tiled_nf, cudaStream_t st);
+
 // forward: own rows from s in factor order (sf), results to z (factor order) and the update vectors (wasm:
 // factor-ordered scratch for fronts assembled ahead of a split product, may be sf itself);
 // backward: reads z and the ancestors' y, writes y (factor order) and sd (node order)

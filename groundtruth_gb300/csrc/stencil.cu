@@ -149,7 +149,11 @@ __device__ __forceinline__ void dinv_apply(const cx<R>* __restrict__ B, int S, i
 template <typename R, int MAXS>
 __global__ void __launch_bounds__(256) pc_node_kernel(Geo g, const cx<R>* __restrict__ r, int64_t ld, cx<R>* __restrict__ sd,
                                                       const int* __restrict__ col_op, const cx<R>* __restrict__ tab,
-                                                      const int* __restrict__ col_list) {
+                                                      const int* __restrict__ col_list, int* __restrict__ cnt,
+                                                      int64_t ncnt) {
+    for (int64_t q = ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x; q < ncnt;
+         q += (int64_t)gridDim.y * gridDim.x * blockDim.x)
+        cnt[q] = 0;
     const int col = col_list ? col_list[blockIdx.y] : blockIdx.y;
     const int op = col_op ? col_op[col] : 0;
     const int S = g.S, nx = g.nx, ny = g.ny, nxy = nx * ny, NC = 1 << S;
@@ -239,12 +243,12 @@ __global__ void __launch_bounds__(256) pc_node_kernel(Geo g, const cx<R>* __rest
 
 template <typename R>
 void launch_pc_node(const Geo& g, const cx<R>* r, int64_t ld, cx<R>* sd, int ncol, const int* col_op, const cx<R>* tab,
-                    const int* col_list, cudaStream_t st) {
+                    const int* col_list, int* cnt, int64_t ncnt, cudaStream_t st) {
     if (g.S > SHEETS_MAX) throw CudaError{cudaErrorInvalidValue, "more sheets than the stencil kernels take"};
     const dim3 grid(ceil_div(g.nx, RPB_NODE), ncol);
-    if (g.S <= 2) pc_node_kernel<R, 2><<<grid, 256, 0, st>>>(g, r, ld, sd, col_op, tab, col_list);
-    else if (g.S <= 4) pc_node_kernel<R, 4><<<grid, 256, 0, st>>>(g, r, ld, sd, col_op, tab, col_list);
-    else pc_node_kernel<R, 8><<<grid, 256, 0, st>>>(g, r, ld, sd, col_op, tab, col_list);
+    if (g.S <= 2) pc_node_kernel<R, 2><<<grid, 256, 0, st>>>(g, r, ld, sd, col_op, tab, col_list, cnt, ncnt);
+    else if (g.S <= 4) pc_node_kernel<R, 4><<<grid, 256, 0, st>>>(g, r, ld, sd, col_op, tab, col_list, cnt, ncnt);
+    else pc_node_kernel<R, 8><<<grid, 256, 0, st>>>(g, r, ld, sd, col_op, tab, col_list, cnt, ncnt);
     GT_LAUNCH_CHECK();
 }
 
@@ -368,8 +372,8 @@ void launch_gather(const int64_t* c2d, int64_t ncomp, const c64* in, int64_t ldi
 
 template void launch_tail<float>(const Geo&, const c32*, const c32*, c32*, int64_t, int, const int*, const c64*, const c64*, int, const int*, cudaStream_t);
 template void launch_tail<double>(const Geo&, const c64*, const c64*, c64*, int64_t, int, const int*, const c64*, const c64*, int, const int*, cudaStream_t);
-template void launch_pc_node<float>(const Geo&, const c32*, int64_t, c32*, int, const int*, const c32*, const int*, cudaStream_t);
-template void launch_pc_node<double>(const Geo&, const c64*, int64_t, c64*, int, const int*, const c64*, const int*, cudaStream_t);
+template void launch_pc_node<float>(const Geo&, const c32*, int64_t, c32*, int, const int*, const c32*, const int*, int*, int64_t, cudaStream_t);
+template void launch_pc_node<double>(const Geo&, const c64*, int64_t, c64*, int, const int*, const c64*, const int*, int*, int64_t, cudaStream_t);
 template void launch_pc_strip<float>(const Geo&, const c32*, int64_t, const c32*, c32*, int64_t, int, const int*, const c32*, const int*, cudaStream_t);
 template void launch_pc_strip<double>(const Geo&, const c64*, int64_t, const c64*, c64*, int64_t, int, const int*, const c64*, const int*, cudaStream_t);
 

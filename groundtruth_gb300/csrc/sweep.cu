@@ -1,0 +1,570 @@
+// The FP32 triangular sweeps of the preconditioner (the solves with the factorised Schur complement, peec.py:3071)
+// as one kernel: every front of the elimination tree, forward and backward, and every column group in one launch.
+//
+// After the factorisation a front's panel is P = [Linv_own; -L_bnd Linv_own] (factor.cu), so its solves are two dense
+// products without a sequential chain:
+//     forward   out = P w_own: own rows z_own = dinv * out, boundary rows (children's updates + out) go up
+//     backward  y_own = P^T [z_own; y_bnd]
+// A task is one output tile of one front: up to 128 rows of the forward product or columns of the backward one, for a
+// group of up to 8 columns that share the operator.  The FP32 panels are stored tile by tile in the order the tasks
+// read them, [inner index][outputs], the zeros above the own block's diagonal left out at tile granularity, so that a
+// task's panel is one contiguous run.
+//
+// Why one launch: a level at a time, the top of the tree (one to a few fronts per level) left the GPU idle between
+// 26-40 dependent launches of ~20 us each; the slotted pair at 256 x 256 took 1.08 ms per application with 32 columns at four
+// frequencies, where its panels are 0.15 ms of HBM time.  Here blocks draw tickets from a counter, and tickets are numbered so that
+// a task's inputs always have smaller ones: leaves to root, then root to leaves.  A block waits (bounded) on a counter
+// of its inputs' finished tiles; whoever holds the smallest unfinished ticket never waits, so the kernel finishes
+// however many of its blocks are resident.  A block's fifth warp runs ahead of the other four: it takes the next
+// ticket and brings its panel run into a ring of shared-memory stages by bulk copies while the present task waits
+// for its inputs or computes, so the panel streams at HBM rate through the tree's dependent steps.
+//
+// The vectors between tasks (update vectors, z, y) are interleaved by column group, a row's columns side by side as
+// pairs (re0 re1 im0 im1), which the gathers read as 16-byte pieces and the packed FP32 FMAs (two per instruction)
+// take as they are.
+//
+// A column's arithmetic is set by the fronts alone (tile, stage and segment sizes), never by the other columns.
+#include "kernels.h"
+
+#include <algorithm>
+#include <map>
+#include <mutex>
+#include <vector>
+
+namespace gt {
+
+constexpr int SWT = 128;               // consumer threads
+constexpr int SWW = SWT / 32;
+constexpr int SW_BLOCK = SWT + 32;     // and the producer warp
+constexpr int SW_STAGES = 2;
+constexpr int SW_STAGE_ENT = 1792;     // panel entries per stage (14 KB)
+constexpr int SW_XROWS = 256;          // inner rows staged at once (16 KB at 8 columns)
+constexpr int SW_HMAX = 128;
+constexpr uint64_t SW_WAIT_NS = 2000000000ull;
+constexpr uint32_t SW_POLLS = 1u << 28;
+
+struct SwDesc {                        // one ring stage, written by the producer
+    int f_dir;                         // 0 forward, 1 backward, -1 no more work
+    int g;                             // column group
+    int ka, kb;                        // inner range of the stage
+    int first, last;
+    SwTask t;
+};
+
+struct alignas(16) SwShared {
+    float2 ring[SW_STAGES][SW_STAGE_ENT];
+    float4 x[SW_XROWS * 4];            // inner rows [row][pair]; then the partial sums [seg][output][pair]
+    float4 eb[SW_HMAX * 4];            // forward: the tile's boundary rows' updates so far [row][pair]
+    float2 dv[SW_HMAX];                // forward: the own rows' pivot reciprocals
+    int node[SW_HMAX];                 // backward: dense node of each output
+    SwDesc desc[SW_STAGES];
+    uint64_t full[SW_STAGES], empty[SW_STAGES];
+};
+static_assert(SW_XROWS * 4 >= 2 * SWT * 4, "the partial sums take the staged rows' place");
+
+__device__ unsigned int g_sweep_timeouts = 0;
+
+__device__ __forceinline__ uint32_t sw_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ uint64_t sw_ns() {
+    uint64_t t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+__device__ __forceinline__ bool sw_try(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                 "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
+// a wait that gives up is counted, and everything after it goes on without its inputs: the launch ends and the
+// host reports GT_TIMEOUT
+__device__ __noinline__ void sw_gave_up() { atomicAdd(&g_sweep_timeouts, 1u); }
+__device__ __forceinline__ void sw_wait_bar(uint64_t* b, uint32_t parity) {
+    const uint32_t bar = sw_smem(b);
+    if (sw_try(bar, parity)) return;
+    const uint64_t t0 = sw_ns();
+    for (uint32_t it = 0; it < SW_POLLS; ++it) {
+        if (sw_try(bar, parity)) return;
+        if (sw_ns() - t0 > 2 * SW_WAIT_NS) break;
+    }
+    sw_gave_up();
+}
+__device__ __forceinline__ int sw_acquire(const int* p) {
+    int v;
+    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void sw_wait_count(const int* p, int need) {
+    if (sw_acquire(p) >= need) return;
+    const uint64_t t0 = sw_ns();
+    for (uint32_t it = 0; it < SW_POLLS; ++it) {
+        if (sw_acquire(p) >= need) return;
+        if ((it & 63) == 63) {
+            if (*(volatile unsigned int*)&g_sweep_timeouts) return;      // someone gave up already
+            if (sw_ns() - t0 > SW_WAIT_NS) break;
+        }
+        __nanosleep(32);
+    }
+    sw_gave_up();
+}
+__device__ __forceinline__ void sw_sync() { asm volatile("bar.sync 1, %0;" ::"n"(SWT) : "memory"); }
+
+// two packed FP32 FMAs: acc.x += a.x b.x, acc.y += a.y b.y
+__device__ __forceinline__ void fma2(float2& acc, float2 a, float2 b) {
+    uint64_t c = reinterpret_cast<uint64_t&>(acc);
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c)
+        : "l"(reinterpret_cast<const uint64_t&>(a)), "l"(reinterpret_cast<const uint64_t&>(b)));
+    acc = reinterpret_cast<float2&>(c);
+}
+
+// (re, im) pairs of a column pair += p * x for the panel entry p
+__device__ __forceinline__ void mac_pair(float2& re, float2& im, float2 pr, float2 pi, float2 npi, float4 x) {
+    const float2 xr = make_float2(x.x, x.y), xi = make_float2(x.z, x.w);
+    fma2(re, pr, xr);
+    fma2(re, npi, xi);
+    fma2(im, pr, xi);
+    fma2(im, pi, xr);
+}
+
+struct SwArgs {
+    const SwTask* tasks;               // nft forward tasks, then nbt backward ones
+    int nft, nbt;
+    int nsrc;
+    int64_t src_rows;
+    const int* src;                    // [nsrc][src_rows] update-vector rows added into a front's rows (-1: none)
+    const int* bidx;                   // boundary rows' factor indices
+    const int64_t* iperm;
+    int64_t nfac, nvec, nnode, ptotal;
+    const float2* pf;                  // [op][ptotal] forward tiles
+    const float2* pb;                  // [op][ptotal] backward tiles
+    const float2* dinv;                // [op][nfac]
+    const float2* s;                   // [slot][nfac] right-hand sides, factor order
+    float4* z;                         // interleaved [group][nfac][pairs]
+    float4* y;
+    float4* u;                         // interleaved [group][nvec][pairs]
+    float2* sd;                        // [slot][nnode] solutions, node order
+    Groups G;
+    int* cnt;                          // [counter][ngroup] finished tiles; the ticket counter in front of them
+    int t0, t1;                        // tickets of this launch
+};
+
+template <int NP>
+__device__ void sw_task(const SwArgs& A, SwShared& sm, uint32_t& it, const SwDesc& d0) {
+    const int tid = threadIdx.x;
+    const SwTask t = d0.t;
+    const int dir = d0.f_dir, g = d0.g, ng = A.G.ngroup;
+    const int* gs = A.G.gslot + A.G.gptr[g];
+    const int gc = A.G.gptr[g + 1] - A.G.gptr[g];
+    const int64_t gb = A.G.pair0[g];                     // column pairs before this group's
+    float4* __restrict__ z = A.z + gb * A.nfac;
+    float4* __restrict__ y = A.y + gb * A.nfac;
+    float4* __restrict__ u = A.u + gb * A.nvec;
+    const int h = t.h, hp = (h + 1) & ~1;
+    const int np2 = hp >> 1;                             // pairs of outputs
+    const int nseg = SWT / np2;
+    const int seg = tid / np2, row2 = tid - seg * np2;
+    const bool act = seg < nseg;
+    if (tid == 0 && t.need > 0) sw_wait_count(A.cnt + (int64_t)t.dep * ng + g, t.need);
+    // what the tile's outputs need besides the product
+    if (dir == 0) {
+        sw_sync();
+        const int64_t op = A.G.op[g];
+        for (int q = tid; q < h; q += SWT)
+            if (t.r0 + q < t.nown) sm.dv[q] = A.dinv[op * A.nfac + t.own0 + t.r0 + q];
+        const int lo = max(0, t.nown - t.r0);
+        for (int q = lo * NP + tid; q < h * NP; q += SWT) {
+            const int r = q / NP, p = q - r * NP;
+            float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int s = 0; s < A.nsrc; ++s) {
+                const int e = A.src[s * A.src_rows + t.goff + t.r0 + r];
+                if (e >= 0) {
+                    const float4 b = __ldcg(u + (int64_t)e * NP + p);
+                    a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+                }
+            }
+            sm.eb[q] = a;
+        }
+    } else {
+        for (int q = tid; q < h; q += SWT) sm.node[q] = (int)A.iperm[t.own0 + t.r0 + q];
+        sw_sync();
+    }
+    float2 re[2][NP], im[2][NP];
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int p = 0; p < NP; ++p) re[r][p] = im[r][p] = make_float2(0.f, 0.f);
+    int xbeg = t.k0, xend = t.k0;
+    bool last;
+    do {
+        const int slot = it % SW_STAGES;
+        const SwDesc& d = sm.desc[slot];
+        sw_wait_bar(&sm.full[slot], (it / SW_STAGES) & 1);
+        const int ka = d.ka, kb = d.kb;
+        last = d.last;
+        const float2* ring = sm.ring[slot];
+        for (int k = ka; k < kb;) {
+            if (k >= xend) {
+                if (xend > t.k0) sw_sync();              // the rows staged before have been read
+                xbeg = k;
+                xend = min(t.k1, k + SW_XROWS);
+                const int tot = (xend - xbeg) * NP;
+                if (dir == 0) {
+                    // own rows: the right-hand side plus the children's updates, in the children's order
+                    for (int q = tid; q < tot; q += SWT) {
+                        const int r = q / NP, p = q - r * NP, row = xbeg + r;
+                        const float2* s = A.s + t.own0 + row;
+                        const float2 zero2 = make_float2(0.f, 0.f);
+                        const float2 a0 = 2 * p < gc ? s[(int64_t)gs[2 * p] * A.nfac] : zero2;
+                        const float2 a1 = 2 * p + 1 < gc ? s[(int64_t)gs[2 * p + 1] * A.nfac] : zero2;
+                        float4 a = make_float4(a0.x, a1.x, a0.y, a1.y);
+                        for (int c = 0; c < A.nsrc; ++c) {
+                            const int e = A.src[c * A.src_rows + t.goff + row];
+                            if (e >= 0) {
+                                const float4 b = __ldcg(u + (int64_t)e * NP + p);
+                                a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+                            }
+                        }
+                        sm.x[q] = a;
+                    }
+                } else {
+#pragma unroll 4
+                    for (int q = tid; q < tot; q += SWT) {
+                        const int r = q / NP, p = q - r * NP, row = xbeg + r;
+                        const float4* src = row < t.nown ? z + (int64_t)(t.own0 + row) * NP
+                                                         : y + (int64_t)A.bidx[t.goff + row - t.nown] * NP;
+                        sm.x[q] = __ldcg(src + p);
+                    }
+                }
+                sw_sync();
+            }
+            const int e = min(kb, xend);
+            if (act) {
+                const float4* P = reinterpret_cast<const float4*>(ring + (k - ka) * hp) + row2;
+                const float4* X = sm.x + (k - xbeg) * NP;
+#pragma unroll 2
+                for (int q = seg; q < e - k; q += nseg) {
+                    const float4 a = P[q * np2];          // outputs 2 row2, 2 row2 + 1
+                    const float2 pr0 = make_float2(a.x, a.x), pi0 = make_float2(a.y, a.y), ni0 = make_float2(-a.y, -a.y);
+                    const float2 pr1 = make_float2(a.z, a.z), pi1 = make_float2(a.w, a.w), ni1 = make_float2(-a.w, -a.w);
+#pragma unroll
+                    for (int p = 0; p < NP; ++p) {
+                        const float4 x = X[q * NP + p];
+                        mac_pair(re[0][p], im[0][p], pr0, pi0, ni0, x);
+                        mac_pair(re[1][p], im[1][p], pr1, pi1, ni1, x);
+                    }
+                }
+            }
+            k = e;
+        }
+        ++it;
+        __syncwarp();
+        if ((tid & 31) == 0)
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sw_smem(&sm.empty[slot])) : "memory");
+    } while (!last);
+    // the segments' partial sums meet in the staged rows' place
+    sw_sync();
+    if (act) {
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+#pragma unroll
+            for (int p = 0; p < NP; ++p)
+                sm.x[(seg * hp + 2 * row2 + r) * NP + p] = make_float4(re[r][p].x, re[r][p].y, im[r][p].x, im[r][p].y);
+    }
+    sw_sync();
+    for (int q = tid; q < h * NP; q += SWT) {
+        float4 v = sm.x[q];
+        for (int sg = 1; sg < nseg; ++sg) {
+            const float4 b = sm.x[sg * hp * NP + q];
+            v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
+        }
+        const int r = q / NP, p = q - r * NP, row = t.r0 + r;
+        if (dir == 0) {
+            if (row < t.nown) {
+                const float2 d = sm.dv[r];
+                z[(int64_t)(t.own0 + row) * NP + p] = make_float4(d.x * v.x - d.y * v.z, d.x * v.y - d.y * v.w,
+                                                                  d.x * v.z + d.y * v.x, d.x * v.w + d.y * v.y);
+            } else {
+                const float4 b = sm.eb[q];
+                u[(int64_t)(t.voff + row - t.nown) * NP + p] = make_float4(b.x + v.x, b.y + v.y, b.z + v.z, b.w + v.w);
+            }
+        } else {
+            y[(int64_t)(t.own0 + row) * NP + p] = v;
+            const int64_t node = sm.node[r];
+            if (2 * p < gc) A.sd[(int64_t)gs[2 * p] * A.nnode + node] = make_float2(v.x, v.z);
+            if (2 * p + 1 < gc) A.sd[(int64_t)gs[2 * p + 1] * A.nnode + node] = make_float2(v.y, v.w);
+        }
+    }
+    sw_sync();                                           // every output of the tile is written
+    if (tid == 0 && t.sig >= 0) {
+        __threadfence();
+        asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(A.cnt + (int64_t)t.sig * ng + g) : "memory");
+    }
+}
+
+__global__ void __launch_bounds__(SW_BLOCK, 4) sweep_kernel(SwArgs A) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    SwShared& sm = *reinterpret_cast<SwShared*>(smem_raw);
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < SW_STAGES; ++s) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sw_smem(&sm.full[s])) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(sw_smem(&sm.empty[s])), "r"(SWW) : "memory");
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    __syncthreads();
+    if (threadIdx.x >= SWT) {
+        if (threadIdx.x != SWT) return;
+        // the producer: tickets in order, each task's panel run stage by stage
+        int* ticket = A.cnt - 1;
+        uint32_t it = 0;
+        for (;;) {
+            const int tk = A.t0 + atomicAdd(ticket, 1);
+            const bool done = tk >= A.t1;
+            SwTask t{};
+            int g = 0, dir = -1;
+            const float2* src = nullptr;
+            if (!done) {
+                const int task = tk / A.G.ngroup;
+                g = tk - task * A.G.ngroup;
+                t = A.tasks[task];
+                dir = task >= A.nft;
+                src = (dir ? A.pb : A.pf) + (int64_t)A.G.op[g] * A.ptotal + t.off;
+            }
+            const int hp = (t.h + 1) & ~1;
+            const int step = done ? 1 : SW_STAGE_ENT / hp;
+            int k = t.k0;
+            do {
+                const int slot = it % SW_STAGES;
+                if (it >= SW_STAGES) sw_wait_bar(&sm.empty[slot], (it / SW_STAGES - 1) & 1);
+                SwDesc& d = sm.desc[slot];
+                const int e = min(t.k1, k + step);
+                d.f_dir = dir;
+                d.g = g;
+                d.ka = k;
+                d.kb = e;
+                d.first = k == t.k0;
+                d.last = e >= t.k1;
+                if (d.first) d.t = t;
+                const uint32_t bytes = (uint32_t)(e - k) * hp * sizeof(float2), bar = sw_smem(&sm.full[slot]);
+                if (bytes) {
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                                 ::"r"(sw_smem(sm.ring[slot])), "l"(src + (int64_t)(k - t.k0) * hp), "r"(bytes), "r"(bar)
+                                 : "memory");
+                } else {
+                    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+                }
+                ++it;
+                k = e;
+            } while (k < t.k1);
+            if (done) return;
+        }
+    }
+    uint32_t it = 0;
+    for (;;) {
+        const int slot = it % SW_STAGES;
+        sw_wait_bar(&sm.full[slot], (it / SW_STAGES) & 1);
+        const SwDesc& d = sm.desc[slot];
+        if (d.f_dir < 0) return;
+        switch (A.G.pair0[d.g + 1] - A.G.pair0[d.g]) {
+            case 1: sw_task<1>(A, sm, it, d); break;
+            case 2: sw_task<2>(A, sm, it, d); break;
+            default: sw_task<4>(A, sm, it, d); break;
+        }
+    }
+}
+
+unsigned int sweep_take_wait_timeouts() {
+    unsigned int h = 0, zero_v = 0;
+    GT_CUDA(cudaMemcpyFromSymbol(&h, g_sweep_timeouts, sizeof(h)));
+    if (h) GT_CUDA(cudaMemcpyToSymbol(g_sweep_timeouts, &zero_v, sizeof(zero_v)));
+    return h;
+}
+
+// blocks of the sweep kernel the current device holds at once
+static int resident_blocks() {
+    static std::mutex lock;
+    static std::map<int, int> held;
+    int dev = 0;
+    GT_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lk(lock);
+    int& n = held[dev];
+    if (!n) {
+        int sms = 0, per = 0;
+        GT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        GT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, sweep_kernel, SW_BLOCK, sizeof(SwShared)));
+        n = std::max(1, sms * std::max(per, 1));
+    }
+    return n;
+}
+
+void launch_sweep(const SweepPlan& S, const Fronts& F, const c32* pf, const c32* pb, const c32* dinv, const c32* s, c32* z,
+                  c32* y, c32* u, c32* sd, const Groups& G, int* cnt, int t0, int t1, cudaStream_t st) {
+    raise_smem((const void*)sweep_kernel, sizeof(SwShared));
+    SwArgs A{};
+    A.tasks = S.tasks;
+    A.nft = S.nft;
+    A.nbt = S.nbt;
+    A.nsrc = S.nsrc;
+    A.src_rows = S.src_rows;
+    A.src = S.src;
+    A.bidx = S.bidx;
+    A.iperm = F.iperm;
+    A.nfac = F.nfac;
+    A.nvec = F.vec_total;
+    A.nnode = F.nnode;
+    A.ptotal = S.ptotal;
+    A.pf = reinterpret_cast<const float2*>(pf);
+    A.pb = reinterpret_cast<const float2*>(pb);
+    A.dinv = reinterpret_cast<const float2*>(dinv);
+    A.s = reinterpret_cast<const float2*>(s);
+    A.z = reinterpret_cast<float4*>(z);
+    A.y = reinterpret_cast<float4*>(y);
+    A.u = reinterpret_cast<float4*>(u);
+    A.sd = reinterpret_cast<float2*>(sd);
+    A.G = G;
+    A.cnt = cnt + 1;
+    A.t0 = t0 * G.ngroup;
+    A.t1 = t1 * G.ngroup;
+    const int64_t tickets = (int64_t)(t1 - t0) * G.ngroup;
+    if (tickets <= 0) return;
+    sweep_kernel<<<(int)std::min<int64_t>(tickets, resident_blocks()), SW_BLOCK, sizeof(SwShared), st>>>(A);
+    GT_LAUNCH_CHECK();
+}
+
+// ------------------------------------------------------------------------------------------ the plan
+// Outputs per tile of a level: whole fronts while the level has tasks enough for the GPU by them, else 128, 64, 32 or 16,
+// the widest that gives a column group 96 tasks (a wide tile gathers its inner rows once for more outputs; the top of the
+// tree, one or a few fronts, takes narrow tiles to spread over the SMs).
+static int tile_of(const int64_t* fronts, int64_t n, const std::vector<int>& ext) {
+    for (int H : {128, 64, 32}) {
+        int64_t tasks = 0;
+        for (int64_t q = 0; q < n; ++q) tasks += (ext[fronts[q]] + H - 1) / H;
+        if (tasks >= 96) return H;
+    }
+    return 16;
+}
+
+SweepPlanHost make_sweep_plan(int nfront, int nlev, const int64_t* level_ptr, const int64_t* order, const int64_t* own_start,
+                              const int64_t* nown, const int64_t* nbnd, const int64_t* bnd_ptr, const int64_t* bnd_idx,
+                              const int64_t* child_ptr, const int64_t* child_idx, const int64_t* cmap_ptr,
+                              const int64_t* cmap_idx, const int64_t* vec_off) {
+    SweepPlanHost S;
+    std::vector<int> nf(nfront), no(nfront), parent(nfront, -1);
+    std::vector<int64_t> roff(nfront + 1, 0);
+    for (int f = 0; f < nfront; ++f) {
+        no[f] = (int)nown[f];
+        nf[f] = (int)(nown[f] + nbnd[f]);
+        roff[f + 1] = roff[f] + nf[f];
+        for (int64_t c = child_ptr[f]; c < child_ptr[f + 1]; ++c) parent[child_idx[c]] = f;
+    }
+    // each front row's sources among the update vectors, in the children's order
+    S.src_rows = std::max<int64_t>(roff[nfront], 1);
+    std::vector<std::vector<int>> lists;
+    std::vector<int> held(S.src_rows, 0);
+    for (int f = 0; f < nfront; ++f)
+        for (int64_t ci = child_ptr[f]; ci < child_ptr[f + 1]; ++ci) {
+            const int64_t c = child_idx[ci];
+            for (int64_t i = 0; i < nbnd[c]; ++i) {
+                const int64_t row = roff[f] + cmap_idx[cmap_ptr[ci] + i];
+                const int k = held[row]++;
+                if (k >= (int)lists.size()) lists.emplace_back(S.src_rows, -1);
+                lists[k][row] = (int)(vec_off[c] + i);
+            }
+        }
+    S.nsrc = (int)lists.size();
+    for (auto& l : lists) S.src.insert(S.src.end(), l.begin(), l.end());
+    S.bidx.assign(bnd_idx, bnd_idx + bnd_ptr[nfront]);
+    // tile widths per front and the tiles' places in the panel copies
+    S.hf.assign(nfront, 16);
+    S.hb.assign(nfront, 16);
+    for (int h = 0; h < nlev; ++h) {
+        const int64_t* fr = order + level_ptr[h];
+        const int64_t n = level_ptr[h + 1] - level_ptr[h];
+        const int tf = tile_of(fr, n, nf), tb = tile_of(fr, n, no);
+        for (int64_t q = 0; q < n; ++q) S.hf[fr[q]] = tf, S.hb[fr[q]] = tb;
+    }
+    S.offf.resize(nfront);
+    S.offb.resize(nfront);
+    std::vector<int> ntf(nfront, 0), ntb(nfront, 0);
+    int64_t pf = 0, pb = 0;
+    for (int f = 0; f < nfront; ++f) {
+        S.offf[f] = pf;
+        S.offb[f] = pb;
+        for (int r = 0; r < nf[f]; r += S.hf[f]) {
+            const int h = std::min(S.hf[f], nf[f] - r);
+            pf += (int64_t)((h + 1) & ~1) * std::min(no[f], r + S.hf[f]);
+            ++ntf[f];
+        }
+        for (int k = 0; k < no[f]; k += S.hb[f]) {
+            const int h = std::min(S.hb[f], no[f] - k);
+            pb += (int64_t)((h + 1) & ~1) * (nf[f] - k);
+            ++ntb[f];
+        }
+    }
+    S.ptotal = std::max<int64_t>({pf, pb, 2});
+    S.ptotal += S.ptotal & 1;
+    // counters: f: tiles of f's children done going up; nfront + f: f's own tiles done coming down; 2 nfront + f: a
+    // root's own tiles done going up
+    std::vector<int> need(nfront, 0);
+    for (int f = 0; f < nfront; ++f)
+        if (parent[f] >= 0) need[parent[f]] += ntf[f];
+    for (int h = 0; h < nlev; ++h) {
+        for (int64_t q = level_ptr[h]; q < level_ptr[h + 1]; ++q) {
+            const int f = (int)order[q];
+            int64_t off = S.offf[f];
+            for (int r = 0; r < nf[f]; r += S.hf[f]) {
+                SwTask t{};
+                t.r0 = r;
+                t.h = std::min(S.hf[f], nf[f] - r);
+                t.k0 = 0;
+                t.k1 = std::min(no[f], r + S.hf[f]);
+                t.dep = f;
+                t.need = need[f];
+                t.sig = parent[f] >= 0 ? parent[f] : 2 * nfront + f;
+                t.nown = no[f];
+                t.own0 = (int)own_start[f];
+                t.voff = (int)vec_off[f];
+                t.goff = roff[f];
+                t.off = off;
+                off += (int64_t)((t.h + 1) & ~1) * t.k1;
+                S.tasks.push_back(t);
+            }
+        }
+        S.level_f.push_back((int)S.tasks.size());
+    }
+    S.nft = (int)S.tasks.size();
+    for (int h = nlev - 1; h >= 0; --h) {
+        for (int64_t q = level_ptr[h]; q < level_ptr[h + 1]; ++q) {
+            const int f = (int)order[q];
+            int a = parent[f];
+            while (a >= 0 && !ntb[a]) a = parent[a];
+            int root = f;
+            while (parent[root] >= 0) root = parent[root];
+            int64_t off = S.offb[f];
+            for (int k = 0; k < no[f]; k += S.hb[f]) {
+                SwTask t{};
+                t.r0 = k;
+                t.h = std::min(S.hb[f], no[f] - k);
+                t.k0 = k;
+                t.k1 = nf[f];
+                t.dep = a >= 0 ? nfront + a : 2 * nfront + root;
+                t.need = a >= 0 ? ntb[a] : ntf[root];
+                t.sig = nfront + f;
+                t.nown = no[f];
+                t.own0 = (int)own_start[f];
+                t.voff = (int)vec_off[f];
+                t.goff = bnd_ptr[f];
+                t.off = off;
+                off += (int64_t)((t.h + 1) & ~1) * (t.k1 - t.k0);
+                S.tasks.push_back(t);
+            }
+        }
+        S.level_b.push_back((int)S.tasks.size());
+    }
+    S.nbt = (int)S.tasks.size() - S.nft;
+    return S;
+}
+
+}  // namespace gt
