@@ -40,7 +40,7 @@ constexpr int SW_STAGES = 2;
 constexpr int SW_STAGE_ENT = 1792;     // panel entries per stage (14 KB)
 constexpr int SW_XROWS = 256;          // inner rows staged at once (16 KB at 8 columns)
 constexpr int SW_HMAX = 128;
-constexpr uint64_t SW_WAIT_NS = 2000000000ull;
+constexpr long long SW_WAIT_CYCLES = 4000000000ll;       // two seconds
 constexpr uint32_t SW_POLLS = 1u << 28;
 
 struct SwDesc {                        // one ring stage, written by the producer
@@ -65,11 +65,6 @@ static_assert(SW_XROWS * 4 >= 2 * SWT * 4, "the partial sums take the staged row
 __device__ unsigned int g_sweep_timeouts = 0;
 
 __device__ __forceinline__ uint32_t sw_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ uint64_t sw_ns() {
-    uint64_t t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
 __device__ __forceinline__ bool sw_try(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
@@ -82,10 +77,10 @@ __device__ __noinline__ void sw_gave_up() { atomicAdd(&g_sweep_timeouts, 1u); }
 __device__ __forceinline__ void sw_wait_bar(uint64_t* b, uint32_t parity) {
     const uint32_t bar = sw_smem(b);
     if (sw_try(bar, parity)) return;
-    const uint64_t t0 = sw_ns();
+    const long long t0 = clock64();
     for (uint32_t it = 0; it < SW_POLLS; ++it) {
         if (sw_try(bar, parity)) return;
-        if (sw_ns() - t0 > 2 * SW_WAIT_NS) break;
+        if (clock64() - t0 > 2 * SW_WAIT_CYCLES) break;
     }
     sw_gave_up();
 }
@@ -96,12 +91,12 @@ __device__ __forceinline__ int sw_acquire(const int* p) {
 }
 __device__ __forceinline__ void sw_wait_count(const int* p, int need) {
     if (sw_acquire(p) >= need) return;
-    const uint64_t t0 = sw_ns();
+    const long long t0 = clock64();
     for (uint32_t it = 0; it < SW_POLLS; ++it) {
         if (sw_acquire(p) >= need) return;
         if ((it & 63) == 63) {
             if (*(volatile unsigned int*)&g_sweep_timeouts) return;      // someone gave up already
-            if (sw_ns() - t0 > SW_WAIT_NS) break;
+            if (clock64() - t0 > SW_WAIT_CYCLES) break;
         }
         __nanosleep(32);
     }
@@ -109,21 +104,37 @@ __device__ __forceinline__ void sw_wait_count(const int* p, int need) {
 }
 __device__ __forceinline__ void sw_sync() { asm volatile("bar.sync 1, %0;" ::"n"(SWT) : "memory"); }
 
-// two packed FP32 FMAs: acc.x += a.x b.x, acc.y += a.y b.y
-__device__ __forceinline__ void fma2(float2& acc, float2 a, float2 b) {
-    uint64_t c = reinterpret_cast<uint64_t&>(acc);
-    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c)
-        : "l"(reinterpret_cast<const uint64_t&>(a)), "l"(reinterpret_cast<const uint64_t&>(b)));
-    acc = reinterpret_cast<float2&>(c);
+// two packed FP32 FMAs: each half of acc += a b
+__device__ __forceinline__ void fma2(uint64_t& acc, uint64_t a, uint64_t b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ uint64_t both(float a) {
+    uint64_t v;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(v) : "f"(a));
+    return v;
+}
+__device__ __forceinline__ float4 halves(uint64_t re, uint64_t im) {
+    float4 v;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(re));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.z), "=f"(v.w) : "l"(im));
+    return v;
+}
+__device__ __forceinline__ void add4(float4& a, float4 b) {
+    a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
 }
 
-// (re, im) pairs of a column pair += p * x for the panel entry p
-__device__ __forceinline__ void mac_pair(float2& re, float2& im, float2 pr, float2 pi, float2 npi, float4 x) {
-    const float2 xr = make_float2(x.x, x.y), xi = make_float2(x.z, x.w);
-    fma2(re, pr, xr);
-    fma2(re, npi, xi);
-    fma2(im, pr, xi);
-    fma2(im, pi, xr);
+// (re, im) of NP column pairs += (pr + j pi) x
+template <int NP>
+__device__ __forceinline__ void mac_row(uint64_t* re, uint64_t* im, float pr, float pi, const ulonglong2* X) {
+    const uint64_t r2 = both(pr), i2 = both(pi), n2 = both(-pi);
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+        const ulonglong2 x = X[p];                       // the pair's real parts, its imaginary parts
+        fma2(re[p], r2, x.x);
+        fma2(im[p], r2, x.y);
+        fma2(re[p], n2, x.y);
+        fma2(im[p], i2, x.x);
+    }
 }
 
 struct SwArgs {
@@ -144,9 +155,17 @@ struct SwArgs {
     float4* u;                         // interleaved [group][nvec][pairs]
     float2* sd;                        // [slot][nnode] solutions, node order
     Groups G;
-    int* cnt;                          // [counter][ngroup] finished tiles; the ticket counter in front of them
+    int* cnt;                          // [counter][ngroup] finished tiles
+    int* ticket;                       // this launch's ticket counter
     int t0, t1;                        // tickets of this launch
 };
+
+// where the partial sum of row pair row2, entry e = row * NP + pair, stands: the entries of a row pair permuted by the row
+// pair, so that the warp that stores one entry of 32 row pairs, and the one that reads them in order, meet all banks
+template <int NP>
+__device__ __forceinline__ int sw_slot(int row2, int e) {
+    return row2 * 2 * NP + (e ^ ((row2 / (4 / NP)) & (2 * NP - 1)));
+}
 
 template <int NP>
 __device__ void sw_task(const SwArgs& A, SwShared& sm, uint32_t& it, const SwDesc& d0) {
@@ -179,7 +198,7 @@ __device__ void sw_task(const SwArgs& A, SwShared& sm, uint32_t& it, const SwDes
                 const int e = A.src[s * A.src_rows + t.goff + t.r0 + r];
                 if (e >= 0) {
                     const float4 b = __ldcg(u + (int64_t)e * NP + p);
-                    a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+                    add4(a, b);
                 }
             }
             sm.eb[q] = a;
@@ -188,11 +207,11 @@ __device__ void sw_task(const SwArgs& A, SwShared& sm, uint32_t& it, const SwDes
         for (int q = tid; q < h; q += SWT) sm.node[q] = (int)A.iperm[t.own0 + t.r0 + q];
         sw_sync();
     }
-    float2 re[2][NP], im[2][NP];
+    uint64_t re[2][NP], im[2][NP];
 #pragma unroll
     for (int r = 0; r < 2; ++r)
 #pragma unroll
-        for (int p = 0; p < NP; ++p) re[r][p] = im[r][p] = make_float2(0.f, 0.f);
+        for (int p = 0; p < NP; ++p) re[r][p] = im[r][p] = 0;
     int xbeg = t.k0, xend = t.k0;
     bool last;
     do {
@@ -221,7 +240,7 @@ __device__ void sw_task(const SwArgs& A, SwShared& sm, uint32_t& it, const SwDes
                             const int e = A.src[c * A.src_rows + t.goff + row];
                             if (e >= 0) {
                                 const float4 b = __ldcg(u + (int64_t)e * NP + p);
-                                a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+                                add4(a, b);
                             }
                         }
                         sm.x[q] = a;
@@ -239,19 +258,13 @@ __device__ void sw_task(const SwArgs& A, SwShared& sm, uint32_t& it, const SwDes
             }
             const int e = min(kb, xend);
             if (act) {
-                const float4* P = reinterpret_cast<const float4*>(ring + (k - ka) * hp) + row2;
-                const float4* X = sm.x + (k - xbeg) * NP;
+                const float4* P = reinterpret_cast<const float4*>(ring) + (k - ka + seg) * np2 + row2;
+                const ulonglong2* X = reinterpret_cast<const ulonglong2*>(sm.x) + (k - xbeg + seg) * NP;
 #pragma unroll 2
-                for (int q = seg; q < e - k; q += nseg) {
-                    const float4 a = P[q * np2];          // outputs 2 row2, 2 row2 + 1
-                    const float2 pr0 = make_float2(a.x, a.x), pi0 = make_float2(a.y, a.y), ni0 = make_float2(-a.y, -a.y);
-                    const float2 pr1 = make_float2(a.z, a.z), pi1 = make_float2(a.w, a.w), ni1 = make_float2(-a.w, -a.w);
-#pragma unroll
-                    for (int p = 0; p < NP; ++p) {
-                        const float4 x = X[q * NP + p];
-                        mac_pair(re[0][p], im[0][p], pr0, pi0, ni0, x);
-                        mac_pair(re[1][p], im[1][p], pr1, pi1, ni1, x);
-                    }
+                for (int q = k + seg; q < e; q += nseg, P += nseg * np2, X += nseg * NP) {
+                    const float4 a = *P;                  // outputs 2 row2, 2 row2 + 1
+                    mac_row<NP>(re[0], im[0], a.x, a.y, X);
+                    mac_row<NP>(re[1], im[1], a.z, a.w, X);
                 }
             }
             k = e;
@@ -267,16 +280,13 @@ __device__ void sw_task(const SwArgs& A, SwShared& sm, uint32_t& it, const SwDes
 #pragma unroll
         for (int r = 0; r < 2; ++r)
 #pragma unroll
-            for (int p = 0; p < NP; ++p)
-                sm.x[(seg * hp + 2 * row2 + r) * NP + p] = make_float4(re[r][p].x, re[r][p].y, im[r][p].x, im[r][p].y);
+            for (int p = 0; p < NP; ++p) sm.x[seg * hp * NP + sw_slot<NP>(row2, r * NP + p)] = halves(re[r][p], im[r][p]);
     }
     sw_sync();
     for (int q = tid; q < h * NP; q += SWT) {
-        float4 v = sm.x[q];
-        for (int sg = 1; sg < nseg; ++sg) {
-            const float4 b = sm.x[sg * hp * NP + q];
-            v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
-        }
+        const int at = sw_slot<NP>(q / (2 * NP), q % (2 * NP));
+        float4 v = sm.x[at];
+        for (int sg = 1; sg < nseg; ++sg) add4(v, sm.x[sg * hp * NP + at]);
         const int r = q / NP, p = q - r * NP, row = t.r0 + r;
         if (dir == 0) {
             if (row < t.nown) {
@@ -316,10 +326,9 @@ __global__ void __launch_bounds__(SW_BLOCK, 4) sweep_kernel(SwArgs A) {
     if (threadIdx.x >= SWT) {
         if (threadIdx.x != SWT) return;
         // the producer: tickets in order, each task's panel run stage by stage
-        int* ticket = A.cnt - 1;
         uint32_t it = 0;
         for (;;) {
-            const int tk = A.t0 + atomicAdd(ticket, 1);
+            const int tk = A.t0 + atomicAdd(A.ticket, 1);
             const bool done = tk >= A.t1;
             SwTask t{};
             int g = 0, dir = -1;
@@ -401,7 +410,6 @@ static int resident_blocks() {
 
 void launch_sweep(const SweepPlan& S, const Fronts& F, const c32* pf, const c32* pb, const c32* dinv, const c32* s, c32* z,
                   c32* y, c32* u, c32* sd, const Groups& G, int* cnt, int t0, int t1, cudaStream_t st) {
-    raise_smem((const void*)sweep_kernel, sizeof(SwShared));
     SwArgs A{};
     A.tasks = S.tasks;
     A.nft = S.nft;
@@ -425,10 +433,12 @@ void launch_sweep(const SweepPlan& S, const Fronts& F, const c32* pf, const c32*
     A.sd = reinterpret_cast<float2*>(sd);
     A.G = G;
     A.cnt = cnt + 1;
+    A.ticket = cnt;
     A.t0 = t0 * G.ngroup;
     A.t1 = t1 * G.ngroup;
     const int64_t tickets = (int64_t)(t1 - t0) * G.ngroup;
     if (tickets <= 0) return;
+    raise_smem((const void*)sweep_kernel, sizeof(SwShared));
     sweep_kernel<<<(int)std::min<int64_t>(tickets, resident_blocks()), SW_BLOCK, sizeof(SwShared), st>>>(A);
     GT_LAUNCH_CHECK();
 }
