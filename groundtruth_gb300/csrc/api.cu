@@ -281,6 +281,23 @@ struct gt_geometry {
     std::unique_ptr<Workspace> ws;
     Profiler prof;
     std::mutex lock;
+    // scratch of the output and coupling calls, kept from call to call (each of them holds the lock and leaves no kernel
+    // running), freed by gt_geometry_trim and with the geometry
+    void* scratch = nullptr;
+    size_t scratch_bytes = 0;
+    template <typename T> T* small_scratch(size_t n) {
+        if (n * sizeof(T) > scratch_bytes) {
+            free_scratch();
+            GT_CUDA(cudaMalloc(&scratch, n * sizeof(T)));
+            scratch_bytes = n * sizeof(T);
+        }
+        return static_cast<T*>(scratch);
+    }
+    void free_scratch() {
+        if (scratch) cudaFree(scratch);
+        scratch = nullptr;
+        scratch_bytes = 0;
+    }
     // the triangular sweeps of independent column groups run on these streams side by side, so that one
     // group's elimination level overlaps another's
     static constexpr int NSUB = 4;
@@ -295,6 +312,7 @@ struct gt_geometry {
         }
     }
     ~gt_geometry() {
+        free_scratch();
         for (int k = 0; k < NSUB; ++k) {
             if (sub[k]) cudaStreamDestroy(sub[k]);
             if (join[k]) cudaEventDestroy(join[k]);
@@ -1525,9 +1543,10 @@ int gt_geometry_trim(gt_geometry* G) {
     GT_GUARD_BEGIN
     if (!G) throw Invalid("null geometry");
     std::lock_guard<std::mutex> lk(G->lock);
-    if (G->ws) {
+    if (G->ws || G->scratch) {
         GT_CUDA(cudaDeviceSynchronize());
         G->ws.reset();
+        G->free_scratch();
     }
     return GT_OK;
     GT_GUARD_END
@@ -2007,15 +2026,17 @@ int gt_strip_coupling(gt_geometry* G, const double* sheet_z, const double* sheet
     std::lock_guard<std::mutex> lk(G->lock);
     const int64_t ns = G->n_strips;
     if (n_strips) *n_strips = ns;
-    Pool tmp;
-    const int S = G->geo.S;
-    double* dz = tmp.upload(sheet_z, S);
-    double* dt = tmp.upload(sheet_t, S);
-    double* dseg = n_seg ? tmp.upload(segments, (size_t)n_seg * 8) : nullptr;
-    double* dpsi = tmp.alloc<double>(std::max<int64_t>(ns, 1));
+    SheetZ z{}, t{};
+    for (int k = 0; k < G->geo.S; ++k) {
+        z.z[k] = sheet_z[k];
+        t.z[k] = sheet_t[k];
+    }
+    double* dseg = G->small_scratch<double>((size_t)n_seg * 8 + std::max<int64_t>(ns, 1));
+    double* dpsi = dseg + (size_t)n_seg * 8;
     cudaStream_t st = 0;
+    if (n_seg) GT_CUDA(cudaMemcpyAsync(dseg, segments, (size_t)n_seg * 8 * sizeof(double), cudaMemcpyHostToDevice, st));
     if (n_seg == 0) GT_CUDA(cudaMemsetAsync(dpsi, 0, std::max<int64_t>(ns, 1) * sizeof(double), st));
-    else launch_strip_coupling(G->geo, G->d_c2d, ns, dz, dt, pitch, dseg, n_seg, dpsi, st);
+    else launch_strip_coupling(G->geo, G->d_c2d, ns, z, t, pitch, dseg, n_seg, dpsi, st);
     GT_CUDA(cudaMemcpy(psi, dpsi, ns * sizeof(double), cudaMemcpyDeviceToHost));
     return GT_OK;
     GT_GUARD_END
@@ -2042,12 +2063,13 @@ int gt_moment(gt_geometry* G, int32_t n_cols, const void* x_device, const double
     if (G->geo.NL != G->geo.S) throw Invalid("the moment of face sheets is taken on the host");
     std::lock_guard<std::mutex> lk(G->lock);
     cudaStream_t st = (cudaStream_t)stream;
-    Pool tmp;
-    double* dz = tmp.upload(sheet_z, G->geo.S);
-    c64* dm = tmp.alloc<c64>((size_t)n_cols * 3);
-    launch_moment(G->geo, static_cast<const c64*>(x_device), G->geo.n, n_cols, dz, pitch, dm, st);
+    SheetZ zs{};
+    for (int k = 0; k < G->geo.S; ++k) zs.z[k] = sheet_z[k];
+    const size_t part = (size_t)n_cols * moment_blocks(G->geo) * 3;
+    c64* dm = G->small_scratch<c64>(part + (size_t)n_cols * 3);
+    launch_moment(G->geo, static_cast<const c64*>(x_device), G->geo.n, n_cols, zs, pitch, dm, dm + part, st);
+    GT_CUDA(cudaMemcpyAsync(m, dm + part, (size_t)n_cols * 3 * sizeof(c64), cudaMemcpyDeviceToHost, st));
     GT_CUDA(cudaStreamSynchronize(st));
-    GT_CUDA(cudaMemcpy(m, dm, (size_t)n_cols * 3 * sizeof(c64), cudaMemcpyDeviceToHost));
     return GT_OK;
     GT_GUARD_END
 }

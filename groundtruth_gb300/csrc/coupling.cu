@@ -14,18 +14,27 @@ namespace gt {
 namespace {
 
 constexpr double MU0_4PI = 1e-7;     // mu0 / (4 pi)
-constexpr int SEG_TILE = 256;
+constexpr int SEG_TILE = 128;
 
 struct Seg {
     double a[3], b[3], width, cur;
+    double u[3], L, iL2, rmin2, lim, zm;     // direction, length, 1 / L^2, r_min^2, the cell average's reach, mean height
 };
 
-__device__ __forceinline__ double vec_pot(const Seg& s, double L, const double* u, double px, double py, double pz,
-                                          double rmin) {
+// A(p) of a segment.  The two terms asinh(a / rho) + asinh(b / rho), a = L - p.u, b = p.u, are one asinh by its addition
+// theorem: sinh of the sum is (a rb + b ra) / rho^2 with ra, rb the distances to the ends, and for ends on either side of
+// the foot (a, b of opposite sign), where that would cancel, L (a - b) / (a rb - b ra).  Half the transcendental work of
+// the sum of two: the kernel is bound by the FP64 pipe (two operations a clock and SM).
+__device__ __forceinline__ double vec_pot(const Seg& s, double px, double py, double pz) {
     const double dx = px - s.a[0], dy = py - s.a[1], dz = pz - s.a[2];
-    const double pu = dx * u[0] + dy * u[1] + dz * u[2];
-    const double rho = sqrt(fmax(dx * dx + dy * dy + dz * dz - pu * pu, rmin * rmin));
-    return MU0_4PI * (asinh((L - pu) / rho) + asinh(pu / rho));
+    const double pu = dx * s.u[0] + dy * s.u[1] + dz * s.u[2];
+    const double h2 = fmax(dx * dx + dy * dy + dz * dz - pu * pu, s.rmin2);
+    const double a = s.L - pu;
+    const double ra = sqrt(a * a + h2), rb = sqrt(pu * pu + h2);
+    const bool within = a >= 0 && pu >= 0;
+    const double num = within ? a * rb + pu * ra : s.L * (a - pu);
+    const double den = within ? h2 : a * rb - pu * ra;
+    return MU0_4PI * asinh(num / den);
 }
 
 __device__ __forceinline__ double dist_to_segment(const Seg& s, double px, double py, double pz) {
@@ -38,8 +47,7 @@ __device__ __forceinline__ double dist_to_segment(const Seg& s, double px, doubl
 }
 
 __global__ void __launch_bounds__(256) strip_coupling_kernel(Geo g, const int64_t* __restrict__ c2d, int64_t ns,
-                                                             const double* __restrict__ sheet_z,
-                                                             const double* __restrict__ sheet_t, double d,
+                                                             SheetZ sheet_z, SheetZ sheet_t, double d,
                                                              const double* __restrict__ segs, int nseg,
                                                              double* __restrict__ psi) {
     __shared__ Seg sh[SEG_TILE];
@@ -67,7 +75,7 @@ __global__ void __launch_bounds__(256) strip_coupling_kernel(Geo g, const int64_
             cy = j * d + 0.5 * d;
         }
     }
-    const double zk = act ? sheet_z[k] : 0.0, half = act ? 0.5 * sheet_t[k] : 0.0;
+    const double zk = act ? sheet_z.z[k] : 0.0, half = act ? 0.5 * sheet_t.z[k] : 0.0;
     // the 3-point Gauss-Legendre rule on [-1/2, 1/2]
     const double gq[3] = {-0.5 * sqrt(0.6), 0.0, 0.5 * sqrt(0.6)};
     const double gw[3] = {5.0 / 9.0, 8.0 / 9.0, 5.0 / 9.0};
@@ -77,7 +85,17 @@ __global__ void __launch_bounds__(256) strip_coupling_kernel(Geo g, const int64_
         __syncthreads();
         for (int q = threadIdx.x; q < nt; q += blockDim.x) {
             const double* r = segs + (int64_t)(t0 + q) * 8;
-            sh[q] = Seg{{r[0], r[1], r[2]}, {r[3], r[4], r[5]}, r[6], r[7]};
+            Seg s{{r[0], r[1], r[2]}, {r[3], r[4], r[5]}, r[6], r[7]};
+            const double ab[3] = {r[3] - r[0], r[4] - r[1], r[5] - r[2]};
+            const double L2 = ab[0] * ab[0] + ab[1] * ab[1] + ab[2] * ab[2];
+            s.L = sqrt(L2);
+            for (int c = 0; c < 3; ++c) s.u[c] = ab[c] / s.L;
+            s.iL2 = 1.0 / L2;
+            const double rmin = fmax(0.5 * r[6], 1e-7);
+            s.rmin2 = rmin * rmin;
+            s.lim = 3 * d + 2 * r[6];
+            s.zm = 0.5 * (r[2] + r[5]);
+            sh[q] = s;
         }
         __syncthreads();
         if (!act) continue;
@@ -85,23 +103,27 @@ __global__ void __launch_bounds__(256) strip_coupling_kernel(Geo g, const int64_
             const Seg& s = sh[q];
             const double ab[3] = {s.b[0] - s.a[0], s.b[1] - s.a[1], s.b[2] - s.a[2]};
             if (ab[0] == 0.0 && ab[1] == 0.0) continue;                  // vertical: not a horizontal segment
-            const double L = sqrt(ab[0] * ab[0] + ab[1] * ab[1] + ab[2] * ab[2]);
-            if (fabs(ab[axis]) < 1e-15 * L) continue;
-            const double u[3] = {ab[0] / L, ab[1] / L, ab[2] / L};
-            const double cz = zk + (0.5 * (s.a[2] + s.b[2]) > zk ? half : -half);
-            const double rmin = fmax(0.5 * s.width, 1e-7);
+            if (fabs(ab[axis]) < 1e-15 * s.L) continue;
+            const double cz = zk + (s.zm > zk ? half : -half);
+            // near: the centre within lim of the segment; by the squared distance, and by the distance itself where the
+            // two are too close for that
+            const double dx = cx - s.a[0], dy = cy - s.a[1], dz = cz - s.a[2];
+            const double tt = fmin(fmax((dx * ab[0] + dy * ab[1] + dz * ab[2]) * s.iL2, 0.0), 1.0);
+            const double qx = dx - tt * ab[0], qy = dy - tt * ab[1], qz = dz - tt * ab[2];
+            const double d2 = qx * qx + qy * qy + qz * qz, l2 = s.lim * s.lim;
+            const bool near = fabs(d2 - l2) > 1e-9 * l2 ? d2 < l2 : dist_to_segment(s, cx, cy, cz) < s.lim;
             double a;
-            if (dist_to_segment(s, cx, cy, cz) < 3 * d + 2 * s.width) {
+            if (near) {
                 a = 0.0;
                 for (int m = 0; m < 3; ++m)
                     for (int n = 0; n < 3; ++n) {
                         const double da = (axis == 0 ? gq[m] : gq[n]) * d, dl = (axis == 0 ? gq[n] : gq[m]) * d;
-                        a += vec_pot(s, L, u, cx + da, cy + dl, cz, rmin) * (gw[m] * gw[n] / 4.0);
+                        a += vec_pot(s, cx + da, cy + dl, cz) * (gw[m] * gw[n] / 4.0);
                     }
             } else {
-                a = vec_pot(s, L, u, cx, cy, cz, rmin);
+                a = vec_pot(s, cx, cy, cz);
             }
-            acc += (s.cur * ab[axis] / L) * a;
+            acc += (s.cur * s.u[axis]) * a;
         }
     }
     if (act) psi[c] = d * acc;
@@ -109,7 +131,7 @@ __global__ void __launch_bounds__(256) strip_coupling_kernel(Geo g, const int64_
 
 }  // namespace
 
-void launch_strip_coupling(const Geo& g, const int64_t* c2d, int64_t ns, const double* sheet_z, const double* sheet_t,
+void launch_strip_coupling(const Geo& g, const int64_t* c2d, int64_t ns, const SheetZ& sheet_z, const SheetZ& sheet_t,
                            double d, const double* segs, int nseg, double* psi, cudaStream_t st) {
     if (ns <= 0) return;
     strip_coupling_kernel<<<ceil_div(ns, 256), 256, 0, st>>>(g, c2d, ns, sheet_z, sheet_t, d, segs, nseg, psi);

@@ -105,13 +105,17 @@ template <typename R>
 void launch_pc_strip(const Geo& g, const cx<R>* r, int64_t ldr, const cx<R>* sd, cx<R>* out, int64_t ldo, int ncol,
                      const int* col_op, const cx<R>* tab, const int* col_list, cudaStream_t st);
 
-// psi of the first ns compact entries (the strips): segments [nseg][8] (a, b, width, current), device FP64
-void launch_strip_coupling(const Geo& g, const int64_t* c2d, int64_t ns, const double* sheet_z, const double* sheet_t,
+// psi of the first ns compact entries (the strips): segments [nseg][8] (a, b, width, current), device FP64; the sheets'
+// heights and thicknesses by value
+struct SheetZ { double z[8]; };
+void launch_strip_coupling(const Geo& g, const int64_t* c2d, int64_t ns, const SheetZ& sheet_z, const SheetZ& sheet_t,
                            double d, const double* segs, int nseg, double* psi, cudaStream_t st);
 
 // post-solve outputs from dense FP64 solutions [col][ld]: node fields kx / ky [col][S][nx][ny]; moments [col][3]
 void launch_node_field(const Geo& g, const c64* x, int64_t ld, int ncol, double d, c64* kx, c64* ky, cudaStream_t st);
-void launch_moment(const Geo& g, const c64* x, int64_t ld, int ncol, const double* zs, double d, c64* m,
+// (part: ncol x moment_blocks x 3 scratch; zs by value)
+int moment_blocks(const Geo& g);
+void launch_moment(const Geo& g, const c64* x, int64_t ld, int ncol, const SheetZ& zs, double d, c64* part, c64* m,
                    cudaStream_t st);
 
 // the real (P0/2+1) x (P1/2+1) spectrum quadrant of a strip kernel (host in / out, device work)
