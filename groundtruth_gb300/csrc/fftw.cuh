@@ -86,6 +86,34 @@ template <typename R, bool INV> __device__ __forceinline__ void w4(cx<R>& a0, cx
     a3 = t1 - t3;
 }
 
+// cos(2 pi i / 24) (sin(2 pi i / 24) is cos24(i - 6)), for the lengths 3, 6, 12 and 24
+template <typename R> __device__ __forceinline__ R cos24(int i) {
+    switch (((i % 24) + 24) % 24) {
+        case 0: return R(1.0);
+        case 1: case 23: return R(9.65925826289068312e-01);
+        case 2: case 22: return R(8.66025403784438708e-01);
+        case 3: case 21: return R(7.07106781186547573e-01);
+        case 4: case 20: return R(0.5);
+        case 5: case 19: return R(2.58819045102520739e-01);
+        case 6: case 18: return R(0.0);
+        case 7: case 17: return R(-2.58819045102520739e-01);
+        case 8: case 16: return R(-0.5);
+        case 9: case 15: return R(-7.07106781186547573e-01);
+        case 10: case 14: return R(-8.66025403784438708e-01);
+        case 11: case 13: return R(-9.65925826289068312e-01);
+    }
+    return R(-1.0);
+}
+
+// a * W_N^m with m known once the loops are unrolled (N divides 24)
+template <typename R, bool INV, int N>
+__device__ __forceinline__ cx<R> wtw3(cx<R> a, int m) {
+    m %= N;
+    if (m == 0) return a;
+    const R c = cos24<R>(m * (24 / N)), s = cos24<R>(m * (24 / N) - 6);
+    return INV ? mk<R>(a.re * c - a.im * s, a.im * c + a.re * s) : mk<R>(a.re * c + a.im * s, a.im * c - a.re * s);
+}
+
 // N-point DFT (N = 4, 8, 16, 32) of v[0 .. N) in natural order, in place, as A x B with A = 4:
 // X[ka + 4 kb] = sum_b W_N^(b ka) W_B^(b kb) sum_a v[B a + b] W_4^(a ka).  HALF: v[N/2 ..] are zero and
 // not read.  LO: only X[0 .. N/2) are wanted (the rest are left undefined).
@@ -137,6 +165,37 @@ __device__ __forceinline__ void rdft(cx<R>* v) {
             rdft<R, INV, B>(t);
 #pragma unroll
             for (int kb = 0; kb < (LO ? B / 2 : B); ++kb) v[ka + A * kb] = t[kb];
+        }
+    }
+}
+
+// N-point DFT of v[0 .. N) in natural order for N = 2^a <= 32 or N = 3 * 2^a <= 24, as 3 x N/3 in the latter case:
+// X[ka + 3 kb] = sum_b W_N^(b ka) W_M^(b kb) sum_a v[M a + b] W_3^(a ka), M = N / 3
+template <typename R, bool INV, int N, bool HALF = false, bool LO = false>
+__device__ __forceinline__ void rdft3(cx<R>* v) {
+    if constexpr (N % 3 != 0) {
+        if constexpr (N > 1) rdft<R, INV, N, HALF, LO>(v);
+    } else {
+        constexpr int M = N / 3;
+        const R s3 = INV ? R(8.66025403784438708e-01) : R(-8.66025403784438708e-01);
+        cx<R> u[N];
+#pragma unroll
+        for (int b = 0; b < M; ++b) {
+            const cx<R> x0 = v[b];
+            const cx<R> x1 = HALF && 2 * (M + b) >= N + 1 ? zero<R>() : v[M + b];
+            const cx<R> x2 = HALF ? zero<R>() : v[2 * M + b];
+            const cx<R> sum = x1 + x2, dif = x1 - x2;
+            const cx<R> m = mk<R>(x0.re - R(0.5) * sum.re, x0.im - R(0.5) * sum.im);
+            const cx<R> j = mk<R>(-s3 * dif.im, s3 * dif.re);
+            u[b] = x0 + sum;
+            u[M + b] = wtw3<R, INV, N>(m + j, b);
+            u[2 * M + b] = wtw3<R, INV, N>(m - j, 2 * b);
+        }
+#pragma unroll
+        for (int ka = 0; ka < 3; ++ka) {
+            if constexpr (M > 1) rdft<R, INV, M>(u + ka * M);
+#pragma unroll
+            for (int kb = 0; kb < M; ++kb) v[ka + 3 * kb] = u[ka * M + kb];
         }
     }
 }
@@ -214,6 +273,58 @@ __device__ __forceinline__ void fft512_inv2(cx<R> (&u)[32], cx<R> (&v)[2][16], c
     tw512_lane2<R, true>(v[0], v[1], lane, tw);
     rdft<R, true, 16, false, LO>(v[0]);
     rdft<R, true, 16, false, LO>(v[1]);
+}
+
+// The same transforms for N = 32 A, A = 2^a or 3 * 2^a up to 32, RR = the rows a warp carries (RR A <= 32 lanes take the
+// 32-point DFTs; with A = 12 or 24 a quarter of them idle).  The upper half of the rows is zero on the way in and not
+// wanted on the way out: with H = ceil(A / 2), lane t holds x_q[t + 32 r] in v[q][r], r < H; lane q A + k1 holds
+// X_q[k1 + A k2] in u[k2].  tw: W_N^m, m < N.  sx: RR x A x 33 slots of the warp's own.
+template <int A> struct WarpFft {
+    static constexpr int N = 32 * A, H = (A + 1) / 2, RR = A >= 24 ? 1 : A >= 12 ? 2 : A >= 6 ? 4 : 8, SLOTS = RR * A * 33;
+};
+
+template <typename R, int A>
+__device__ __forceinline__ void fftw_fwd(cx<R> (&v)[WarpFft<A>::RR][A], cx<R> (&u)[32], cx<R>* sx, const cx<R>* __restrict__ tw) {
+    constexpr int RR = WarpFft<A>::RR;
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int q = 0; q < RR; ++q) rdft3<R, false, A, true>(v[q]);
+#pragma unroll
+    for (int k1 = 0; k1 < A; ++k1) {
+        const cx<R> w = tw[lane * k1];
+#pragma unroll
+        for (int q = 0; q < RR; ++q) sx[(q * A + k1) * 33 + lane] = k1 ? v[q][k1] * w : v[q][k1];
+    }
+    __syncwarp();
+    const int at = lane < RR * A ? lane : 0;
+#pragma unroll
+    for (int t = 0; t < 32; ++t) u[t] = sx[at * 33 + t];
+    __syncwarp();
+    rdft<R, false, 32>(u);
+}
+
+template <typename R, int A>
+__device__ __forceinline__ void fftw_inv(cx<R> (&u)[32], cx<R> (&v)[WarpFft<A>::RR][A], cx<R>* sx, const cx<R>* __restrict__ tw) {
+    constexpr int RR = WarpFft<A>::RR;
+    const int lane = threadIdx.x & 31;
+    rdft<R, true, 32>(u);
+    if (lane < RR * A) {
+#pragma unroll
+        for (int t = 0; t < 32; ++t) sx[lane * 33 + t] = u[t];
+    }
+    __syncwarp();
+#pragma unroll
+    for (int k1 = 0; k1 < A; ++k1) {
+        const cx<R> w = tw[lane * k1];
+#pragma unroll
+        for (int q = 0; q < RR; ++q) {
+            const cx<R> a = sx[(q * A + k1) * 33 + lane];
+            v[q][k1] = k1 ? twm<R, true>(a, w) : a;
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < RR; ++q) rdft3<R, true, A, false, true>(v[q]);
 }
 
 }  // namespace gt

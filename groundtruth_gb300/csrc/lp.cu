@@ -59,8 +59,12 @@ __global__ void __launch_bounds__(1024) lp_pass_a(const cx<R>* __restrict__ x, i
     }
 }
 
+// threads of a block of the generic column pass: half as many in FP64, whose values take twice the registers (at 1024 it
+// spilled 3-5 KB a thread); the runtime-length form takes any length, up to 1024 threads for one row
+template <typename R, int PL> __host__ __device__ constexpr int lp_threads() { return sizeof(R) == 8 && PL ? 512 : 1024; }
+
 template <typename R, int PL>
-__global__ void __launch_bounds__(1024) lp_pass_b(int S, int n0, int P0, int P1, int ncol, int bt, const R* __restrict__ spec,
+__global__ void __launch_bounds__(lp_threads<R, PL>()) lp_pass_b(int S, int n0, int P0, int P1, int ncol, int bt, const R* __restrict__ spec,
                           const cx<R>* __restrict__ tw, cx<R>* __restrict__ T, int ldt) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cx<R>* buf = reinterpret_cast<cx<R>*>(smem_raw);
@@ -337,6 +341,85 @@ __global__ void __launch_bounds__(BW_WARPS * 32, GT_BW_MINB) lp_pass_bw(int n0, 
             const int j = lane + 32 * r;
             if (ok[q] && j < n0) row[q][j] = v[q][r];
         }
+}
+
+// Pass B in FP32 for the other lengths of 32 A (and for 512 with more than two sheets): warps transform RR rows each
+// (fftw.cuh), a row being one sheet of one column; the transforms pass through the block's shared rows for the S x S
+// multiply, one thread per pixel of a column, and back.  A block takes as many columns as give it about four warps.
+// The Stockham form of these lengths (lp_pass_b) moves every value through shared memory four times per transform under
+// block-wide barriers and spills: 103 us for six columns of a four-sheet 131 x 203 board at length 384.
+template <int A>
+__global__ void __launch_bounds__(256, 2) lp_pass_bg(int S, int n0, int P1, int ncol, int bt, const float* __restrict__ spec,
+                                                     const c32* __restrict__ tw, c32* __restrict__ T, int ldt) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr int N = 32 * A, Q0 = N / 2 + 1, RR = WarpFft<A>::RR, H = WarpFft<A>::H, RS = A * 33;
+    c32* Z = reinterpret_cast<c32*>(smem_raw);           // [row][k1 * 33 + k2], pixel k1 + A k2
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int c = blockIdx.x, b0 = blockIdx.y * bt, nb = min(bt, ncol - b0), nrow = nb * S;
+    c32* sx = Z + warp * RR * RS;
+    const c32* src[RR];
+    bool ok[RR];
+#pragma unroll
+    for (int q = 0; q < RR; ++q) {
+        const int row = warp * RR + q, b = row / S;
+        ok[q] = row < nrow;
+        src[q] = T + (((int64_t)(b0 + min(b, nb - 1)) * S + (row - b * S)) * P1 + c) * ldt;
+    }
+    c32 u[32];
+    {
+        c32 v[RR][A];
+#pragma unroll
+        for (int q = 0; q < RR; ++q)
+#pragma unroll
+            for (int r = 0; r < A; ++r) {
+                const int j = lane + 32 * r;
+                v[q][r] = r < H && ok[q] && j < n0 ? src[q][j] : zero<float>();
+            }
+        fftw_fwd<float, A>(v, u, sx, tw);
+    }
+    if (lane < RR * A)
+#pragma unroll
+        for (int k2 = 0; k2 < 32; ++k2) sx[lane * 33 + k2] = u[k2];
+    __syncthreads();
+    const float* Kc = spec + (int64_t)min(c, P1 - c) * Q0 * S * S;
+    for (int idx = threadIdx.x; idx < nb * N; idx += blockDim.x) {
+        const int b = idx / N, e = idx - b * N, k1 = e >> 5, k2 = e & 31, p = k1 + A * k2;
+        const float* K = Kc + (int64_t)min(p, N - p) * S * S;
+        c32* z = Z + b * S * RS + k1 * 33 + k2;
+        c32 w[MAXS];
+#pragma unroll
+        for (int s = 0; s < MAXS; ++s)
+            if (s < S) w[s] = z[s * RS];
+#pragma unroll
+        for (int t = 0; t < MAXS; ++t) {
+            if (t >= S) break;
+            c32 acc = zero<float>();
+#pragma unroll
+            for (int s = 0; s < MAXS; ++s)
+                if (s < S) {
+                    const float k = __ldg(K + t * S + s);
+                    acc.re += k * w[s].re;
+                    acc.im += k * w[s].im;
+                }
+            z[t * RS] = acc;
+        }
+    }
+    __syncthreads();
+    const int at = lane < RR * A ? lane : 0;
+#pragma unroll
+    for (int k2 = 0; k2 < 32; ++k2) u[k2] = sx[at * 33 + k2];
+    __syncwarp();
+    {
+        c32 v[RR][A];
+        fftw_inv<float, A>(u, v, sx, tw);
+#pragma unroll
+        for (int q = 0; q < RR; ++q)
+#pragma unroll
+            for (int r = 0; r < H; ++r) {
+                const int j = lane + 32 * r;
+                if (ok[q] && j < n0) const_cast<c32*>(src[q])[j] = v[q][r];
+            }
+    }
 }
 
 // Row passes for P1 = 512 in FP32 (n1 <= 256): a block of RW_WARPS warps takes RW_ROWS = 16 consecutive rows
@@ -902,31 +985,47 @@ static void launch_bw(const LpArgs<float>& a, cudaStream_t st) {
     GT_LAUNCH_CHECK();
 }
 
+template <int A>
+static void launch_bg(const LpArgs<float>& a, cudaStream_t st) {
+    constexpr int RR = WarpFft<A>::RR;
+    const int bt = std::max(1, std::min(a.ncol, (4 * RR + a.S - 1) / a.S));
+    const int warps = ceil_div(bt * a.S, RR);
+    const size_t sm = (size_t)warps * WarpFft<A>::SLOTS * sizeof(c32);
+    set_smem<float>((const void*)lp_pass_bg<A>, sm);
+    lp_pass_bg<A><<<dim3(a.P1, ceil_div(a.ncol, bt)), warps * 32, sm, st>>>(a.S, a.n0, a.P1, a.ncol, bt, a.spec, a.tw0, a.T,
+                                                                          ldt_of(a));
+    GT_LAUNCH_CHECK();
+}
+
 template <typename R, int PB>
 static void launch_b(const LpArgs<R>& a, int bt, cudaStream_t st) {
-    if constexpr (PB == 512 && std::is_same<R, float>::value) {
-        if (a.n0 <= PB / 2 && a.S <= 2) {
-            if (a.S == 2) launch_bw<2>(a, st);
-            else launch_bw<1>(a, st);
-            return;
+    // FP32: warp transforms for the lengths of 32 A (every length P0 >= 2 n0 - 1 is even, so n0 <= P0 / 2)
+    constexpr bool warp = std::is_same<R, float>::value && (PB == 96 || PB == 128 || PB == 192 || PB == 256 || PB == 384 ||
+                                                            PB == 512 || PB == 768 || PB == 1024);
+    if constexpr (warp) {
+        if constexpr (PB == 512) {
+            if (a.S == 2) return launch_bw<2>(a, st);
+            if (a.S == 1) return launch_bw<1>(a, st);
         }
-    }
-    if constexpr (PB == 64 || PB == 512) {
-        if (b8_fits(a)) {
-            switch (a.S) {
-                case 1: launch_b8<R, PB, 1>(a, bt, st); return;
-                case 2: launch_b8<R, PB, 2>(a, bt, st); return;
-                case 3: launch_b8<R, PB, 3>(a, bt, st); return;
-                default: launch_b8<R, PB, 4>(a, bt, st); return;
+        launch_bg<PB / 32>(a, st);
+    } else {
+        if constexpr (PB == 64 || PB == 512) {
+            if (b8_fits(a)) {
+                switch (a.S) {
+                    case 1: launch_b8<R, PB, 1>(a, bt, st); return;
+                    case 2: launch_b8<R, PB, 2>(a, bt, st); return;
+                    case 3: launch_b8<R, PB, 3>(a, bt, st); return;
+                    default: launch_b8<R, PB, 4>(a, bt, st); return;
+                }
             }
         }
+        size_t smB = (size_t)bt * a.S * srow(a.P0) * sizeof(cx<R>);
+        dim3 gB(a.P1, ceil_div(a.ncol, bt));
+        const int team = a.P0 / 8, threads = std::min(bt * a.S, lp_threads<R, PB>() / team) * team;
+        set_smem<R>((const void*)lp_pass_b<R, PB>, smB);
+        lp_pass_b<R, PB><<<gB, threads, smB, st>>>(a.S, a.n0, a.P0, a.P1, a.ncol, bt, a.spec, a.tw0, a.T, ldt_of(a));
+        GT_LAUNCH_CHECK();
     }
-    size_t smB = (size_t)bt * a.S * srow(a.P0) * sizeof(cx<R>);
-    dim3 gB(a.P1, ceil_div(a.ncol, bt));
-    const int team = a.P0 / 8, threads = std::min(bt * a.S, 1024 / team) * team;
-    set_smem<R>((const void*)lp_pass_b<R, PB>, smB);
-    lp_pass_b<R, PB><<<gB, threads, smB, st>>>(a.S, a.n0, a.P0, a.P1, a.ncol, bt, a.spec, a.tw0, a.T, ldt_of(a));
-    GT_LAUNCH_CHECK();
 }
 
 // cuTensorMapEncodeTiled from the driver (no link against libcuda: the runtime hands out its entry point)
