@@ -256,11 +256,13 @@ struct gt_geometry {
     std::vector<double> level_panel;   // panel entries (sum of nf x nown) of each level
     int max_nf = 0;
     int64_t* d_order = nullptr;
-    // the factorisation's order: each level's small fronts, then its large ones (nf >= tiled_nf, the blocked
-    // multi-CTA elimination), with the large ones' counts and extents per level
+    // the factorisation's order: each level's small fronts (one CTA each), then its large ones (the blocked multi-CTA
+    // elimination), with the small ones' shared memory and the large ones' counts and extents per level
     int64_t* d_forder = nullptr;
-    std::vector<int> level_nbig, level_bigmaxnf, level_bigmaxnown, level_smallmaxnf;
-    int tiled_nf = 256;
+    std::vector<int> level_nbig, level_bigmaxnf, level_bigmaxnown;
+    std::vector<size_t> level_smem;
+    int* d_xfirst = nullptr;           // the large fronts' first diagonal block among all of theirs
+    int64_t xtotal = 0;
     // every large front (all levels), for the blocked selective inversion
     int64_t* d_bigfronts = nullptr;
     int nbig = 0, bigmax_nf = 1, bigmax_nown = 1;
@@ -1439,22 +1441,36 @@ int gt_geometry_create(const gt_geometry_desc* d, gt_geometry** out) {
         G->max_nf = std::max(G->max_nf, mx);
     }
     {
-        if (const char* e = std::getenv("GT_TILED_NF")) G->tiled_nf = std::max(1, std::atoi(e));
+        // Large: fronts of tiled_nf rows (a CTA's share of the FP64 rate, 1 / 152, would be the level's time), those whose
+        // own columns do not fit a CTA's shared memory, and fronts of LONE_NF rows or more on levels too narrow to give
+        // every SM one (at LONE_OPS operators, the same for any number so that a factorisation does not depend on its
+        // company).
+        constexpr int LONE_NF = 96, LONE_OPS = 4, SMS = 152;
+        int tiled_nf = 256;
+        const char* tiled_env = std::getenv("GT_TILED_NF");
+        if (tiled_env) tiled_nf = std::max(1, std::atoi(tiled_env));
+        std::vector<int> xfirst(std::max(nf, 1), -1);
         std::vector<int64_t> ord;
         ord.reserve(nf);
         for (int h = 0; h < d->n_levels; ++h) {
             std::vector<int64_t> small, big;
-            int bmx = 1, bmo = 1, smx = 1;
+            int bmx = 1, bmo = 1;
+            size_t smem = 0;
+            const int64_t width = d->level_ptr[h + 1] - d->level_ptr[h];
             for (int64_t q = d->level_ptr[h]; q < d->level_ptr[h + 1]; ++q) {
                 const int64_t f = d->front_order[q];
                 const int nff = (int)(d->nown[f] + d->nbnd[f]);
-                if (nff >= G->tiled_nf) {
+                const int no = (int)d->nown[f];
+                if (nff >= tiled_nf || !small_front_fits(no, nff - no) ||
+                    (!tiled_env && width * LONE_OPS < SMS && nff >= LONE_NF)) {
                     big.push_back(f);
+                    xfirst[f] = (int)G->xtotal;
+                    G->xtotal += ceil_div(no, FACTOR_BLOCK);
                     bmx = std::max(bmx, nff);
                     bmo = std::max<int>(bmo, (int)d->nown[f]);
                 } else {
                     small.push_back(f);
-                    smx = std::max(smx, nff);
+                    smem = std::max(smem, small_front_smem(no, nff - no));
                 }
             }
             ord.insert(ord.end(), small.begin(), small.end());
@@ -1462,19 +1478,20 @@ int gt_geometry_create(const gt_geometry_desc* d, gt_geometry** out) {
             G->level_nbig.push_back((int)big.size());
             G->level_bigmaxnf.push_back(bmx);
             G->level_bigmaxnown.push_back(bmo);
-            G->level_smallmaxnf.push_back(smx);
+            G->level_smem.push_back(smem);
         }
         G->d_forder = p.upload(ord.data(), ord.size());
         std::vector<int64_t> big;
         for (int f = 0; f < nf; ++f) {
             const int nff = (int)(d->nown[f] + d->nbnd[f]);
-            if (nff < G->tiled_nf) continue;
+            if (xfirst[f] < 0) continue;
             big.push_back(f);
             G->bigmax_nf = std::max(G->bigmax_nf, nff);
             G->bigmax_nown = std::max<int>(G->bigmax_nown, (int)d->nown[f]);
         }
         G->nbig = (int)big.size();
         G->d_bigfronts = p.upload(big.data(), big.size());
+        G->d_xfirst = p.upload(xfirst.data(), xfirst.size());
     }
     {
         const SweepPlanHost H = make_sweep_plan(nf, d->n_levels, d->level_ptr, d->front_order, d->own_start, d->nown, d->nbnd,
@@ -1637,6 +1654,7 @@ int gt_operators_create_ex(gt_geometry* G, int32_t n_ops, const double* omega, c
     Pool tmp;
     c64* svals = tmp.alloc<c64>((size_t)n_ops * F.nsv);
     c64* upd = tmp.alloc<c64>((size_t)n_ops * std::max<int64_t>(F.upd_total, 1));
+    c64* xinv = tmp.alloc<c64>((size_t)n_ops * G->xtotal * FACTOR_BLOCK * FACTOR_BLOCK);
     int* status = tmp.alloc<int>(1);
     GT_CUDA(cudaMemsetAsync(status, 0, sizeof(int), st));
     O->panel64 = (keep64 ? p : tmp).alloc<c64>((size_t)n_ops * F.panel_total);
@@ -1659,29 +1677,22 @@ int gt_operators_create_ex(gt_geometry* G, int32_t n_ops, const double* omega, c
         const int nbig = G->level_nbig[h], nsmall = nfl - nbig;
         const int64_t* lst = G->d_forder + G->level_ptr[h];
         Scope sc(P, P->levels ? ("factor.L" + std::to_string(h)).c_str() : "factor_levels", st);
-        if (nsmall) launch_factor_level(F, lst, nsmall, G->level_smallmaxnf[h], svals, O->panel64, upd, n_ops, status, st);
+        if (nsmall)
+            launch_small_fronts(F, G->sweep, lst, nsmall, G->level_smem[h], svals, O->panel64, upd, O->panel64_rm, O->dinv64,
+                                O->dinv32, O->panel32, O->panel32_b, n_ops, status, st);
         if (nbig)
-            launch_factor_tiled(F, lst + nsmall, nbig, G->level_bigmaxnf[h], G->level_bigmaxnown[h], svals, O->panel64,
-                                upd, n_ops, status, st);
-    }
-    int max_nown = 1;
-    for (int h = 0; h < nlev; ++h) max_nown = std::max(max_nown, G->level_maxnown[h]);
-    {
-        Scope sc(P, "factor_invert", st);
-        launch_invert_own(F, O->panel64, max_nown, n_ops, G->tiled_nf, st);
-    }
-    {
-        Scope sc(P, "factor_bnd_inv", st);
-        launch_bnd_inv(F, O->panel64, G->max_nf, n_ops, G->tiled_nf, st);
+            launch_factor_tiled(F, lst + nsmall, nbig, G->level_bigmaxnf[h], G->level_bigmaxnown[h], svals, O->panel64, upd,
+                                xinv, G->d_xfirst, G->xtotal, n_ops, status, st);
     }
     {
         Scope sc(P, "factor_invert_tiled", st);
-        launch_invert_tiled(F, G->d_bigfronts, G->nbig, G->bigmax_nf, G->bigmax_nown, O->panel64, n_ops, st);
+        launch_invert_tiled(F, G->d_bigfronts, G->nbig, G->bigmax_nf, G->bigmax_nown, O->panel64, xinv, G->d_xfirst, G->xtotal,
+                            n_ops, st);
     }
     {
         Scope sc(P, "factor_convert", st);
-        launch_panel_convert(F, G->sweep, O->panel64, O->panel32, O->panel32_b, O->panel64_rm, O->dinv64, O->dinv32, n_ops,
-                             G->tiled_nf, st);
+        launch_panel_convert(F, G->sweep, G->d_bigfronts, G->nbig, O->panel64, O->panel32, O->panel32_b, O->panel64_rm,
+                             O->dinv64, O->dinv32, n_ops, st);
     }
     int h_status = 0;
     GT_CUDA(cudaMemcpyAsync(&h_status, status, sizeof(int), cudaMemcpyDeviceToHost, st));

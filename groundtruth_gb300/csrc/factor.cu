@@ -6,8 +6,8 @@
 //
 //   assemble   S values = sum of coef * admittance table entries (a fixed sparse map, per frequency)
 //   front      F = own columns of S + children's update matrices (extend-add)
-//   eliminate  the own columns of F by rank-1 updates; L and D go to the front's panel (nf x nown,
-//              column-major, D on its diagonal), the trailing block is the front's update matrix
+//   eliminate  the own columns of F; L and D go to the front's panel (nf x nown, column-major, D on its diagonal),
+//              the trailing block is the front's update matrix
 //
 // FP64 throughout (a floating plane coupled only by plane-pair capacitance makes S nearly singular in one
 // mode whose pivot is ~1e-10 of the strips' admittance); the panels are also rounded to FP32 for the
@@ -18,7 +18,7 @@
 
 namespace gt {
 
-// Complex multiply-accumulate as four explicit FMAs (acc += a u; cfms: acc -= a u): written out, the
+// Complex multiply-accumulate as four explicit FMAs (acc += a u): written out, the
 // product and the sum round as separate operations (six instructions instead of four on the FP64 pipe).
 __device__ __forceinline__ void cfma(c32& acc, c32 a, c32 u) {
     acc.re = __fmaf_rn(a.re, u.re, acc.re);
@@ -32,13 +32,6 @@ __device__ __forceinline__ void cfma(c64& acc, c64 a, c64 u) {
     acc.im = __fma_rn(a.re, u.im, acc.im);
     acc.im = __fma_rn(a.im, u.re, acc.im);
 }
-__device__ __forceinline__ void cfms(c64& acc, c64 a, c64 u) {
-    acc.re = __fma_rn(-a.re, u.re, acc.re);
-    acc.re = __fma_rn(a.im, u.im, acc.re);
-    acc.im = __fma_rn(-a.re, u.im, acc.im);
-    acc.im = __fma_rn(-a.im, u.re, acc.im);
-}
-
 __global__ void assemble_s_kernel(const int64_t* __restrict__ ptr, const int* __restrict__ tab_idx,
                                   const double* __restrict__ coef, int64_t nsv, const c64* __restrict__ table, int ntab,
                                   c64* __restrict__ svals) {
@@ -68,12 +61,263 @@ struct FrontView {
     }
 };
 
-// A front's entries before elimination: the own columns of S and the children's update matrices, one child
+// 1 / d for a positive normal d: an FP32 seed of the mantissa and two Newton steps r += r (1 - d r) (within 2 ulp; the
+// compiler's division occupies the FP64 pipe, two operations a clock and SM, three times as long, on the pivots' chain)
+__device__ __forceinline__ double recip64(double d) {
+    const long long bits = __double_as_longlong(d);
+    const int e = (int)(bits >> 52) - 1023;
+    const double m = __longlong_as_double((bits & 0xfffffffffffffll) | 0x3ff0000000000000ll);      // in [1, 2)
+    double r = (double)(1.0f / (float)m);
+    r = __fma_rn(r, __fma_rn(-m, r, 1.0), r);
+    r = __fma_rn(r, __fma_rn(-m, r, 1.0), r);
+    return r * __longlong_as_double((long long)(1023 - e) << 52);
+}
+
+__device__ __forceinline__ c64 pivot_inverse(c64 d, int* status) {
+    double dd = d.re * d.re + d.im * d.im;
+    if (!(dd > 1e-300) || !isfinite(dd)) {
+        atomicOr(status, 1);
+        d = mk<double>(1e-150, 0.0);
+        dd = 1e-300;
+    }
+    const double r = recip64(dd);
+    return mk<double>(d.re * r, -d.im * r);
+}
+
+__device__ __forceinline__ FrontView front_view(const Fronts& F, int f, int op, c64* panel, c64* upd) {
+    const int nown = (int)F.nown[f], nbnd = (int)F.nbnd[f];
+    return FrontView{panel + (int64_t)op * F.panel_total + F.panel_off[f], upd + (int64_t)op * F.upd_total + F.upd_off[f],
+                     nown + nbnd, nown, nbnd};
+}
+
+// tile t of the lower triangle of a T x T tile grid: (bi, bj), bj <= bi
+__device__ __forceinline__ void lower_tile(int t, int& bi, int& bj) {
+    int b = (int)((sqrtf(8.0f * t + 1.0f) - 1.0f) * 0.5f);
+    while ((int64_t)b * (b + 1) / 2 > t) --b;
+    while ((int64_t)(b + 1) * (b + 2) / 2 <= t) ++b;
+    bi = b;
+    bj = t - b * (b + 1) / 2;
+}
+
+// The sweeps' copies of a front's finished panel P = [Linv_own; -L_bnd Linv_own] (unit diagonal, zeros above it):
+// element (i, k) into its FP32 forward tile (rows gH .., inner k < min(nown, (g + 1) H)) and backward tile (columns
+// tC .., inner i >= tC), see sweep.cu.
+struct SweepTiles {
+    int nf, nown, H, C;
+    c32 *tf, *tb;
+    __device__ SweepTiles(const SweepPlan& S, int f, int op, int nf_, int nown_, c32* pf, c32* pb)
+        : nf(nf_), nown(nown_), H(S.hf[f]), C(S.hb[f]), tf(pf + (int64_t)op * S.ptotal + S.offf[f]),
+          tb(pb + (int64_t)op * S.ptotal + S.offb[f]) {}
+    __device__ __forceinline__ void fwd(int i, int k, c32 v) const {
+        const int g = i / H;
+        if (k >= min(nown, (g + 1) * H)) return;
+        const int m = min(g, nown / H), h = min(H, nf - g * H);
+        tf[(int64_t)H * H * m * (m + 1) / 2 + (int64_t)H * nown * (g - m) + (int64_t)k * ((h + 1) & ~1) + (i - g * H)] = v;
+    }
+    __device__ __forceinline__ void bwd(int i, int k, c32 v) const {
+        const int t = k / C;
+        if (i < t * C) return;
+        const int h = min(C, nown - t * C);
+        tb[(int64_t)C * ((int64_t)t * nf - (int64_t)C * t * (t - 1) / 2) + (int64_t)(i - t * C) * ((h + 1) & ~1) + (k - t * C)] = v;
+    }
+};
+
+// Small fronts: one CTA per (front, operator) with the front's own columns in shared memory from assembly to the finished
+// solve panel.  An SM of GB300 retires two FP64 FMAs a clock, a warp's instruction holding its quarter of the pipe for 64
+// cycles however few lanes it has, so the work is laid out flat over the threads (the elimination column by column as dot
+// products over row x segment, the update matrix and the inverse entry by entry), with no complex product in the inner
+// loops but the FMAs themselves:
+//   assemble   own columns of S plus the children's entries; what falls into the update matrix goes to global memory
+//   column k   a(i,k) - sum_{m<k} l(i,m) w(k,m), w = l d held unscaled in the upper triangle; l = that / d_k
+//   update     U(i,j) -= sum_k l(i,k) w(j,k)
+//   inverse    X = L_own^-1 row by row in place, M = -L_bnd X
+// and the sweeps' copies are written straight from shared memory.  Rank-1 updates in global memory and three passes for the
+// inversion and the copies took 41 of the 127 ms of four factorisations of the 256 x 256 pair.
+constexpr int SF_THREADS = 256;
+constexpr size_t SF_SMEM_MAX = 224 * 1024;
+
+size_t small_front_smem(int nown, int nbnd) {
+    const size_t ldp = (size_t)(nown + nbnd) | 1, ldb = (size_t)nbnd | 1;
+    return ((size_t)nown * (ldp + ldb + 1) + SF_THREADS) * sizeof(c64);
+}
+bool small_front_fits(int nown, int nbnd) { return small_front_smem(nown, nbnd) <= SF_SMEM_MAX; }
+
+__global__ void __launch_bounds__(SF_THREADS) small_front_kernel(Fronts F, SweepPlan S, const int64_t* __restrict__ front_list,
+                                                                 const c64* __restrict__ svals, c64* __restrict__ panel,
+                                                                 c64* __restrict__ upd, c64* __restrict__ r64,
+                                                                 c64* __restrict__ d64, c32* __restrict__ d32,
+                                                                 c32* __restrict__ pf, c32* __restrict__ pb,
+                                                                 int* __restrict__ status) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int f = (int)front_list[blockIdx.x], op = blockIdx.y, tid = threadIdx.x;
+    const FrontView Fv = front_view(F, f, op, panel, upd);
+    const int nf = Fv.nf, nown = Fv.nown, nbnd = Fv.nbnd, ldp = nf | 1, ldb = nbnd | 1;
+    c64* P = reinterpret_cast<c64*>(smem_raw);            // [k][i]: L, the unscaled rows above its diagonal; then the inverse
+    c64* W = P + nown * ldp;                              // [k][j]: the boundary rows unscaled (l d); then M
+    c64* di = W + nown * ldb;                             // 1 / d
+    c64* red = di + nown;
+    const int64_t ch0 = F.child_ptr[f], ch1 = F.child_ptr[f + 1];
+    const bool kids = ch1 > ch0;
+    for (int q = tid; q < nown * ldp; q += SF_THREADS) P[q] = zero<double>();
+    if (kids)
+        for (int q = tid; q < nbnd * nbnd; q += SF_THREADS) Fv.upd[q] = zero<double>();
+    __syncthreads();
+    {
+        const c64* sv = svals + (int64_t)op * F.nsv;
+        for (int64_t e = F.ent_ptr[f] + tid; e < F.ent_ptr[f + 1]; e += SF_THREADS)
+            P[F.ent_col[e] * ldp + F.ent_row[e]] += sv[F.ent_s[e]];
+    }
+    __syncthreads();
+    for (int64_t ci = ch0; ci < ch1; ++ci) {
+        const int c = (int)F.child_idx[ci], nb = (int)F.nbnd[c];
+        const int64_t* map = F.cmap_idx + F.cmap_ptr[ci];
+        const c64* U = upd + (int64_t)op * F.upd_total + F.upd_off[c];
+        for (int q = tid; q < nb * nb; q += SF_THREADS) {
+            const int j = q / nb, i = q - j * nb;
+            if (i < j) continue;
+            const int mi = (int)map[i], mj = (int)map[j];
+            if (mj < nown) P[mj * ldp + mi] += U[q];
+            else Fv.upd[(mj - nown) * nbnd + (mi - nown)] += U[q];
+        }
+        __syncthreads();
+    }
+    // the own columns
+    for (int k = 0; k < nown; ++k) {
+        const int R = nf - k, nseg = R >= SF_THREADS ? 1 : min(SF_THREADS / R, max(1, k / 4));
+        c64* pk = P + k * ldp;
+        for (int t0 = 0; t0 < R; t0 += SF_THREADS) {       // (a front of more rows than threads takes them in turns)
+            const int seg = nseg > 1 ? tid / R : 0, i = k + t0 + tid - seg * R;
+            c64 acc = zero<double>();
+            const bool act = seg < nseg && i < nf;
+            if (act)
+                for (int m = seg; m < k; m += nseg) cfma(acc, P[m * ldp + i], pk[m]);
+            if (nseg > 1) {
+                red[tid] = acc;
+                __syncthreads();
+                if (act && seg == 0)
+                    for (int q = 1; q < nseg; ++q) acc += red[q * R + tid];
+            }
+            if (act && seg == 0) {
+                const c64 v = pk[i] - acc;
+                pk[i] = v;
+                if (i == k) di[k] = pivot_inverse(v, status);
+            }
+        }
+        __syncthreads();
+        const c64 dk = di[k];
+        for (int i = k + 1 + tid; i < nf; i += SF_THREADS) {
+            const c64 v = pk[i];
+            if (i < nown) P[i * ldp + k] = v;              // w(i, k), above the diagonal of column i
+            else W[k * ldb + i - nown] = v;
+            pk[i] = v * dk;
+        }
+        __syncthreads();
+    }
+    // the update matrix, lower triangle; threads run down its columns
+    const int ntri = nbnd * (nbnd + 1) / 2;
+    for (int e = tid; e < ntri; e += SF_THREADS) {
+        int a, b;
+        lower_tile(e, a, b);
+        const int i = nbnd - 1 - b, j = nbnd - 1 - a;
+        c64 acc = zero<double>();
+        for (int k = 0; k < nown; ++k) cfma(acc, P[k * ldp + nown + i], W[k * ldb + j]);
+        c64& u = Fv.upd[j * nbnd + i];
+        u = (kids ? u : zero<double>()) - acc;
+    }
+    // X = L_own^-1, row i from the rows above it: X(i,c) = -(L(i,c) + sum_{c<m<i} L(i,m) X(m,c))
+    __syncthreads();
+    for (int i = 1; i < nown; ++i) {
+        const int nseg = i >= SF_THREADS ? 1 : min(SF_THREADS / i, max(1, i / 4));
+        c64 keep = zero<double>();
+        for (int t0 = 0; t0 < i; t0 += SF_THREADS) {
+            const int seg = nseg > 1 ? tid / i : 0, c = t0 + tid - seg * i;
+            const bool act = seg < nseg && c < i;
+            c64 acc = zero<double>();
+            if (act)
+                for (int m = c + 1 + seg; m < i; m += nseg) cfma(acc, P[m * ldp + i], P[c * ldp + m]);
+            if (nseg > 1) {
+                red[tid] = acc;
+                __syncthreads();
+                if (act && seg == 0)
+                    for (int q = 1; q < nseg; ++q) acc += red[q * i + tid];
+            }
+            if (act && seg == 0) {
+                acc += P[c * ldp + i];
+                keep = mk<double>(-acc.re, -acc.im);
+            }
+        }
+        __syncthreads();                                   // every term has read row i of L (nown <= SF_THREADS here)
+        if (tid < i) P[tid * ldp + i] = keep;
+        __syncthreads();
+    }
+    // M = -L_bnd X, over the unscaled rows
+    for (int e = tid; e < nown * nbnd; e += SF_THREADS) {
+        const int c = e / nbnd, j = e - c * nbnd;
+        c64 acc = P[c * ldp + nown + j];
+        for (int m = c + 1; m < nown; ++m) cfma(acc, P[m * ldp + nown + j], P[c * ldp + m]);
+        W[c * ldb + j] = mk<double>(-acc.re, -acc.im);
+    }
+    __syncthreads();
+    auto at = [&](int i, int k) {
+        return i < k ? zero<double>() : i == k ? mk<double>(1.0, 0.0) : i < nown ? P[k * ldp + i] : W[k * ldb + i - nown];
+    };
+    const SweepTiles T(S, f, op, nf, nown, pf, pb);
+    const int64_t base = (int64_t)op * F.panel_total + F.panel_off[f], dbase = (int64_t)op * F.nfac + F.own_start[f];
+    for (int q = tid; q < nf * nown; q += SF_THREADS) {
+        const int k = q / nf, i = q - k * nf;
+        const c64 v = at(i, k);
+        if (r64) Fv.panel[q] = v;
+        T.fwd(i, k, cvt<float>(v));
+    }
+    for (int q = tid; q < nf * nown; q += SF_THREADS) {
+        const int i = q / nown, k = q - i * nown;
+        const c64 v = at(i, k);
+        if (r64) r64[base + q] = v;
+        T.bwd(i, k, cvt<float>(v));
+    }
+    for (int k = tid; k < nown; k += SF_THREADS) {
+        d64[dbase + k] = di[k];
+        d32[dbase + k] = cvt<float>(di[k]);
+    }
+}
+
+void launch_small_fronts(const Fronts& F, const SweepPlan& S, const int64_t* front_list, int nfront, size_t smem,
+                         const c64* svals, c64* panel, c64* upd, c64* r64, c64* d64, c32* d32, c32* pf, c32* pb, int nops,
+                         int* status, cudaStream_t st) {
+    raise_smem((const void*)small_front_kernel, smem);
+    small_front_kernel<<<dim3(nfront, nops), SF_THREADS, smem, st>>>(F, S, front_list, svals, panel, upd, r64, d64, d32, pf, pb,
+                                                                     status);
+    GT_LAUNCH_CHECK();
+}
+
+// Large fronts: blocked elimination, FB own columns per step, every step over many CTAs (the top of the tree
+// has a few fronts per operator, and an SM's FP64 rate is 1/152 of the GPU's):
+//   diag   one CTA per (front, operator) factors the FB x FB diagonal block in shared memory and inverts its L11
+//   rows   W21 = A21 L11^-T as a product with the inverse, L21 = W21 D^-1, 32 rows per CTA
+//   trail  A22 -= L21 D L21^T over FT x FT tiles of the trailing lower triangle, one tile per CTA
+// Tiles of 32 x 32 (32 us of an SM's FP64 pipe each; 64 x 64 took 127): the last steps of a top front have a few tiles
+// for 152 SMs.  A warp's FP64 instruction holds its quarter of the pipe for 64 cycles whatever its active lanes, so no step
+// leaves a product chain to one thread: rows by substitution, a thread a row, took 90 us a step.
+constexpr int FB = FACTOR_BLOCK, FT = 32;
+
+// the inverses of the diagonal blocks' L11: [op][first block of the front + kb / FB][FB x FB], row-major
+struct DiagInv {
+    c64* x;
+    const int* first;          // [nfront] first block of each large front
+    int64_t total;             // blocks per operator
+    __device__ __forceinline__ c64* of(int f, int op, int kb) const {
+        return x + ((int64_t)op * total + first[f] + kb / FB) * (FB * FB);
+    }
+};
+
+// A large front's entries before elimination: the own columns of S and the children's update matrices, one child
 // at a time (their boundaries overlap).  The panels start zeroed (one memset before the first level); the
 // update matrix's slot is shared with matrices of other levels (its last owner's was assembled into its
 // parent at an earlier level) and is cleared here.
-__device__ void assemble_front(const Fronts& F, int f, int op, const c64* __restrict__ svals, const FrontView& Fv,
-                               const c64* __restrict__ upd) {
+__global__ void assemble_fronts_kernel(Fronts F, const int64_t* __restrict__ front_list, const c64* __restrict__ svals,
+                                       c64* __restrict__ panel, c64* __restrict__ upd) {
+    const int f = (int)front_list[blockIdx.x], op = blockIdx.y;
+    const FrontView Fv = front_view(F, f, op, panel, upd);
     const int tid = threadIdx.x, nth = blockDim.x;
     for (int64_t q = tid; q < (int64_t)Fv.nbnd * Fv.nbnd; q += nth) Fv.upd[q] = zero<double>();
     __syncthreads();
@@ -85,154 +329,126 @@ __device__ void assemble_front(const Fronts& F, int f, int op, const c64* __rest
         const int nb = (int)F.nbnd[c];
         const int64_t* map = F.cmap_idx + F.cmap_ptr[ci];
         const c64* U = upd + (int64_t)op * F.upd_total + F.upd_off[c];
-        for (int64_t q = tid; q < (int64_t)nb * nb; q += nth) {
-            int j = int(q / nb), i = int(q - (int64_t)j * nb);
-            if (i >= j) Fv.at((int)map[i], (int)map[j]) += U[q];
+        const int warp = tid >> 5, lane = tid & 31;
+        for (int j = warp; j < nb; j += nth >> 5) {
+            const int mj = (int)map[j];
+            for (int i = j + lane; i < nb; i += 32) Fv.at((int)map[i], mj) += U[(int64_t)j * nb + i];
         }
         __syncthreads();
     }
 }
 
-__device__ __forceinline__ FrontView front_view(const Fronts& F, int f, int op, c64* panel, c64* upd) {
-    const int nown = (int)F.nown[f], nbnd = (int)F.nbnd[f];
-    return FrontView{panel + (int64_t)op * F.panel_total + F.panel_off[f], upd + (int64_t)op * F.upd_total + F.upd_off[f],
-                     nown + nbnd, nown, nbnd};
-}
-
-__device__ __forceinline__ c64 pivot_inverse(c64 d, int* status) {
-    const double dd = d.re * d.re + d.im * d.im;
-    if (!(dd > 1e-300) || !isfinite(dd)) {
-        atomicOr(status, 1);
-        d = mk<double>(1e-150, 0.0);
-    }
-    return cdiv(mk<double>(1.0, 0.0), d);
-}
-
-// Small fronts: one CTA per (front, operator) assembles the front and eliminates its own columns by rank-1
-// updates in place.
-__global__ void factor_level_kernel(Fronts F, const int64_t* __restrict__ front_list, const c64* __restrict__ svals,
-                                    c64* __restrict__ panel, c64* __restrict__ upd, int* __restrict__ status) {
-    const int f = (int)front_list[blockIdx.x];
-    const int op = blockIdx.y;
-    const FrontView Fv = front_view(F, f, op, panel, upd);
-    const int nf = Fv.nf, nown = Fv.nown;
-    assemble_front(F, f, op, svals, Fv, upd);
-    const int tid = threadIdx.x, nth = blockDim.x;
-    const int warp = tid >> 5, lane = tid & 31, nwarp = nth >> 5;
-    for (int k = 0; k < nown; ++k) {
-        const c64 d = Fv.panel[(int64_t)k * nf + k];
-        const double dd = d.re * d.re + d.im * d.im;
-        if ((!(dd > 1e-300) || !isfinite(dd)) && tid == 0) atomicOr(status, 1);
-        const c64 dinv = (!(dd > 1e-300) || !isfinite(dd)) ? cdiv(mk<double>(1.0, 0.0), mk<double>(1e-150, 0.0))
-                                                            : cdiv(mk<double>(1.0, 0.0), d);
-        const c64* colk = Fv.panel + (int64_t)k * nf;
-        for (int j = k + 1 + warp; j < nf; j += nwarp) {
-            const c64 ljd = colk[j] * dinv;
-            for (int i = j + lane; i < nf; i += 32) {
-                c64& v = Fv.at(i, j);
-                cfms(v, colk[i], ljd);
-            }
-        }
-        __syncthreads();
-        for (int i = k + 1 + tid; i < nf; i += nth) Fv.panel[(int64_t)k * nf + i] = Fv.panel[(int64_t)k * nf + i] * dinv;
-        __syncthreads();
-    }
-}
-
-void launch_factor_level(const Fronts& F, const int64_t* front_list, int nf_level, int max_nf, const c64* svals,
-                         c64* panel, c64* upd, int nops, int* status, cudaStream_t st) {
-    int threads = max_nf >= 256 ? 512 : 256;
-    factor_level_kernel<<<dim3(nf_level, nops), threads, 0, st>>>(F, front_list, svals, panel, upd, status);
-    GT_LAUNCH_CHECK();
-}
-
-// Large fronts: blocked elimination, FB own columns per step, every step over many CTAs (the top of the tree
-// has a few fronts per operator, and an SM's FP64 rate is 1/152 of the GPU's):
-//   diag   one warp per (front, operator) factors the FB x FB diagonal block in shared memory (lane = row)
-//   rows   L21 = A21 L11^-T D^-1 for the rows below it, one thread per row, 128 rows per CTA
-//   trail  A22 -= L21 D L21^T over 64 x 64 tiles of the trailing lower triangle, one tile per CTA
-// The arithmetic is the rank-1 kernel's, the updates of a block summed before they are subtracted.
-constexpr int FB = 32, FT = 64, ROWS_CTA = 128;
-
-__global__ void assemble_fronts_kernel(Fronts F, const int64_t* __restrict__ front_list, const c64* __restrict__ svals,
-                                       c64* __restrict__ panel, c64* __restrict__ upd) {
-    const int f = (int)front_list[blockIdx.x];
-    const int op = blockIdx.y;
-    assemble_front(F, f, op, svals, front_view(F, f, op, panel, upd), upd);
-}
-
-__global__ void __launch_bounds__(32) tiled_diag_kernel(Fronts F, const int64_t* __restrict__ front_list, int kb,
-                                                        c64* __restrict__ panel, c64* __restrict__ upd,
-                                                        int* __restrict__ status) {
+__global__ void __launch_bounds__(256) tiled_diag_kernel(Fronts F, const int64_t* __restrict__ front_list, int kb,
+                                                         c64* __restrict__ panel, c64* __restrict__ upd, DiagInv X,
+                                                         int* __restrict__ status) {
     __shared__ c64 a[FB][FB + 1];
-    const int f = (int)front_list[blockIdx.x];
-    const FrontView Fv = front_view(F, f, blockIdx.y, panel, upd);
+    __shared__ c64 x[FB][FB + 1];
+    __shared__ c64 red[256];
+    __shared__ c64 sd;
+    const int f = (int)front_list[blockIdx.x], op = blockIdx.y;
+    const FrontView Fv = front_view(F, f, op, panel, upd);
     const int nb = min(FB, Fv.nown - kb);
     if (nb <= 0) return;
-    const int i = threadIdx.x;
-    for (int j = 0; j < nb; ++j)
+    const int tid = threadIdx.x;
+    for (int q = tid; q < FB * FB; q += 256) {
+        const int j = q / FB, i = q - j * FB;
         a[i][j] = (i < nb && j <= i) ? Fv.panel[(int64_t)(kb + j) * Fv.nf + kb + i] : zero<double>();
-    __syncwarp();
-    for (int k = 0; k < nb; ++k) {
-        const c64 dinv = pivot_inverse(a[k][k], status);
-        const c64 lik = a[i][k];
-        for (int j = k + 1; j <= i && i < nb; ++j) a[i][j] -= lik * (a[j][k] * dinv);
-        __syncwarp();
-        if (i > k && i < nb) a[i][k] = lik * dinv;
-        __syncwarp();
-    }
-    if (i < nb)
-        for (int j = 0; j <= i; ++j) Fv.panel[(int64_t)(kb + j) * Fv.nf + kb + i] = a[i][j];
-}
-
-__global__ void __launch_bounds__(ROWS_CTA) tiled_rows_kernel(Fronts F, const int64_t* __restrict__ front_list, int kb,
-                                                              c64* __restrict__ panel, c64* __restrict__ upd) {
-    __shared__ c64 l11[FB][FB];
-    __shared__ c64 dv[FB];
-    const int f = (int)front_list[blockIdx.y];
-    const FrontView Fv = front_view(F, f, blockIdx.z, panel, upd);
-    const int nb = min(FB, Fv.nown - kb);
-    if (nb <= 0) return;
-    const int i = kb + nb + blockIdx.x * ROWS_CTA + threadIdx.x;
-    if (kb + nb + blockIdx.x * ROWS_CTA >= Fv.nf) return;             // the whole CTA is past the front
-    for (int q = threadIdx.x; q < FB * FB; q += ROWS_CTA) {
-        const int r = q / FB, c = q - r * FB;
-        l11[r][c] = (r < nb && c < r) ? Fv.panel[(int64_t)(kb + c) * Fv.nf + kb + r] : zero<double>();
-        if (r == c) dv[r] = r < nb ? Fv.panel[(int64_t)(kb + r) * Fv.nf + kb + r] : mk<double>(1.0, 0.0);
     }
     __syncthreads();
-    if (i >= Fv.nf) return;
-    c64 w[FB];                                                          // w = l D: the row's updates to come
-#pragma unroll
-    for (int k = 0; k < FB; ++k) {
-        if (k < nb) {
-            c64 t = Fv.panel[(int64_t)(kb + k) * Fv.nf + i];
-#pragma unroll
-            for (int m = 0; m < k; ++m) cfms(t, w[m], l11[k][m]);
-            w[k] = t;
+    for (int k = 0; k < nb; ++k) {
+        // column k as dot products over the columns before it; w = l d unscaled in the upper triangle
+        const int R = nb - k, nseg = min(256 / R, max(1, k / 4)), seg = tid / R, i = k + tid - seg * R;
+        c64 acc = zero<double>();
+        if (seg < nseg)
+            for (int m = seg; m < k; m += nseg) cfma(acc, a[i][m], a[m][k]);
+        red[tid] = acc;
+        __syncthreads();
+        if (tid < R) {
+            for (int q = 1; q < nseg; ++q) acc += red[q * R + tid];
+            const c64 v = a[i][k] - acc;
+            a[i][k] = v;
+            if (i == k) sd = pivot_inverse(v, status);
         }
+        __syncthreads();
+        if (tid < R && i > k) {
+            const c64 v = a[i][k];
+            a[k][i] = v;
+            a[i][k] = v * sd;
+        }
+        __syncthreads();
     }
+    for (int q = tid; q < FB * FB; q += 256) {
+        const int j = q / FB, i = q - j * FB;
+        if (i < nb && j <= i) Fv.panel[(int64_t)(kb + j) * Fv.nf + kb + i] = a[i][j];
+        x[i][j] = i == j ? mk<double>(1.0, 0.0) : zero<double>();
+    }
+    __syncthreads();
+    for (int i = 1; i < nb; ++i) {                        // X(i,c) = -sum_{c<=m<i} L(i,m) X(m,c)
+        const int nseg = min(256 / i, max(1, i / 4)), seg = tid / i, c = tid - seg * i;
+        c64 acc = zero<double>();
+        if (seg < nseg)
+            for (int m = c + seg; m < i; m += nseg) cfma(acc, a[i][m], x[m][c]);
+        red[tid] = acc;
+        __syncthreads();
+        if (tid < i) {
+            for (int q = 1; q < nseg; ++q) acc += red[q * i + tid];
+            x[i][c] = mk<double>(-acc.re, -acc.im);
+        }
+        __syncthreads();
+    }
+    c64* out = X.of(f, op, kb);
+    for (int q = tid; q < FB * FB; q += 256) out[q] = x[q / FB][q % FB];
+}
+
+// rows of the front below the block: 32 per CTA
+__global__ void __launch_bounds__(256) tiled_rows_kernel(Fronts F, const int64_t* __restrict__ front_list, int kb,
+                                                         c64* __restrict__ panel, c64* __restrict__ upd, DiagInv X) {
+    __shared__ c64 x[FB][FB];
+    __shared__ c64 ar[FB][FB + 1];                        // [row][column]
+    __shared__ c64 dv[FB];
+    const int f = (int)front_list[blockIdx.y], op = blockIdx.z;
+    const FrontView Fv = front_view(F, f, op, panel, upd);
+    const int nb = min(FB, Fv.nown - kb);
+    if (nb <= 0) return;
+    const int i0 = kb + nb + blockIdx.x * 32, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (i0 >= Fv.nf) return;
+    const c64* xi = X.of(f, op, kb);
+    for (int q = tid; q < FB * FB; q += 256) {
+        x[q / FB][q % FB] = xi[q];
+        const int m = q / FB, r = q - m * FB;
+        ar[r][m] = m < nb && i0 + r < Fv.nf ? Fv.panel[(int64_t)(kb + m) * Fv.nf + i0 + r] : zero<double>();
+    }
+    if (tid < FB) {
+        const c64 d = tid < nb ? Fv.panel[(int64_t)(kb + tid) * Fv.nf + kb + tid] : mk<double>(1.0, 0.0);
+        dv[tid] = cdiv(mk<double>(1.0, 0.0), d);
+    }
+    __syncthreads();
+    if (i0 + lane >= Fv.nf) return;
 #pragma unroll
-    for (int k = 0; k < FB; ++k)
-        if (k < nb) Fv.panel[(int64_t)(kb + k) * Fv.nf + i] = cdiv(w[k], dv[k]);
+    for (int e = 0; e < FB / 8; ++e) {
+        // columns e, 15 - e ... of the warp: the short and the long sums mixed
+        const int k = (e & 1) ? FB - 1 - warp - 8 * (e >> 1) : warp + 8 * (e >> 1);
+        if (k >= nb) continue;
+        c64 w = ar[lane][k];
+        for (int m = 0; m < k; ++m) cfma(w, ar[lane][m], x[k][m]);
+        Fv.panel[(int64_t)(kb + k) * Fv.nf + i0 + lane] = w * dv[k];
+    }
 }
 
-// tile t of the lower triangle of a T x T tile grid: (bi, bj), bj <= bi
-__device__ __forceinline__ void lower_tile(int t, int& bi, int& bj) {
-    int b = (int)((sqrt(8.0 * t + 1.0) - 1.0) * 0.5);
-    while ((int64_t)b * (b + 1) / 2 > t) --b;
-    while ((int64_t)(b + 1) * (b + 2) / 2 <= t) ++b;
-    bi = b;
-    bj = t - b * (b + 1) / 2;
+// 2 x 2 outputs per thread of a 32 x 32 tile: acc += A(m, 2 tx ..) B(m, 2 ty ..) over m < nb
+__device__ __forceinline__ void tile_mac(const c64* As, const c64* Bs, int nb, int tx, int ty, c64 (&acc)[2][2]) {
+    for (int m = 0; m < nb; ++m) {
+        const c64 a0 = As[m * FT + tx], a1 = As[m * FT + tx + 16], b0 = Bs[m * FT + ty], b1 = Bs[m * FT + ty + 16];
+        cfma(acc[0][0], a0, b0);
+        cfma(acc[0][1], a0, b1);
+        cfma(acc[1][0], a1, b0);
+        cfma(acc[1][1], a1, b1);
+    }
 }
-
-constexpr size_t TRAIL_SMEM = 2 * (size_t)FB * FT * sizeof(c64);
 
 __global__ void __launch_bounds__(256) tiled_trail_kernel(Fronts F, const int64_t* __restrict__ front_list, int kb,
                                                           c64* __restrict__ panel, c64* __restrict__ upd) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    c64* As = reinterpret_cast<c64*>(smem_raw);          // [m][FT]: L(i0 + r, kb + m)
-    c64* Bs = As + FB * FT;                              // [m][FT]: L(j0 + c, kb + m) d_m
+    __shared__ c64 As[FB * FT], Bs[FB * FT];             // [m][r]: L(i0 + r, kb + m); [m][c]: L(j0 + c, kb + m) d_m
     const int f = (int)front_list[blockIdx.y];
     const FrontView Fv = front_view(F, f, blockIdx.z, panel, upd);
     const int nb = min(FB, Fv.nown - kb);
@@ -256,195 +472,84 @@ __global__ void __launch_bounds__(256) tiled_trail_kernel(Fronts F, const int64_
     }
     __syncthreads();
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    c64 acc[4][4];
+    c64 acc[2][2] = {{zero<double>(), zero<double>()}, {zero<double>(), zero<double>()}};
+    tile_mac(As, Bs, nb, tx, ty, acc);
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
+    for (int c = 0; c < 2; ++c)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) acc[r][c] = zero<double>();
-    for (int m = 0; m < nb; ++m) {
-        c64 a[4], b[4];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) a[r] = As[m * FT + tx + 16 * r];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) b[c] = Bs[m * FT + ty + 16 * c];
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) cfma(acc[r][c], a[r], b[c]);
-    }
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        const int j = j0 + ty + 16 * c;
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const int i = i0 + tx + 16 * r;
+        for (int r = 0; r < 2; ++r) {
+            const int i = i0 + tx + 16 * r, j = j0 + ty + 16 * c;
             if (i < Fv.nf && j <= i) Fv.at(i, j) -= acc[r][c];
         }
-    }
 }
 
 void launch_factor_tiled(const Fronts& F, const int64_t* front_list, int nf_level, int max_nf, int max_nown,
-                         const c64* svals, c64* panel, c64* upd, int nops, int* status, cudaStream_t st) {
+                         const c64* svals, c64* panel, c64* upd, c64* xinv, const int* xfirst, int64_t xtotal, int nops,
+                         int* status, cudaStream_t st) {
+    const DiagInv X{xinv, xfirst, xtotal};
     assemble_fronts_kernel<<<dim3(nf_level, nops), 512, 0, st>>>(F, front_list, svals, panel, upd);
     GT_LAUNCH_CHECK();
-    raise_smem((const void*)tiled_trail_kernel, TRAIL_SMEM);
     for (int kb = 0; kb < max_nown; kb += FB) {
-        tiled_diag_kernel<<<dim3(nf_level, nops), 32, 0, st>>>(F, front_list, kb, panel, upd, status);
+        tiled_diag_kernel<<<dim3(nf_level, nops), 256, 0, st>>>(F, front_list, kb, panel, upd, X, status);
         GT_LAUNCH_CHECK();
         const int below = max_nf - kb - 1;              // rows below the block (at least this front's nb of them)
         if (below <= 0) continue;
-        tiled_rows_kernel<<<dim3(ceil_div(below, ROWS_CTA), nf_level, nops), ROWS_CTA, 0, st>>>(F, front_list, kb, panel,
-                                                                                                 upd);
+        tiled_rows_kernel<<<dim3(ceil_div(below, 32), nf_level, nops), 256, 0, st>>>(F, front_list, kb, panel, upd, X);
         GT_LAUNCH_CHECK();
         const int T = ceil_div(below, FT);
-        tiled_trail_kernel<<<dim3((unsigned)((int64_t)T * (T + 1) / 2), nf_level, nops), 256, TRAIL_SMEM, st>>>(
-            F, front_list, kb, panel, upd);
+        tiled_trail_kernel<<<dim3((unsigned)((int64_t)T * (T + 1) / 2), nf_level, nops), 256, 0, st>>>(F, front_list, kb, panel,
+                                                                                                     upd);
         GT_LAUNCH_CHECK();
     }
-}
-
-// Selective inversion: the inverse X of each front's own block (unit lower triangular; D on the diagonal
-// kept as is), FP64.  Rows are independent: X[i, k] = -(L[i, k] + sum_{k < m < i} X[i, m] L[m, k]) for k
-// descending.  X[i, k] is written to the unused upper triangle, transposed (position (k, i)), so the factor's
-// lower triangle stays intact while other rows read it; panel_convert moves X into place.  One thread per
-// row, rows of large fronts over several blocks, no barriers.
-constexpr int INV_ROWS = 128;
-__global__ void __launch_bounds__(INV_ROWS) invert_own_kernel(Fronts F, c64* __restrict__ panel, int nchunk, int tiled_nf) {
-    const int f = blockIdx.x / nchunk, chunk = blockIdx.x - f * nchunk, op = blockIdx.y;
-    const int nown = (int)F.nown[f], nf = nown + (int)F.nbnd[f];
-    if (chunk * INV_ROWS >= nown || nf >= tiled_nf) return;      // large fronts: the blocked inversion
-    const int i = chunk * INV_ROWS + threadIdx.x;
-    c64* L = panel + (int64_t)op * F.panel_total + F.panel_off[f];
-    const int kmax = min(nown, chunk * INV_ROWS + INV_ROWS) - 2;   // the block's largest row - 1
-    c64* Xi = L + (int64_t)min(i, nown - 1) * nf;                   // X[i, m] at Xi[m], m < i
-    for (int k = kmax; k >= 0; --k) {
-        if (k >= i || i >= nown) continue;
-        c64 acc = L[(int64_t)k * nf + i];
-        const c64* Lk = L + (int64_t)k * nf;
-        for (int m = k + 1; m < i; ++m) cfma(acc, Xi[m], Lk[m]);
-        Xi[k] = mk<double>(-acc.re, -acc.im);
-    }
-}
-
-void launch_invert_own(const Fronts& F, c64* panel, int max_nown, int nops, int tiled_nf, cudaStream_t st) {
-    const int nchunk = std::max(1, ceil_div(max_nown, INV_ROWS));
-    invert_own_kernel<<<dim3(F.nfront * nchunk, nops), INV_ROWS, 0, st>>>(F, panel, nchunk, tiled_nf);
-    GT_LAUNCH_CHECK();
-}
-
-// Boundary rows of each front replaced by M = -L_bnd Linv_own (in place, FP64; after invert_own_kernel,
-// Linv read from the upper triangle).  Every boundary row is independent: M[j, k] = -(L[j, k] + sum_{m > k} L[j, m] Linv[m, k]) for k ascending reads only entries
-// m > k of its own row, which are still the factor's.  One thread per row (rows of a warp consecutive, so
-// the row loads coalesce and the Linv loads broadcast); the rows of large fronts spread over many blocks.
-constexpr int BND_ROWS = 128;
-__global__ void __launch_bounds__(BND_ROWS) bnd_inv_kernel(Fronts F, c64* __restrict__ panel, int nchunk, int tiled_nf) {
-    const int f = blockIdx.x / nchunk, chunk = blockIdx.x - f * nchunk, op = blockIdx.y;
-    const int nown = (int)F.nown[f], nbnd = (int)F.nbnd[f], nf = nown + nbnd;
-    const int j = nown + chunk * BND_ROWS + threadIdx.x;
-    if (chunk * BND_ROWS >= nbnd || nf >= tiled_nf) return;
-    c64* L = panel + (int64_t)op * F.panel_total + F.panel_off[f];
-    const bool act = j < nf;
-    const int jr = act ? j : nf - 1;
-    for (int k = 0; k < nown; ++k) {
-        c64 acc = L[(int64_t)k * nf + jr];
-        // Linv[m, k] (m > k) is held transposed at position (k, m): L[m * nf + k]
-        int m = k + 1;
-        for (; m + 4 <= nown; m += 4) {
-            const c64 a0 = L[(int64_t)m * nf + jr], a1 = L[(int64_t)(m + 1) * nf + jr];
-            const c64 a2 = L[(int64_t)(m + 2) * nf + jr], a3 = L[(int64_t)(m + 3) * nf + jr];
-            cfma(acc, a0, L[(int64_t)m * nf + k]);
-            cfma(acc, a1, L[(int64_t)(m + 1) * nf + k]);
-            cfma(acc, a2, L[(int64_t)(m + 2) * nf + k]);
-            cfma(acc, a3, L[(int64_t)(m + 3) * nf + k]);
-        }
-        for (; m < nown; ++m) cfma(acc, L[(int64_t)m * nf + jr], L[(int64_t)m * nf + k]);
-        if (act) L[(int64_t)k * nf + j] = mk<double>(-acc.re, -acc.im);
-    }
-}
-
-void launch_bnd_inv(const Fronts& F, c64* panel, int max_nbnd, int nops, int tiled_nf, cudaStream_t st) {
-    const int nchunk = std::max(1, ceil_div(max_nbnd, BND_ROWS));
-    bnd_inv_kernel<<<dim3(F.nfront * nchunk, nops), BND_ROWS, 0, st>>>(F, panel, nchunk, tiled_nf);
-    GT_LAUNCH_CHECK();
 }
 
 // Selective inversion of large fronts, blocked.  The inverted panel [Linv_own; -L_bnd Linv_own] is the first
 // nown columns of the inverse of the unit lower triangular T = [L_own 0; L_bnd I], so it is computed in place
 // as the forward substitution T Y = [I; 0], FB rows of T per step (kb = FB k, nb = the step's rows):
-//   inv_rows   Y[kb.., c] = L_kk^-1 Y[kb.., c] for columns c < kb (their right-hand sides accumulated so far)
-//   inv_diag   L_kk -> its inverse, in place, by one warp (a lane per row; D stays on the diagonal)
+//   inv_rows   Y[kb.., c] = L_kk^-1 Y[kb.., c] for columns c < kb (their right-hand sides accumulated so far), with
+//              the inverses the elimination left; the block's own entries become that inverse (D stays on the diagonal)
 //   inv_trail  Y[i, c] -= L[i, kb..] Y[kb.., c] for the rows i below the block: first the columns c < kb,
 //              then the block's own columns, whose Y takes the place of the L it is made from (each tile
 //              reads its rows of L before it writes; the c < kb pass has read them all by then).
 // The panel's upper triangle stays zero; the diagonal keeps D for panel_convert.
-__global__ void __launch_bounds__(ROWS_CTA) inv_rows_kernel(Fronts F, const int64_t* __restrict__ front_list, int kb,
-                                                            c64* __restrict__ panel) {
-    __shared__ c64 l11[FB][FB];
-    const int f = (int)front_list[blockIdx.y];
-    const int op = blockIdx.z;
+__global__ void __launch_bounds__(256) inv_rows_kernel(Fronts F, const int64_t* __restrict__ front_list, int kb,
+                                                       c64* __restrict__ panel, DiagInv X) {
+    __shared__ c64 x[FB][FB];
+    __shared__ c64 y[FB][FB + 1];                         // [column][row]
+    const int f = (int)front_list[blockIdx.y], op = blockIdx.z;
     const int nown = (int)F.nown[f], nf = nown + (int)F.nbnd[f];
     const int nb = min(FB, nown - kb);
-    if (nb <= 0 || blockIdx.x * ROWS_CTA >= kb) return;
+    const int c0 = blockIdx.x * 32, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (nb <= 0 || c0 > kb) return;
     c64* P = panel + (int64_t)op * F.panel_total + F.panel_off[f];
-    for (int q = threadIdx.x; q < FB * FB; q += ROWS_CTA) {
-        const int r = q / FB, c = q - r * FB;
-        l11[r][c] = (r < nb && c < r) ? P[(int64_t)(kb + c) * nf + kb + r] : zero<double>();
+    const c64* xi = X.of(f, op, kb);
+    if (c0 == kb) {                                       // the block's own columns
+        for (int q = tid; q < FB * FB; q += 256) {
+            const int k = q / FB, i = q - k * FB;
+            if (i < nb && k < i) P[(int64_t)(kb + k) * nf + kb + i] = xi[i * FB + k];
+        }
+        return;
+    }
+    for (int q = tid; q < FB * FB; q += 256) {
+        x[q / FB][q % FB] = xi[q];
+        const int c = q / FB, r = q - c * FB;
+        y[c][r] = r < nb ? P[(int64_t)(c0 + c) * nf + kb + r] : zero<double>();
     }
     __syncthreads();
-    const int c = blockIdx.x * ROWS_CTA + threadIdx.x;
-    if (c >= kb) return;
-    c64* col = P + (int64_t)c * nf + kb;
-    c64 y[FB];
 #pragma unroll
-    for (int r = 0; r < FB; ++r) {
-        if (r < nb) {
-            c64 t = col[r];
-#pragma unroll
-            for (int m = 0; m < r; ++m) cfms(t, l11[r][m], y[m]);
-            y[r] = t;
-        }
+    for (int e = 0; e < FB / 8; ++e) {
+        const int r = (e & 1) ? FB - 1 - warp - 8 * (e >> 1) : warp + 8 * (e >> 1);
+        if (r >= nb) continue;
+        c64 t = y[lane][r];
+        for (int m = 0; m < r; ++m) cfma(t, x[r][m], y[lane][m]);
+        P[(int64_t)(c0 + lane) * nf + kb + r] = t;
     }
-#pragma unroll
-    for (int r = 0; r < FB; ++r)
-        if (r < nb) col[r] = y[r];
-}
-
-__global__ void __launch_bounds__(32) inv_diag_kernel(Fronts F, const int64_t* __restrict__ front_list, int kb,
-                                                      c64* __restrict__ panel) {
-    __shared__ c64 a[FB][FB + 1];
-    const int f = (int)front_list[blockIdx.x];
-    const int op = blockIdx.y;
-    const int nown = (int)F.nown[f], nf = nown + (int)F.nbnd[f];
-    const int nb = min(FB, nown - kb);
-    if (nb <= 0) return;
-    c64* P = panel + (int64_t)op * F.panel_total + F.panel_off[f];
-    const int i = threadIdx.x;
-    for (int j = 0; j < FB; ++j) a[i][j] = (i < nb && j < i) ? P[(int64_t)(kb + j) * nf + kb + i] : zero<double>();
-    __syncwarp();
-    if (i >= nb) return;
-    // X[i, k] = -(L[i, k] + sum_{k < m < i} X[i, m] L[m, k]), k descending: lane i needs only its own row of X
-    c64 x[FB];
-#pragma unroll
-    for (int k = FB - 1; k >= 0; --k) {
-        if (k < i) {
-            c64 acc = a[i][k];
-#pragma unroll
-            for (int m = k + 1; m < FB; ++m)
-                if (m < i) cfma(acc, x[m], a[m][k]);
-            x[k] = mk<double>(-acc.re, -acc.im);
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < FB; ++k)
-        if (k < i) P[(int64_t)(kb + k) * nf + kb + i] = x[k];
 }
 
 // rows i >= kb + nb of the front; mode 0: columns c < kb (tile grid rt x ct), mode 1: the block's columns
 __global__ void __launch_bounds__(256) inv_trail_kernel(Fronts F, const int64_t* __restrict__ front_list, int kb,
                                                         c64* __restrict__ panel, int mode) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    c64* As = reinterpret_cast<c64*>(smem_raw);          // [m][FT]: L(i0 + r, kb + m)
-    c64* Bs = As + FB * FT;                              // [m][FT]: Y(kb + m, c0 + c)
+    __shared__ c64 As[FB * FT], Bs[FB * FT];             // [m][r]: L(i0 + r, kb + m); [m][c]: Y(kb + m, c0 + c)
     const int f = (int)front_list[blockIdx.y];
     const int op = blockIdx.z;
     const int nown = (int)F.nown[f], nf = nown + (int)F.nbnd[f];
@@ -463,42 +568,24 @@ __global__ void __launch_bounds__(256) inv_trail_kernel(Fronts F, const int64_t*
     c64* P = panel + (int64_t)op * F.panel_total + F.panel_off[f];
     for (int q = threadIdx.x; q < FB * FT; q += 256) {
         const int m = q / FT, r = q - m * FT;
-        c64 a = zero<double>(), b = zero<double>();
-        if (m < nb) {
-            if (i0 + r < nf) a = P[(int64_t)(kb + m) * nf + i0 + r];
-            const int c = c0 + r;
-            // Y(kb + m, c): the block row's solved entries; in mode 1 the block's inverse, unit diagonal
-            if (c < c1) b = (mode == 1 && c - kb == m) ? mk<double>(1.0, 0.0)
-                                                       : (mode == 1 && c - kb > m) ? zero<double>()
-                                                                                   : P[(int64_t)c * nf + kb + m];
-        }
-        As[q] = a;
-        Bs[q] = b;
+        As[q] = m < nb && i0 + r < nf ? P[(int64_t)(kb + m) * nf + i0 + r] : zero<double>();
+        // Y(kb + m, c), read down the columns: the block row's solved entries; in mode 1 the block's inverse, unit diagonal
+        const int cl = q / FB, mm = q - cl * FB, c = c0 + cl;
+        c64 b = zero<double>();
+        if (mm < nb && c < c1) b = mode == 0 || c - kb < mm ? P[(int64_t)c * nf + kb + mm]
+                                   : c - kb == mm ? mk<double>(1.0, 0.0) : zero<double>();
+        Bs[mm * FT + cl] = b;
     }
     __syncthreads();
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    c64 acc[4][4];
+    c64 acc[2][2] = {{zero<double>(), zero<double>()}, {zero<double>(), zero<double>()}};
+    tile_mac(As, Bs, nb, tx, ty, acc);
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) acc[r][c] = zero<double>();
-    for (int m = 0; m < nb; ++m) {
-        c64 a[4], b[4];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) a[r] = As[m * FT + tx + 16 * r];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) b[c] = Bs[m * FT + ty + 16 * c];
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) cfma(acc[r][c], a[r], b[c]);
-    }
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
+    for (int c = 0; c < 2; ++c) {
         const int j = c0 + ty + 16 * c;
         if (j >= c1) continue;
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
+        for (int r = 0; r < 2; ++r) {
             const int i = i0 + tx + 16 * r;
             if (i >= nf) continue;
             c64& y = P[(int64_t)j * nf + i];
@@ -508,91 +595,56 @@ __global__ void __launch_bounds__(256) inv_trail_kernel(Fronts F, const int64_t*
 }
 
 void launch_invert_tiled(const Fronts& F, const int64_t* front_list, int nfront, int max_nf, int max_nown, c64* panel,
-                         int nops, cudaStream_t st) {
+                         const c64* xinv, const int* xfirst, int64_t xtotal, int nops, cudaStream_t st) {
     if (nfront <= 0) return;
-    raise_smem((const void*)inv_trail_kernel, TRAIL_SMEM);
+    const DiagInv X{const_cast<c64*>(xinv), xfirst, xtotal};
     for (int kb = 0; kb < max_nown; kb += FB) {
-        if (kb > 0) {
-            inv_rows_kernel<<<dim3(ceil_div(kb, ROWS_CTA), nfront, nops), ROWS_CTA, 0, st>>>(F, front_list, kb, panel);
-            GT_LAUNCH_CHECK();
-        }
-        inv_diag_kernel<<<dim3(nfront, nops), 32, 0, st>>>(F, front_list, kb, panel);
+        inv_rows_kernel<<<dim3(kb / 32 + 1, nfront, nops), 256, 0, st>>>(F, front_list, kb, panel, X);
         GT_LAUNCH_CHECK();
         const int below = max_nf - kb - 1;
         if (below <= 0) continue;
         const int rt = ceil_div(below, FT);
         if (kb > 0) {
-            inv_trail_kernel<<<dim3(rt * ceil_div(kb, FT), nfront, nops), 256, TRAIL_SMEM, st>>>(F, front_list, kb, panel, 0);
+            inv_trail_kernel<<<dim3(rt * ceil_div(kb, FT), nfront, nops), 256, 0, st>>>(F, front_list, kb, panel, 0);
             GT_LAUNCH_CHECK();
         }
-        inv_trail_kernel<<<dim3(rt, nfront, nops), 256, TRAIL_SMEM, st>>>(F, front_list, kb, panel, 1);
+        inv_trail_kernel<<<dim3(rt, nfront, nops), 256, 0, st>>>(F, front_list, kb, panel, 1);
         GT_LAUNCH_CHECK();
     }
 }
 
-// Finish the solve panels: the own block gets its inverse below an explicit unit diagonal (moved from the
-// upper triangle, which becomes zero; the pivots go to dinv as 1/D), and the copies the sweeps read are written: the
-// FP32 forward and backward tiles (sweep.cu) and the FP64 row-major panel.
+// Finish the large fronts' solve panels: an explicit unit diagonal (the pivots go to dinv as 1/D) and the copies the sweeps
+// read: the FP32 forward and backward tiles and the FP64 row-major panel.
 // r64 (the FP64 row-major copy) may be null: operators that keep their FP32 panels only
-__global__ void panel_convert_kernel(Fronts F, SweepPlan S, c64* __restrict__ p64, c32* __restrict__ pf, c32* __restrict__ pb,
-                                     c64* __restrict__ r64, c64* __restrict__ d64, c32* __restrict__ d32, int tiled_nf) {
-    const int f = blockIdx.x;
-    const int op = blockIdx.y;
+__global__ void panel_convert_kernel(Fronts F, SweepPlan S, const int64_t* __restrict__ front_list, c64* __restrict__ p64,
+                                     c32* __restrict__ pf, c32* __restrict__ pb, c64* __restrict__ r64, c64* __restrict__ d64,
+                                     c32* __restrict__ d32) {
+    const int f = (int)front_list[blockIdx.y];
+    const int op = blockIdx.z;
     const int nown = (int)F.nown[f], nf = nown + (int)F.nbnd[f];
-    const bool in_place = nf >= tiled_nf;                       // the blocked inversion: X below the diagonal
     const int64_t base = (int64_t)op * F.panel_total + F.panel_off[f];
     const int64_t dbase = (int64_t)op * F.nfac + F.own_start[f];
-    const int H = S.hf[f], C = S.hb[f];
-    c32* tf = pf + (int64_t)op * S.ptotal + S.offf[f];
-    c32* tb = pb + (int64_t)op * S.ptotal + S.offb[f];
-    // element (i, k) into its forward tile (rows gH .., inner k < min(nown, (g + 1) H)) and its backward one (columns
-    // tC .., inner i >= tC)
-    auto put = [&](int i, int k, c32 v) {
-        const int g = i / H;
-        if (k < min(nown, (g + 1) * H)) {
-            const int m = min(g, nown / H), h = min(H, nf - g * H);
-            tf[(int64_t)H * H * m * (m + 1) / 2 + (int64_t)H * nown * (g - m) + (int64_t)k * ((h + 1) & ~1) + (i - g * H)] = v;
-        }
-        const int t = k / C;
-        if (i >= t * C) {
-            const int h = min(C, nown - t * C);
-            tb[(int64_t)C * ((int64_t)t * nf - (int64_t)C * t * (t - 1) / 2) + (int64_t)(i - t * C) * ((h + 1) & ~1) +
-               (k - t * C)] = v;
-        }
-    };
-    for (int64_t q = threadIdx.x; q < (int64_t)nf * nown; q += blockDim.x) {
-        int k = int(q / nf), i = int(q - (int64_t)k * nf);      // column-major element (i, k)
-        if (i < k) {                                             // the upper triangle: zero
-            if (in_place) {
-                put(i, k, zero<float>());
-                if (r64) r64[base + (int64_t)i * nown + k] = zero<double>();
-            }
-            continue;                                            // (else with its partner below)
-        }
-        c64 v = p64[base + q];
+    const SweepTiles T(S, f, op, nf, nown, pf, pb);
+    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < (int64_t)nf * nown; q += (int64_t)gridDim.x * blockDim.x) {
+        const int k = int(q / nf), i = int(q - (int64_t)k * nf);      // column-major element (i, k)
+        c64 v = i < k ? zero<double>() : p64[base + q];
         if (i == k) {
             const c64 dv = cdiv(mk<double>(1.0, 0.0), v);
             d64[dbase + i] = dv;
             d32[dbase + i] = cvt<float>(dv);
             v = mk<double>(1.0, 0.0);
             p64[base + q] = v;
-        } else if (i < nown && !in_place) {
-            // X[i, k] from its transposed position (k, i), which becomes zero
-            const int64_t qt = (int64_t)i * nf + k;
-            v = p64[base + qt];
-            p64[base + q] = v;
-            p64[base + qt] = zero<double>();
-            put(k, i, zero<float>());
-            if (r64) r64[base + (int64_t)k * nown + i] = zero<double>();
         }
-        put(i, k, cvt<float>(v));
+        T.fwd(i, k, cvt<float>(v));
+        T.bwd(i, k, cvt<float>(v));
         if (r64) r64[base + (int64_t)i * nown + k] = v;
     }
 }
 
-void launch_panel_convert(const Fronts& F, const SweepPlan& S, c64* p64, c32* pf, c32* pb, c64* r64, c64* d64, c32* d32, int nops,
-                          int tiled_nf, cudaStream_t st) {
-    panel_convert_kernel<<<dim3(F.nfront, nops), 256, 0, st>>>(F, S, p64, pf, pb, r64, d64, d32, tiled_nf);
+void launch_panel_convert(const Fronts& F, const SweepPlan& S, const int64_t* front_list, int nfront, c64* p64, c32* pf, c32* pb,
+                          c64* r64, c64* d64, c32* d32, int nops, cudaStream_t st) {
+    if (nfront <= 0) return;
+    panel_convert_kernel<<<dim3(16, nfront, nops), 256, 0, st>>>(F, S, front_list, p64, pf, pb, r64, d64, d32);
     GT_LAUNCH_CHECK();
 }
 

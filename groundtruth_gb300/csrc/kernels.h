@@ -154,20 +154,6 @@ struct Fronts {
 
 void launch_assemble_s(const int64_t* ptr, const int* tab_idx, const double* coef, int64_t nsv, const c64* table,
                        int ntab, c64* svals, int nops, cudaStream_t st);
-// one elimination level: fronts front_list[0..nf) for each operator
-void launch_factor_level(const Fronts& F, const int64_t* front_list, int nf_level, int max_nf, const c64* svals,
-                         c64* panel, c64* upd, int nops, int* status, cudaStream_t st);
-// one level's large fronts (blocked elimination over many CTAs); the fronts start zeroed
-void launch_factor_tiled(const Fronts& F, const int64_t* front_list, int nf_level, int max_nf, int max_nown,
-                         const c64* svals, c64* panel, c64* upd, int nops, int* status, cudaStream_t st);
-// each front's own block replaced by its inverse (in place, FP64; the unit diagonal and the pivots untouched)
-void launch_invert_own(const Fronts& F, c64* panel, int max_nown, int nops, int tiled_nf, cudaStream_t st);
-// each front's boundary rows replaced by -L_bnd Linv_own (in place, FP64; after launch_invert_own)
-void launch_bnd_inv(const Fronts& F, c64* panel, int max_nbnd, int nops, int tiled_nf, cudaStream_t st);
-// both at once for the listed (large) fronts, blocked over many CTAs; the two above skip fronts of tiled_nf rows
-// or more, and panel_convert takes their inverse in place
-void launch_invert_tiled(const Fronts& F, const int64_t* front_list, int nfront, int max_nf, int max_nown, c64* panel,
-                         int nops, cudaStream_t st);
 // triangular solves; groups of columns sharing an operator
 struct Groups {
     int ngroup;
@@ -219,8 +205,27 @@ void launch_sweep(const SweepPlan& S, const Fronts& F, const c32* pf, const c32*
 unsigned int sweep_take_wait_timeouts();
 // the solve panels: own blocks get a unit diagonal and zeros above it (pivot reciprocals to d64 / d32,
 // [op][nfac]); the FP32 sweeps' forward and backward tiles (pf, pb) and the FP64 row-major copy
-void launch_panel_convert(const Fronts& F, const SweepPlan& S, c64* p64, c32* pf, c32* pb, c64* r64, c64* d64, c32* d32, int nops,
-                          int tiled_nf, cudaStream_t st);
+// the small fronts of a level: from assembly to the finished solve panels (small_front_smem bytes for the largest; r64 null:
+// FP32 copies only)
+size_t small_front_smem(int nown, int nbnd);
+bool small_front_fits(int nown, int nbnd);
+void launch_small_fronts(const Fronts& F, const SweepPlan& S, const int64_t* front_list, int nfront, size_t smem,
+                         const c64* svals, c64* panel, c64* upd, c64* r64, c64* d64, c32* d32, c32* pf, c32* pb, int nops,
+                         int* status, cudaStream_t st);
+// one level's large fronts (blocked elimination over many CTAs); the fronts start zeroed.  xinv: the inverses of their
+// diagonal blocks, xtotal blocks of FACTOR_BLOCK^2 per operator, a front's from block xfirst[front] on
+constexpr int FACTOR_BLOCK = 32;
+void launch_factor_tiled(const Fronts& F, const int64_t* front_list, int nf_level, int max_nf, int max_nown,
+                         const c64* svals, c64* panel, c64* upd, c64* xinv, const int* xfirst, int64_t xtotal, int nops,
+                         int* status, cudaStream_t st);
+// the listed (large) fronts' own blocks replaced by their inverses and the boundary rows by -L_bnd Linv_own, in place
+void launch_invert_tiled(const Fronts& F, const int64_t* front_list, int nfront, int max_nf, int max_nown, c64* panel,
+                         const c64* xinv, const int* xfirst, int64_t xtotal, int nops, cudaStream_t st);
+// their solve panels: unit diagonal (pivot reciprocals to d64 / d32, [op][nfac]), the FP32 sweeps' forward and backward
+// tiles (pf, pb) and the FP64 row-major copy
+void launch_panel_convert(const Fronts& F, const SweepPlan& S, const int64_t* front_list, int nfront, c64* p64, c32* pf, c32* pb,
+                          c64* r64, c64* d64, c32* d32, int nops, cudaStream_t st);
+
 
 // forward: own rows from s in factor order (sf), results to z (factor order) and the update vectors (wasm:
 // factor-ordered scratch for fronts assembled ahead of a split product, may be sf itself);
