@@ -357,6 +357,17 @@ __global__ void __launch_bounds__(256, 2) lp_pass_bg(int S, int n0, int P1, int 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int c = blockIdx.x, b0 = blockIdx.y * bt, nb = min(bt, ncol - b0), nrow = nb * S;
     c32* sx = Z + warp * RR * RS;
+    // the spectrum's column, [Q0][S S] padded to an odd stride: read from global memory by the pixels' threads, each S x S
+    // block a strided run, it took 77 us of the same six columns, 43 so
+    const int SS = S * S, KS = SS | 1;
+    float* Ks = reinterpret_cast<float*>(Z + (blockDim.x >> 5) * RR * RS);
+    {
+        const float* Kc = spec + (int64_t)min(c, P1 - c) * Q0 * SS;
+        for (int q = threadIdx.x; q < Q0 * SS; q += blockDim.x) {
+            const int p = q / SS;
+            Ks[p * KS + q - p * SS] = __ldg(Kc + q);
+        }
+    }
     const c32* src[RR];
     bool ok[RR];
 #pragma unroll
@@ -381,10 +392,9 @@ __global__ void __launch_bounds__(256, 2) lp_pass_bg(int S, int n0, int P1, int 
 #pragma unroll
         for (int k2 = 0; k2 < 32; ++k2) sx[lane * 33 + k2] = u[k2];
     __syncthreads();
-    const float* Kc = spec + (int64_t)min(c, P1 - c) * Q0 * S * S;
     for (int idx = threadIdx.x; idx < nb * N; idx += blockDim.x) {
-        const int b = idx / N, e = idx - b * N, k1 = e >> 5, k2 = e & 31, p = k1 + A * k2;
-        const float* K = Kc + (int64_t)min(p, N - p) * S * S;
+        const int b = idx / N, p = idx - b * N, k2 = p / A, k1 = p - k2 * A;
+        const float* K = Ks + min(p, N - p) * KS;
         c32* z = Z + b * S * RS + k1 * 33 + k2;
         c32 w[MAXS];
 #pragma unroll
@@ -397,7 +407,7 @@ __global__ void __launch_bounds__(256, 2) lp_pass_bg(int S, int n0, int P1, int 
 #pragma unroll
             for (int s = 0; s < MAXS; ++s)
                 if (s < S) {
-                    const float k = __ldg(K + t * S + s);
+                    const float k = K[t * S + s];
                     acc.re += k * w[s].re;
                     acc.im += k * w[s].im;
                 }
@@ -990,7 +1000,7 @@ static void launch_bg(const LpArgs<float>& a, cudaStream_t st) {
     constexpr int RR = WarpFft<A>::RR;
     const int bt = std::max(1, std::min(a.ncol, (4 * RR + a.S - 1) / a.S));
     const int warps = ceil_div(bt * a.S, RR);
-    const size_t sm = (size_t)warps * WarpFft<A>::SLOTS * sizeof(c32);
+    const size_t sm = (size_t)warps * WarpFft<A>::SLOTS * sizeof(c32) + (size_t)(16 * A + 1) * ((a.S * a.S) | 1) * sizeof(float);
     set_smem<float>((const void*)lp_pass_bg<A>, sm);
     lp_pass_bg<A><<<dim3(a.P1, ceil_div(a.ncol, bt)), warps * 32, sm, st>>>(a.S, a.n0, a.P1, a.ncol, bt, a.spec, a.tw0, a.T,
                                                                           ldt_of(a));
