@@ -226,7 +226,9 @@ struct Workspace {
     int *slot_col = nullptr, *slot_op = nullptr, *g_ptr = nullptr, *g_slot = nullptr, *g_op = nullptr, *g_pair = nullptr, *col_op = nullptr;
     int* slot_pc = nullptr;      // each slot's factorisation (the preconditioner's tables, panels and pivots)
     int* act = nullptr;
-    int* act_host = nullptr;
+    double* togo_host = nullptr; // [2][ncol]: GmresState::to_go after the last two steps
+    cudaEvent_t togo_ev[2] = {}; // their copies' arrival
+    int* done = nullptr;         // per slot, for the reductions' last blocks
     // outer GCR: directions P (corrections) and Q = K P, per column, k-major; step sizes; active columns
     int kmax = 0;
     c64 *gP = nullptr, *gQ = nullptr, *gbeta = nullptr, *galpha = nullptr, *gnu2 = nullptr;
@@ -236,7 +238,9 @@ struct Workspace {
     int* its_col = nullptr;
     ~Workspace() {
         if (flag_host) cudaFreeHost(flag_host);
-        if (act_host) cudaFreeHost(act_host);
+        if (togo_host) cudaFreeHost(togo_host);
+        for (cudaEvent_t e : togo_ev)
+            if (e) cudaEventDestroy(e);
     }
 };
 
@@ -833,7 +837,7 @@ static void fill_ws(Workspace& W, gt_geometry* G, int ncol, int m, int prec, int
     s.reorth = p.alloc<int>(ncol);
     s.eta = p.alloc<double>(ncol);
     s.inv_hn = p.alloc<double>(ncol);
-    s.resid_est = p.alloc<double>(ncol);
+    s.to_go = p.alloc<double>(ncol);
     W.slot_col = p.alloc<int>(ncol);
     W.slot_op = p.alloc<int>(ncol);
     W.slot_pc = p.alloc<int>(ncol);
@@ -842,7 +846,12 @@ static void fill_ws(Workspace& W, gt_geometry* G, int ncol, int m, int prec, int
     W.g_op = p.alloc<int>(ncol);
     W.g_pair = p.alloc<int>(ncol + 1);
     W.act = p.alloc<int>(ncol);
-    if (!dry) GT_CUDA(cudaMallocHost(&W.act_host, ncol * sizeof(int)));
+    W.done = p.alloc<int>(ncol);
+    if (!dry) {
+        GT_CUDA(cudaMemsetAsync(W.done, 0, ncol * sizeof(int), st));
+        GT_CUDA(cudaMallocHost(&W.togo_host, 2 * ncol * sizeof(double)));
+        for (cudaEvent_t& e : W.togo_ev) GT_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    }
     W.gP = p.alloc<c64>((size_t)kmax * ncol * n);
     W.gQ = p.alloc<c64>((size_t)kmax * ncol * n);
     W.gbeta = p.alloc<c64>((size_t)ncol * (kmax + 1));
@@ -861,8 +870,7 @@ static void fill_ws(Workspace& W, gt_geometry* G, int ncol, int m, int prec, int
 static void norms64(gt_geometry* G, const c64* v, int64_t ld, int ncol, double* out, cudaStream_t st) {
     Workspace& W = *G->ws;
     const int nch = nchunks(G->geo.n);
-    launch_dots<double>(v, 0, ld, 0, v, ld, G->geo.n, ncol, nullptr, W.npart, nch, st);
-    launch_reduce(W.npart, nch, 0, ncol, nullptr, W.nred, 1, 0, st);
+    launch_dots<double>(v, 0, ld, 0, v, ld, G->geo.n, ncol, nullptr, W.npart, nch, W.nred, 1, W.done, st);
     launch_sqrt_norms(W.nred, 1, ncol, out, st);
 }
 
@@ -993,6 +1001,8 @@ static int solve_impl(gt_geometry* G, gt_operators* ops, int ncol, const int* h_
             launch_init_cycle<R, B>(ST, W.r64, n, W.slot_col, W.rho, n, st);
         }
         int jdone = 0;
+        constexpr double FAR = 8;
+        double togo = 2 * FAR;       // the slowest slot's, as last seen
         for (int j = 0; j < m; ++j) {
             // the products run on the slots still iterating in this cycle (W.act, grp)
             const int na = (int)act.size();
@@ -1013,35 +1023,44 @@ static int solve_impl(gt_geometry* G, gt_operators* ops, int ncol, const int* h_
             {
                 Scope sc(P, narrow ? "gs_dots_f32_b16" : sizeof(R) == 4 ? "gs_dots_f32" : "gs_dots_f64", st,
                          (double)ns * n * ((j + 1.0) * sizeof(B) + sizeof(cx<R>)));
-                launch_dots<R, B>(V, n, lds, j + 1, w, n, n, ns, S.active, W.partial, nch, st, vs);
-                launch_reduce(W.partial, nch, j + 1, ns, S.active, S.hvec, S.ldh, 0, st);
+                launch_dots<R, B>(V, n, lds, j + 1, w, n, n, ns, S.active, W.partial, nch, S.hvec, S.ldh, W.done, st, vs);
             }
             {
                 Scope sc(P, narrow ? "gs_update_f32_b16" : sizeof(R) == 4 ? "gs_update_f32" : "gs_update_f64", st,
                          (double)ns * n * ((j + 1.0) * sizeof(B) + 2.0 * sizeof(cx<R>)));
-                launch_update<R, B>(V, n, lds, j + 1, S.hvec, S.ldh, w, n, n, ns, S.active, W.partial, -1, st, vs);
-                launch_reduce(W.partial, nchu, 0, ns, S.active, S.hn2, 1, 0, st);
-                launch_dgks(S, j, st);
+                launch_gram_schmidt<R, B>(V, n, lds, 1, w, n, n, W.partial, W.done, S, j, st, vs);
             }
-            if (o.reorth > 0) {         // DGKS second pass (the slots launch_dgks flagged)
+            if (o.reorth > 0) {         // DGKS second pass (the slots the first one flagged)
                 Scope sc(P, "gs_reorth", st);
-                launch_dots<R, B>(V, n, lds, j + 1, w, n, n, ns, S.reorth, W.partial, nch, st, vs);
-                launch_reduce(W.partial, nch, j + 1, ns, S.reorth, S.h2vec, S.ldh, 0, st);
-                launch_update<R, B>(V, n, lds, j + 1, S.h2vec, S.ldh, w, n, n, ns, S.reorth, W.partial, -1, st, vs);
-                launch_reduce(W.partial, nchu, 0, ns, S.reorth, S.hn2b, 1, 0, st);
+                launch_dots<R, B>(V, n, lds, j + 1, w, n, n, ns, S.reorth, W.partial, nch, S.h2vec, S.ldh, W.done, st, vs);
+                launch_gram_schmidt<R, B>(V, n, lds, 2, w, n, n, W.partial, W.done, S, j, st, vs);
             }
-            {
+            if (j + 1 < m) {
                 Scope sc(P, "gmres_small", st);
-                launch_givens(S, j, st);
-                if (j + 1 < m) launch_scale<R, B>(ST, j, n, st);
+                launch_scale<R, B>(ST, j, n, st);
             }
-            GT_CUDA(cudaMemcpyAsync(W.act_host, S.active, ns * sizeof(int), cudaMemcpyDeviceToHost, st));
-            GT_CUDA(cudaStreamSynchronize(st));
+            GT_CUDA(cudaMemcpyAsync(W.togo_host + (j & 1) * W.ncol, S.to_go, ns * sizeof(double), cudaMemcpyDeviceToHost, st));
+            GT_CUDA(cudaEventRecord(W.togo_ev[j & 1], st));
             jdone = j + 1;
+            // which slots go on.  While the slowest is far from its target (a step gains a factor of two or so) this step's
+            // outcome is not waited for: the next one is launched behind it on the flags of the step before, a finished
+            // slot's products done once more for nothing and its state untouched (its flag holds the rest back), and the
+            // GPU never stands while the host looks.  Near the end each step is looked at before the next.
+            const int seen = togo > FAR ? j - 1 : j;
+            if (seen < 0) continue;
+            GT_CUDA(cudaEventSynchronize(W.togo_ev[seen & 1]));
+            const double* left = W.togo_host + (seen & 1) * W.ncol;
             std::vector<int> still;
+            togo = 0;
             for (int q : act)
-                if (W.act_host[q]) still.push_back(q);
-            if (still.empty()) break;
+                if (left[q] != 0) {
+                    still.push_back(q);
+                    togo = std::max(togo, left[q]);
+                }
+            if (still.empty()) {
+                jdone = seen + 1;
+                break;
+            }
             if (still.size() < act.size()) {
                 act.swap(still);
                 grp = upload_groups(act);
@@ -1055,7 +1074,7 @@ static int solve_impl(gt_geometry* G, gt_operators* ops, int ncol, const int* h_
         GT_CUDA(cudaMemsetAsync(w, 0, (size_t)ns * n * sizeof(cx<R>), st));
         {
             Scope sc(P, "combine", st, (double)ns * n * (jdone * sizeof(B) + 2.0 * sizeof(cx<R>)));
-            launch_update<R, B>(V, n, lds, jdone, S.y, S.ldh, w, n, n, ns, nullptr, nullptr, 1, st, vs);
+            launch_update<R, B>(V, n, lds, jdone, S.y, S.ldh, w, n, n, ns, nullptr, nullptr, nullptr, nullptr, 1, st, vs);
         }
         act.resize(ns);
         for (int q = 0; q < ns; ++q) act[q] = q;
@@ -1078,21 +1097,16 @@ static int solve_impl(gt_geometry* G, gt_operators* ops, int ncol, const int* h_
         {
             Scope sc(P, "gcr", st, 0.0);
             if (k > 0) {
-                launch_dots<double>(W.gQ, ldk, n, k, Qk, n, n, ncol, W.colact, W.npart_k, nch, st);
-                launch_reduce(W.npart_k, nch, k, ncol, W.colact, W.gbeta, K + 1, 0, st);
-                launch_update<double>(W.gQ, ldk, n, k, W.gbeta, K + 1, Qk, n, n, ncol, W.colact, W.npart, -1, st);
-                launch_update<double>(W.gP, ldk, n, k, W.gbeta, K + 1, Pk, n, n, ncol, W.colact, nullptr, -1, st);
-                launch_reduce(W.npart, nchu, 0, ncol, W.colact, W.gnu2, 1, 0, st);
+                launch_dots<double>(W.gQ, ldk, n, k, Qk, n, n, ncol, W.colact, W.npart_k, nch, W.gbeta, K + 1, W.done, st);
+                launch_update<double>(W.gQ, ldk, n, k, W.gbeta, K + 1, Qk, n, n, ncol, W.colact, W.npart, W.gnu2, W.done, -1, st);
+                launch_update<double>(W.gP, ldk, n, k, W.gbeta, K + 1, Pk, n, n, ncol, W.colact, nullptr, nullptr, nullptr, -1, st);
             } else {
-                launch_dots<double>(Qk, 0, n, 0, Qk, n, n, ncol, W.colact, W.npart, nch, st);
-                launch_reduce(W.npart, nch, 0, ncol, W.colact, W.gnu2, 1, 0, st);
+                launch_dots<double>(Qk, 0, n, 0, Qk, n, n, ncol, W.colact, W.npart, nch, W.gnu2, 1, W.done, st);
             }
             launch_gcr_scale(Pk, Qk, n, W.gnu2, W.colact, n, ncol, st);
-            launch_dots<double>(Qk, 0, n, 1, W.r64, n, n, ncol, W.colact, W.npart_k, nch, st);
-            launch_reduce(W.npart_k, nch, 1, ncol, W.colact, W.galpha, 2, 0, st);
-            launch_update<double>(Pk, 0, n, 1, W.galpha, 2, W.x64, n, n, ncol, W.colact, nullptr, 1, st);
-            launch_update<double>(Qk, 0, n, 1, W.galpha, 2, W.r64, n, n, ncol, W.colact, W.npart, -1, st);
-            launch_reduce(W.npart, nchu, 0, ncol, W.colact, W.nred, 1, 0, st);
+            launch_dots<double>(Qk, 0, n, 1, W.r64, n, n, ncol, W.colact, W.npart_k, nch, W.galpha, 2, W.done, st);
+            launch_update<double>(Pk, 0, n, 1, W.galpha, 2, W.x64, n, n, ncol, W.colact, nullptr, nullptr, nullptr, 1, st);
+            launch_update<double>(Qk, 0, n, 1, W.galpha, 2, W.r64, n, n, ncol, W.colact, W.npart, W.nred, W.done, -1, st);
             launch_sqrt_norms_active(W.nred, 1, ncol, W.colact, W.rho, st);
         }
         ++k;

@@ -37,12 +37,29 @@ constexpr int UPD_CHUNK = DOT_THREADS * UPD_EPT;
 int update_chunks(int64_t n) { return (int)((n + UPD_CHUNK - 1) / UPD_CHUNK); }
 constexpr int MAXV = 256;
 
-// partial[(slot * nchunk + chunk) * (nv + 1) + i] = sum over the chunk of conj(V_i) w, i < nv; index nv: |w|^2
+// Whether the calling block is the last of the slot's nblk to get here (its partial results, and the others', are then
+// visible to it); it leaves the slot's counter at zero for the next kernel.
+__device__ __forceinline__ bool last_of_slot(int* done, int slot, int nblk) {
+    __shared__ int last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last = atomicAdd(done + slot, 1) == nblk - 1;
+        if (last) done[slot] = 0;
+    }
+    __syncthreads();
+    if (last) __threadfence();
+    return last;
+}
+
+// partial[(slot * nchunk + chunk) * (nv + 1) + i] = sum over the chunk of conj(V_i) w, i < nv; index nv: |w|^2.  The
+// slot's last block adds the chunks in a fixed order to out[slot * ldo + i]: a reduction kernel of its own, one block per
+// slot, was a launch more on a chain of short ones.
 template <typename R, typename B>
 __global__ void __launch_bounds__(DOT_THREADS) dots_kernel(const B* __restrict__ V, int64_t ldv, int64_t lds, int nv,
                                                            const cx<R>* __restrict__ w, int64_t ldw, int64_t n,
                                                            const int* __restrict__ active, c64* __restrict__ partial,
-                                                           int nchunk, R vs) {
+                                                           int nchunk, R vs, c64* __restrict__ out, int ldo, int* done) {
     __shared__ c64 red[DOT_THREADS / 32][MAXV + 1];
     const int slot = blockIdx.y;
     if (active && !active[slot]) return;
@@ -104,45 +121,120 @@ __global__ void __launch_bounds__(DOT_THREADS) dots_kernel(const B* __restrict__
         for (int q = 0; q < DOT_THREADS / 32; ++q) acc += red[q][i];
         partial[((int64_t)slot * nchunk + chunk) * (nv + 1) + i] = acc;
     }
+    if (!last_of_slot(done, slot, nchunk)) return;
+    const c64* ps = partial + (int64_t)slot * nchunk * (nv + 1);
+    constexpr int PER = 4;                               // threads per sum
+    for (int b = 0; b <= nv; b += DOT_THREADS / PER) {
+        const int i = b + tid / PER, sub = tid % PER;
+        c64 acc = zero<double>();
+        if (i <= nv)
+            for (int c = sub; c < nchunk; c += PER) {
+                const double2 v = __ldcg(reinterpret_cast<const double2*>(ps + (int64_t)c * (nv + 1) + i));
+                acc += mk<double>(v.x, v.y);
+            }
+        for (int o = 1; o < PER; o <<= 1) {
+            acc.re += __shfl_xor_sync(0xffffffffu, acc.re, o);
+            acc.im += __shfl_xor_sync(0xffffffffu, acc.im, o);
+        }
+        if (i <= nv && sub == 0) out[(int64_t)slot * ldo + i] = acc;
+    }
 }
 
 template <typename R, typename B>
 void launch_dots(const B* V, int64_t ldv, int64_t lds, int nv, const cx<R>* w, int64_t ldw, int64_t n, int nslot,
-                 const int* active, c64* partial, int nchunk, cudaStream_t st, R vs) {
+                 const int* active, c64* partial, int nchunk, c64* out, int ldo, int* done, cudaStream_t st, R vs) {
     dots_kernel<R, B><<<dim3(nchunk, nslot), DOT_THREADS, 0, st>>>(V, ldv, lds, nv, w, ldw, n, active, partial, nchunk,
-                                                                    vs);
+                                                                    vs, out, ldo, done);
     GT_LAUNCH_CHECK();
 }
 
-// out[slot * ldo + i] = sum over chunks of partial (i <= nv); mode 1 adds to out
-__global__ void reduce_kernel(const c64* __restrict__ partial, int nchunk, int nv, const int* __restrict__ active,
-                              c64* __restrict__ out, int ldo, int mode) {
-    const int slot = blockIdx.x;
-    if (active && !active[slot]) return;
-    for (int i = threadIdx.x; i <= nv; i += blockDim.x) {
-        c64 acc = zero<double>();
-        for (int c = 0; c < nchunk; ++c) acc += partial[((int64_t)slot * nchunk + c) * (nv + 1) + i];
-        if (mode == 1) out[(int64_t)slot * ldo + i] += acc;
-        else out[(int64_t)slot * ldo + i] = acc;
+// The Hessenberg column j of a slot by one warp: rotate, new rotation, residual estimate, convergence.  The rotations are a
+// chain, x_{i+1} = cs_i h_{i+1} - conj(sn_i) x_i; its first term and the rotated entries cs_i x_i + sn_i h_{i+1} are made
+// side by side, so that a step of the chain is two FP64 multiply-adds on a lane for each component (an FP64 instruction
+// holds its pipe for 64 cycles).  sm: 3 (MAXV + 1) complex values.
+__device__ void givens_column(const GmresState& s, int j, int slot, bool re, double hn, c64* sm) {
+    const int lane = threadIdx.x & 31, m = s.m;
+    c64* hs = sm;                                        // h_0 .. h_j
+    c64* ts = sm + MAXV + 1;                             // cs_i h_{i+1}
+    c64* xs = sm + 2 * (MAXV + 1);                       // the chain
+    c64* H = s.H + (int64_t)slot * (m + 1) * m + (int64_t)j * (m + 1);
+    const c64* h = s.hvec + (int64_t)slot * s.ldh;
+    const c64* h2 = s.h2vec + (int64_t)slot * s.ldh;
+    double* cs = s.cs + (int64_t)slot * m;
+    c64* sn = s.sn + (int64_t)slot * m;
+    c64* g = s.g + (int64_t)slot * (m + 1);
+    double hnorm2 = 0;
+    for (int i = lane; i <= j; i += 32) {
+        c64 v = h[i];
+        if (re) v += h2[i];
+        hs[i] = v;
+        hnorm2 += norm2(v);
     }
-}
-
-void launch_reduce(const c64* partial, int nchunk, int nv, int nslot, const int* active, c64* out, int ldo, int mode,
-                   cudaStream_t st) {
-    reduce_kernel<<<nslot, 128, 0, st>>>(partial, nchunk, nv, active, out, ldo, mode);
-    GT_LAUNCH_CHECK();
+    hnorm2 = shfl_sum(hnorm2);
+    __syncwarp();
+    for (int i = lane; i < j; i += 32) ts[i] = cs[i] * hs[i + 1];
+    __syncwarp();
+    // lanes 0 and 1: the real and the imaginary part
+    double x = lane & 1 ? hs[0].im : hs[0].re;
+    for (int i = 0; i < j; ++i) {
+        if (lane < 2) reinterpret_cast<double*>(xs + i)[lane] = x;
+        const double o = __shfl_xor_sync(0xffffffffu, x, 1);
+        const c64 sv = sn[i];
+        const double t = lane & 1 ? ts[i].im : ts[i].re;
+        x = __fma_rn(lane & 1 ? sv.im : -sv.im, o, __fma_rn(-sv.re, x, t));
+    }
+    __syncwarp();
+    for (int i = lane; i < j; i += 32) H[i] = cs[i] * xs[i] + sn[i] * hs[i + 1];
+    const c64 a = mk<double>(__shfl_sync(0xffffffffu, x, 0), __shfl_sync(0xffffffffu, x, 1));
+    if (lane) return;
+    const double aa = sqrt(norm2(a));
+    const double rho = hypot(aa, hn);
+    double c = 1.0;
+    c64 sj = zero<double>(), hj = a;
+    if (rho != 0.0) {
+        if (aa == 0.0) {
+            c = 0.0;
+            sj = mk<double>(1.0, 0.0);
+            hj = mk<double>(hn, 0.0);
+        } else {
+            const c64 ph = mk<double>(a.re / aa, a.im / aa);
+            c = aa / rho;
+            sj = (hn / rho) * ph;
+            hj = rho * ph;
+        }
+    }
+    cs[j] = c;
+    sn[j] = sj;
+    H[j] = hj;
+    H[j + 1] = zero<double>();
+    const c64 gj = g[j], gn = mk<double>(-1.0, 0.0) * (conj(sj) * gj);
+    g[j + 1] = gn;
+    g[j] = c * gj;
+    s.it[slot] = j + 1;
+    const int total = s.its_total[slot] + 1;
+    s.its_total[slot] = total;
+    const double res = sqrt(norm2(gn));
+    const bool breakdown = hn <= 1e-14 * sqrt(hnorm2);
+    s.inv_hn[slot] = (hn > 0 && !breakdown) ? 1.0 / hn : 0.0;
+    const bool over = res <= s.eta[slot] || breakdown || j + 1 >= m || total >= s.max_its;
+    if (over) s.active[slot] = s.reorth[slot] = 0;       // (no second pass on a later step either)
+    s.to_go[slot] = over ? 0.0 : res / s.eta[slot];
 }
 
 // w += sign * sum_i h_i V_i (sign -1: Gram-Schmidt; +1: the cycle's combination); partial |w|^2 per chunk of
-// UPD_CHUNK elements (nchunk = update_chunks(n))
+// UPD_CHUNK elements (nchunk = update_chunks(n)).  The slot's last block finishes: tail 1: |w|^2 to out[slot]; 2: as that,
+// for the first Gram-Schmidt pass: decide the second one (DGKS) and, without it, the Hessenberg column; 3: as that, for
+// the second pass.
 template <typename R, typename B>
 __global__ void __launch_bounds__(DOT_THREADS) update_kernel(const B* __restrict__ V, int64_t ldv, int64_t lds,
                                                              int nv, const c64* __restrict__ h, int ldh,
                                                              cx<R>* __restrict__ w, int64_t ldw, int64_t n,
                                                              const int* __restrict__ active, c64* __restrict__ partial,
-                                                             int nchunk, int sign, R vs) {
+                                                             int nchunk, int sign, R vs, int tail, c64* __restrict__ out,
+                                                             int* done, GmresState s, int j) {
     __shared__ cx<R> hs[MAXV];
     __shared__ double red[DOT_THREADS / 32];
+    __shared__ c64 gv[3 * (MAXV + 1)];
     const int slot = blockIdx.y;
     if (active && !active[slot]) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -198,99 +290,68 @@ __global__ void __launch_bounds__(DOT_THREADS) update_kernel(const B* __restrict
     nrm = shfl_sum(nrm);
     if (lane == 0) red[warp] = nrm;
     __syncthreads();
-    if (tid == 0 && partial) {
-        double s = 0;
-        for (int q = 0; q < DOT_THREADS / 32; ++q) s += red[q];
-        partial[(int64_t)slot * nchunk + blockIdx.x] = mk<double>(s, 0.0);
+    if (!tail) return;
+    if (tid == 0) {
+        double t = 0;
+        for (int q = 0; q < DOT_THREADS / 32; ++q) t += red[q];
+        partial[(int64_t)slot * nchunk + blockIdx.x] = mk<double>(t, 0.0);
     }
+    if (!last_of_slot(done, slot, nchunk)) return;
+    double t = 0;
+    for (int c = tid; c < nchunk; c += DOT_THREADS) t += __ldcg(&partial[(int64_t)slot * nchunk + c].re);
+    t = shfl_sum(t);
+    if (lane == 0) red[warp] = t;
+    __syncthreads();
+    if (warp) return;
+    t = 0;
+    for (int q = 0; q < DOT_THREADS / 32; ++q) t += red[q];
+    if (lane == 0) out[slot] = mk<double>(t, 0.0);
+    if (tail == 1) return;
+    bool re = tail == 3;
+    if (tail == 2) {
+        re = sqrt(t) < s.reorth_ratio * sqrt(s.hvec[(int64_t)slot * s.ldh + j + 1].re);
+        if (lane == 0) s.reorth[slot] = re;
+        if (re) return;
+    }
+    givens_column(s, j, slot, re, sqrt(t), gv);
+}
+
+template <typename R, typename B>
+static void update_launch(const B* V, int64_t ldv, int64_t lds, int nv, const c64* h, int ldh, cx<R>* w, int64_t ldw, int64_t n,
+                          int nslot, const int* active, c64* partial, int sign, R vs, int tail, c64* out, int* done,
+                          const GmresState& s, int j, cudaStream_t st) {
+    const int nchunk = update_chunks(n);
+    update_kernel<R, B><<<dim3(nchunk, nslot), DOT_THREADS, 0, st>>>(V, ldv, lds, nv, h, ldh, w, ldw, n, active,
+                                                                      partial, nchunk, sign, vs, tail, out, done, s, j);
+    GT_LAUNCH_CHECK();
 }
 
 template <typename R, typename B>
 void launch_update(const B* V, int64_t ldv, int64_t lds, int nv, const c64* h, int ldh, cx<R>* w, int64_t ldw,
-                   int64_t n, int nslot, const int* active, c64* partial, int sign, cudaStream_t st, R vs) {
-    const int nchunk = update_chunks(n);
-    update_kernel<R, B><<<dim3(nchunk, nslot), DOT_THREADS, 0, st>>>(V, ldv, lds, nv, h, ldh, w, ldw, n, active,
-                                                                      partial, nchunk, sign, vs);
-    GT_LAUNCH_CHECK();
+                   int64_t n, int nslot, const int* active, c64* partial, c64* nrm2, int* done, int sign, cudaStream_t st, R vs) {
+    update_launch<R, B>(V, ldv, lds, nv, h, ldh, w, ldw, n, nslot, active, partial, sign, vs, nrm2 ? 1 : 0, nrm2, done,
+                        GmresState{}, 0, st);
 }
 
-template void launch_dots<float, c32>(const c32*, int64_t, int64_t, int, const c32*, int64_t, int64_t, int, const int*, c64*, int, cudaStream_t, float);
-template void launch_dots<float, h16c>(const h16c*, int64_t, int64_t, int, const c32*, int64_t, int64_t, int, const int*, c64*, int, cudaStream_t, float);
-template void launch_dots<double, c64>(const c64*, int64_t, int64_t, int, const c64*, int64_t, int64_t, int, const int*, c64*, int, cudaStream_t, double);
-template void launch_update<float, c32>(const c32*, int64_t, int64_t, int, const c64*, int, c32*, int64_t, int64_t, int, const int*, c64*, int, cudaStream_t, float);
-template void launch_update<float, h16c>(const h16c*, int64_t, int64_t, int, const c64*, int, c32*, int64_t, int64_t, int, const int*, c64*, int, cudaStream_t, float);
-template void launch_update<double, c64>(const c64*, int64_t, int64_t, int, const c64*, int, c64*, int64_t, int64_t, int, const int*, c64*, int, cudaStream_t, double);
+template <typename R, typename B>
+void launch_gram_schmidt(const B* V, int64_t ldv, int64_t lds, int pass, cx<R>* w, int64_t ldw, int64_t n, c64* partial, int* done,
+                         const GmresState& s, int j, cudaStream_t st, R vs) {
+    update_launch<R, B>(V, ldv, lds, j + 1, pass == 2 ? s.h2vec : s.hvec, s.ldh, w, ldw, n, s.nslot,
+                        pass == 2 ? s.reorth : s.active, partial, -1, vs, pass + 1, pass == 2 ? s.hn2b : s.hn2, done, s, j, st);
+}
+
+template void launch_dots<float, c32>(const c32*, int64_t, int64_t, int, const c32*, int64_t, int64_t, int, const int*, c64*, int, c64*, int, int*, cudaStream_t, float);
+template void launch_dots<float, h16c>(const h16c*, int64_t, int64_t, int, const c32*, int64_t, int64_t, int, const int*, c64*, int, c64*, int, int*, cudaStream_t, float);
+template void launch_dots<double, c64>(const c64*, int64_t, int64_t, int, const c64*, int64_t, int64_t, int, const int*, c64*, int, c64*, int, int*, cudaStream_t, double);
+template void launch_update<float, c32>(const c32*, int64_t, int64_t, int, const c64*, int, c32*, int64_t, int64_t, int, const int*, c64*, c64*, int*, int, cudaStream_t, float);
+template void launch_update<float, h16c>(const h16c*, int64_t, int64_t, int, const c64*, int, c32*, int64_t, int64_t, int, const int*, c64*, c64*, int*, int, cudaStream_t, float);
+template void launch_update<double, c64>(const c64*, int64_t, int64_t, int, const c64*, int, c64*, int64_t, int64_t, int, const int*, c64*, c64*, int*, int, cudaStream_t, double);
+
+template void launch_gram_schmidt<float, c32>(const c32*, int64_t, int64_t, int, c32*, int64_t, int64_t, c64*, int*, const GmresState&, int, cudaStream_t, float);
+template void launch_gram_schmidt<float, h16c>(const h16c*, int64_t, int64_t, int, c32*, int64_t, int64_t, c64*, int*, const GmresState&, int, cudaStream_t, float);
+template void launch_gram_schmidt<double, c64>(const c64*, int64_t, int64_t, int, c64*, int64_t, int64_t, c64*, int*, const GmresState&, int, cudaStream_t, double);
 
 // ------------------------------------------------------------------------------------------ per-slot scalars
-// After the first Gram-Schmidt pass: hvec[0..j] = h, hvec[j+1] = |w_before|^2; hn2 = |w_after|^2 (reduced
-// from the update's partials).  Decide the re-orthogonalisation.
-__global__ void dgks_kernel(GmresState s, int j) {
-    int slot = blockIdx.x * blockDim.x + threadIdx.x;
-    if (slot >= s.nslot) return;
-    int re = 0;
-    if (s.active[slot]) {
-        double before = sqrt(s.hvec[(int64_t)slot * s.ldh + j + 1].re);
-        double after = sqrt(s.hn2[slot].re);
-        re = after < s.reorth_ratio * before;
-    }
-    s.reorth[slot] = re;
-}
-
-// The Hessenberg column j of each active slot: rotate, new rotation, residual estimate, convergence.
-__global__ void givens_kernel(GmresState s, int j) {
-    int slot = blockIdx.x * blockDim.x + threadIdx.x;
-    if (slot >= s.nslot || !s.active[slot]) return;
-    const int m = s.m;
-    c64* H = s.H + (int64_t)slot * (m + 1) * m + (int64_t)j * (m + 1);
-    const c64* h = s.hvec + (int64_t)slot * s.ldh;
-    const c64* h2 = s.h2vec + (int64_t)slot * s.ldh;
-    const bool re = s.reorth[slot];
-    double hnorm2 = 0;
-    for (int i = 0; i <= j; ++i) {
-        c64 v = h[i];
-        if (re) v += h2[i];
-        H[i] = v;
-        hnorm2 += norm2(v);
-    }
-    double hn = sqrt(re ? s.hn2b[slot].re : s.hn2[slot].re);
-    double* cs = s.cs + (int64_t)slot * m;
-    c64* sn = s.sn + (int64_t)slot * m;
-    c64* g = s.g + (int64_t)slot * (m + 1);
-    for (int i = 0; i < j; ++i) {
-        c64 a = H[i], c = H[i + 1];
-        H[i] = cs[i] * a + sn[i] * c;
-        H[i + 1] = cs[i] * c - conj(sn[i]) * a;
-    }
-    c64 a = H[j];
-    double aa = sqrt(norm2(a));
-    double rho = hypot(aa, hn);
-    if (rho == 0.0) {
-        cs[j] = 1.0;
-        sn[j] = zero<double>();
-    } else if (aa == 0.0) {
-        cs[j] = 0.0;
-        sn[j] = mk<double>(1.0, 0.0);
-        H[j] = mk<double>(hn, 0.0);
-    } else {
-        c64 ph = mk<double>(a.re / aa, a.im / aa);
-        cs[j] = aa / rho;
-        sn[j] = (hn / rho) * ph;
-        H[j] = rho * ph;
-    }
-    H[j + 1] = zero<double>();
-    c64 gj = g[j];
-    g[j + 1] = mk<double>(-1.0, 0.0) * (conj(sn[j]) * gj);
-    g[j] = cs[j] * gj;
-    s.it[slot] = j + 1;
-    s.its_total[slot] += 1;
-    double res = sqrt(norm2(g[j + 1]));
-    bool breakdown = hn <= 1e-14 * sqrt(hnorm2);
-    bool done = res <= s.eta[slot] || breakdown || j + 1 >= m || s.its_total[slot] >= s.max_its;
-    s.inv_hn[slot] = (hn > 0 && !breakdown) ? 1.0 / hn : 0.0;
-    if (done) s.active[slot] = 0;
-    s.resid_est[slot] = res;
-}
-
 // store v (a basis vector, unscaled) at p[q]; with a narrower basis type also the stored value, unscaled,
 // to vc[q] (the vector the next product is applied to)
 template <typename R, typename B>
@@ -454,14 +515,6 @@ void launch_gcr_scale(c64* p, c64* q, int64_t ld, const c64* nu2, const int* act
     GT_LAUNCH_CHECK();
 }
 
-void launch_dgks(const GmresState& s, int j, cudaStream_t st) {
-    dgks_kernel<<<ceil_div(s.nslot, 128), 128, 0, st>>>(s, j);
-    GT_LAUNCH_CHECK();
-}
-void launch_givens(const GmresState& s, int j, cudaStream_t st) {
-    givens_kernel<<<ceil_div(s.nslot, 64), 64, 0, st>>>(s, j);
-    GT_LAUNCH_CHECK();
-}
 template <typename R, typename B>
 void launch_scale(const GmresStateT<R, B>& s, int j, int64_t n, cudaStream_t st) {
     int blocks = (int)std::min<int64_t>((n + 255) / 256, 1024);

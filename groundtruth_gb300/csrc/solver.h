@@ -22,7 +22,7 @@ struct GmresState {
     int* reorth;       // [slot]
     double* eta;       // [slot] the cycle's relative target
     double* inv_hn;    // [slot]
-    double* resid_est; // [slot]
+    double* to_go;     // [slot] the residual estimate over the cycle's target after the last step, 0 once the cycle is over
 };
 
 template <typename R, typename B = cx<R>> struct GmresStateT {
@@ -36,8 +36,12 @@ template <typename R, typename B = cx<R>> struct GmresStateT {
     cx<R>* vcur;       // [slot][ldv]: the newest basis vector as stored, unscaled (B != cx<R> only)
 };
 
-void launch_dgks(const GmresState& s, int j, cudaStream_t st);
-void launch_givens(const GmresState& s, int j, cudaStream_t st);
+// the update of Gram-Schmidt pass 1 or 2 of step j with what follows it per slot: after pass 1 (s.hvec) the decision on a
+// second one (s.reorth) and, where there is none, the Hessenberg column and convergence; after pass 2 (s.h2vec, the
+// flagged slots) the column
+template <typename R, typename B>
+void launch_gram_schmidt(const B* V, int64_t ldv, int64_t lds, int pass, cx<R>* w, int64_t ldw, int64_t n, c64* partial, int* done,
+                         const GmresState& s, int j, cudaStream_t st, R vs);
 template <typename R, typename B> void launch_scale(const GmresStateT<R, B>& s, int j, int64_t n, cudaStream_t st);
 void launch_hsolve(const GmresState& s, cudaStream_t st);
 template <typename R, typename B>
