@@ -30,7 +30,8 @@ __device__ __forceinline__ void bstore(h16c* p, c32 v) { p->v = __floats2half2_r
 constexpr int DOT_THREADS = 256;
 constexpr int DOT_EPT = 8;
 constexpr int DOT_CHUNK = DOT_THREADS * DOT_EPT;
-// the update keeps fewer elements per thread (more blocks resident, several basis vectors in flight)
+// the update keeps fewer elements per thread (more blocks resident, more basis vectors in flight); with 2 or 1 it is slower
+// where it matters (128 columns of 100,000 unknowns: 243 and 412 ms of updates against 207) and 1 us faster on one small column
 constexpr int UPD_EPT = 4;
 constexpr int UPD_CHUNK = DOT_THREADS * UPD_EPT;
 
@@ -59,7 +60,7 @@ template <typename R, typename B>
 __global__ void __launch_bounds__(DOT_THREADS) dots_kernel(const B* __restrict__ V, int64_t ldv, int64_t lds, int nv,
                                                            const cx<R>* __restrict__ w, int64_t ldw, int64_t n,
                                                            const int* __restrict__ active, c64* __restrict__ partial,
-                                                           int nchunk, R vs, c64* __restrict__ out, int ldo, int* done) {
+                                                           int nchunk, int vpb, R vs, c64* __restrict__ out, int ldo, int* done) {
     __shared__ c64 red[DOT_THREADS / 32][MAXV + 1];
     const int slot = blockIdx.y;
     if (active && !active[slot]) return;
@@ -75,53 +76,40 @@ __global__ void __launch_bounds__(DOT_THREADS) dots_kernel(const B* __restrict__
         nrm += norm2(wv[e]);
     }
     const B* Vs = V + (int64_t)slot * lds;
-    int i = 0;
-    // full chunks: UN basis vectors' loads in flight together (FP32 arithmetic; FP64 keeps one)
+    // UN basis vectors' loads in flight together (FP32 arithmetic; FP64 keeps one)
     constexpr int UN = sizeof(R) == 4 ? 2 : 1;
-    if (base + DOT_CHUNK <= n) {
-        for (; i + UN <= nv; i += UN) {
-            cx<R> v[UN][DOT_EPT];
+    const int i0 = blockIdx.z * vpb, i1 = min(nv, i0 + vpb);
+    for (int i = i0; i < i1; i += UN) {
+        cx<R> v[UN][DOT_EPT];
 #pragma unroll
-            for (int u = 0; u < UN; ++u)
+        for (int u = 0; u < UN; ++u)
 #pragma unroll
-                for (int e = 0; e < DOT_EPT; ++e) v[u][e] = bload(Vs + (int64_t)(i + u) * ldv + base + e * DOT_THREADS + tid);
-#pragma unroll
-            for (int u = 0; u < UN; ++u) {
-                R ar = 0, ai = 0;
-#pragma unroll
-                for (int e = 0; e < DOT_EPT; ++e) {
-                    ar += v[u][e].re * wv[e].re + v[u][e].im * wv[e].im;
-                    ai += v[u][e].re * wv[e].im - v[u][e].im * wv[e].re;
-                }
-                ar = shfl_sum(ar);
-                ai = shfl_sum(ai);
-                if (lane == 0) red[warp][i + u] = mk<double>((double)ar * vs, (double)ai * vs);
+            for (int e = 0; e < DOT_EPT; ++e) {
+                const int64_t q = base + e * DOT_THREADS + tid;
+                v[u][e] = i + u < i1 && q < n ? bload(Vs + (int64_t)(i + u) * ldv + q) : zero<R>();
             }
-        }
-    }
-    for (; i < nv; ++i) {
-        const B* Vi = Vs + (int64_t)i * ldv;
-        R ar = 0, ai = 0;
 #pragma unroll
-        for (int e = 0; e < DOT_EPT; ++e) {
-            int64_t q = base + e * DOT_THREADS + tid;
-            cx<R> v = q < n ? bload(Vi + q) : zero<R>();
-            ar += v.re * wv[e].re + v.im * wv[e].im;
-            ai += v.re * wv[e].im - v.im * wv[e].re;
+        for (int u = 0; u < UN; ++u) {
+            R ar = 0, ai = 0;
+#pragma unroll
+            for (int e = 0; e < DOT_EPT; ++e) {
+                ar += v[u][e].re * wv[e].re + v[u][e].im * wv[e].im;
+                ai += v[u][e].re * wv[e].im - v[u][e].im * wv[e].re;
+            }
+            ar = shfl_sum(ar);
+            ai = shfl_sum(ai);
+            if (lane == 0 && i + u < i1) red[warp][i + u] = mk<double>((double)ar * vs, (double)ai * vs);
         }
-        ar = shfl_sum(ar);
-        ai = shfl_sum(ai);
-        if (lane == 0) red[warp][i] = mk<double>((double)ar * vs, (double)ai * vs);
     }
     nrm = shfl_sum(nrm);
     if (lane == 0) red[warp][nv] = mk<double>(nrm, 0.0);
     __syncthreads();
-    for (int i = tid; i <= nv; i += DOT_THREADS) {
+    for (int i = i0 + tid; i < i1 + (i1 == nv); i += DOT_THREADS) {
         c64 acc = zero<double>();
         for (int q = 0; q < DOT_THREADS / 32; ++q) acc += red[q][i];
         partial[((int64_t)slot * nchunk + chunk) * (nv + 1) + i] = acc;
     }
-    if (!last_of_slot(done, slot, nchunk)) return;
+    if (!last_of_slot(done, slot, nchunk * gridDim.z)) return;
     const c64* ps = partial + (int64_t)slot * nchunk * (nv + 1);
     constexpr int PER = 4;                               // threads per sum
     for (int b = 0; b <= nv; b += DOT_THREADS / PER) {
@@ -143,8 +131,13 @@ __global__ void __launch_bounds__(DOT_THREADS) dots_kernel(const B* __restrict__
 template <typename R, typename B>
 void launch_dots(const B* V, int64_t ldv, int64_t lds, int nv, const cx<R>* w, int64_t ldw, int64_t n, int nslot,
                  const int* active, c64* partial, int nchunk, c64* out, int ldo, int* done, cudaStream_t st, R vs) {
-    dots_kernel<R, B><<<dim3(nchunk, nslot), DOT_THREADS, 0, st>>>(V, ldv, lds, nv, w, ldw, n, active, partial, nchunk,
-                                                                    vs, out, ldo, done);
+    // few chunks of few slots: the vectors over blocks too, two at least to each (a block's loop over 50 vectors waits 25
+    // times for memory: 14 us on average at 3,700 unknowns, 10 us so), up to three blocks for each of the 152 SMs.  A sum is
+    // the same however the vectors are dealt out.
+    const int groups = std::max(1, std::min((nv + 1) / 2, 456 / (nchunk * nslot)));
+    const int vpb = std::max(2, (ceil_div(nv, groups) + 1) / 2 * 2);
+    dots_kernel<R, B><<<dim3(nchunk, nslot, std::max(1, ceil_div(nv, vpb))), DOT_THREADS, 0, st>>>(
+        V, ldv, lds, nv, w, ldw, n, active, partial, nchunk, vpb, vs, out, ldo, done);
     GT_LAUNCH_CHECK();
 }
 
@@ -232,14 +225,17 @@ __global__ void __launch_bounds__(DOT_THREADS) update_kernel(const B* __restrict
                                                              const int* __restrict__ active, c64* __restrict__ partial,
                                                              int nchunk, int sign, R vs, int tail, c64* __restrict__ out,
                                                              int* done, GmresState s, int j) {
-    __shared__ cx<R> hs[MAXV];
+    __shared__ cx<R> hs[MAXV + 16];
     __shared__ double red[DOT_THREADS / 32];
     __shared__ c64 gv[3 * (MAXV + 1)];
     const int slot = blockIdx.y;
     if (active && !active[slot]) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int i = tid; i < nv; i += DOT_THREADS) {
-        c64 v = h[(int64_t)slot * ldh + i];
+    // UN basis vectors' loads in flight together (FP32 arithmetic; FP64 keeps fewer); the coefficients' last group of UN is
+    // filled up with zeros
+    constexpr int UN = (sizeof(R) == 4 ? 16 : 4) / UPD_EPT;
+    for (int i = tid; i < (nv + UN - 1) / UN * UN; i += DOT_THREADS) {
+        const c64 v = i < nv ? h[(int64_t)slot * ldh + i] : zero<double>();
         hs[i] = mk<R>(R(sign * v.re * vs), R(sign * v.im * vs));
     }
     __syncthreads();
@@ -251,31 +247,20 @@ __global__ void __launch_bounds__(DOT_THREADS) update_kernel(const B* __restrict
         acc[e] = q < n ? w[(int64_t)slot * ldw + q] : zero<R>();
     }
     const B* Vs = V + (int64_t)slot * lds;
-    int i = 0;
-    // full chunks: UN basis vectors' loads in flight together (FP32 arithmetic; FP64 keeps one)
-    constexpr int UN = sizeof(R) == 4 ? 4 : 1;
-    if (base + UPD_CHUNK <= n) {
-        for (; i + UN <= nv; i += UN) {
-            cx<R> v[UN][UPD_EPT];
+    for (int i = 0; i < nv; i += UN) {
+        cx<R> v[UN][UPD_EPT];
 #pragma unroll
-            for (int u = 0; u < UN; ++u)
+        for (int u = 0; u < UN; ++u)
 #pragma unroll
-                for (int e = 0; e < UPD_EPT; ++e) v[u][e] = bload(Vs + (int64_t)(i + u) * ldv + base + e * DOT_THREADS + tid);
-#pragma unroll
-            for (int u = 0; u < UN; ++u) {
-                const cx<R> hi = hs[i + u];
-#pragma unroll
-                for (int e = 0; e < UPD_EPT; ++e) acc[e] += hi * v[u][e];
+            for (int e = 0; e < UPD_EPT; ++e) {
+                const int64_t q = base + e * DOT_THREADS + tid;
+                v[u][e] = i + u < nv && q < n ? bload(Vs + (int64_t)(i + u) * ldv + q) : zero<R>();
             }
-        }
-    }
-    for (; i < nv; ++i) {
-        const cx<R> hi = hs[i];
-        const B* Vi = Vs + (int64_t)i * ldv;
 #pragma unroll
-        for (int e = 0; e < UPD_EPT; ++e) {
-            int64_t q = base + e * DOT_THREADS + tid;
-            if (q < n) acc[e] += hi * bload(Vi + q);
+        for (int u = 0; u < UN; ++u) {
+            const cx<R> hi = hs[i + u];
+#pragma unroll
+            for (int e = 0; e < UPD_EPT; ++e) acc[e] += hi * v[u][e];
         }
     }
     R nrm = 0;
