@@ -467,8 +467,8 @@ static void tune_lp(Orient& o, LpArgs<R> a, int pr, cudaStream_t st) {
 
 // System product out = K x (mode 0), rhs - K x (1), or the L_p product of the strips (2).
 template <typename R>
-static void matvec(gt_geometry* G, gt_operators* ops, const cx<R>* x, const cx<R>* rhs, cx<R>* out, int64_t ld, int ncol,
-                   const int* col_op, int mode, cx<R>* T, cudaStream_t st, const int* col_list = nullptr) {
+static void matvec(gt_geometry* G, gt_operators* ops, const cx<R>* x, const cx<R>* rhs, cx<R>* out, int64_t ld, int64_t ldo,
+                   int ncol, const int* col_op, int mode, cx<R>* T, cudaStream_t st, const int* col_list = nullptr) {
     Profiler* P = &G->prof;
     for (int k = 0; k < 2; ++k) {
         Orient& o = G->o[k];
@@ -478,6 +478,7 @@ static void matvec(gt_geometry* G, gt_operators* ops, const cx<R>* x, const cx<R
         a.rhs = rhs;
         a.out = out;
         a.ld = ld;
+        a.ldo = ldo;
         a.off = o.off;
         a.off_v = G->geo.off_v;
         a.S = G->geo.S;
@@ -530,11 +531,11 @@ static void matvec(gt_geometry* G, gt_operators* ops, const cx<R>* x, const cx<R
         const double nXY = (double)(G->geo.off_c - G->geo.off_x);
         Scope s(P, sizeof(R) == 4 ? "tail_f32" : "tail_f64", st,
                 ncol * (double)sizeof(cx<R>) * (2.0 * (G->geo.n - nXY) + nXY));
-        launch_tail<R>(G->geo, x, rhs, out, ld, ncol, col_op, ops->zcap, ops->zbr, mode, col_list, st);
+        launch_tail<R>(G->geo, x, rhs, out, ld, ldo, ncol, col_op, ops->zcap, ops->zbr, mode, col_list, st);
     }
     if (G->narrow.nrow) {
         Scope s(P, "narrow", st);
-        launch_narrow<R>(G->narrow, x, out, ld, ncol, G->geo.S, col_op, ops->omega, ops->zs, ops->zmut, mode,
+        launch_narrow<R>(G->narrow, x, out, ld, ldo, ncol, G->geo.S, col_op, ops->omega, ops->zs, ops->zmut, mode,
                          col_list, st);
     }
 }
@@ -620,7 +621,8 @@ static void sweep64(gt_geometry* G, const gt_operators* ops, const Groups& grp, 
 template <typename R>
 static void precond(gt_geometry* G, gt_operators* ops, const cx<R>* r, int64_t ldr, cx<R>* out, int64_t ldo, int nslot,
                     const int* slot_op, const Groups& grp, int gmax, cx<R>* zfac, cx<R>* yfac, cx<R>* uvec, cx<R>* sd,
-                    c32* yint, int* cnt, cudaStream_t st, const int* col_list = nullptr) {
+                    c32* yint, int* cnt, cudaStream_t st, const int* col_list = nullptr,
+                    const double* rscale = nullptr) {
     constexpr bool f32 = sizeof(R) == 4;
     Profiler* P = &G->prof;
     if (!f32 && (!ops->panel64 || !ops->panel64_rm))
@@ -630,7 +632,7 @@ static void precond(gt_geometry* G, gt_operators* ops, const cx<R>* r, int64_t l
     {
         Scope s(P, "pc_node", st, nslot * es * (nXYC + nodes + nfac));
         launch_pc_node<R>(G->geo, r, ldr, yfac, nslot, slot_op, tab_of<R>(ops), col_list, f32 ? cnt : nullptr,
-                          f32 ? sweep_counters(G->F.nfront, grp.ngroup) : 0, st);
+                          f32 ? sweep_counters(G->F.nfront, grp.ngroup) : 0, rscale, st);
     }
     if constexpr (f32) sweep32(G, ops, grp, yfac, zfac, yint, uvec, sd, cnt, nslot, st);
     else sweep64(G, ops, grp, gmax, yfac, zfac, uvec, sd, nslot, st);
@@ -642,7 +644,7 @@ static void precond(gt_geometry* G, gt_operators* ops, const cx<R>* r, int64_t l
     }
     {
         Scope s(P, "pc_strip", st, nslot * es * (2 * n + nfac));
-        launch_pc_strip<R>(G->geo, r, ldr, sd, out, ldo, nslot, slot_op, tab_of<R>(ops), col_list, st);
+        launch_pc_strip<R>(G->geo, r, ldr, sd, out, ldo, nslot, slot_op, tab_of<R>(ops), col_list, rscale, st);
     }
 }
 
@@ -837,6 +839,7 @@ static void fill_ws(Workspace& W, gt_geometry* G, int ncol, int m, int prec, int
     s.reorth = p.alloc<int>(ncol);
     s.eta = p.alloc<double>(ncol);
     s.inv_hn = p.alloc<double>(ncol);
+    s.vinv = p.alloc<double>((size_t)ncol * (m + 1));
     s.to_go = p.alloc<double>(ncol);
     W.slot_col = p.alloc<int>(ncol);
     W.slot_op = p.alloc<int>(ncol);
@@ -890,7 +893,7 @@ static int solve_impl(gt_geometry* G, gt_operators* ops, int ncol, const int* h_
     norms64(G, W.b64, n, ncol, W.bnorm, st);
     if (o.use_guess) {
         // x holds the starting points: r = b - K x in FP64
-        matvec<double>(G, ops, W.x64, W.b64, W.r64, n, ncol, W.col_op, 1, W.T64, st);
+        matvec<double>(G, ops, W.x64, W.b64, W.r64, n, n, ncol, W.col_op, 1, W.T64, st);
         norms64(G, W.r64, n, ncol, W.rho, st);
     } else {
         GT_CUDA(cudaMemsetAsync(W.x64, 0, (size_t)ncol * n * sizeof(c64), st));
@@ -917,17 +920,17 @@ static int solve_impl(gt_geometry* G, gt_operators* ops, int ncol, const int* h_
     const int64_t lds = (int64_t)(m + 1) * n;
     // the preconditioner on nsl listed slots (outputs n apart): in precision R, or, for stiff factorisations
     // (pc64), in FP64 on FP64 copies of the vectors, its result rounded back to R
-    auto apply_pc = [&](const cx<R>* rin, int64_t ldr, cx<R>* out, int nsl, const Groups& g, const int* list) {
+    auto apply_pc = [&](const cx<R>* rin, int64_t ldr, const double* rscale, cx<R>* out, int nsl, const Groups& g, const int* list) {
         if constexpr (std::is_same<R, float>::value) {
             if (pc64) {
-                launch_recast<double, float>(W.pr64, n, rin, ldr, list, n, nsl, st);
+                launch_recast<double, float>(W.pr64, n, rin, ldr, list, n, nsl, rscale, st);
                 precond<double>(G, ops, W.pr64, n, W.pz64, n, nsl, W.slot_pc, g, gmax, W.zfac64, W.yfac64, W.uvec64,
                                 W.sd64, nullptr, nullptr, st, list);
-                launch_recast<float, double>(out, n, W.pz64, n, list, n, nsl, st);
+                launch_recast<float, double>(out, n, W.pz64, n, list, n, nsl, nullptr, st);
                 return;
             }
         }
-        precond<R>(G, ops, rin, ldr, out, n, nsl, W.slot_pc, g, gmax, zfac, yfac, uvec, sd, W.yint, W.cnt, st, list);
+        precond<R>(G, ops, rin, ldr, out, n, nsl, W.slot_pc, g, gmax, zfac, yfac, uvec, sd, W.yint, W.cnt, st, list, rscale);
     };
     std::vector<int> slot_col, slot_op, slot_pc, gptr, gslot, gop, gpair, act;
     auto upload_groups = [&](const std::vector<int>& slots) {
@@ -946,7 +949,7 @@ static int solve_impl(gt_geometry* G, gt_operators* ops, int ncol, const int* h_
     std::vector<int> colact(ncol);
     // the true residual r = b - K x in FP64 (and its norms), which also restarts the GCR directions
     auto true_residual = [&]() {
-        matvec<double>(G, ops, W.x64, W.b64, W.r64, n, ncol, W.col_op, 1, W.T64, st);
+        matvec<double>(G, ops, W.x64, W.b64, W.r64, n, n, ncol, W.col_op, 1, W.T64, st);
         {
             Scope sc(P, "norms", st, 16.0 * ncol * n);
             norms64(G, W.r64, n, ncol, W.rho, st);
@@ -1000,44 +1003,53 @@ static int solve_impl(gt_geometry* G, gt_operators* ops, int ncol, const int* h_
             launch_init_state(S, W.slot_col, W.rho, W.bnorm, o.tol, o.inner_tol, st);
             launch_init_cycle<R, B>(ST, W.r64, n, W.slot_col, W.rho, n, st);
         }
+        const double* vinv = narrow ? nullptr : S.vinv;
         int jdone = 0;
         constexpr double FAR = 8;
         double togo = 2 * FAR;       // the slowest slot's, as last seen
         for (int j = 0; j < m; ++j) {
             // the products run on the slots still iterating in this cycle (W.act, grp)
             const int na = (int)act.size();
-            // the product is applied to the basis vector as stored
+            // The product is applied to the basis vector as stored.  A basis of the arithmetic's type is made in place, the
+            // product's result being its next vector until the Gram-Schmidt passes have turned it into one, and is not
+            // normalised: whoever reads a vector applies its 1 / norm (vinv) to a sum, a coefficient or an input that it
+            // has in registers, which saves a pass over the vector.
             const cx<R>* vin;
-            int64_t ldin;
+            cx<R>* wj;
+            int64_t ldin, ldw;
             if constexpr (narrow) {
                 vin = vcur;
-                ldin = n;
+                wj = w;
+                ldin = ldw = n;
             } else {
                 vin = V + (int64_t)j * n;
-                ldin = lds;
+                wj = V + (int64_t)(j + 1) * n;
+                ldin = ldw = lds;
             }
-            apply_pc(vin, ldin, z, na, grp, W.act);
-            matvec<R>(G, ops, z, nullptr, w, n, na, W.slot_op, 0, T, st, W.act);
+            apply_pc(vin, ldin, narrow ? nullptr : S.inv_hn, z, na, grp, W.act);
+            matvec<R>(G, ops, z, nullptr, wj, n, ldw, na, W.slot_op, 0, T, st, W.act);
             // classical Gram-Schmidt: the dot products read the j+1 basis vectors and w; the update reads
             // them again, reads w and writes it
             {
                 Scope sc(P, narrow ? "gs_dots_f32_b16" : sizeof(R) == 4 ? "gs_dots_f32" : "gs_dots_f64", st,
                          (double)ns * n * ((j + 1.0) * sizeof(B) + sizeof(cx<R>)));
-                launch_dots<R, B>(V, n, lds, j + 1, w, n, n, ns, S.active, W.partial, nch, S.hvec, S.ldh, W.done, st, vs);
+                launch_dots<R, B>(V, n, lds, j + 1, wj, ldw, n, ns, S.active, W.partial, nch, S.hvec, S.ldh, W.done, st, vs, vinv, m + 1);
             }
             {
                 Scope sc(P, narrow ? "gs_update_f32_b16" : sizeof(R) == 4 ? "gs_update_f32" : "gs_update_f64", st,
                          (double)ns * n * ((j + 1.0) * sizeof(B) + 2.0 * sizeof(cx<R>)));
-                launch_gram_schmidt<R, B>(V, n, lds, 1, w, n, n, W.partial, W.done, S, j, st, vs);
+                launch_gram_schmidt<R, B>(V, n, lds, 1, wj, ldw, n, W.partial, W.done, S, j, st, vs);
             }
             if (o.reorth > 0) {         // DGKS second pass (the slots the first one flagged)
                 Scope sc(P, "gs_reorth", st);
-                launch_dots<R, B>(V, n, lds, j + 1, w, n, n, ns, S.reorth, W.partial, nch, S.h2vec, S.ldh, W.done, st, vs);
-                launch_gram_schmidt<R, B>(V, n, lds, 2, w, n, n, W.partial, W.done, S, j, st, vs);
+                launch_dots<R, B>(V, n, lds, j + 1, wj, ldw, n, ns, S.reorth, W.partial, nch, S.h2vec, S.ldh, W.done, st, vs, vinv, m + 1);
+                launch_gram_schmidt<R, B>(V, n, lds, 2, wj, ldw, n, W.partial, W.done, S, j, st, vs);
             }
-            if (j + 1 < m) {
-                Scope sc(P, "gmres_small", st);
-                launch_scale<R, B>(ST, j, n, st);
+            if constexpr (narrow) {
+                if (j + 1 < m) {
+                    Scope sc(P, "gmres_small", st);
+                    launch_scale<R, B>(ST, j, n, st);
+                }
             }
             GT_CUDA(cudaMemcpyAsync(W.togo_host + (j & 1) * W.ncol, S.to_go, ns * sizeof(double), cudaMemcpyDeviceToHost, st));
             GT_CUDA(cudaEventRecord(W.togo_ev[j & 1], st));
@@ -1074,12 +1086,12 @@ static int solve_impl(gt_geometry* G, gt_operators* ops, int ncol, const int* h_
         GT_CUDA(cudaMemsetAsync(w, 0, (size_t)ns * n * sizeof(cx<R>), st));
         {
             Scope sc(P, "combine", st, (double)ns * n * (jdone * sizeof(B) + 2.0 * sizeof(cx<R>)));
-            launch_update<R, B>(V, n, lds, jdone, S.y, S.ldh, w, n, n, ns, nullptr, nullptr, nullptr, nullptr, 1, st, vs);
+            launch_update<R, B>(V, n, lds, jdone, S.y, S.ldh, w, n, n, ns, nullptr, nullptr, nullptr, nullptr, 1, st, vs, vinv, m + 1);
         }
         act.resize(ns);
         for (int q = 0; q < ns; ++q) act[q] = q;
         grp = upload_groups(act);
-        apply_pc(w, n, z, ns, grp, W.act);
+        apply_pc(w, n, nullptr, z, ns, grp, W.act);
         // GCR step in FP64: p = the cycle's correction, q = K p, both orthogonalised against the directions
         // held (q orthonormal); then x += alpha p, r -= alpha q with alpha = q^H r
         if (k == K) k = 0;
@@ -1093,7 +1105,7 @@ static int solve_impl(gt_geometry* G, gt_operators* ops, int ncol, const int* h_
             GT_CUDA(cudaMemsetAsync(Pk, 0, (size_t)ldk * sizeof(c64), st));
             launch_to64<R>(Pk, n, z, n, W.slot_col, n, ns, st);
         }
-        matvec<double>(G, ops, Pk, nullptr, Qk, n, ns, W.col_op, 0, W.T64, st, W.slot_col);
+        matvec<double>(G, ops, Pk, nullptr, Qk, n, n, ns, W.col_op, 0, W.T64, st, W.slot_col);
         {
             Scope sc(P, "gcr", st, 0.0);
             if (k > 0) {
@@ -1171,7 +1183,7 @@ void lp_with_scratch(gt_geometry* G, int ncol, const c64* x, c64* y, void* scrat
         LpArgs<double> a{};
         a.x = x;
         a.out = y;
-        a.ld = G->geo.n;
+        a.ld = a.ldo = G->geo.n;
         a.off = o.off;
         a.off_v = G->geo.off_v;
         a.S = G->geo.S;
@@ -1194,7 +1206,7 @@ void lp_with_scratch(gt_geometry* G, int ncol, const c64* x, c64* y, void* scrat
         launch_lp<double>(a, st);
     }
     if (G->narrow.nrow)
-        launch_narrow<double>(G->narrow, x, y, G->geo.n, ncol, G->geo.S, nullptr, nullptr, nullptr, nullptr, 2,
+        launch_narrow<double>(G->narrow, x, y, G->geo.n, G->geo.n, ncol, G->geo.S, nullptr, nullptr, nullptr, nullptr, 2,
                               nullptr, st);
 }
 
@@ -2003,7 +2015,7 @@ int gt_apply(gt_geometry* G, gt_operators* ops, int32_t kind, int32_t precision,
         }
         if (kind == 0 || kind == 2) {
             cx<R>* T = tmp.alloc<cx<R>>((size_t)n_cols * G->maxT);
-            matvec<R>(G, ops, xi, nullptr, yo, n, n_cols, d_op, kind == 0 ? 0 : 2, T, st);
+            matvec<R>(G, ops, xi, nullptr, yo, n, n, n_cols, d_op, kind == 0 ? 0 : 2, T, st);
         } else {
             std::vector<int> gptr, gslot, gop, gpair, all(n_cols);
             for (int c = 0; c < n_cols; ++c) all[c] = c;

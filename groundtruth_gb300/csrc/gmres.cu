@@ -60,7 +60,8 @@ template <typename R, typename B>
 __global__ void __launch_bounds__(DOT_THREADS) dots_kernel(const B* __restrict__ V, int64_t ldv, int64_t lds, int nv,
                                                            const cx<R>* __restrict__ w, int64_t ldw, int64_t n,
                                                            const int* __restrict__ active, c64* __restrict__ partial,
-                                                           int nchunk, int vpb, R vs, c64* __restrict__ out, int ldo, int* done) {
+                                                           int nchunk, int vpb, R vs, const double* __restrict__ vinv, int ldi,
+                                                           c64* __restrict__ out, int ldo, int* done) {
     __shared__ c64 red[DOT_THREADS / 32][MAXV + 1];
     const int slot = blockIdx.y;
     if (active && !active[slot]) return;
@@ -124,20 +125,22 @@ __global__ void __launch_bounds__(DOT_THREADS) dots_kernel(const B* __restrict__
             acc.re += __shfl_xor_sync(0xffffffffu, acc.re, o);
             acc.im += __shfl_xor_sync(0xffffffffu, acc.im, o);
         }
-        if (i <= nv && sub == 0) out[(int64_t)slot * ldo + i] = acc;
+        if (i <= nv && sub == 0)
+            out[(int64_t)slot * ldo + i] = vinv && i < nv ? vinv[(int64_t)slot * ldi + i] * acc : acc;
     }
 }
 
 template <typename R, typename B>
 void launch_dots(const B* V, int64_t ldv, int64_t lds, int nv, const cx<R>* w, int64_t ldw, int64_t n, int nslot,
-                 const int* active, c64* partial, int nchunk, c64* out, int ldo, int* done, cudaStream_t st, R vs) {
+                 const int* active, c64* partial, int nchunk, c64* out, int ldo, int* done, cudaStream_t st, R vs,
+                 const double* vinv, int ldi) {
     // few chunks of few slots: the vectors over blocks too, two at least to each (a block's loop over 50 vectors waits 25
     // times for memory: 14 us on average at 3,700 unknowns, 10 us so), up to three blocks for each of the 152 SMs.  A sum is
     // the same however the vectors are dealt out.
     const int groups = std::max(1, std::min((nv + 1) / 2, 456 / (nchunk * nslot)));
     const int vpb = std::max(2, (ceil_div(nv, groups) + 1) / 2 * 2);
     dots_kernel<R, B><<<dim3(nchunk, nslot, std::max(1, ceil_div(nv, vpb))), DOT_THREADS, 0, st>>>(
-        V, ldv, lds, nv, w, ldw, n, active, partial, nchunk, vpb, vs, out, ldo, done);
+        V, ldv, lds, nv, w, ldw, n, active, partial, nchunk, vpb, vs, vinv, ldi, out, ldo, done);
     GT_LAUNCH_CHECK();
 }
 
@@ -208,7 +211,9 @@ __device__ void givens_column(const GmresState& s, int j, int slot, bool re, dou
     s.its_total[slot] = total;
     const double res = sqrt(norm2(gn));
     const bool breakdown = hn <= 1e-14 * sqrt(hnorm2);
-    s.inv_hn[slot] = (hn > 0 && !breakdown) ? 1.0 / hn : 0.0;
+    const double inv = (hn > 0 && !breakdown) ? 1.0 / hn : 0.0;
+    s.inv_hn[slot] = inv;
+    s.vinv[(int64_t)slot * (m + 1) + j + 1] = inv;
     const bool over = res <= s.eta[slot] || breakdown || j + 1 >= m || total >= s.max_its;
     if (over) s.active[slot] = s.reorth[slot] = 0;       // (no second pass on a later step either)
     s.to_go[slot] = over ? 0.0 : res / s.eta[slot];
@@ -223,8 +228,8 @@ __global__ void __launch_bounds__(DOT_THREADS) update_kernel(const B* __restrict
                                                              int nv, const c64* __restrict__ h, int ldh,
                                                              cx<R>* __restrict__ w, int64_t ldw, int64_t n,
                                                              const int* __restrict__ active, c64* __restrict__ partial,
-                                                             int nchunk, int sign, R vs, int tail, c64* __restrict__ out,
-                                                             int* done, GmresState s, int j) {
+                                                             int nchunk, int sign, R vs, const double* __restrict__ vinv, int ldi,
+                                                             int tail, c64* __restrict__ out, int* done, GmresState s, int j) {
     __shared__ cx<R> hs[MAXV + 16];
     __shared__ double red[DOT_THREADS / 32];
     __shared__ c64 gv[3 * (MAXV + 1)];
@@ -235,7 +240,8 @@ __global__ void __launch_bounds__(DOT_THREADS) update_kernel(const B* __restrict
     // filled up with zeros
     constexpr int UN = (sizeof(R) == 4 ? 16 : 4) / UPD_EPT;
     for (int i = tid; i < (nv + UN - 1) / UN * UN; i += DOT_THREADS) {
-        const c64 v = i < nv ? h[(int64_t)slot * ldh + i] : zero<double>();
+        c64 v = i < nv ? h[(int64_t)slot * ldh + i] : zero<double>();
+        if (vinv && i < nv) v = vinv[(int64_t)slot * ldi + i] * v;
         hs[i] = mk<R>(R(sign * v.re * vs), R(sign * v.im * vs));
     }
     __syncthreads();
@@ -303,18 +309,19 @@ __global__ void __launch_bounds__(DOT_THREADS) update_kernel(const B* __restrict
 
 template <typename R, typename B>
 static void update_launch(const B* V, int64_t ldv, int64_t lds, int nv, const c64* h, int ldh, cx<R>* w, int64_t ldw, int64_t n,
-                          int nslot, const int* active, c64* partial, int sign, R vs, int tail, c64* out, int* done,
+                          int nslot, const int* active, c64* partial, int sign, R vs, const double* vinv, int ldi, int tail, c64* out, int* done,
                           const GmresState& s, int j, cudaStream_t st) {
     const int nchunk = update_chunks(n);
     update_kernel<R, B><<<dim3(nchunk, nslot), DOT_THREADS, 0, st>>>(V, ldv, lds, nv, h, ldh, w, ldw, n, active,
-                                                                      partial, nchunk, sign, vs, tail, out, done, s, j);
+                                                                      partial, nchunk, sign, vs, vinv, ldi, tail, out, done, s, j);
     GT_LAUNCH_CHECK();
 }
 
 template <typename R, typename B>
 void launch_update(const B* V, int64_t ldv, int64_t lds, int nv, const c64* h, int ldh, cx<R>* w, int64_t ldw,
-                   int64_t n, int nslot, const int* active, c64* partial, c64* nrm2, int* done, int sign, cudaStream_t st, R vs) {
-    update_launch<R, B>(V, ldv, lds, nv, h, ldh, w, ldw, n, nslot, active, partial, sign, vs, nrm2 ? 1 : 0, nrm2, done,
+                   int64_t n, int nslot, const int* active, c64* partial, c64* nrm2, int* done, int sign, cudaStream_t st, R vs,
+                   const double* vinv, int ldi) {
+    update_launch<R, B>(V, ldv, lds, nv, h, ldh, w, ldw, n, nslot, active, partial, sign, vs, vinv, ldi, nrm2 ? 1 : 0, nrm2, done,
                         GmresState{}, 0, st);
 }
 
@@ -322,15 +329,16 @@ template <typename R, typename B>
 void launch_gram_schmidt(const B* V, int64_t ldv, int64_t lds, int pass, cx<R>* w, int64_t ldw, int64_t n, c64* partial, int* done,
                          const GmresState& s, int j, cudaStream_t st, R vs) {
     update_launch<R, B>(V, ldv, lds, j + 1, pass == 2 ? s.h2vec : s.hvec, s.ldh, w, ldw, n, s.nslot,
-                        pass == 2 ? s.reorth : s.active, partial, -1, vs, pass + 1, pass == 2 ? s.hn2b : s.hn2, done, s, j, st);
+                        pass == 2 ? s.reorth : s.active, partial, -1, vs, std::is_same<B, cx<R>>::value ? s.vinv : nullptr, s.m + 1,
+                        pass + 1, pass == 2 ? s.hn2b : s.hn2, done, s, j, st);
 }
 
-template void launch_dots<float, c32>(const c32*, int64_t, int64_t, int, const c32*, int64_t, int64_t, int, const int*, c64*, int, c64*, int, int*, cudaStream_t, float);
-template void launch_dots<float, h16c>(const h16c*, int64_t, int64_t, int, const c32*, int64_t, int64_t, int, const int*, c64*, int, c64*, int, int*, cudaStream_t, float);
-template void launch_dots<double, c64>(const c64*, int64_t, int64_t, int, const c64*, int64_t, int64_t, int, const int*, c64*, int, c64*, int, int*, cudaStream_t, double);
-template void launch_update<float, c32>(const c32*, int64_t, int64_t, int, const c64*, int, c32*, int64_t, int64_t, int, const int*, c64*, c64*, int*, int, cudaStream_t, float);
-template void launch_update<float, h16c>(const h16c*, int64_t, int64_t, int, const c64*, int, c32*, int64_t, int64_t, int, const int*, c64*, c64*, int*, int, cudaStream_t, float);
-template void launch_update<double, c64>(const c64*, int64_t, int64_t, int, const c64*, int, c64*, int64_t, int64_t, int, const int*, c64*, c64*, int*, int, cudaStream_t, double);
+template void launch_dots<float, c32>(const c32*, int64_t, int64_t, int, const c32*, int64_t, int64_t, int, const int*, c64*, int, c64*, int, int*, cudaStream_t, float, const double*, int);
+template void launch_dots<float, h16c>(const h16c*, int64_t, int64_t, int, const c32*, int64_t, int64_t, int, const int*, c64*, int, c64*, int, int*, cudaStream_t, float, const double*, int);
+template void launch_dots<double, c64>(const c64*, int64_t, int64_t, int, const c64*, int64_t, int64_t, int, const int*, c64*, int, c64*, int, int*, cudaStream_t, double, const double*, int);
+template void launch_update<float, c32>(const c32*, int64_t, int64_t, int, const c64*, int, c32*, int64_t, int64_t, int, const int*, c64*, c64*, int*, int, cudaStream_t, float, const double*, int);
+template void launch_update<float, h16c>(const h16c*, int64_t, int64_t, int, const c64*, int, c32*, int64_t, int64_t, int, const int*, c64*, c64*, int*, int, cudaStream_t, float, const double*, int);
+template void launch_update<double, c64>(const c64*, int64_t, int64_t, int, const c64*, int, c64*, int64_t, int64_t, int, const int*, c64*, c64*, int*, int, cudaStream_t, double, const double*, int);
 
 template void launch_gram_schmidt<float, c32>(const c32*, int64_t, int64_t, int, c32*, int64_t, int64_t, c64*, int*, const GmresState&, int, cudaStream_t, float);
 template void launch_gram_schmidt<float, h16c>(const h16c*, int64_t, int64_t, int, c32*, int64_t, int64_t, c64*, int*, const GmresState&, int, cudaStream_t, float);
@@ -349,6 +357,7 @@ __device__ __forceinline__ void put_basis(const GmresStateT<R, B>& s, B* p, cx<R
     }
 }
 
+// the next vector of a narrow basis: w normalised and rounded
 template <typename R, typename B>
 __global__ void scale_kernel(GmresStateT<R, B> s, int j, int64_t n) {
     const int slot = blockIdx.y;
@@ -402,6 +411,9 @@ __global__ void init_state_kernel(GmresState s, const int* __restrict__ slot_col
     for (int i = 1; i <= s.m; ++i) g[i] = zero<double>();
     s.it[slot] = 0;
     s.active[slot] = 1;
+    // the cycle's first vector is stored normalised; no later one is weighted before it is made
+    s.inv_hn[slot] = 1.0;
+    for (int i = 0; i <= s.m; ++i) s.vinv[(int64_t)slot * (s.m + 1) + i] = i ? 0.0 : 1.0;
     // the cycle needs to reach the outer tolerance at most (half of it, as a margin), never below inner_tol
     double need = rho[col] > 0 ? 0.5 * tol * bnorm[col] / rho[col] : 1.0;
     s.eta[slot] = fmax(inner_tol, need);
@@ -449,12 +461,13 @@ __global__ void to64_kernel(c64* __restrict__ dst, int64_t ldd, const cx<R>* __r
 // solve's vectors into and out of an FP64 preconditioner apply
 template <typename D, typename S>
 __global__ void recast_kernel(cx<D>* __restrict__ dst, int64_t ldd, const cx<S>* __restrict__ src, int64_t lds,
-                              const int* __restrict__ list, int64_t n) {
+                              const int* __restrict__ list, int64_t n, const double* __restrict__ scale) {
     const int c = list ? list[blockIdx.y] : (int)blockIdx.y;
+    const double f = scale ? scale[c] : 1.0;
     cx<D>* d = dst + (int64_t)c * ldd;
     const cx<S>* x = src + (int64_t)c * lds;
     for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x)
-        d[q] = cvt<D>(x[q]);
+        d[q] = cvt<D>(f * cvt<double>(x[q]));
 }
 
 __global__ void gcr_scale_kernel(c64* __restrict__ p, c64* __restrict__ q, int64_t ld, const c64* __restrict__ nu2,
@@ -484,14 +497,14 @@ template void launch_to64<double>(c64*, int64_t, const c64*, int64_t, const int*
 
 template <typename D, typename S>
 void launch_recast(cx<D>* dst, int64_t ldd, const cx<S>* src, int64_t lds, const int* list, int64_t n, int nslot,
-                   cudaStream_t st) {
+                   const double* scale, cudaStream_t st) {
     if (nslot <= 0) return;
     int blocks = (int)std::min<int64_t>((n + 255) / 256, 1024);
-    recast_kernel<D, S><<<dim3(blocks, nslot), 256, 0, st>>>(dst, ldd, src, lds, list, n);
+    recast_kernel<D, S><<<dim3(blocks, nslot), 256, 0, st>>>(dst, ldd, src, lds, list, n, scale);
     GT_LAUNCH_CHECK();
 }
-template void launch_recast<double, float>(c64*, int64_t, const c32*, int64_t, const int*, int64_t, int, cudaStream_t);
-template void launch_recast<float, double>(c32*, int64_t, const c64*, int64_t, const int*, int64_t, int, cudaStream_t);
+template void launch_recast<double, float>(c64*, int64_t, const c32*, int64_t, const int*, int64_t, int, const double*, cudaStream_t);
+template void launch_recast<float, double>(c32*, int64_t, const c64*, int64_t, const int*, int64_t, int, const double*, cudaStream_t);
 
 void launch_gcr_scale(c64* p, c64* q, int64_t ld, const c64* nu2, const int* active, int64_t n, int ncol,
                       cudaStream_t st) {
@@ -549,9 +562,7 @@ void launch_sqrt_norms(const c64* nrm2, int ld, int n, double* out, cudaStream_t
     GT_LAUNCH_CHECK();
 }
 
-template void launch_scale<float, c32>(const GmresStateT<float, c32>&, int, int64_t, cudaStream_t);
 template void launch_scale<float, h16c>(const GmresStateT<float, h16c>&, int, int64_t, cudaStream_t);
-template void launch_scale<double, c64>(const GmresStateT<double, c64>&, int, int64_t, cudaStream_t);
 template void launch_init_cycle<float, c32>(const GmresStateT<float, c32>&, const c64*, int64_t, const int*, const double*, int64_t, cudaStream_t);
 template void launch_init_cycle<float, h16c>(const GmresStateT<float, h16c>&, const c64*, int64_t, const int*, const double*, int64_t, cudaStream_t);
 template void launch_init_cycle<double, c64>(const GmresStateT<double, c64>&, const c64*, int64_t, const int*, const double*, int64_t, cudaStream_t);

@@ -55,7 +55,7 @@ struct Narrow {
     const double* twre = nullptr;
 };
 template <typename R>
-void launch_narrow(const Narrow& nw, const cx<R>* x, cx<R>* out, int64_t ld, int ncol, int S, const int* col_op,
+void launch_narrow(const Narrow& nw, const cx<R>* x, cx<R>* out, int64_t ld, int64_t ldo, int ncol, int S, const int* col_op,
                    const double* omega, const c64* zs, const c64* zmut, int mode, const int* col_list,
                    cudaStream_t st);
 
@@ -63,7 +63,7 @@ template <typename R> struct LpArgs {
     const cx<R>* x;
     const cx<R>* rhs;
     cx<R>* out;
-    int64_t ld, off, off_v;
+    int64_t ld, ldo, off, off_v;   // columns of x and rhs are ld apart, of out ldo
     int S, n0, n1, nx, ny, di, dj, P0, P1, ncol;
     const cx<R>* tw0;      // twiddles of the column length P0
     const cx<R>* tw1;      // of the row length P1
@@ -92,18 +92,18 @@ template <typename R> void lp_shapes(const LpArgs<R>& a, int* rows, int* bt);
 // capacitance / branch / node rows of the system product (mode 0: K x, 1: rhs - K x); also zeroes the
 // padding between segments
 template <typename R>
-void launch_tail(const Geo& g, const cx<R>* x, const cx<R>* rhs, cx<R>* out, int64_t ld, int ncol, const int* col_op,
-                 const c64* zcap, const c64* zbr, int mode, const int* col_list, cudaStream_t st);
+void launch_tail(const Geo& g, const cx<R>* x, const cx<R>* rhs, cx<R>* out, int64_t ld, int64_t ldo, int ncol,
+                 const int* col_op, const c64* zcap, const c64* zbr, int mode, const int* col_list, cudaStream_t st);
 
 // preconditioner: s = r_V - Ar^T D^-1 r_1 into factor order (sd [col][nfac]); then, with y in node order in
 // sd [col][S*nx*ny] (zero at nodes that are not kept), out = [D^-1 (r_1 + Ar y); y]
-// (cnt: ncnt counters of the sweep that follows, cleared by the way)
+// (cnt: ncnt counters of the sweep that follows, cleared by the way).  rscale (or null): r is taken times rscale[column].
 template <typename R>
 void launch_pc_node(const Geo& g, const cx<R>* r, int64_t ld, cx<R>* sd, int ncol, const int* col_op,
-                    const cx<R>* tab, const int* col_list, int* cnt, int64_t ncnt, cudaStream_t st);
+                    const cx<R>* tab, const int* col_list, int* cnt, int64_t ncnt, const double* rscale, cudaStream_t st);
 template <typename R>
 void launch_pc_strip(const Geo& g, const cx<R>* r, int64_t ldr, const cx<R>* sd, cx<R>* out, int64_t ldo, int ncol,
-                     const int* col_op, const cx<R>* tab, const int* col_list, cudaStream_t st);
+                     const int* col_op, const cx<R>* tab, const int* col_list, const double* rscale, cudaStream_t st);
 
 // psi of the first ns compact entries (the strips): segments [nseg][8] (a, b, width, current), device FP64; the sheets'
 // heights and thicknesses by value
@@ -253,10 +253,10 @@ void launch_lowrank_rhs(cx<R>* s, int64_t nfac, int c0, int ncol, int k, const i
 // U^T W entries g[c][i] of ncol node-ordered columns
 void launch_lowrank_gather(const c64* w, int64_t nnode, int ncol, int k, const int* ends, c64* g, cudaStream_t st);
 void launch_lowrank_to32(const c64* a, c32* b, int64_t n, cudaStream_t st);
-// dst[c] = src[c] (n entries, converted) for c = list[0 .. nslot) (0 .. nslot when list is null)
+// dst[c] = src[c] (n entries, times scale[c] if given, converted) for c = list[0 .. nslot) (0 .. nslot when list is null)
 template <typename D, typename S>
 void launch_recast(cx<D>* dst, int64_t ldd, const cx<S>* src, int64_t lds, const int* list, int64_t n, int nslot,
-                   cudaStream_t st);
+                   const double* scale, cudaStream_t st);
 void launch_lowrank_to64(const c32* a, c64* b, int64_t n, cudaStream_t st);
 
 // --- Krylov vector work (batched, one basis per slot)
@@ -266,15 +266,17 @@ struct h16c {
     __half2 v;
 };
 // Basis vectors are stored as B (cx<R>, or h16c for R = float) times the scale; vs = 1 / scale undoes it.
-// done: one counter per slot, zero between kernels; out[slot * ldo + i]: the reduced sums (i <= nv; nv: |w|^2)
+// done: one counter per slot, zero between kernels; out[slot * ldo + i]: the reduced sums (i <= nv; nv: |w|^2).
+// vinv (or null): vector i of a slot is taken times vinv[slot * ldi + i].
 template <typename R, typename B>
 void launch_dots(const B* V, int64_t ldv, int64_t lds, int nv, const cx<R>* w, int64_t ldw, int64_t n, int nslot,
-                 const int* active, c64* partial, int nchunk, c64* out, int ldo, int* done, cudaStream_t st, R vs = R(1));
+                 const int* active, c64* partial, int nchunk, c64* out, int ldo, int* done, cudaStream_t st, R vs = R(1),
+                 const double* vinv = nullptr, int ldi = 0);
 // nrm2 (if not null): |w|^2 after the update per slot (partial: update_chunks(n) per slot)
 int update_chunks(int64_t n);
 template <typename R, typename B>
 void launch_update(const B* V, int64_t ldv, int64_t lds, int nv, const c64* h, int ldh, cx<R>* w, int64_t ldw,
                    int64_t n, int nslot, const int* active, c64* partial, c64* nrm2, int* done, int sign, cudaStream_t st,
-                   R vs = R(1));
+                   R vs = R(1), const double* vinv = nullptr, int ldi = 0);
 
 }  // namespace gt

@@ -495,7 +495,7 @@ constexpr size_t CW_SMEM = (size_t)CW_WARPS * WX_SLOTS * sizeof(c32);
 __global__ void __launch_bounds__(CW_WARPS * 32, GT_CW_MINB) lp_pass_cw(const c32* __restrict__ T,
                                                                const c32* __restrict__ x,
                                                                const c32* __restrict__ rhs, c32* __restrict__ out,
-                                                               int64_t ld, int64_t off, int64_t off_v, int S, int n0,
+                                                               int64_t ld, int64_t ldo, int64_t off, int64_t off_v, int S, int n0,
                                                                int n1, int nx, int ny, int di, int dj, int ldt,
                                                                const c32* __restrict__ tw, const uint8_t* __restrict__ mask,
                                                                const int* __restrict__ col_op,
@@ -553,7 +553,7 @@ __global__ void __launch_bounds__(CW_WARPS * 32, GT_CW_MINB) lp_pass_cw(const c3
                 y = z * x[base + pos] + w * jmul(L) - (x[base + va] - x[base + vb]);
                 if (mode == 1) y = rhs[base + pos] - y;
             }
-            out[base + pos] = y;
+            out[(int64_t)col * ldo + pos] = y;
         }
     }
 }
@@ -600,7 +600,7 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
 __global__ void __launch_bounds__(CT_WARPS * 32, GT_RW_MINB) lp_pass_ct(const __grid_constant__ CUtensorMap tmap,
                                                                 const c32* __restrict__ x,
                                                                 const c32* __restrict__ rhs, c32* __restrict__ out,
-                                                                int64_t ld, int64_t off, int64_t off_v, int S, int n0,
+                                                                int64_t ld, int64_t ldo, int64_t off, int64_t off_v, int S, int n0,
                                                                 int n1, int nx, int ny, int di, int dj,
                                                                 const c32* __restrict__ tw, const uint8_t* __restrict__ mask,
                                                                 const int* __restrict__ col_op,
@@ -711,7 +711,7 @@ __global__ void __launch_bounds__(CT_WARPS * 32, GT_RW_MINB) lp_pass_ct(const __
                 yv = z * x[base + pos] + w * jmul(L) - (x[base + va] - x[base + vb]);
                 if (mode == 1) yv = rhs[base + pos] - yv;
             }
-            out[base + pos] = yv;
+            out[(int64_t)col * ldo + pos] = yv;
         }
     }
 }
@@ -780,7 +780,7 @@ __global__ void __launch_bounds__(1024) lp_pass_a8(const cx<R>* __restrict__ x, 
 
 template <typename R, int P>
 __global__ void __launch_bounds__(1024) lp_pass_c8(const cx<R>* __restrict__ T, const cx<R>* __restrict__ x,
-                                                   const cx<R>* __restrict__ rhs, cx<R>* __restrict__ out, int64_t ld,
+                                                   const cx<R>* __restrict__ rhs, cx<R>* __restrict__ out, int64_t ld, int64_t ldo,
                                                    int64_t off, int64_t off_v, int S, int n0, int n1, int nx, int ny,
                                                    int di, int dj, int rows, const cx<R>* __restrict__ tw,
                                                    const uint8_t* __restrict__ mask, const int* __restrict__ col_op,
@@ -858,14 +858,14 @@ __global__ void __launch_bounds__(1024) lp_pass_c8(const cx<R>* __restrict__ T, 
             y = z * xv + w * jmul(L[r]) - dv;
             if (mode == 1) y = rhs[base + pos] - y;
         }
-        out[base + pos] = y;
+        out[(int64_t)col * ldo + pos] = y;
     }
 }
 
 // mode 0: out = R_t x + j w L - (V[a] - V[b]); 1: out = rhs - (that); 2: out = L
 template <typename R, int PL>
 __global__ void __launch_bounds__(1024) lp_pass_c(const cx<R>* __restrict__ T, const cx<R>* __restrict__ x, const cx<R>* __restrict__ rhs,
-                          cx<R>* __restrict__ out, int64_t ld, int64_t off, int64_t off_v, int S, int n0, int n1,
+                          cx<R>* __restrict__ out, int64_t ld, int64_t ldo, int64_t off, int64_t off_v, int S, int n0, int n1,
                           int nx, int ny, int di, int dj, int P1, int rows, const cx<R>* __restrict__ tw,
                           const uint8_t* __restrict__ mask, const int* __restrict__ col_op,
                           const double* __restrict__ omega, const c64* __restrict__ zs, int mode,
@@ -912,7 +912,7 @@ __global__ void __launch_bounds__(1024) lp_pass_c(const cx<R>* __restrict__ T, c
             y = z * xv + w * jmul(L) - dv;
             if (mode == 1) y = rhs[base + pos] - y;
         }
-        out[base + pos] = y;
+        out[(int64_t)col * ldo + pos] = y;
     }
 }
 
@@ -1085,7 +1085,7 @@ static void launch_c(const LpArgs<R>& a, int rows, cudaStream_t st) {
             const bool shortfall = t && t[0] == '1';
             set_smem<float>((const void*)lp_pass_ct, CT_SMEM);
             lp_pass_ct<<<dim3(ceil_div(a.n0, 16), a.S, a.ncol), CT_WARPS * 32, CT_SMEM, st>>>(
-                m, a.x, a.rhs, a.out, a.ld, a.off, a.off_v, a.S, a.n0, a.n1, a.nx, a.ny, a.di, a.dj, a.tw1, a.mask,
+                m, a.x, a.rhs, a.out, a.ld, a.ldo, a.off, a.off_v, a.S, a.n0, a.n1, a.nx, a.ny, a.di, a.dj, a.tw1, a.mask,
                 a.col_op, a.omega, a.zs, a.mode, a.col_list, a.sheet_layer, shortfall ? 16u : 0u,
                 shortfall ? 1000000ull : CT_WAIT_NS);
             GT_LAUNCH_CHECK();
@@ -1094,7 +1094,7 @@ static void launch_c(const LpArgs<R>& a, int rows, cudaStream_t st) {
         if (rw_fits(a)) {
             set_smem<float>((const void*)lp_pass_cw, CW_SMEM);
             lp_pass_cw<<<dim3(ceil_div(a.n0, 2 * CW_WARPS), a.S, a.ncol), CW_WARPS * 32, CW_SMEM, st>>>(
-                a.T, a.x, a.rhs, a.out, a.ld, a.off, a.off_v, a.S, a.n0, a.n1, a.nx, a.ny, a.di, a.dj, a.ldt, a.tw1,
+                a.T, a.x, a.rhs, a.out, a.ld, a.ldo, a.off, a.off_v, a.S, a.n0, a.n1, a.nx, a.ny, a.di, a.dj, a.ldt, a.tw1,
                 a.mask, a.col_op, a.omega, a.zs, a.mode, a.col_list, a.sheet_layer);
             GT_LAUNCH_CHECK();
             return;
@@ -1104,7 +1104,7 @@ static void launch_c(const LpArgs<R>& a, int rows, cudaStream_t st) {
         const size_t sm = (size_t)2 * rows * lp_srow(PA) * sizeof(cx<R>);
         set_smem<R>((const void*)lp_pass_c8<R, PA>, sm);
         lp_pass_c8<R, PA><<<dim3(ceil_div(a.n0, rows), a.S, a.ncol), rows * (PA / 8), sm, st>>>(
-            a.T, a.x, a.rhs, a.out, a.ld, a.off, a.off_v, a.S, a.n0, a.n1, a.nx, a.ny, a.di, a.dj, rows, a.tw1, a.mask,
+            a.T, a.x, a.rhs, a.out, a.ld, a.ldo, a.off, a.off_v, a.S, a.n0, a.n1, a.nx, a.ny, a.di, a.dj, rows, a.tw1, a.mask,
             a.col_op, a.omega, a.zs, a.mode, a.col_list, a.sheet_layer, ldt_of(a));
         GT_LAUNCH_CHECK();
         return;
@@ -1112,7 +1112,7 @@ static void launch_c(const LpArgs<R>& a, int rows, cudaStream_t st) {
     size_t smA = (size_t)rows * srow(a.P1) * sizeof(cx<R>);
     dim3 gA(ceil_div(a.n0, rows), a.S, a.ncol);
     set_smem<R>((const void*)lp_pass_c<R, PA>, smA);
-    lp_pass_c<R, PA><<<gA, rows * (a.P1 / 8), smA, st>>>(a.T, a.x, a.rhs, a.out, a.ld, a.off, a.off_v, a.S, a.n0, a.n1,
+    lp_pass_c<R, PA><<<gA, rows * (a.P1 / 8), smA, st>>>(a.T, a.x, a.rhs, a.out, a.ld, a.ldo, a.off, a.off_v, a.S, a.n0, a.n1,
                                                           a.nx, a.ny, a.di, a.dj, a.P1, rows, a.tw1, a.mask, a.col_op,
                                                           a.omega, a.zs, a.mode, a.col_list, a.sheet_layer, ldt_of(a));
     GT_LAUNCH_CHECK();

@@ -13,7 +13,7 @@ namespace gt {
 // one thread per (row, column); grid (row chunks, columns)
 template <typename R>
 __global__ void __launch_bounds__(128) narrow_kernel(Narrow nw, const cx<R>* __restrict__ x, cx<R>* __restrict__ out,
-                                                    int64_t ld, int S, const int* __restrict__ col_op,
+                                                    int64_t ld, int64_t ldo, int S, const int* __restrict__ col_op,
                                                     const double* __restrict__ omega, const c64* __restrict__ zs,
                                                     const c64* __restrict__ zmut, int mode,
                                                     const int* __restrict__ col_list) {
@@ -39,22 +39,22 @@ __global__ void __launch_bounds__(128) narrow_kernel(Narrow nw, const cx<R>* __r
         }
         if (mode == 1) y = zero<R>() - y;
     }
-    out[(int64_t)col * ld + p] += y;
+    out[(int64_t)col * ldo + p] += y;
 }
 
 template <typename R>
-void launch_narrow(const Narrow& nw, const cx<R>* x, cx<R>* out, int64_t ld, int ncol, int S, const int* col_op,
+void launch_narrow(const Narrow& nw, const cx<R>* x, cx<R>* out, int64_t ld, int64_t ldo, int ncol, int S, const int* col_op,
                    const double* omega, const c64* zs, const c64* zmut, int mode, const int* col_list,
                    cudaStream_t st) {
     if (nw.nrow == 0 || ncol < 1) return;
-    narrow_kernel<R><<<dim3((unsigned)((nw.nrow + 127) / 128), ncol), 128, 0, st>>>(nw, x, out, ld, S, col_op, omega,
+    narrow_kernel<R><<<dim3((unsigned)((nw.nrow + 127) / 128), ncol), 128, 0, st>>>(nw, x, out, ld, ldo, S, col_op, omega,
                                                                                    zs, zmut, mode, col_list);
     GT_LAUNCH_CHECK();
 }
 
-template void launch_narrow<float>(const Narrow&, const c32*, c32*, int64_t, int, int, const int*, const double*,
+template void launch_narrow<float>(const Narrow&, const c32*, c32*, int64_t, int64_t, int, int, const int*, const double*,
                                    const c64*, const c64*, int, const int*, cudaStream_t);
-template void launch_narrow<double>(const Narrow&, const c64*, c64*, int64_t, int, int, const int*, const double*,
+template void launch_narrow<double>(const Narrow&, const c64*, c64*, int64_t, int64_t, int, int, const int*, const double*,
                                     const c64*, const c64*, int, const int*, cudaStream_t);
 
 }  // namespace gt

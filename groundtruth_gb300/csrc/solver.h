@@ -21,7 +21,8 @@ struct GmresState {
     int* active;       // [slot]
     int* reorth;       // [slot]
     double* eta;       // [slot] the cycle's relative target
-    double* inv_hn;    // [slot]
+    double* inv_hn;    // [slot] 1 / norm of the newest basis vector, which is stored as the last step left it (1 for the cycle's first)
+    double* vinv;      // [slot][m+1] the same of all of them (a narrow basis is stored normalised and has none)
     double* to_go;     // [slot] the residual estimate over the cycle's target after the last step, 0 once the cycle is over
 };
 
@@ -42,6 +43,7 @@ template <typename R, typename B = cx<R>> struct GmresStateT {
 template <typename R, typename B>
 void launch_gram_schmidt(const B* V, int64_t ldv, int64_t lds, int pass, cx<R>* w, int64_t ldw, int64_t n, c64* partial, int* done,
                          const GmresState& s, int j, cudaStream_t st, R vs);
+// V_{j+1} = w / norm rounded to a narrow basis (others are made in place and not normalised)
 template <typename R, typename B> void launch_scale(const GmresStateT<R, B>& s, int j, int64_t n, cudaStream_t st);
 void launch_hsolve(const GmresState& s, cudaStream_t st);
 template <typename R, typename B>

@@ -36,7 +36,7 @@ __device__ __forceinline__ int seg_of(const Geo& g, int64_t pos, int64_t nX, int
 // padding between segments.  The strips are written by the FFT pass.
 template <typename R>
 __global__ void __launch_bounds__(256) tail_kernel(Geo g, const cx<R>* __restrict__ x, const cx<R>* __restrict__ rhs,
-                                                   cx<R>* __restrict__ out, int64_t ld, const int* __restrict__ col_op,
+                                                   cx<R>* __restrict__ out, int64_t ld, int64_t ldo, const int* __restrict__ col_op,
                                                    const c64* __restrict__ zcap, const c64* __restrict__ zbr, int mode,
                                                    const int* __restrict__ col_list) {
     const int col = col_list ? col_list[blockIdx.z] : blockIdx.z;
@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(256) tail_kernel(Geo g, const cx<R>* __restric
     const cx<R>* xc = x + (int64_t)col * ld;
     const cx<R>* V = xc + g.off_v;
     const cx<R>* bc = rhs ? rhs + (int64_t)col * ld : nullptr;
-    cx<R>* oc = out + (int64_t)col * ld;
+    cx<R>* oc = out + (int64_t)col * ldo;
     const int part = blockIdx.y;
     auto put = [&](int64_t pos, cx<R> y) { oc[pos] = mode == 1 ? bc[pos] - y : y; };
     if (part == 0) for (int bx = blockIdx.x * RPB; bx < blockIdx.x * RPB + RPB; ++bx) {
@@ -120,10 +120,10 @@ __global__ void __launch_bounds__(256) tail_kernel(Geo g, const cx<R>* __restric
 }
 
 template <typename R>
-void launch_tail(const Geo& g, const cx<R>* x, const cx<R>* rhs, cx<R>* out, int64_t ld, int ncol, const int* col_op,
-                 const c64* zcap, const c64* zbr, int mode, const int* col_list, cudaStream_t st) {
+void launch_tail(const Geo& g, const cx<R>* x, const cx<R>* rhs, cx<R>* out, int64_t ld, int64_t ldo, int ncol,
+                 const int* col_op, const c64* zcap, const c64* zbr, int mode, const int* col_list, cudaStream_t st) {
     const dim3 grid(std::max(ceil_div((int64_t)g.nx * std::max(g.np, g.S), RPB), 1), 3, ncol);
-    tail_kernel<R><<<grid, 256, 0, st>>>(g, x, rhs, out, ld, col_op, zcap, zbr, mode, col_list);
+    tail_kernel<R><<<grid, 256, 0, st>>>(g, x, rhs, out, ld, ldo, col_op, zcap, zbr, mode, col_list);
     GT_LAUNCH_CHECK();
 }
 
@@ -150,7 +150,7 @@ template <typename R, int MAXS>
 __global__ void __launch_bounds__(256) pc_node_kernel(Geo g, const cx<R>* __restrict__ r, int64_t ld, cx<R>* __restrict__ sd,
                                                       const int* __restrict__ col_op, const cx<R>* __restrict__ tab,
                                                       const int* __restrict__ col_list, int* __restrict__ cnt,
-                                                      int64_t ncnt) {
+                                                      int64_t ncnt, const double* __restrict__ rscale) {
     for (int64_t q = ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x; q < ncnt;
          q += (int64_t)gridDim.y * gridDim.x * blockDim.x)
         cnt[q] = 0;
@@ -162,6 +162,7 @@ __global__ void __launch_bounds__(256) pc_node_kernel(Geo g, const cx<R>* __rest
     const cx<R>* X = rc + g.off_x;
     const cx<R>* Y = rc + g.off_y;
     cx<R>* sc = sd + (int64_t)col * g.nfac;
+    const R f = rscale ? R(rscale[col]) : R(1);          // (the result is linear in r)
     for (int i = blockIdx.x * RPB_NODE; i < min(nx, blockIdx.x * RPB_NODE + RPB_NODE); ++i)
     for (int j = threadIdx.x; j < ny; j += blockDim.x) {
         const int ij = i * ny + j;
@@ -236,19 +237,19 @@ __global__ void __launch_bounds__(256) pc_node_kernel(Geo g, const cx<R>* __rest
                 const cx<R> v = T[g.tab_br0 + bb] * rc[g.off_b + bb];
                 acc = bq > 0 ? acc + v : acc - v;
             }
-            sc[g.perm[node]] = rc[g.off_v + node] - acc;
+            sc[g.perm[node]] = f * (rc[g.off_v + node] - acc);
         }
     }
 }
 
 template <typename R>
 void launch_pc_node(const Geo& g, const cx<R>* r, int64_t ld, cx<R>* sd, int ncol, const int* col_op, const cx<R>* tab,
-                    const int* col_list, int* cnt, int64_t ncnt, cudaStream_t st) {
+                    const int* col_list, int* cnt, int64_t ncnt, const double* rscale, cudaStream_t st) {
     if (g.S > SHEETS_MAX) throw CudaError{cudaErrorInvalidValue, "more sheets than the stencil kernels take"};
     const dim3 grid(ceil_div(g.nx, RPB_NODE), ncol);
-    if (g.S <= 2) pc_node_kernel<R, 2><<<grid, 256, 0, st>>>(g, r, ld, sd, col_op, tab, col_list, cnt, ncnt);
-    else if (g.S <= 4) pc_node_kernel<R, 4><<<grid, 256, 0, st>>>(g, r, ld, sd, col_op, tab, col_list, cnt, ncnt);
-    else pc_node_kernel<R, 8><<<grid, 256, 0, st>>>(g, r, ld, sd, col_op, tab, col_list, cnt, ncnt);
+    if (g.S <= 2) pc_node_kernel<R, 2><<<grid, 256, 0, st>>>(g, r, ld, sd, col_op, tab, col_list, cnt, ncnt, rscale);
+    else if (g.S <= 4) pc_node_kernel<R, 4><<<grid, 256, 0, st>>>(g, r, ld, sd, col_op, tab, col_list, cnt, ncnt, rscale);
+    else pc_node_kernel<R, 8><<<grid, 256, 0, st>>>(g, r, ld, sd, col_op, tab, col_list, cnt, ncnt, rscale);
     GT_LAUNCH_CHECK();
 }
 
@@ -259,9 +260,10 @@ template <typename R, int MAXS>
 __global__ void __launch_bounds__(256) pc_strip_kernel(Geo g, const cx<R>* __restrict__ r, int64_t ldr,
                                                        const cx<R>* __restrict__ sd, cx<R>* __restrict__ out, int64_t ldo,
                                                        const int* __restrict__ col_op, const cx<R>* __restrict__ tab,
-                                                       const int* __restrict__ col_list) {
+                                                       const int* __restrict__ col_list, const double* __restrict__ rscale) {
     const int col = col_list ? col_list[blockIdx.z] : blockIdx.z;
     const int op = col_op ? col_op[col] : 0;
+    const R f = rscale ? R(rscale[col]) : R(1);
     const int S = g.S, nx = g.nx, ny = g.ny, nxy = nx * ny, NC = 1 << S;
     const cx<R>* T = tab + (int64_t)op * g.ntab;
     const cx<R>* rc = r + (int64_t)col * ldr;
@@ -283,7 +285,7 @@ __global__ void __launch_bounds__(256) pc_strip_kernel(Geo g, const cx<R>* __res
 #pragma unroll
             for (int l = 0; l < MAXS; ++l)
                 u[l] = (l < S && ((code >> l) & 1))
-                           ? rc[seg + (int64_t)l * lstride + pq] +
+                           ? f * rc[seg + (int64_t)l * lstride + pq] +
                                  (yc[g.sheet_layer[l] * nxy + na] - yc[g.sheet_layer[l] * nxy + na + dn])
                            : zero<R>();
             const int* ovr = xo ? g.ovr_x : g.ovr_y;
@@ -304,7 +306,7 @@ __global__ void __launch_bounds__(256) pc_strip_kernel(Geo g, const cx<R>* __res
             const int ij = i * ny + j;
             const int64_t pos = g.off_c + (int64_t)p * nxy + ij;
             const cx<R> y = g.cap_fill ? R(g.cap_fill[(int64_t)p * nxy + ij]) * zc : zc;
-            oc[pos] = g.mask[pos] ? y * (rc[pos] + (yc[up * nxy + ij] - yc[lo * nxy + ij])) : zero<R>();
+            oc[pos] = g.mask[pos] ? y * (f * rc[pos] + (yc[up * nxy + ij] - yc[lo * nxy + ij])) : zero<R>();
         }
     } else if (part == 3) for (int bx = blockIdx.x * RPB; bx < blockIdx.x * RPB + RPB; ++bx) {
         const int k = bx / nx, i = bx - k * nx;
@@ -323,7 +325,7 @@ __global__ void __launch_bounds__(256) pc_strip_kernel(Geo g, const cx<R>* __res
         const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
         for (int b = tid; b < g.nbr; b += nth) {
             const int64_t pos = g.off_b + b;
-            oc[pos] = g.mask[pos] ? T[g.tab_br0 + b] * (rc[pos] + (yc[g.branch_nodes[2 * b]] - yc[g.branch_nodes[2 * b + 1]]))
+            oc[pos] = g.mask[pos] ? T[g.tab_br0 + b] * (f * rc[pos] + (yc[g.branch_nodes[2 * b]] - yc[g.branch_nodes[2 * b + 1]]))
                                   : zero<R>();
         }
         for (int q = 0; q < 5; ++q)
@@ -333,12 +335,12 @@ __global__ void __launch_bounds__(256) pc_strip_kernel(Geo g, const cx<R>* __res
 
 template <typename R>
 void launch_pc_strip(const Geo& g, const cx<R>* r, int64_t ldr, const cx<R>* sd, cx<R>* out, int64_t ldo, int ncol,
-                     const int* col_op, const cx<R>* tab, const int* col_list, cudaStream_t st) {
+                     const int* col_op, const cx<R>* tab, const int* col_list, const double* rscale, cudaStream_t st) {
     if (g.S > SHEETS_MAX) throw CudaError{cudaErrorInvalidValue, "more sheets than the stencil kernels take"};
     const dim3 grid(std::max(ceil_div((int64_t)g.nx * std::max(g.np, g.S), RPB), 1), 5, ncol);
-    if (g.S <= 2) pc_strip_kernel<R, 2><<<grid, 256, 0, st>>>(g, r, ldr, sd, out, ldo, col_op, tab, col_list);
-    else if (g.S <= 4) pc_strip_kernel<R, 4><<<grid, 256, 0, st>>>(g, r, ldr, sd, out, ldo, col_op, tab, col_list);
-    else pc_strip_kernel<R, 8><<<grid, 256, 0, st>>>(g, r, ldr, sd, out, ldo, col_op, tab, col_list);
+    if (g.S <= 2) pc_strip_kernel<R, 2><<<grid, 256, 0, st>>>(g, r, ldr, sd, out, ldo, col_op, tab, col_list, rscale);
+    else if (g.S <= 4) pc_strip_kernel<R, 4><<<grid, 256, 0, st>>>(g, r, ldr, sd, out, ldo, col_op, tab, col_list, rscale);
+    else pc_strip_kernel<R, 8><<<grid, 256, 0, st>>>(g, r, ldr, sd, out, ldo, col_op, tab, col_list, rscale);
     GT_LAUNCH_CHECK();
 }
 
@@ -370,11 +372,11 @@ void launch_gather(const int64_t* c2d, int64_t ncomp, const c64* in, int64_t ldi
     GT_LAUNCH_CHECK();
 }
 
-template void launch_tail<float>(const Geo&, const c32*, const c32*, c32*, int64_t, int, const int*, const c64*, const c64*, int, const int*, cudaStream_t);
-template void launch_tail<double>(const Geo&, const c64*, const c64*, c64*, int64_t, int, const int*, const c64*, const c64*, int, const int*, cudaStream_t);
-template void launch_pc_node<float>(const Geo&, const c32*, int64_t, c32*, int, const int*, const c32*, const int*, int*, int64_t, cudaStream_t);
-template void launch_pc_node<double>(const Geo&, const c64*, int64_t, c64*, int, const int*, const c64*, const int*, int*, int64_t, cudaStream_t);
-template void launch_pc_strip<float>(const Geo&, const c32*, int64_t, const c32*, c32*, int64_t, int, const int*, const c32*, const int*, cudaStream_t);
-template void launch_pc_strip<double>(const Geo&, const c64*, int64_t, const c64*, c64*, int64_t, int, const int*, const c64*, const int*, cudaStream_t);
+template void launch_tail<float>(const Geo&, const c32*, const c32*, c32*, int64_t, int64_t, int, const int*, const c64*, const c64*, int, const int*, cudaStream_t);
+template void launch_tail<double>(const Geo&, const c64*, const c64*, c64*, int64_t, int64_t, int, const int*, const c64*, const c64*, int, const int*, cudaStream_t);
+template void launch_pc_node<float>(const Geo&, const c32*, int64_t, c32*, int, const int*, const c32*, const int*, int*, int64_t, const double*, cudaStream_t);
+template void launch_pc_node<double>(const Geo&, const c64*, int64_t, c64*, int, const int*, const c64*, const int*, int*, int64_t, const double*, cudaStream_t);
+template void launch_pc_strip<float>(const Geo&, const c32*, int64_t, const c32*, c32*, int64_t, int, const int*, const c32*, const int*, const double*, cudaStream_t);
+template void launch_pc_strip<double>(const Geo&, const c64*, int64_t, const c64*, c64*, int64_t, int, const int*, const c64*, const int*, const double*, cudaStream_t);
 
 }  // namespace gt
