@@ -226,8 +226,8 @@ struct Workspace {
     int *slot_col = nullptr, *slot_op = nullptr, *g_ptr = nullptr, *g_slot = nullptr, *g_op = nullptr, *g_pair = nullptr, *col_op = nullptr;
     int* slot_pc = nullptr;      // each slot's factorisation (the preconditioner's tables, panels and pivots)
     int* act = nullptr;
-    double* togo_host = nullptr; // [2][ncol]: GmresState::to_go after the last two steps
-    cudaEvent_t togo_ev[2] = {}; // their copies' arrival
+    double* togo_host = nullptr; // [m][ncol], pinned: GmresState::to_go after each step of the cycle, written by the GPU
+    cudaEvent_t togo_ev[2] = {}; // after the even and the odd steps' kernels
     int* done = nullptr;         // per slot, for the reductions' last blocks
     // outer GCR: directions P (corrections) and Q = K P, per column, k-major; step sizes; active columns
     int kmax = 0;
@@ -840,7 +840,6 @@ static void fill_ws(Workspace& W, gt_geometry* G, int ncol, int m, int prec, int
     s.eta = p.alloc<double>(ncol);
     s.inv_hn = p.alloc<double>(ncol);
     s.vinv = p.alloc<double>((size_t)ncol * (m + 1));
-    s.to_go = p.alloc<double>(ncol);
     W.slot_col = p.alloc<int>(ncol);
     W.slot_op = p.alloc<int>(ncol);
     W.slot_pc = p.alloc<int>(ncol);
@@ -852,7 +851,7 @@ static void fill_ws(Workspace& W, gt_geometry* G, int ncol, int m, int prec, int
     W.done = p.alloc<int>(ncol);
     if (!dry) {
         GT_CUDA(cudaMemsetAsync(W.done, 0, ncol * sizeof(int), st));
-        GT_CUDA(cudaMallocHost(&W.togo_host, 2 * ncol * sizeof(double)));
+        GT_CUDA(cudaMallocHost(&W.togo_host, (size_t)m * ncol * sizeof(double)));
         for (cudaEvent_t& e : W.togo_ev) GT_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
     W.gP = p.alloc<c64>((size_t)kmax * ncol * n);
@@ -1004,10 +1003,13 @@ static int solve_impl(gt_geometry* G, gt_operators* ops, int ncol, const int* h_
             launch_init_cycle<R, B>(ST, W.r64, n, W.slot_col, W.rho, n, st);
         }
         const double* vinv = narrow ? nullptr : S.vinv;
+        // (the GPU is done with the cycle before: its outcome has been read)
+        std::fill(W.togo_host, W.togo_host + (size_t)m * W.ncol, 0.0);
         int jdone = 0;
         constexpr double FAR = 8;
         double togo = 2 * FAR;       // the slowest slot's, as last seen
         for (int j = 0; j < m; ++j) {
+            S.to_go = W.togo_host + (size_t)j * W.ncol;
             // the products run on the slots still iterating in this cycle (W.act, grp)
             const int na = (int)act.size();
             // The product is applied to the basis vector as stored.  A basis of the arithmetic's type is made in place, the
@@ -1051,7 +1053,6 @@ static int solve_impl(gt_geometry* G, gt_operators* ops, int ncol, const int* h_
                     launch_scale<R, B>(ST, j, n, st);
                 }
             }
-            GT_CUDA(cudaMemcpyAsync(W.togo_host + (j & 1) * W.ncol, S.to_go, ns * sizeof(double), cudaMemcpyDeviceToHost, st));
             GT_CUDA(cudaEventRecord(W.togo_ev[j & 1], st));
             jdone = j + 1;
             // which slots go on.  While the slowest is far from its target (a step gains a factor of two or so) this step's
@@ -1061,7 +1062,7 @@ static int solve_impl(gt_geometry* G, gt_operators* ops, int ncol, const int* h_
             const int seen = togo > FAR ? j - 1 : j;
             if (seen < 0) continue;
             GT_CUDA(cudaEventSynchronize(W.togo_ev[seen & 1]));
-            const double* left = W.togo_host + (seen & 1) * W.ncol;
+            const double* left = W.togo_host + (size_t)seen * W.ncol;
             std::vector<int> still;
             togo = 0;
             for (int q : act)

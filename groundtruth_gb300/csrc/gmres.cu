@@ -62,6 +62,7 @@ __global__ void __launch_bounds__(DOT_THREADS) dots_kernel(const B* __restrict__
                                                            const int* __restrict__ active, c64* __restrict__ partial,
                                                            int nchunk, int vpb, R vs, const double* __restrict__ vinv, int ldi,
                                                            c64* __restrict__ out, int ldo, int* done) {
+    pdl_enter();
     __shared__ c64 red[DOT_THREADS / 32][MAXV + 1];
     const int slot = blockIdx.y;
     if (active && !active[slot]) return;
@@ -139,7 +140,7 @@ void launch_dots(const B* V, int64_t ldv, int64_t lds, int nv, const cx<R>* w, i
     // the same however the vectors are dealt out.
     const int groups = std::max(1, std::min((nv + 1) / 2, 456 / (nchunk * nslot)));
     const int vpb = std::max(2, (ceil_div(nv, groups) + 1) / 2 * 2);
-    dots_kernel<R, B><<<dim3(nchunk, nslot, std::max(1, ceil_div(nv, vpb))), DOT_THREADS, 0, st>>>(
+    pdl_launch(dots_kernel<R, B>, dim3(nchunk, nslot, std::max(1, ceil_div(nv, vpb))), DOT_THREADS, 0, st, 
         V, ldv, lds, nv, w, ldw, n, active, partial, nchunk, vpb, vs, vinv, ldi, out, ldo, done);
     GT_LAUNCH_CHECK();
 }
@@ -216,7 +217,7 @@ __device__ void givens_column(const GmresState& s, int j, int slot, bool re, dou
     s.vinv[(int64_t)slot * (m + 1) + j + 1] = inv;
     const bool over = res <= s.eta[slot] || breakdown || j + 1 >= m || total >= s.max_its;
     if (over) s.active[slot] = s.reorth[slot] = 0;       // (no second pass on a later step either)
-    s.to_go[slot] = over ? 0.0 : res / s.eta[slot];
+    if (!over) s.to_go[slot] = res / s.eta[slot];
 }
 
 // w += sign * sum_i h_i V_i (sign -1: Gram-Schmidt; +1: the cycle's combination); partial |w|^2 per chunk of
@@ -230,6 +231,7 @@ __global__ void __launch_bounds__(DOT_THREADS) update_kernel(const B* __restrict
                                                              const int* __restrict__ active, c64* __restrict__ partial,
                                                              int nchunk, int sign, R vs, const double* __restrict__ vinv, int ldi,
                                                              int tail, c64* __restrict__ out, int* done, GmresState s, int j) {
+    pdl_enter();
     __shared__ cx<R> hs[MAXV + 16];
     __shared__ double red[DOT_THREADS / 32];
     __shared__ c64 gv[3 * (MAXV + 1)];
@@ -312,7 +314,7 @@ static void update_launch(const B* V, int64_t ldv, int64_t lds, int nv, const c6
                           int nslot, const int* active, c64* partial, int sign, R vs, const double* vinv, int ldi, int tail, c64* out, int* done,
                           const GmresState& s, int j, cudaStream_t st) {
     const int nchunk = update_chunks(n);
-    update_kernel<R, B><<<dim3(nchunk, nslot), DOT_THREADS, 0, st>>>(V, ldv, lds, nv, h, ldh, w, ldw, n, active,
+    pdl_launch(update_kernel<R, B>, dim3(nchunk, nslot), DOT_THREADS, 0, st, V, ldv, lds, nv, h, ldh, w, ldw, n, active,
                                                                       partial, nchunk, sign, vs, vinv, ldi, tail, out, done, s, j);
     GT_LAUNCH_CHECK();
 }
@@ -360,6 +362,7 @@ __device__ __forceinline__ void put_basis(const GmresStateT<R, B>& s, B* p, cx<R
 // the next vector of a narrow basis: w normalised and rounded
 template <typename R, typename B>
 __global__ void scale_kernel(GmresStateT<R, B> s, int j, int64_t n) {
+    pdl_enter();
     const int slot = blockIdx.y;
     if (!s.active[slot]) return;
     const R f = R(s.inv_hn[slot]);
@@ -462,6 +465,7 @@ __global__ void to64_kernel(c64* __restrict__ dst, int64_t ldd, const cx<R>* __r
 template <typename D, typename S>
 __global__ void recast_kernel(cx<D>* __restrict__ dst, int64_t ldd, const cx<S>* __restrict__ src, int64_t lds,
                               const int* __restrict__ list, int64_t n, const double* __restrict__ scale) {
+    pdl_enter();
     const int c = list ? list[blockIdx.y] : (int)blockIdx.y;
     const double f = scale ? scale[c] : 1.0;
     cx<D>* d = dst + (int64_t)c * ldd;
@@ -500,7 +504,7 @@ void launch_recast(cx<D>* dst, int64_t ldd, const cx<S>* src, int64_t lds, const
                    const double* scale, cudaStream_t st) {
     if (nslot <= 0) return;
     int blocks = (int)std::min<int64_t>((n + 255) / 256, 1024);
-    recast_kernel<D, S><<<dim3(blocks, nslot), 256, 0, st>>>(dst, ldd, src, lds, list, n, scale);
+    pdl_launch(recast_kernel<D, S>, dim3(blocks, nslot), 256, 0, st, dst, ldd, src, lds, list, n, scale);
     GT_LAUNCH_CHECK();
 }
 template void launch_recast<double, float>(c64*, int64_t, const c32*, int64_t, const int*, int64_t, int, const double*, cudaStream_t);
@@ -516,7 +520,7 @@ void launch_gcr_scale(c64* p, c64* q, int64_t ld, const c64* nu2, const int* act
 template <typename R, typename B>
 void launch_scale(const GmresStateT<R, B>& s, int j, int64_t n, cudaStream_t st) {
     int blocks = (int)std::min<int64_t>((n + 255) / 256, 1024);
-    scale_kernel<R, B><<<dim3(blocks, s.nslot), 256, 0, st>>>(s, j, n);
+    pdl_launch(scale_kernel<R, B>, dim3(blocks, s.nslot), 256, 0, st, s, j, n);
     GT_LAUNCH_CHECK();
 }
 void launch_hsolve(const GmresState& s, cudaStream_t st) {

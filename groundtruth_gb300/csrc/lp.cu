@@ -32,6 +32,7 @@ template <typename R, int PL>
 __global__ void __launch_bounds__(1024) lp_pass_a(const cx<R>* __restrict__ x, int64_t ldx, int64_t off, int S, int n0, int n1, int P1,
                           int rows, const cx<R>* __restrict__ tw, cx<R>* __restrict__ T, const int* __restrict__ col_list,
                           int ldt) {
+    pdl_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cx<R>* buf = reinterpret_cast<cx<R>*>(smem_raw);
     const int P = PL ? PL : P1;                  // compile-time when specialised
@@ -66,6 +67,7 @@ template <typename R, int PL> __host__ __device__ constexpr int lp_threads() { r
 template <typename R, int PL>
 __global__ void __launch_bounds__(lp_threads<R, PL>()) lp_pass_b(int S, int n0, int P0, int P1, int ncol, int bt, const R* __restrict__ spec,
                           const cx<R>* __restrict__ tw, cx<R>* __restrict__ T, int ldt) {
+    pdl_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cx<R>* buf = reinterpret_cast<cx<R>*>(smem_raw);
     const int P = PL ? PL : P0;                  // compile-time when specialised
@@ -174,6 +176,7 @@ __device__ __forceinline__ int b8_stages(cx<R>* b0, cx<R>* b1, int cur, int t, c
 template <typename R, int P, int S>
 __global__ void __launch_bounds__(512) lp_pass_b8(int n0, int P1, int ncol, int bt, const R* __restrict__ spec,
                                                   const cx<R>* __restrict__ tw, cx<R>* __restrict__ T, int ldt) {
+    pdl_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int TEAM = P / 8, NBF = P / 8, ST = lp_srow(P), Q0 = P / 2 + 1;
     const int c = blockIdx.x;
@@ -286,6 +289,7 @@ constexpr int BW_WARPS = 4;
 template <int S>
 __global__ void __launch_bounds__(BW_WARPS * 32, GT_BW_MINB) lp_pass_bw(int n0, int P1, int ncol, const float* __restrict__ spec,
                                                             const c32* __restrict__ tw, c32* __restrict__ T, int ldt) {
+    pdl_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int P = 512, Q0 = P / 2 + 1, CPW = S == 2 ? 1 : 2;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -351,6 +355,7 @@ __global__ void __launch_bounds__(BW_WARPS * 32, GT_BW_MINB) lp_pass_bw(int n0, 
 template <int A>
 __global__ void __launch_bounds__(256, 2) lp_pass_bg(int S, int n0, int P1, int ncol, int bt, const float* __restrict__ spec,
                                                      const c32* __restrict__ tw, c32* __restrict__ T, int ldt) {
+    pdl_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int N = 32 * A, Q0 = N / 2 + 1, RR = WarpFft<A>::RR, H = WarpFft<A>::H, RS = A * 33;
     c32* Z = reinterpret_cast<c32*>(smem_raw);           // [row][k1 * 33 + k2], pixel k1 + A k2
@@ -446,6 +451,7 @@ constexpr size_t RW_SMEM = (size_t)(RW_WARPS * WX_SLOTS > 512 * RW_TS ? RW_WARPS
 __global__ void __launch_bounds__(RW_WARPS * 32, GT_RW_MINB) lp_pass_aw(const c32* __restrict__ x, int64_t ldx, int64_t off, int S,
                                                                int n0, int n1, int ldt, const c32* __restrict__ tw,
                                                                c32* __restrict__ T, const int* __restrict__ col_list) {
+    pdl_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     c32* sm = reinterpret_cast<c32*>(smem_raw);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -502,6 +508,7 @@ __global__ void __launch_bounds__(CW_WARPS * 32, GT_CW_MINB) lp_pass_cw(const c3
                                                                const double* __restrict__ omega, const c64* __restrict__ zs,
                                                                int mode, const int* __restrict__ col_list,
                                                                const int* __restrict__ sheet_layer) {
+    pdl_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     c32* sm = reinterpret_cast<c32*>(smem_raw);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -608,6 +615,7 @@ __global__ void __launch_bounds__(CT_WARPS * 32, GT_RW_MINB) lp_pass_ct(const __
                                                                 int mode, const int* __restrict__ col_list,
                                                                 const int* __restrict__ sheet_layer,
                                                                 uint32_t missing_bytes, uint64_t wait_ns) {
+    pdl_enter();
     // missing_bytes: 0, except when a test makes the wait run out (the barrier then expects bytes no load
     // brings; the loads themselves are the usual two)
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -729,6 +737,7 @@ template <typename R, int P>
 __global__ void __launch_bounds__(1024) lp_pass_a8(const cx<R>* __restrict__ x, int64_t ldx, int64_t off, int S, int n0,
                                                    int n1, int rows, const cx<R>* __restrict__ tw, cx<R>* __restrict__ T,
                                                    const int* __restrict__ col_list, int ldt) {
+    pdl_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int TEAM = P / 8, NBF = P / 8, ST = lp_srow(P);
     cx<R>* buf = reinterpret_cast<cx<R>*>(smem_raw);
@@ -787,6 +796,7 @@ __global__ void __launch_bounds__(1024) lp_pass_c8(const cx<R>* __restrict__ T, 
                                                    const double* __restrict__ omega, const c64* __restrict__ zs, int mode,
                                                    const int* __restrict__ col_list, const int* __restrict__ sheet_layer,
                                                    int ldt) {
+    pdl_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int TEAM = P / 8, NBF = P / 8, ST = lp_srow(P);
     cx<R>* buf = reinterpret_cast<cx<R>*>(smem_raw);
@@ -870,6 +880,7 @@ __global__ void __launch_bounds__(1024) lp_pass_c(const cx<R>* __restrict__ T, c
                           const uint8_t* __restrict__ mask, const int* __restrict__ col_op,
                           const double* __restrict__ omega, const c64* __restrict__ zs, int mode,
                           const int* __restrict__ col_list, const int* __restrict__ sheet_layer, int ldt) {
+    pdl_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cx<R>* buf = reinterpret_cast<cx<R>*>(smem_raw);
     const int P = PL ? PL : P1;                  // compile-time when specialised
@@ -951,7 +962,7 @@ static void launch_a(const LpArgs<R>& a, int rows, cudaStream_t st) {
     if constexpr (PA == 512 && std::is_same<R, float>::value) {
         if (rw_fits(a)) {
             set_smem<float>((const void*)lp_pass_aw, RW_SMEM);
-            lp_pass_aw<<<dim3(ceil_div(a.n0, RW_ROWS), a.S, a.ncol), RW_WARPS * 32, RW_SMEM, st>>>(
+            pdl_launch(lp_pass_aw, dim3(ceil_div(a.n0, RW_ROWS), a.S, a.ncol), RW_WARPS * 32, RW_SMEM, st, 
                 a.x, a.ld, a.off, a.S, a.n0, a.n1, a.ldt, a.tw1, a.T, a.col_list);
             GT_LAUNCH_CHECK();
             return;
@@ -960,7 +971,7 @@ static void launch_a(const LpArgs<R>& a, int rows, cudaStream_t st) {
     if constexpr (PA == 64 || PA == 512) {
         const size_t sm = (size_t)2 * rows * lp_srow(PA) * sizeof(cx<R>);
         set_smem<R>((const void*)lp_pass_a8<R, PA>, sm);
-        lp_pass_a8<R, PA><<<dim3(ceil_div(a.n0, rows), a.S, a.ncol), rows * (PA / 8), sm, st>>>(
+        pdl_launch(lp_pass_a8<R, PA>, dim3(ceil_div(a.n0, rows), a.S, a.ncol), rows * (PA / 8), sm, st, 
             a.x, a.ld, a.off, a.S, a.n0, a.n1, rows, a.tw1, a.T, a.col_list, ldt_of(a));
         GT_LAUNCH_CHECK();
         return;
@@ -968,7 +979,7 @@ static void launch_a(const LpArgs<R>& a, int rows, cudaStream_t st) {
     size_t smA = (size_t)rows * srow(a.P1) * sizeof(cx<R>);
     dim3 gA(ceil_div(a.n0, rows), a.S, a.ncol);
     set_smem<R>((const void*)lp_pass_a<R, PA>, smA);
-    lp_pass_a<R, PA><<<gA, rows * (a.P1 / 8), smA, st>>>(a.x, a.ld, a.off, a.S, a.n0, a.n1, a.P1, rows, a.tw1, a.T,
+    pdl_launch(lp_pass_a<R, PA>, gA, rows * (a.P1 / 8), smA, st, a.x, a.ld, a.off, a.S, a.n0, a.n1, a.P1, rows, a.tw1, a.T,
                                                           a.col_list, ldt_of(a));
     GT_LAUNCH_CHECK();
 }
@@ -977,7 +988,7 @@ template <typename R, int P, int S>
 static void launch_b8(const LpArgs<R>& a, int bt, cudaStream_t st) {
     const size_t sm = (size_t)2 * bt * S * lp_srow(P) * sizeof(cx<R>);
     set_smem<R>((const void*)lp_pass_b8<R, P, S>, sm);
-    lp_pass_b8<R, P, S><<<dim3(a.P1, ceil_div(a.ncol, bt)), bt * (P / 8), sm, st>>>(a.n0, a.P1, a.ncol, bt, a.spec, a.tw0,
+    pdl_launch(lp_pass_b8<R, P, S>, dim3(a.P1, ceil_div(a.ncol, bt)), bt * (P / 8), sm, st, a.n0, a.P1, a.ncol, bt, a.spec, a.tw0,
                                                                                   a.T, ldt_of(a));
     GT_LAUNCH_CHECK();
 }
@@ -990,7 +1001,7 @@ static void launch_bw(const LpArgs<float>& a, cudaStream_t st) {
     constexpr int CPW = S == 2 ? 1 : 2;
     const size_t sm = (size_t)BW_WARPS * WX_SLOTS * sizeof(c32);
     set_smem<float>((const void*)lp_pass_bw<S>, sm);
-    lp_pass_bw<S><<<dim3(a.P1, ceil_div(a.ncol, BW_WARPS * CPW)), BW_WARPS * 32, sm, st>>>(a.n0, a.P1, a.ncol, a.spec,
+    pdl_launch(lp_pass_bw<S>, dim3(a.P1, ceil_div(a.ncol, BW_WARPS * CPW)), BW_WARPS * 32, sm, st, a.n0, a.P1, a.ncol, a.spec,
                                                                                          a.tw0, a.T, ldt_of(a));
     GT_LAUNCH_CHECK();
 }
@@ -1002,7 +1013,7 @@ static void launch_bg(const LpArgs<float>& a, cudaStream_t st) {
     const int warps = ceil_div(bt * a.S, RR);
     const size_t sm = (size_t)warps * WarpFft<A>::SLOTS * sizeof(c32) + (size_t)(16 * A + 1) * ((a.S * a.S) | 1) * sizeof(float);
     set_smem<float>((const void*)lp_pass_bg<A>, sm);
-    lp_pass_bg<A><<<dim3(a.P1, ceil_div(a.ncol, bt)), warps * 32, sm, st>>>(a.S, a.n0, a.P1, a.ncol, bt, a.spec, a.tw0, a.T,
+    pdl_launch(lp_pass_bg<A>, dim3(a.P1, ceil_div(a.ncol, bt)), warps * 32, sm, st, a.S, a.n0, a.P1, a.ncol, bt, a.spec, a.tw0, a.T,
                                                                           ldt_of(a));
     GT_LAUNCH_CHECK();
 }
@@ -1033,7 +1044,7 @@ static void launch_b(const LpArgs<R>& a, int bt, cudaStream_t st) {
         dim3 gB(a.P1, ceil_div(a.ncol, bt));
         const int team = a.P0 / 8, threads = std::min(bt * a.S, lp_threads<R, PB>() / team) * team;
         set_smem<R>((const void*)lp_pass_b<R, PB>, smB);
-        lp_pass_b<R, PB><<<gB, threads, smB, st>>>(a.S, a.n0, a.P0, a.P1, a.ncol, bt, a.spec, a.tw0, a.T, ldt_of(a));
+        pdl_launch(lp_pass_b<R, PB>, gB, threads, smB, st, a.S, a.n0, a.P0, a.P1, a.ncol, bt, a.spec, a.tw0, a.T, ldt_of(a));
         GT_LAUNCH_CHECK();
     }
 }
@@ -1084,7 +1095,7 @@ static void launch_c(const LpArgs<R>& a, int rows, cudaStream_t st) {
             const char* t = std::getenv("GT_LP_TMA_TEST_SHORTFALL");
             const bool shortfall = t && t[0] == '1';
             set_smem<float>((const void*)lp_pass_ct, CT_SMEM);
-            lp_pass_ct<<<dim3(ceil_div(a.n0, 16), a.S, a.ncol), CT_WARPS * 32, CT_SMEM, st>>>(
+            pdl_launch(lp_pass_ct, dim3(ceil_div(a.n0, 16), a.S, a.ncol), CT_WARPS * 32, CT_SMEM, st, 
                 m, a.x, a.rhs, a.out, a.ld, a.ldo, a.off, a.off_v, a.S, a.n0, a.n1, a.nx, a.ny, a.di, a.dj, a.tw1, a.mask,
                 a.col_op, a.omega, a.zs, a.mode, a.col_list, a.sheet_layer, shortfall ? 16u : 0u,
                 shortfall ? 1000000ull : CT_WAIT_NS);
@@ -1093,7 +1104,7 @@ static void launch_c(const LpArgs<R>& a, int rows, cudaStream_t st) {
         }
         if (rw_fits(a)) {
             set_smem<float>((const void*)lp_pass_cw, CW_SMEM);
-            lp_pass_cw<<<dim3(ceil_div(a.n0, 2 * CW_WARPS), a.S, a.ncol), CW_WARPS * 32, CW_SMEM, st>>>(
+            pdl_launch(lp_pass_cw, dim3(ceil_div(a.n0, 2 * CW_WARPS), a.S, a.ncol), CW_WARPS * 32, CW_SMEM, st, 
                 a.T, a.x, a.rhs, a.out, a.ld, a.ldo, a.off, a.off_v, a.S, a.n0, a.n1, a.nx, a.ny, a.di, a.dj, a.ldt, a.tw1,
                 a.mask, a.col_op, a.omega, a.zs, a.mode, a.col_list, a.sheet_layer);
             GT_LAUNCH_CHECK();
@@ -1103,7 +1114,7 @@ static void launch_c(const LpArgs<R>& a, int rows, cudaStream_t st) {
     if constexpr (PA == 64 || PA == 512) {
         const size_t sm = (size_t)2 * rows * lp_srow(PA) * sizeof(cx<R>);
         set_smem<R>((const void*)lp_pass_c8<R, PA>, sm);
-        lp_pass_c8<R, PA><<<dim3(ceil_div(a.n0, rows), a.S, a.ncol), rows * (PA / 8), sm, st>>>(
+        pdl_launch(lp_pass_c8<R, PA>, dim3(ceil_div(a.n0, rows), a.S, a.ncol), rows * (PA / 8), sm, st, 
             a.T, a.x, a.rhs, a.out, a.ld, a.ldo, a.off, a.off_v, a.S, a.n0, a.n1, a.nx, a.ny, a.di, a.dj, rows, a.tw1, a.mask,
             a.col_op, a.omega, a.zs, a.mode, a.col_list, a.sheet_layer, ldt_of(a));
         GT_LAUNCH_CHECK();
@@ -1112,7 +1123,7 @@ static void launch_c(const LpArgs<R>& a, int rows, cudaStream_t st) {
     size_t smA = (size_t)rows * srow(a.P1) * sizeof(cx<R>);
     dim3 gA(ceil_div(a.n0, rows), a.S, a.ncol);
     set_smem<R>((const void*)lp_pass_c<R, PA>, smA);
-    lp_pass_c<R, PA><<<gA, rows * (a.P1 / 8), smA, st>>>(a.T, a.x, a.rhs, a.out, a.ld, a.ldo, a.off, a.off_v, a.S, a.n0, a.n1,
+    pdl_launch(lp_pass_c<R, PA>, gA, rows * (a.P1 / 8), smA, st, a.T, a.x, a.rhs, a.out, a.ld, a.ldo, a.off, a.off_v, a.S, a.n0, a.n1,
                                                           a.nx, a.ny, a.di, a.dj, a.P1, rows, a.tw1, a.mask, a.col_op,
                                                           a.omega, a.zs, a.mode, a.col_list, a.sheet_layer, ldt_of(a));
     GT_LAUNCH_CHECK();

@@ -17,6 +17,7 @@ __global__ void __launch_bounds__(128) narrow_kernel(Narrow nw, const cx<R>* __r
                                                     const double* __restrict__ omega, const c64* __restrict__ zs,
                                                     const c64* __restrict__ zmut, int mode,
                                                     const int* __restrict__ col_list) {
+    pdl_enter();
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= nw.nrow) return;
     const int col = col_list ? col_list[blockIdx.y] : blockIdx.y;
@@ -47,7 +48,7 @@ void launch_narrow(const Narrow& nw, const cx<R>* x, cx<R>* out, int64_t ld, int
                    const double* omega, const c64* zs, const c64* zmut, int mode, const int* col_list,
                    cudaStream_t st) {
     if (nw.nrow == 0 || ncol < 1) return;
-    narrow_kernel<R><<<dim3((unsigned)((nw.nrow + 127) / 128), ncol), 128, 0, st>>>(nw, x, out, ld, ldo, S, col_op, omega,
+    pdl_launch(narrow_kernel<R>, dim3((unsigned)((nw.nrow + 127) / 128), ncol), 128, 0, st, nw, x, out, ld, ldo, S, col_op, omega,
                                                                                    zs, zmut, mode, col_list);
     GT_LAUNCH_CHECK();
 }

@@ -23,7 +23,8 @@ struct GmresState {
     double* eta;       // [slot] the cycle's relative target
     double* inv_hn;    // [slot] 1 / norm of the newest basis vector, which is stored as the last step left it (1 for the cycle's first)
     double* vinv;      // [slot][m+1] the same of all of them (a narrow basis is stored normalised and has none)
-    double* to_go;     // [slot] the residual estimate over the cycle's target after the last step, 0 once the cycle is over
+    double* to_go;     // [slot] pinned host memory: the residual estimate over the cycle's target after this step, left at 0
+                       // for a slot whose cycle is over
 };
 
 template <typename R, typename B = cx<R>> struct GmresStateT {

@@ -39,6 +39,7 @@ __global__ void __launch_bounds__(256) tail_kernel(Geo g, const cx<R>* __restric
                                                    cx<R>* __restrict__ out, int64_t ld, int64_t ldo, const int* __restrict__ col_op,
                                                    const c64* __restrict__ zcap, const c64* __restrict__ zbr, int mode,
                                                    const int* __restrict__ col_list) {
+    pdl_enter();
     const int col = col_list ? col_list[blockIdx.z] : blockIdx.z;
     const int op = col_op ? col_op[col] : 0;
     const int S = g.S, nx = g.nx, ny = g.ny, nxy = nx * ny;
@@ -123,7 +124,7 @@ template <typename R>
 void launch_tail(const Geo& g, const cx<R>* x, const cx<R>* rhs, cx<R>* out, int64_t ld, int64_t ldo, int ncol,
                  const int* col_op, const c64* zcap, const c64* zbr, int mode, const int* col_list, cudaStream_t st) {
     const dim3 grid(std::max(ceil_div((int64_t)g.nx * std::max(g.np, g.S), RPB), 1), 3, ncol);
-    tail_kernel<R><<<grid, 256, 0, st>>>(g, x, rhs, out, ld, ldo, col_op, zcap, zbr, mode, col_list);
+    pdl_launch(tail_kernel<R>, grid, 256, 0, st, g, x, rhs, out, ld, ldo, col_op, zcap, zbr, mode, col_list);
     GT_LAUNCH_CHECK();
 }
 
@@ -151,6 +152,7 @@ __global__ void __launch_bounds__(256) pc_node_kernel(Geo g, const cx<R>* __rest
                                                       const int* __restrict__ col_op, const cx<R>* __restrict__ tab,
                                                       const int* __restrict__ col_list, int* __restrict__ cnt,
                                                       int64_t ncnt, const double* __restrict__ rscale) {
+    pdl_enter();
     for (int64_t q = ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x; q < ncnt;
          q += (int64_t)gridDim.y * gridDim.x * blockDim.x)
         cnt[q] = 0;
@@ -247,9 +249,9 @@ void launch_pc_node(const Geo& g, const cx<R>* r, int64_t ld, cx<R>* sd, int nco
                     const int* col_list, int* cnt, int64_t ncnt, const double* rscale, cudaStream_t st) {
     if (g.S > SHEETS_MAX) throw CudaError{cudaErrorInvalidValue, "more sheets than the stencil kernels take"};
     const dim3 grid(ceil_div(g.nx, RPB_NODE), ncol);
-    if (g.S <= 2) pc_node_kernel<R, 2><<<grid, 256, 0, st>>>(g, r, ld, sd, col_op, tab, col_list, cnt, ncnt, rscale);
-    else if (g.S <= 4) pc_node_kernel<R, 4><<<grid, 256, 0, st>>>(g, r, ld, sd, col_op, tab, col_list, cnt, ncnt, rscale);
-    else pc_node_kernel<R, 8><<<grid, 256, 0, st>>>(g, r, ld, sd, col_op, tab, col_list, cnt, ncnt, rscale);
+    if (g.S <= 2) pdl_launch(pc_node_kernel<R, 2>, grid, 256, 0, st, g, r, ld, sd, col_op, tab, col_list, cnt, ncnt, rscale);
+    else if (g.S <= 4) pdl_launch(pc_node_kernel<R, 4>, grid, 256, 0, st, g, r, ld, sd, col_op, tab, col_list, cnt, ncnt, rscale);
+    else pdl_launch(pc_node_kernel<R, 8>, grid, 256, 0, st, g, r, ld, sd, col_op, tab, col_list, cnt, ncnt, rscale);
     GT_LAUNCH_CHECK();
 }
 
@@ -261,6 +263,7 @@ __global__ void __launch_bounds__(256) pc_strip_kernel(Geo g, const cx<R>* __res
                                                        const cx<R>* __restrict__ sd, cx<R>* __restrict__ out, int64_t ldo,
                                                        const int* __restrict__ col_op, const cx<R>* __restrict__ tab,
                                                        const int* __restrict__ col_list, const double* __restrict__ rscale) {
+    pdl_enter();
     const int col = col_list ? col_list[blockIdx.z] : blockIdx.z;
     const int op = col_op ? col_op[col] : 0;
     const R f = rscale ? R(rscale[col]) : R(1);
@@ -338,9 +341,9 @@ void launch_pc_strip(const Geo& g, const cx<R>* r, int64_t ldr, const cx<R>* sd,
                      const int* col_op, const cx<R>* tab, const int* col_list, const double* rscale, cudaStream_t st) {
     if (g.S > SHEETS_MAX) throw CudaError{cudaErrorInvalidValue, "more sheets than the stencil kernels take"};
     const dim3 grid(std::max(ceil_div((int64_t)g.nx * std::max(g.np, g.S), RPB), 1), 5, ncol);
-    if (g.S <= 2) pc_strip_kernel<R, 2><<<grid, 256, 0, st>>>(g, r, ldr, sd, out, ldo, col_op, tab, col_list, rscale);
-    else if (g.S <= 4) pc_strip_kernel<R, 4><<<grid, 256, 0, st>>>(g, r, ldr, sd, out, ldo, col_op, tab, col_list, rscale);
-    else pc_strip_kernel<R, 8><<<grid, 256, 0, st>>>(g, r, ldr, sd, out, ldo, col_op, tab, col_list, rscale);
+    if (g.S <= 2) pdl_launch(pc_strip_kernel<R, 2>, grid, 256, 0, st, g, r, ldr, sd, out, ldo, col_op, tab, col_list, rscale);
+    else if (g.S <= 4) pdl_launch(pc_strip_kernel<R, 4>, grid, 256, 0, st, g, r, ldr, sd, out, ldo, col_op, tab, col_list, rscale);
+    else pdl_launch(pc_strip_kernel<R, 8>, grid, 256, 0, st, g, r, ldr, sd, out, ldo, col_op, tab, col_list, rscale);
     GT_LAUNCH_CHECK();
 }
 

@@ -312,6 +312,7 @@ __device__ void sw_task(const SwArgs& A, SwShared& sm, uint32_t& it, const SwDes
 }
 
 __global__ void __launch_bounds__(SW_BLOCK, 4) sweep_kernel(SwArgs A) {
+    pdl_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SwShared& sm = *reinterpret_cast<SwShared*>(smem_raw);
     if (threadIdx.x == 0) {
@@ -439,7 +440,7 @@ void launch_sweep(const SweepPlan& S, const Fronts& F, const c32* pf, const c32*
     const int64_t tickets = (int64_t)(t1 - t0) * G.ngroup;
     if (tickets <= 0) return;
     raise_smem((const void*)sweep_kernel, sizeof(SwShared));
-    sweep_kernel<<<(int)std::min<int64_t>(tickets, resident_blocks()), SW_BLOCK, sizeof(SwShared), st>>>(A);
+    pdl_launch(sweep_kernel, (int)std::min<int64_t>(tickets, resident_blocks()), SW_BLOCK, sizeof(SwShared), st, A);
     GT_LAUNCH_CHECK();
 }
 

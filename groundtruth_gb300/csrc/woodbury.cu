@@ -19,6 +19,7 @@ __global__ void __launch_bounds__(LOWRANK_MAX) lowrank_coef_kernel(const cx<R>* 
                                                                     const int* __restrict__ col_fact,
                                                                     const int* __restrict__ col_list,
                                                                     cx<R>* __restrict__ cbuf, int64_t ldc) {
+    pdl_enter();
     __shared__ cx<R> t[LOWRANK_MAX];
     const int col = col_list ? col_list[blockIdx.x] : blockIdx.x;
     const int f = col_fact[col];
@@ -41,6 +42,7 @@ __global__ void __launch_bounds__(256) lowrank_apply_kernel(cx<R>* __restrict__ 
                                                             const int* __restrict__ col_fact,
                                                             const int* __restrict__ col_list,
                                                             const cx<R>* __restrict__ cbuf, int64_t ldc) {
+    pdl_enter();
     __shared__ cx<R> c[LOWRANK_MAX];
     const int col = col_list ? col_list[blockIdx.y] : blockIdx.y;
     const int f = col_fact[col];
@@ -59,10 +61,10 @@ template <typename R>
 void launch_lowrank(cx<R>* sd, int64_t nnode, int ncol, int k, const int* ends, const cx<R>* w, const cx<R>* minv,
                     const int* col_fact, const int* col_list, cx<R>* cbuf, int64_t ldc, cudaStream_t st) {
     if (k < 1 || k > LOWRANK_MAX || ncol < 1) return;
-    lowrank_coef_kernel<R><<<ncol, LOWRANK_MAX, 0, st>>>(sd, nnode, k, ends, minv, col_fact, col_list, cbuf, ldc);
+    pdl_launch(lowrank_coef_kernel<R>, ncol, LOWRANK_MAX, 0, st, sd, nnode, k, ends, minv, col_fact, col_list, cbuf, ldc);
     GT_LAUNCH_CHECK();
     const int chunks = (int)std::min<int64_t>((nnode + 255) / 256, 304);
-    lowrank_apply_kernel<R><<<dim3(chunks, ncol), 256, 0, st>>>(sd, nnode, k, w, col_fact, col_list, cbuf, ldc);
+    pdl_launch(lowrank_apply_kernel<R>, dim3(chunks, ncol), 256, 0, st, sd, nnode, k, w, col_fact, col_list, cbuf, ldc);
     GT_LAUNCH_CHECK();
 }
 
