@@ -167,6 +167,47 @@ __device__ __forceinline__ int sw_slot(int row2, int e) {
     return row2 * 2 * NP + (e ^ ((row2 / (4 / NP)) & (2 * NP - 1)));
 }
 
+// out[row][pair] = the right-hand sides (OWN) plus the children's updates of the front's rows row0 + r, r0 <= r < r1, in the
+// children's order.  The row indices, then the values, of GA entries per thread are loaded together: an entry at a time,
+// the three dependent loads of each were most of a tile's time near the root.
+constexpr int GA = 4;
+template <int NP, bool OWN>
+__device__ __forceinline__ void sw_gather(const SwArgs& A, int64_t row0, int r0, int r1, const float4* u, float4* out,
+                                          const float2* s, const int* gs, int gc, int tid) {
+    for (int q0 = r0 * NP + tid; q0 < r1 * NP; q0 += GA * SWT) {
+        float4 a[GA];
+#pragma unroll
+        for (int i = 0; i < GA; ++i) {
+            const int q = q0 + i * SWT, r = q / NP, p = q - r * NP;
+            float2 a0 = make_float2(0.f, 0.f), a1 = a0;
+            if (OWN && q < r1 * NP) {
+                if (2 * p < gc) a0 = s[(int64_t)gs[2 * p] * A.nfac + r];
+                if (2 * p + 1 < gc) a1 = s[(int64_t)gs[2 * p + 1] * A.nfac + r];
+            }
+            a[i] = make_float4(a0.x, a1.x, a0.y, a1.y);
+        }
+        for (int c = 0; c < A.nsrc; ++c) {
+            const int* src = A.src + c * A.src_rows + row0;
+            int e[GA];
+#pragma unroll
+            for (int i = 0; i < GA; ++i) {
+                const int q = q0 + i * SWT;
+                e[i] = q < r1 * NP ? src[q / NP] : -1;
+            }
+            float4 b[GA];
+#pragma unroll
+            for (int i = 0; i < GA; ++i)
+                b[i] = e[i] >= 0 ? __ldcg(u + (int64_t)e[i] * NP + (q0 + i * SWT) % NP) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int i = 0; i < GA; ++i)
+                if (e[i] >= 0) add4(a[i], b[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < GA; ++i)
+            if (q0 + i * SWT < r1 * NP) out[q0 + i * SWT] = a[i];
+    }
+}
+
 template <int NP>
 __device__ void sw_task(const SwArgs& A, SwShared& sm, uint32_t& it, const SwDesc& d0) {
     const int tid = threadIdx.x;
@@ -191,18 +232,7 @@ __device__ void sw_task(const SwArgs& A, SwShared& sm, uint32_t& it, const SwDes
         for (int q = tid; q < h; q += SWT)
             if (t.r0 + q < t.nown) sm.dv[q] = A.dinv[op * A.nfac + t.own0 + t.r0 + q];
         const int lo = max(0, t.nown - t.r0);
-        for (int q = lo * NP + tid; q < h * NP; q += SWT) {
-            const int r = q / NP, p = q - r * NP;
-            float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int s = 0; s < A.nsrc; ++s) {
-                const int e = A.src[s * A.src_rows + t.goff + t.r0 + r];
-                if (e >= 0) {
-                    const float4 b = __ldcg(u + (int64_t)e * NP + p);
-                    add4(a, b);
-                }
-            }
-            sm.eb[q] = a;
-        }
+        sw_gather<NP, false>(A, t.goff + t.r0, lo, h, u, sm.eb, nullptr, nullptr, 0, tid);
     } else {
         for (int q = tid; q < h; q += SWT) sm.node[q] = (int)A.iperm[t.own0 + t.r0 + q];
         sw_sync();
@@ -229,22 +259,7 @@ __device__ void sw_task(const SwArgs& A, SwShared& sm, uint32_t& it, const SwDes
                 const int tot = (xend - xbeg) * NP;
                 if (dir == 0) {
                     // own rows: the right-hand side plus the children's updates, in the children's order
-                    for (int q = tid; q < tot; q += SWT) {
-                        const int r = q / NP, p = q - r * NP, row = xbeg + r;
-                        const float2* s = A.s + t.own0 + row;
-                        const float2 zero2 = make_float2(0.f, 0.f);
-                        const float2 a0 = 2 * p < gc ? s[(int64_t)gs[2 * p] * A.nfac] : zero2;
-                        const float2 a1 = 2 * p + 1 < gc ? s[(int64_t)gs[2 * p + 1] * A.nfac] : zero2;
-                        float4 a = make_float4(a0.x, a1.x, a0.y, a1.y);
-                        for (int c = 0; c < A.nsrc; ++c) {
-                            const int e = A.src[c * A.src_rows + t.goff + row];
-                            if (e >= 0) {
-                                const float4 b = __ldcg(u + (int64_t)e * NP + p);
-                                add4(a, b);
-                            }
-                        }
-                        sm.x[q] = a;
-                    }
+                    sw_gather<NP, true>(A, t.goff + xbeg, 0, xend - xbeg, u, sm.x, A.s + t.own0 + xbeg, gs, gc, tid);
                 } else {
 #pragma unroll 4
                     for (int q = tid; q < tot; q += SWT) {
