@@ -373,21 +373,29 @@ __global__ void scale_kernel(GmresStateT<R, B> s, int j, int64_t n) {
         put_basis(s, v, vc, q, f * w[q]);
 }
 
-// y = R^-1 g over the slot's k = it columns (back substitution, FP64)
-__global__ void hsolve_kernel(GmresState s) {
-    int slot = blockIdx.x * blockDim.x + threadIdx.x;
-    if (slot >= s.nslot) return;
-    const int m = s.m, k = s.it[slot];
+// y = R^-1 g over the slot's k = it columns (back substitution, FP64), a warp per slot, column by column: the divisions
+// are made beforehand, side by side, and each column is taken off the rest of g by all lanes.  By one thread, row by row,
+// it took 0.1 ms at 50 steps, every load waited for.
+__global__ void __launch_bounds__(32) hsolve_kernel(GmresState s) {
+    __shared__ c64 gs[MAXV], di[MAXV];
+    const int slot = blockIdx.x, lane = threadIdx.x, m = s.m, k = s.it[slot];
     const c64* H = s.H + (int64_t)slot * (m + 1) * m;
     const c64* g = s.g + (int64_t)slot * (m + 1);
     c64* y = s.y + (int64_t)slot * s.ldh;
-    for (int i = k - 1; i >= 0; --i) {
-        c64 acc = g[i];
-        for (int q = i + 1; q < k; ++q) acc -= H[(int64_t)q * (m + 1) + i] * y[q];
-        c64 d = H[(int64_t)i * (m + 1) + i];
-        y[i] = (norm2(d) > 0) ? cdiv(acc, d) : zero<double>();
+    for (int i = lane; i < k; i += 32) {
+        const c64 d = H[(int64_t)i * (m + 1) + i];
+        di[i] = norm2(d) > 0 ? cdiv(mk<double>(1.0, 0.0), d) : zero<double>();
+        gs[i] = g[i];
     }
-    for (int i = k; i < m; ++i) y[i] = zero<double>();
+    __syncwarp();
+    for (int q = k - 1; q >= 0; --q) {
+        const c64 v = gs[q] * di[q];
+        if (lane == 0) y[q] = v;
+        const c64* h = H + (int64_t)q * (m + 1);
+        for (int i = lane; i < q; i += 32) gs[i] -= h[i] * v;
+        __syncwarp();
+    }
+    for (int i = k + lane; i < m; i += 32) y[i] = zero<double>();
 }
 
 // a slot's cycle starts from r / rho: V_0 = r / rho, g = (1, 0, ...), rotations cleared
@@ -524,7 +532,7 @@ void launch_scale(const GmresStateT<R, B>& s, int j, int64_t n, cudaStream_t st)
     GT_LAUNCH_CHECK();
 }
 void launch_hsolve(const GmresState& s, cudaStream_t st) {
-    hsolve_kernel<<<ceil_div(s.nslot, 64), 64, 0, st>>>(s);
+    hsolve_kernel<<<s.nslot, 32, 0, st>>>(s);
     GT_LAUNCH_CHECK();
 }
 template <typename R, typename B>
