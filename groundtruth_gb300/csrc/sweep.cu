@@ -54,9 +54,10 @@ struct SwDesc {                        // one ring stage, written by the produce
 struct alignas(16) SwShared {
     float2 ring[SW_STAGES][SW_STAGE_ENT];
     float4 x[SW_XROWS * 4];            // inner rows [row][pair]; then the partial sums [seg][output][pair]
-    float4 eb[SW_HMAX * 4];            // forward: the tile's boundary rows' updates so far [row][pair]
-    float2 dv[SW_HMAX];                // forward: the own rows' pivot reciprocals
-    int node[SW_HMAX];                 // backward: dense node of each output
+    float4 ext[SW_HMAX * 4];           // per output entry, its thread's own: forward, the pivot's reciprocal of an own row or
+                                       // the updates so far of a boundary row; backward, the dense node
+    int xrow[2][SW_XROWS];             // staged rows' sources: forward, the first two children's update rows; backward [0]
+    int hrow[2][SW_HMAX];              // forward: the outputs' sources
     SwDesc desc[SW_STAGES];
     uint64_t full[SW_STAGES], empty[SW_STAGES];
 };
@@ -167,44 +168,100 @@ __device__ __forceinline__ int sw_slot(int row2, int e) {
     return row2 * 2 * NP + (e ^ ((row2 / (4 / NP)) & (2 * NP - 1)));
 }
 
-// out[row][pair] = the right-hand sides (OWN) plus the children's updates of the front's rows row0 + r, r0 <= r < r1, in the
-// children's order.  The row indices, then the values, of GA entries per thread are loaded together: an entry at a time,
-// the three dependent loads of each were most of a tile's time near the root.
-constexpr int GA = 4;
-template <int NP, bool OWN>
-__device__ __forceinline__ void sw_gather(const SwArgs& A, int64_t row0, int r0, int r1, const float4* u, float4* out,
-                                          const float2* s, const int* gs, int gc, int tid) {
-    for (int q0 = r0 * NP + tid; q0 < r1 * NP; q0 += GA * SWT) {
-        float4 a[GA];
+// The update rows that the first two children have for the front's rows row0 .. row0 + n, into rows (a barrier follows).
+__device__ __forceinline__ void sw_sources(const SwArgs& A, int nsrc, int64_t row0, int n, int (*rows)[SW_XROWS], int tid) {
 #pragma unroll
-        for (int i = 0; i < GA; ++i) {
-            const int q = q0 + i * SWT, r = q / NP, p = q - r * NP;
-            float2 a0 = make_float2(0.f, 0.f), a1 = a0;
-            if (OWN && q < r1 * NP) {
-                if (2 * p < gc) a0 = s[(int64_t)gs[2 * p] * A.nfac + r];
-                if (2 * p + 1 < gc) a1 = s[(int64_t)gs[2 * p + 1] * A.nfac + r];
-            }
-            a[i] = make_float4(a0.x, a1.x, a0.y, a1.y);
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int i = 0; i < SW_XROWS / SWT; ++i) {
+            const int r = tid + i * SWT;
+            if (r < n) rows[c][r] = c < nsrc ? A.src[c * A.src_rows + row0 + r] : -1;
         }
-        for (int c = 0; c < A.nsrc; ++c) {
-            const int* src = A.src + c * A.src_rows + row0;
-            int e[GA];
+}
+
+// out += the children's updates of n rows (from row `from` on), in the children's order: the thread's entries tid + i SWT, i < N, each a column
+// pair p of row rt + i RS.  Two entries' values of two children are in flight together; four spill registers (1929 us per
+// application with 128 columns against 2608).
+template <int NP, int N>
+__device__ __forceinline__ void sw_add_children(const SwArgs& A, int nsrc, int64_t row0, int n, int from, const int* rows0,
+                                                const int* rows1, const float4* u, float4* out, int tid) {
+    constexpr int RS = SWT / NP, B = N < 2 ? N : 2;
+    const int p = tid % NP, rt = tid / NP;
+#pragma unroll 1
+    for (int i0 = 0; i0 < N; i0 += B) {
+        if (rt + i0 * RS >= n) break;
+        int e[2][B];
+        float4 a[B], b[2][B];
 #pragma unroll
-            for (int i = 0; i < GA; ++i) {
-                const int q = q0 + i * SWT;
-                e[i] = q < r1 * NP ? src[q / NP] : -1;
-            }
-            float4 b[GA];
-#pragma unroll
-            for (int i = 0; i < GA; ++i)
-                b[i] = e[i] >= 0 ? __ldcg(u + (int64_t)e[i] * NP + (q0 + i * SWT) % NP) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int i = 0; i < GA; ++i)
-                if (e[i] >= 0) add4(a[i], b[i]);
+        for (int i = 0; i < B; ++i) {
+            const int r = rt + (i0 + i) * RS;
+            e[0][i] = r < n ? rows0[r] : -1;
+            e[1][i] = r < n ? rows1[r] : -1;
         }
 #pragma unroll
-        for (int i = 0; i < GA; ++i)
-            if (q0 + i * SWT < r1 * NP) out[q0 + i * SWT] = a[i];
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int i = 0; i < B; ++i)
+                b[c][i] = e[c][i] >= 0 ? __ldcg(u + (int64_t)e[c][i] * NP + p) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < B; ++i) {
+            const int r = rt + (i0 + i) * RS;
+            if (r >= n) continue;
+            a[i] = out[tid + (i0 + i) * SWT];
+            if (e[0][i] >= 0) add4(a[i], b[0][i]);
+            if (e[1][i] >= 0) add4(a[i], b[1][i]);
+#pragma unroll 1
+            for (int c = 2; c < nsrc; ++c) {             // a front with more than two children
+                const int f = r >= from ? A.src[c * A.src_rows + row0 + r] : -1;
+                if (f >= 0) add4(a[i], __ldcg(u + (int64_t)f * NP + p));
+            }
+            out[tid + (i0 + i) * SWT] = a[i];
+        }
+    }
+}
+
+// the backward sweep's inner rows k .. k + n into sm.x: own rows from z, boundary rows from y, the row's index from rows
+template <int NP, int N>
+__device__ __forceinline__ void sw_stage_back(const float4* z, const float4* y, int n, int own, const int* rows, float4* x, int tid) {
+    constexpr int RS = SWT / NP;
+    const int p = tid % NP, rt = tid / NP;
+    constexpr int B = N < 4 ? N : 4;
+#pragma unroll 1
+    for (int i0 = 0; i0 < N; i0 += B) {
+        if (rt + i0 * RS >= n) break;
+        float4 a[B];
+#pragma unroll
+        for (int i = 0; i < B; ++i) {
+            const int r = rt + (i0 + i) * RS;
+            a[i] = r < n ? __ldcg((r < own ? z : y) + (int64_t)rows[r] * NP + p) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int i = 0; i < B; ++i)
+            if (rt + (i0 + i) * RS < n) x[tid + (i0 + i) * SWT] = a[i];
+    }
+}
+
+// forward: the right-hand sides of n rows (s: the first one's in slot 0; c0, c1: the pair's slots or -1) into x
+template <int NP, int N>
+__device__ __forceinline__ void sw_stage_own(const float2* s, int64_t nfac, int c0, int c1, int n, float4* x, int tid) {
+    constexpr int RS = SWT / NP;
+    const int rt = tid / NP;
+    const float2 none = make_float2(0.f, 0.f);
+#pragma unroll 4
+    for (int i = 0; i < N; ++i) {
+        const int r = rt + i * RS;
+        if (r >= n) break;
+        const float2 a0 = c0 >= 0 ? s[c0 * nfac + r] : none, a1 = c1 >= 0 ? s[c1 * nfac + r] : none;
+        x[tid + i * SWT] = make_float4(a0.x, a1.x, a0.y, a1.y);
+    }
+}
+
+// backward: where the inner rows k .. k + n stand, own rows in z, boundary rows in y
+__device__ __forceinline__ void sw_back_rows(const int* bidx, int own0, int nown, int k, int n, int* rows, int tid) {
+#pragma unroll
+    for (int i = 0; i < SW_XROWS / SWT; ++i) {
+        const int r = tid + i * SWT, row = k + r;
+        if (r < n) rows[r] = row < nown ? own0 + row : bidx[row - nown];
     }
 }
 
@@ -224,25 +281,53 @@ __device__ void sw_task(const SwArgs& A, SwShared& sm, uint32_t& it, const SwDes
     const int nseg = SWT / np2;
     const int seg = tid / np2, row2 = tid - seg * np2;
     const bool act = seg < nseg;
-    if (tid == 0 && t.need > 0) sw_wait_count(A.cnt + (int64_t)t.dep * ng + g, t.need);
-    // what the tile's outputs need besides the product
+    // A thread's entries (of the staged rows and of the outputs) are one column pair of every RS-th row.  All that does not
+    // depend on other tasks is fetched before their results are waited for: the rows' sources, the right-hand sides, what
+    // the outputs need besides the product.  A tile's time is in these chains of loads (row index, then value), not in its
+    // product: fetched one entry after the other, after the wait, they made an application 708 us with 32 columns (534
+    // now), 2316 with 128 (1787), 393 with 6 on the stack (309), 77 and 56 with one column on small planes (49 and 38).
+    constexpr int RS = SWT / NP, XE = SW_XROWS / RS, HE = SW_HMAX / RS;
+    const int p = tid % NP, rt = tid / NP;
+    const int c0 = 2 * p < gc ? gs[2 * p] : -1, c1 = 2 * p + 1 < gc ? gs[2 * p + 1] : -1;
+    const int nsrc = t.need > 0 ? A.nsrc : 0;            // (forward: a front without children waits for nobody)
+    const int lo = min(h, max(0, t.nown - t.r0));        // forward: the tile's first boundary row
+    int xbeg = t.k0, xend = min(t.k1, t.k0 + SW_XROWS);
     if (dir == 0) {
-        sw_sync();
         const int64_t op = A.G.op[g];
-        for (int q = tid; q < h; q += SWT)
-            if (t.r0 + q < t.nown) sm.dv[q] = A.dinv[op * A.nfac + t.own0 + t.r0 + q];
-        const int lo = max(0, t.nown - t.r0);
-        sw_gather<NP, false>(A, t.goff + t.r0, lo, h, u, sm.eb, nullptr, nullptr, 0, tid);
+        if (nsrc) {
+            sw_sources(A, nsrc, t.goff + t.k0, xend - xbeg, sm.xrow, tid);
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+                if (tid < h) sm.hrow[c][tid] = tid >= lo && c < nsrc ? A.src[c * A.src_rows + t.goff + t.r0 + tid] : -1;
+        }
+        sw_stage_own<NP, XE>(A.s + t.own0 + t.k0, A.nfac, c0, c1, xend - xbeg, sm.x, tid);
+#pragma unroll
+        for (int i = 0; i < HE; ++i) {
+            const int r = rt + i * RS;
+            const float2 d = r < lo ? A.dinv[op * A.nfac + t.own0 + t.r0 + r] : make_float2(0.f, 0.f);
+            sm.ext[tid + i * SWT] = make_float4(d.x, d.y, 0.f, 0.f);
+        }
+        if (nsrc) {
+            if (tid == 0) sw_wait_count(A.cnt + (int64_t)t.dep * ng + g, t.need);
+            sw_sync();
+            sw_add_children<NP, HE>(A, nsrc, t.goff + t.r0, h, lo, sm.hrow[0], sm.hrow[1], u, sm.ext, tid);
+            sw_add_children<NP, XE>(A, nsrc, t.goff + t.k0, xend - xbeg, 0, sm.xrow[0], sm.xrow[1], u, sm.x, tid);
+        }
     } else {
-        for (int q = tid; q < h; q += SWT) sm.node[q] = (int)A.iperm[t.own0 + t.r0 + q];
+        sw_back_rows(A.bidx + t.goff, t.own0, t.nown, xbeg, xend - xbeg, sm.xrow[0], tid);
+#pragma unroll
+        for (int i = 0; i < HE; ++i)
+            if (rt + i * RS < h) sm.ext[tid + i * SWT].x = __int_as_float((int)A.iperm[t.own0 + t.r0 + rt + i * RS]);
+        if (tid == 0 && t.need > 0) sw_wait_count(A.cnt + (int64_t)t.dep * ng + g, t.need);
         sw_sync();
+        sw_stage_back<NP, XE>(z, y, xend - xbeg, t.nown - xbeg, sm.xrow[0], sm.x, tid);
     }
+    sw_sync();
     uint64_t re[2][NP], im[2][NP];
 #pragma unroll
     for (int r = 0; r < 2; ++r)
 #pragma unroll
         for (int p = 0; p < NP; ++p) re[r][p] = im[r][p] = 0;
-    int xbeg = t.k0, xend = t.k0;
     bool last;
     do {
         const int slot = it % SW_STAGES;
@@ -253,21 +338,20 @@ __device__ void sw_task(const SwArgs& A, SwShared& sm, uint32_t& it, const SwDes
         const float2* ring = sm.ring[slot];
         for (int k = ka; k < kb;) {
             if (k >= xend) {
-                if (xend > t.k0) sw_sync();              // the rows staged before have been read
+                sw_sync();                               // the rows staged before have been read
                 xbeg = k;
                 xend = min(t.k1, k + SW_XROWS);
-                const int tot = (xend - xbeg) * NP;
                 if (dir == 0) {
-                    // own rows: the right-hand side plus the children's updates, in the children's order
-                    sw_gather<NP, true>(A, t.goff + xbeg, 0, xend - xbeg, u, sm.x, A.s + t.own0 + xbeg, gs, gc, tid);
-                } else {
-#pragma unroll 4
-                    for (int q = tid; q < tot; q += SWT) {
-                        const int r = q / NP, p = q - r * NP, row = xbeg + r;
-                        const float4* src = row < t.nown ? z + (int64_t)(t.own0 + row) * NP
-                                                         : y + (int64_t)A.bidx[t.goff + row - t.nown] * NP;
-                        sm.x[q] = __ldcg(src + p);
+                    if (nsrc) sw_sources(A, nsrc, t.goff + k, xend - k, sm.xrow, tid);
+                    sw_stage_own<NP, XE>(A.s + t.own0 + k, A.nfac, c0, c1, xend - k, sm.x, tid);
+                    if (nsrc) {
+                        sw_sync();
+                        sw_add_children<NP, XE>(A, nsrc, t.goff + k, xend - k, 0, sm.xrow[0], sm.xrow[1], u, sm.x, tid);
                     }
+                } else {
+                    sw_back_rows(A.bidx + t.goff, t.own0, t.nown, k, xend - k, sm.xrow[0], tid);
+                    sw_sync();
+                    sw_stage_back<NP, XE>(z, y, xend - k, t.nown - k, sm.xrow[0], sm.x, tid);
                 }
                 sw_sync();
             }
@@ -275,7 +359,7 @@ __device__ void sw_task(const SwArgs& A, SwShared& sm, uint32_t& it, const SwDes
             if (act) {
                 const float4* P = reinterpret_cast<const float4*>(ring) + (k - ka + seg) * np2 + row2;
                 const ulonglong2* X = reinterpret_cast<const ulonglong2*>(sm.x) + (k - xbeg + seg) * NP;
-#pragma unroll 2
+#pragma unroll 1
                 for (int q = k + seg; q < e; q += nseg, P += nseg * np2, X += nseg * NP) {
                     const float4 a = *P;                  // outputs 2 row2, 2 row2 + 1
                     mac_row<NP>(re[0], im[0], a.x, a.y, X);
@@ -298,32 +382,31 @@ __device__ void sw_task(const SwArgs& A, SwShared& sm, uint32_t& it, const SwDes
             for (int p = 0; p < NP; ++p) sm.x[seg * hp * NP + sw_slot<NP>(row2, r * NP + p)] = halves(re[r][p], im[r][p]);
     }
     sw_sync();
-    for (int q = tid; q < h * NP; q += SWT) {
+#pragma unroll
+    for (int i = 0; i < HE; ++i) {
+        const int r = rt + i * RS, q = tid + i * SWT, row = t.r0 + r;
+        if (r >= h) continue;
         const int at = sw_slot<NP>(q / (2 * NP), q % (2 * NP));
         float4 v = sm.x[at];
         for (int sg = 1; sg < nseg; ++sg) add4(v, sm.x[sg * hp * NP + at]);
-        const int r = q / NP, p = q - r * NP, row = t.r0 + r;
         if (dir == 0) {
-            if (row < t.nown) {
-                const float2 d = sm.dv[r];
-                z[(int64_t)(t.own0 + row) * NP + p] = make_float4(d.x * v.x - d.y * v.z, d.x * v.y - d.y * v.w,
-                                                                  d.x * v.z + d.y * v.x, d.x * v.w + d.y * v.y);
-            } else {
-                const float4 b = sm.eb[q];
+            const float4 b = sm.ext[tid + i * SWT];
+            if (r < lo)
+                z[(int64_t)(t.own0 + row) * NP + p] = make_float4(b.x * v.x - b.y * v.z, b.x * v.y - b.y * v.w,
+                                                                  b.x * v.z + b.y * v.x, b.x * v.w + b.y * v.y);
+            else
                 u[(int64_t)(t.voff + row - t.nown) * NP + p] = make_float4(b.x + v.x, b.y + v.y, b.z + v.z, b.w + v.w);
-            }
         } else {
             y[(int64_t)(t.own0 + row) * NP + p] = v;
-            const int64_t node = sm.node[r];
-            if (2 * p < gc) A.sd[(int64_t)gs[2 * p] * A.nnode + node] = make_float2(v.x, v.z);
-            if (2 * p + 1 < gc) A.sd[(int64_t)gs[2 * p + 1] * A.nnode + node] = make_float2(v.y, v.w);
+            const int node = __float_as_int(sm.ext[tid + i * SWT].x);
+            if (c0 >= 0) A.sd[(int64_t)c0 * A.nnode + node] = make_float2(v.x, v.z);
+            if (c1 >= 0) A.sd[(int64_t)c1 * A.nnode + node] = make_float2(v.y, v.w);
         }
     }
     sw_sync();                                           // every output of the tile is written
-    if (tid == 0 && t.sig >= 0) {
-        __threadfence();
+    // (the release carries the whole block's outputs, ordered before it by the barrier)
+    if (tid == 0 && t.sig >= 0)
         asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(A.cnt + (int64_t)t.sig * ng + g) : "memory");
-    }
 }
 
 __global__ void __launch_bounds__(SW_BLOCK, 4) sweep_kernel(SwArgs A) {
