@@ -35,6 +35,7 @@ __device__ __forceinline__ void cfma(c64& acc, c64 a, c64 u) {
 __global__ void assemble_s_kernel(const int64_t* __restrict__ ptr, const int* __restrict__ tab_idx,
                                   const double* __restrict__ coef, int64_t nsv, const c64* __restrict__ table, int ntab,
                                   c64* __restrict__ svals) {
+    pdl_enter();
     const int op = blockIdx.y;
     const c64* T = table + (int64_t)op * ntab;
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nsv; e += (int64_t)gridDim.x * blockDim.x) {
@@ -47,7 +48,7 @@ __global__ void assemble_s_kernel(const int64_t* __restrict__ ptr, const int* __
 void launch_assemble_s(const int64_t* ptr, const int* tab_idx, const double* coef, int64_t nsv, const c64* table,
                        int ntab, c64* svals, int nops, cudaStream_t st) {
     int blocks = (int)std::min<int64_t>((nsv + 255) / 256, 2048);
-    assemble_s_kernel<<<dim3(std::max(blocks, 1), nops), 256, 0, st>>>(ptr, tab_idx, coef, nsv, table, ntab, svals);
+    pdl_launch(assemble_s_kernel, dim3(std::max(blocks, 1), nops), 256, 0, st, ptr, tab_idx, coef, nsv, table, ntab, svals);
     GT_LAUNCH_CHECK();
 }
 
@@ -148,6 +149,7 @@ __global__ void __launch_bounds__(SF_THREADS) small_front_kernel(Fronts F, Sweep
                                                                  c64* __restrict__ d64, c32* __restrict__ d32,
                                                                  c32* __restrict__ pf, c32* __restrict__ pb,
                                                                  int* __restrict__ status) {
+    pdl_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int f = (int)front_list[blockIdx.x], op = blockIdx.y, tid = threadIdx.x;
     const FrontView Fv = front_view(F, f, op, panel, upd);
@@ -285,7 +287,7 @@ void launch_small_fronts(const Fronts& F, const SweepPlan& S, const int64_t* fro
                          const c64* svals, c64* panel, c64* upd, c64* r64, c64* d64, c32* d32, c32* pf, c32* pb, int nops,
                          int* status, cudaStream_t st) {
     raise_smem((const void*)small_front_kernel, smem);
-    small_front_kernel<<<dim3(nfront, nops), SF_THREADS, smem, st>>>(F, S, front_list, svals, panel, upd, r64, d64, d32, pf, pb,
+    pdl_launch(small_front_kernel, dim3(nfront, nops), SF_THREADS, smem, st, F, S, front_list, svals, panel, upd, r64, d64, d32, pf, pb,
                                                                      status);
     GT_LAUNCH_CHECK();
 }
@@ -316,6 +318,7 @@ struct DiagInv {
 // parent at an earlier level) and is cleared here.
 __global__ void assemble_fronts_kernel(Fronts F, const int64_t* __restrict__ front_list, const c64* __restrict__ svals,
                                        c64* __restrict__ panel, c64* __restrict__ upd) {
+    pdl_enter();
     const int f = (int)front_list[blockIdx.x], op = blockIdx.y;
     const FrontView Fv = front_view(F, f, op, panel, upd);
     const int tid = threadIdx.x, nth = blockDim.x;
@@ -341,6 +344,7 @@ __global__ void assemble_fronts_kernel(Fronts F, const int64_t* __restrict__ fro
 __global__ void __launch_bounds__(256) tiled_diag_kernel(Fronts F, const int64_t* __restrict__ front_list, int kb,
                                                          c64* __restrict__ panel, c64* __restrict__ upd, DiagInv X,
                                                          int* __restrict__ status) {
+    pdl_enter();
     __shared__ c64 a[FB][FB + 1];
     __shared__ c64 x[FB][FB + 1];
     __shared__ c64 red[256];
@@ -403,6 +407,7 @@ __global__ void __launch_bounds__(256) tiled_diag_kernel(Fronts F, const int64_t
 // rows of the front below the block: 32 per CTA
 __global__ void __launch_bounds__(256) tiled_rows_kernel(Fronts F, const int64_t* __restrict__ front_list, int kb,
                                                          c64* __restrict__ panel, c64* __restrict__ upd, DiagInv X) {
+    pdl_enter();
     __shared__ c64 x[FB][FB];
     __shared__ c64 ar[FB][FB + 1];                        // [row][column]
     __shared__ c64 dv[FB];
@@ -448,6 +453,7 @@ __device__ __forceinline__ void tile_mac(const c64* As, const c64* Bs, int nb, i
 
 __global__ void __launch_bounds__(256) tiled_trail_kernel(Fronts F, const int64_t* __restrict__ front_list, int kb,
                                                           c64* __restrict__ panel, c64* __restrict__ upd) {
+    pdl_enter();
     __shared__ c64 As[FB * FT], Bs[FB * FT];             // [m][r]: L(i0 + r, kb + m); [m][c]: L(j0 + c, kb + m) d_m
     const int f = (int)front_list[blockIdx.y];
     const FrontView Fv = front_view(F, f, blockIdx.z, panel, upd);
@@ -487,17 +493,17 @@ void launch_factor_tiled(const Fronts& F, const int64_t* front_list, int nf_leve
                          const c64* svals, c64* panel, c64* upd, c64* xinv, const int* xfirst, int64_t xtotal, int nops,
                          int* status, cudaStream_t st) {
     const DiagInv X{xinv, xfirst, xtotal};
-    assemble_fronts_kernel<<<dim3(nf_level, nops), 512, 0, st>>>(F, front_list, svals, panel, upd);
+    pdl_launch(assemble_fronts_kernel, dim3(nf_level, nops), 512, 0, st, F, front_list, svals, panel, upd);
     GT_LAUNCH_CHECK();
     for (int kb = 0; kb < max_nown; kb += FB) {
-        tiled_diag_kernel<<<dim3(nf_level, nops), 256, 0, st>>>(F, front_list, kb, panel, upd, X, status);
+        pdl_launch(tiled_diag_kernel, dim3(nf_level, nops), 256, 0, st, F, front_list, kb, panel, upd, X, status);
         GT_LAUNCH_CHECK();
         const int below = max_nf - kb - 1;              // rows below the block (at least this front's nb of them)
         if (below <= 0) continue;
-        tiled_rows_kernel<<<dim3(ceil_div(below, 32), nf_level, nops), 256, 0, st>>>(F, front_list, kb, panel, upd, X);
+        pdl_launch(tiled_rows_kernel, dim3(ceil_div(below, 32), nf_level, nops), 256, 0, st, F, front_list, kb, panel, upd, X);
         GT_LAUNCH_CHECK();
         const int T = ceil_div(below, FT);
-        tiled_trail_kernel<<<dim3((unsigned)((int64_t)T * (T + 1) / 2), nf_level, nops), 256, 0, st>>>(F, front_list, kb, panel,
+        pdl_launch(tiled_trail_kernel, dim3((unsigned)((int64_t)T * (T + 1) / 2), nf_level, nops), 256, 0, st, F, front_list, kb, panel,
                                                                                                      upd);
         GT_LAUNCH_CHECK();
     }
@@ -514,6 +520,7 @@ void launch_factor_tiled(const Fronts& F, const int64_t* front_list, int nf_leve
 // The panel's upper triangle stays zero; the diagonal keeps D for panel_convert.
 __global__ void __launch_bounds__(256) inv_rows_kernel(Fronts F, const int64_t* __restrict__ front_list, int kb,
                                                        c64* __restrict__ panel, DiagInv X) {
+    pdl_enter();
     __shared__ c64 x[FB][FB];
     __shared__ c64 y[FB][FB + 1];                         // [column][row]
     const int f = (int)front_list[blockIdx.y], op = blockIdx.z;
@@ -549,6 +556,7 @@ __global__ void __launch_bounds__(256) inv_rows_kernel(Fronts F, const int64_t* 
 // rows i >= kb + nb of the front; mode 0: columns c < kb (tile grid rt x ct), mode 1: the block's columns
 __global__ void __launch_bounds__(256) inv_trail_kernel(Fronts F, const int64_t* __restrict__ front_list, int kb,
                                                         c64* __restrict__ panel, int mode) {
+    pdl_enter();
     __shared__ c64 As[FB * FT], Bs[FB * FT];             // [m][r]: L(i0 + r, kb + m); [m][c]: Y(kb + m, c0 + c)
     const int f = (int)front_list[blockIdx.y];
     const int op = blockIdx.z;
@@ -599,16 +607,16 @@ void launch_invert_tiled(const Fronts& F, const int64_t* front_list, int nfront,
     if (nfront <= 0) return;
     const DiagInv X{const_cast<c64*>(xinv), xfirst, xtotal};
     for (int kb = 0; kb < max_nown; kb += FB) {
-        inv_rows_kernel<<<dim3(kb / 32 + 1, nfront, nops), 256, 0, st>>>(F, front_list, kb, panel, X);
+        pdl_launch(inv_rows_kernel, dim3(kb / 32 + 1, nfront, nops), 256, 0, st, F, front_list, kb, panel, X);
         GT_LAUNCH_CHECK();
         const int below = max_nf - kb - 1;
         if (below <= 0) continue;
         const int rt = ceil_div(below, FT);
         if (kb > 0) {
-            inv_trail_kernel<<<dim3(rt * ceil_div(kb, FT), nfront, nops), 256, 0, st>>>(F, front_list, kb, panel, 0);
+            pdl_launch(inv_trail_kernel, dim3(rt * ceil_div(kb, FT), nfront, nops), 256, 0, st, F, front_list, kb, panel, 0);
             GT_LAUNCH_CHECK();
         }
-        inv_trail_kernel<<<dim3(rt, nfront, nops), 256, 0, st>>>(F, front_list, kb, panel, 1);
+        pdl_launch(inv_trail_kernel, dim3(rt, nfront, nops), 256, 0, st, F, front_list, kb, panel, 1);
         GT_LAUNCH_CHECK();
     }
 }
@@ -619,6 +627,7 @@ void launch_invert_tiled(const Fronts& F, const int64_t* front_list, int nfront,
 __global__ void panel_convert_kernel(Fronts F, SweepPlan S, const int64_t* __restrict__ front_list, c64* __restrict__ p64,
                                      c32* __restrict__ pf, c32* __restrict__ pb, c64* __restrict__ r64, c64* __restrict__ d64,
                                      c32* __restrict__ d32) {
+    pdl_enter();
     const int f = (int)front_list[blockIdx.y];
     const int op = blockIdx.z;
     const int nown = (int)F.nown[f], nf = nown + (int)F.nbnd[f];
@@ -644,7 +653,7 @@ __global__ void panel_convert_kernel(Fronts F, SweepPlan S, const int64_t* __res
 void launch_panel_convert(const Fronts& F, const SweepPlan& S, const int64_t* front_list, int nfront, c64* p64, c32* pf, c32* pb,
                           c64* r64, c64* d64, c32* d32, int nops, cudaStream_t st) {
     if (nfront <= 0) return;
-    panel_convert_kernel<<<dim3(16, nfront, nops), 256, 0, st>>>(F, S, front_list, p64, pf, pb, r64, d64, d32);
+    pdl_launch(panel_convert_kernel, dim3(16, nfront, nops), 256, 0, st, F, S, front_list, p64, pf, pb, r64, d64, d32);
     GT_LAUNCH_CHECK();
 }
 
