@@ -14,9 +14,18 @@
 
 namespace gt {
 
-// grid rows per block of the stencil kernels (fewer, fuller blocks)
+// Grid rows per block of the stencil kernels: as many as RPB (pc_node: RPB_NODE, its threads carry more work per row), which
+// makes fewer, fuller blocks, and fewer while there are less than four blocks for each of the 152 SMs: a thread's rows are
+// one after the other, each a chain of loads.  One column, 32 x 32 x 2: the tail 15.7 -> 7.6 us, pc_strip 12 -> 7.4, pc_node
+// 12.8 -> 10.1; 96 x 96: 14.7 -> 6.7, 11.9 -> 7.6, 10.1 -> 8.5 (with events around them).
 constexpr int RPB = 8;
-constexpr int RPB_NODE = 2;     // pc_node's threads carry more work per row
+constexpr int RPB_NODE = 2;
+
+static int rows_per_block(int64_t rows, int64_t others, int most) {
+    return (int)std::max<int64_t>(1, std::min<int64_t>(most, rows * others / (4 * 152)));
+}
+// threads of a block: the row's length, in whole warps
+static int row_threads(int ny) { return std::min(256, std::max(1, ceil_div(ny, 32)) * 32); }
 
 namespace {
 
@@ -38,7 +47,7 @@ template <typename R>
 __global__ void __launch_bounds__(256) tail_kernel(Geo g, const cx<R>* __restrict__ x, const cx<R>* __restrict__ rhs,
                                                    cx<R>* __restrict__ out, int64_t ld, int64_t ldo, const int* __restrict__ col_op,
                                                    const c64* __restrict__ zcap, const c64* __restrict__ zbr, int mode,
-                                                   const int* __restrict__ col_list) {
+                                                   const int* __restrict__ col_list, int rpb) {
     pdl_enter();
     const int col = col_list ? col_list[blockIdx.z] : blockIdx.z;
     const int op = col_op ? col_op[col] : 0;
@@ -49,7 +58,7 @@ __global__ void __launch_bounds__(256) tail_kernel(Geo g, const cx<R>* __restric
     cx<R>* oc = out + (int64_t)col * ldo;
     const int part = blockIdx.y;
     auto put = [&](int64_t pos, cx<R> y) { oc[pos] = mode == 1 ? bc[pos] - y : y; };
-    if (part == 0) for (int bx = blockIdx.x * RPB; bx < blockIdx.x * RPB + RPB; ++bx) {
+    if (part == 0) for (int bx = blockIdx.x * rpb; bx < blockIdx.x * rpb + rpb; ++bx) {
         // node (KCL) rows: I_x(k,i,j) - I_x(k,i-1,j) + I_y(k,i,j) - I_y(k,i,j-1) + caps + branches, the strips of
         // every sheet on layer k (a split layer's two faces)
         const int k = bx / nx, i = bx - k * nx;
@@ -83,7 +92,7 @@ __global__ void __launch_bounds__(256) tail_kernel(Geo g, const cx<R>* __restric
             }
             put(pos, s);
         }
-    } else if (part == 1) for (int bx = blockIdx.x * RPB; bx < blockIdx.x * RPB + RPB; ++bx) {
+    } else if (part == 1) for (int bx = blockIdx.x * rpb; bx < blockIdx.x * rpb + rpb; ++bx) {
         // capacitance rows: z_cap I_c - (V[upper] - V[lower])
         const int p = bx / nx, i = bx - p * nx;
         if (p >= g.np) break;
@@ -123,8 +132,10 @@ __global__ void __launch_bounds__(256) tail_kernel(Geo g, const cx<R>* __restric
 template <typename R>
 void launch_tail(const Geo& g, const cx<R>* x, const cx<R>* rhs, cx<R>* out, int64_t ld, int64_t ldo, int ncol,
                  const int* col_op, const c64* zcap, const c64* zbr, int mode, const int* col_list, cudaStream_t st) {
-    const dim3 grid(std::max(ceil_div((int64_t)g.nx * std::max(g.np, g.S), RPB), 1), 3, ncol);
-    pdl_launch(tail_kernel<R>, grid, 256, 0, st, g, x, rhs, out, ld, ldo, col_op, zcap, zbr, mode, col_list);
+    const int64_t rows = (int64_t)g.nx * std::max(g.np, g.S);
+    const int rpb = rows_per_block(rows, ncol, RPB);
+    pdl_launch(tail_kernel<R>, dim3(std::max(ceil_div(rows, rpb), 1), 3, ncol), row_threads(g.ny), 0, st, g, x, rhs, out, ld, ldo,
+               col_op, zcap, zbr, mode, col_list, rpb);
     GT_LAUNCH_CHECK();
 }
 
@@ -151,7 +162,7 @@ template <typename R, int MAXS>
 __global__ void __launch_bounds__(256) pc_node_kernel(Geo g, const cx<R>* __restrict__ r, int64_t ld, cx<R>* __restrict__ sd,
                                                       const int* __restrict__ col_op, const cx<R>* __restrict__ tab,
                                                       const int* __restrict__ col_list, int* __restrict__ cnt,
-                                                      int64_t ncnt, const double* __restrict__ rscale) {
+                                                      int64_t ncnt, const double* __restrict__ rscale, int rpb) {
     pdl_enter();
     for (int64_t q = ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x; q < ncnt;
          q += (int64_t)gridDim.y * gridDim.x * blockDim.x)
@@ -165,7 +176,7 @@ __global__ void __launch_bounds__(256) pc_node_kernel(Geo g, const cx<R>* __rest
     const cx<R>* Y = rc + g.off_y;
     cx<R>* sc = sd + (int64_t)col * g.nfac;
     const R f = rscale ? R(rscale[col]) : R(1);          // (the result is linear in r)
-    for (int i = blockIdx.x * RPB_NODE; i < min(nx, blockIdx.x * RPB_NODE + RPB_NODE); ++i)
+    for (int i = blockIdx.x * rpb; i < min(nx, blockIdx.x * rpb + rpb); ++i)
     for (int j = threadIdx.x; j < ny; j += blockDim.x) {
         const int ij = i * ny + j;
         cx<R> kcl[MAXS], u[4][MAXS], t[MAXS];
@@ -248,10 +259,11 @@ template <typename R>
 void launch_pc_node(const Geo& g, const cx<R>* r, int64_t ld, cx<R>* sd, int ncol, const int* col_op, const cx<R>* tab,
                     const int* col_list, int* cnt, int64_t ncnt, const double* rscale, cudaStream_t st) {
     if (g.S > SHEETS_MAX) throw CudaError{cudaErrorInvalidValue, "more sheets than the stencil kernels take"};
-    const dim3 grid(ceil_div(g.nx, RPB_NODE), ncol);
-    if (g.S <= 2) pdl_launch(pc_node_kernel<R, 2>, grid, 256, 0, st, g, r, ld, sd, col_op, tab, col_list, cnt, ncnt, rscale);
-    else if (g.S <= 4) pdl_launch(pc_node_kernel<R, 4>, grid, 256, 0, st, g, r, ld, sd, col_op, tab, col_list, cnt, ncnt, rscale);
-    else pdl_launch(pc_node_kernel<R, 8>, grid, 256, 0, st, g, r, ld, sd, col_op, tab, col_list, cnt, ncnt, rscale);
+    const int rpb = rows_per_block(g.nx, ncol, RPB_NODE), threads = row_threads(g.ny);
+    const dim3 grid(ceil_div(g.nx, rpb), ncol);
+    if (g.S <= 2) pdl_launch(pc_node_kernel<R, 2>, grid, threads, 0, st, g, r, ld, sd, col_op, tab, col_list, cnt, ncnt, rscale, rpb);
+    else if (g.S <= 4) pdl_launch(pc_node_kernel<R, 4>, grid, threads, 0, st, g, r, ld, sd, col_op, tab, col_list, cnt, ncnt, rscale, rpb);
+    else pdl_launch(pc_node_kernel<R, 8>, grid, threads, 0, st, g, r, ld, sd, col_op, tab, col_list, cnt, ncnt, rscale, rpb);
     GT_LAUNCH_CHECK();
 }
 
@@ -262,7 +274,7 @@ template <typename R, int MAXS>
 __global__ void __launch_bounds__(256) pc_strip_kernel(Geo g, const cx<R>* __restrict__ r, int64_t ldr,
                                                        const cx<R>* __restrict__ sd, cx<R>* __restrict__ out, int64_t ldo,
                                                        const int* __restrict__ col_op, const cx<R>* __restrict__ tab,
-                                                       const int* __restrict__ col_list, const double* __restrict__ rscale) {
+                                                       const int* __restrict__ col_list, const double* __restrict__ rscale, int rpb) {
     pdl_enter();
     const int col = col_list ? col_list[blockIdx.z] : blockIdx.z;
     const int op = col_op ? col_op[col] : 0;
@@ -273,7 +285,7 @@ __global__ void __launch_bounds__(256) pc_strip_kernel(Geo g, const cx<R>* __res
     const cx<R>* yc = sd + (int64_t)col * g.NL * nxy;    // zero at nodes that are not kept
     cx<R>* oc = out + (int64_t)col * ldo;
     const int part = blockIdx.y;
-    if (part <= 1) for (int bx = blockIdx.x * RPB; bx < blockIdx.x * RPB + RPB; ++bx) {
+    if (part <= 1) for (int bx = blockIdx.x * rpb; bx < blockIdx.x * rpb + rpb; ++bx) {
         const bool xo = part == 0;
         const int i = bx;
         if (i >= (xo ? nx - 1 : nx)) break;
@@ -300,7 +312,7 @@ __global__ void __launch_bounds__(256) pc_strip_kernel(Geo g, const cx<R>* __res
             for (int k = 0; k < MAXS; ++k)
                 if (k < S) oc[seg + (int64_t)k * lstride + pq] = t[k];      // zero where the strip is absent
         }
-    } else if (part == 2) for (int bx = blockIdx.x * RPB; bx < blockIdx.x * RPB + RPB; ++bx) {
+    } else if (part == 2) for (int bx = blockIdx.x * rpb; bx < blockIdx.x * rpb + rpb; ++bx) {
         const int p = bx / nx, i = bx - p * nx;
         if (p >= g.np) break;
         const int up = g.pair_layers[2 * p], lo = g.pair_layers[2 * p + 1];
@@ -311,7 +323,7 @@ __global__ void __launch_bounds__(256) pc_strip_kernel(Geo g, const cx<R>* __res
             const cx<R> y = g.cap_fill ? R(g.cap_fill[(int64_t)p * nxy + ij]) * zc : zc;
             oc[pos] = g.mask[pos] ? y * (f * rc[pos] + (yc[up * nxy + ij] - yc[lo * nxy + ij])) : zero<R>();
         }
-    } else if (part == 3) for (int bx = blockIdx.x * RPB; bx < blockIdx.x * RPB + RPB; ++bx) {
+    } else if (part == 3) for (int bx = blockIdx.x * rpb; bx < blockIdx.x * rpb + rpb; ++bx) {
         const int k = bx / nx, i = bx - k * nx;
         if (k >= g.NL) break;
         for (int j = threadIdx.x; j < ny; j += blockDim.x) {
@@ -340,10 +352,12 @@ template <typename R>
 void launch_pc_strip(const Geo& g, const cx<R>* r, int64_t ldr, const cx<R>* sd, cx<R>* out, int64_t ldo, int ncol,
                      const int* col_op, const cx<R>* tab, const int* col_list, const double* rscale, cudaStream_t st) {
     if (g.S > SHEETS_MAX) throw CudaError{cudaErrorInvalidValue, "more sheets than the stencil kernels take"};
-    const dim3 grid(std::max(ceil_div((int64_t)g.nx * std::max(g.np, g.S), RPB), 1), 5, ncol);
-    if (g.S <= 2) pdl_launch(pc_strip_kernel<R, 2>, grid, 256, 0, st, g, r, ldr, sd, out, ldo, col_op, tab, col_list, rscale);
-    else if (g.S <= 4) pdl_launch(pc_strip_kernel<R, 4>, grid, 256, 0, st, g, r, ldr, sd, out, ldo, col_op, tab, col_list, rscale);
-    else pdl_launch(pc_strip_kernel<R, 8>, grid, 256, 0, st, g, r, ldr, sd, out, ldo, col_op, tab, col_list, rscale);
+    const int64_t rows = (int64_t)g.nx * std::max(g.np, g.S);
+    const int rpb = rows_per_block(rows, ncol, RPB), threads = row_threads(g.ny);
+    const dim3 grid(std::max(ceil_div(rows, rpb), 1), 5, ncol);
+    if (g.S <= 2) pdl_launch(pc_strip_kernel<R, 2>, grid, threads, 0, st, g, r, ldr, sd, out, ldo, col_op, tab, col_list, rscale, rpb);
+    else if (g.S <= 4) pdl_launch(pc_strip_kernel<R, 4>, grid, threads, 0, st, g, r, ldr, sd, out, ldo, col_op, tab, col_list, rscale, rpb);
+    else pdl_launch(pc_strip_kernel<R, 8>, grid, threads, 0, st, g, r, ldr, sd, out, ldo, col_op, tab, col_list, rscale, rpb);
     GT_LAUNCH_CHECK();
 }
 
