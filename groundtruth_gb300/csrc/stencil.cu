@@ -66,31 +66,34 @@ __global__ void __launch_bounds__(256) tail_kernel(Geo g, const cx<R>* __restric
         for (int j = threadIdx.x; j < ny; j += blockDim.x) {
             const int ij = i * ny + j, node = k * nxy + ij;
             const int64_t pos = g.off_v + node;
-            if (!g.mask[pos]) {
-                oc[pos] = zero<R>();
-                continue;
-            }
+            // (everything is loaded whether the node is kept or not: behind the mask's test each load waited for one more)
+            const bool on = g.mask[pos];
+            const int e0 = g.node_br_ptr[node], e1 = on ? g.node_br_ptr[node + 1] : e0;
             cx<R> s = zero<R>();
             for (int sh = g.NL == S ? k : 0; sh < (g.NL == S ? k + 1 : S); ++sh) {
                 if (g.sheet_layer[sh] != k) continue;
                 const cx<R>* X = xc + g.off_x + (int64_t)sh * (nx - 1) * ny;
                 const cx<R>* Y = xc + g.off_y + (int64_t)sh * nx * (ny - 1);
-                if (i < nx - 1) s += X[i * ny + j];
-                if (i > 0) s -= X[(i - 1) * ny + j];
-                if (j < ny - 1) s += Y[i * (ny - 1) + j];
-                if (j > 0) s -= Y[i * (ny - 1) + j - 1];
+                const cx<R> xa = i < nx - 1 ? X[i * ny + j] : zero<R>(), xb = i > 0 ? X[(i - 1) * ny + j] : zero<R>();
+                const cx<R> ya = j < ny - 1 ? Y[i * (ny - 1) + j] : zero<R>(), yb = j > 0 ? Y[i * (ny - 1) + j - 1] : zero<R>();
+                s += xa;
+                s -= xb;
+                s += ya;
+                s -= yb;
             }
             for (int p = 0; p < g.np; ++p) {
                 const int u = g.pair_layers[2 * p], l = g.pair_layers[2 * p + 1];
-                if (u == k) s += xc[g.off_c + (int64_t)p * nxy + ij];
-                if (l == k) s -= xc[g.off_c + (int64_t)p * nxy + ij];
+                const cx<R> c = u == k || l == k ? xc[g.off_c + (int64_t)p * nxy + ij] : zero<R>();
+                if (u == k) s += c;
+                if (l == k) s -= c;
             }
-            for (int e = g.node_br_ptr[node]; e < g.node_br_ptr[node + 1]; ++e) {
+            for (int e = e0; e < e1; ++e) {
                 const int b = g.node_br_idx[e];
                 if (b > 0) s += xc[g.off_b + b - 1];
                 else s -= xc[g.off_b - b - 1];
             }
-            put(pos, s);
+            if (on) put(pos, s);
+            else oc[pos] = zero<R>();
         }
     } else if (part == 1) for (int bx = blockIdx.x * rpb; bx < blockIdx.x * rpb + rpb; ++bx) {
         // capacitance rows: z_cap I_c - (V[upper] - V[lower])
@@ -183,6 +186,25 @@ __global__ void __launch_bounds__(256) pc_node_kernel(Geo g, const cx<R>* __rest
         int code[4], pq[4];
 #pragma unroll
         for (int k = 0; k < MAXS; ++k) kcl[k] = zero<R>();
+        // what the nodes need at the end, asked for now (up to four layers: the registers)
+        constexpr bool PRE = MAXS <= 4;
+        constexpr int NPRE = PRE ? MAXS : 1;
+        cx<R> rv[NPRE];
+        int64_t to[NPRE];
+        int b0[NPRE], b1[NPRE];
+        bool on[NPRE];
+        if constexpr (PRE) {
+#pragma unroll
+            for (int k = 0; k < MAXS; ++k) {
+                const bool in = k < g.NL;
+                const int node = in ? k * nxy + ij : ij;
+                on[k] = in && g.mask[g.off_v + node];
+                rv[k] = rc[g.off_v + node];
+                to[k] = g.perm[node];
+                b0[k] = g.node_br_ptr[node];
+                b1[k] = g.node_br_ptr[node + 1];
+            }
+        }
         // x strips (., i, j) [their a end] and (., i-1, j) [b end]; y strips (., i, j) and (., i, j-1):
         // all codes, then all strip loads, then the products
 #pragma unroll
@@ -229,8 +251,9 @@ __global__ void __launch_bounds__(256) pc_node_kernel(Geo g, const cx<R>* __rest
         for (int p = 0; p < g.np; ++p) {
             const int up = g.pair_layers[2 * p], lo = g.pair_layers[2 * p + 1];
             const int64_t pos = g.off_c + (int64_t)p * nxy + ij;
-            if (!g.mask[pos]) continue;
+            const bool here = g.mask[pos];
             cx<R> v = T[g.tab_cap0 + p] * rc[pos];
+            if (!here) continue;
             if (g.cap_fill) v = R(g.cap_fill[(int64_t)p * nxy + ij]) * v;
 #pragma unroll
             for (int k = 0; k < MAXS; ++k) {
@@ -242,15 +265,16 @@ __global__ void __launch_bounds__(256) pc_node_kernel(Geo g, const cx<R>* __rest
         for (int k = 0; k < MAXS; ++k) {
             if (k >= g.NL) break;
             const int node = k * nxy + ij;
-            if (!g.mask[g.off_v + node]) continue;
+            if (PRE ? !on[k % NPRE] : !g.mask[g.off_v + node]) continue;
             cx<R> acc = kcl[k];
-            for (int e = g.node_br_ptr[node]; e < g.node_br_ptr[node + 1]; ++e) {
+            const int e0 = PRE ? b0[k % NPRE] : g.node_br_ptr[node], e1 = PRE ? b1[k % NPRE] : g.node_br_ptr[node + 1];
+            for (int e = e0; e < e1; ++e) {
                 const int bq = g.node_br_idx[e];
                 const int bb = (bq > 0 ? bq : -bq) - 1;
                 const cx<R> v = T[g.tab_br0 + bb] * rc[g.off_b + bb];
                 acc = bq > 0 ? acc + v : acc - v;
             }
-            sc[g.perm[node]] = f * (rc[g.off_v + node] - acc);
+            sc[PRE ? to[k % NPRE] : g.perm[node]] = f * ((PRE ? rv[k % NPRE] : rc[g.off_v + node]) - acc);
         }
     }
 }
