@@ -465,14 +465,35 @@ static void tune_lp(Orient& o, LpArgs<R> a, int pr, cudaStream_t st) {
     o.bt[pr] = bb;
 }
 
+// Whether the two orientations' L_p passes run side by side, the second's on a stream and in a part of T of its own: while
+// their grids are small, three passes leave most of the GPU idle and the other three cost nothing beside them, nor do the
+// tail's rows.  Solves of 1 column at 32 x 32 and 96 x 96: 10.5 -> 9.5 and 11.0 -> 10.1 ms; 4 columns at 128 x 128 22.8 -> 21.4,
+// 8 there and 2 at 256 x 256 (the line, 8 + 16 MB of T) 2 % and 4 at 256 x 256 1 %.  The profiler's regions are timed one
+// after the other.
+constexpr int64_t SIDE_ENTRIES = 1 << 20;
+static bool side_by_side(const gt_geometry* G, int ncol) { return (int64_t)ncol * G->maxT <= SIDE_ENTRIES; }
+// entries of T for products of up to ncol columns
+static size_t t_entries(const gt_geometry* G, int ncol) {
+    const size_t one = (size_t)ncol * G->maxT;
+    return std::max(one, std::min<size_t>(2 * one, 2 * SIDE_ENTRIES));
+}
+
 // System product out = K x (mode 0), rhs - K x (1), or the L_p product of the strips (2).
 template <typename R>
 static void matvec(gt_geometry* G, gt_operators* ops, const cx<R>* x, const cx<R>* rhs, cx<R>* out, int64_t ld, int64_t ldo,
                    int ncol, const int* col_op, int mode, cx<R>* T, cudaStream_t st, const int* col_list = nullptr) {
     Profiler* P = &G->prof;
+    const cudaStream_t main = st;
+    const bool fork = !P->on && side_by_side(G, ncol);
+    if (fork) {
+        G->make_streams();
+        GT_CUDA(cudaEventRecord(G->fork, main));
+        GT_CUDA(cudaStreamWaitEvent(G->sub[0], G->fork, 0));
+    }
     for (int k = 0; k < 2; ++k) {
         Orient& o = G->o[k];
         if ((int64_t)o.n0 * o.n1 == 0) continue;
+        const cudaStream_t st = fork && k ? G->sub[0] : main;
         LpArgs<R> a{};
         a.x = x;
         a.rhs = rhs;
@@ -494,7 +515,7 @@ static void matvec(gt_geometry* G, gt_operators* ops, const cx<R>* x, const cx<R
         a.tw0 = tw0_of<R>(o);
         a.tw1 = tw1_of<R>(o);
         a.spec = spec_of<R>(o);
-        a.T = T;
+        a.T = T + (fork && k ? (int64_t)ncol * G->maxT : 0);
         a.ldt = o.ld0;
         a.mask = G->geo.mask;
         a.col_op = col_op;
@@ -532,6 +553,10 @@ static void matvec(gt_geometry* G, gt_operators* ops, const cx<R>* x, const cx<R
         Scope s(P, sizeof(R) == 4 ? "tail_f32" : "tail_f64", st,
                 ncol * (double)sizeof(cx<R>) * (2.0 * (G->geo.n - nXY) + nXY));
         launch_tail<R>(G->geo, x, rhs, out, ld, ldo, ncol, col_op, ops->zcap, ops->zbr, mode, col_list, st);
+    }
+    if (fork) {
+        GT_CUDA(cudaEventRecord(G->join[0], G->sub[0]));
+        GT_CUDA(cudaStreamWaitEvent(main, G->join[0], 0));
     }
     if (G->narrow.nrow) {
         Scope s(P, "narrow", st);
@@ -786,7 +811,7 @@ static void fill_ws(Workspace& W, gt_geometry* G, int ncol, int m, int prec, int
     W.x64 = p.alloc<c64>((size_t)ncol * n);
     W.r64 = p.alloc<c64>((size_t)ncol * n);
     W.b64 = p.alloc<c64>((size_t)ncol * n);
-    W.T64 = p.alloc<c64>((size_t)ncol * G->maxT);
+    W.T64 = p.alloc<c64>(t_entries(G, ncol));
     W.rho = p.alloc<double>(ncol);
     W.bnorm = p.alloc<double>(ncol);
     const int nch = nchunks(n);
@@ -797,7 +822,7 @@ static void fill_ws(Workspace& W, gt_geometry* G, int ncol, int m, int prec, int
     if (prec == 2) W.vcur = p.alloc<unsigned char>((size_t)ncol * n * es);
     W.w = p.alloc<unsigned char>((size_t)ncol * n * es);
     W.z = p.alloc<unsigned char>((size_t)ncol * n * es);
-    W.T = p.alloc<unsigned char>((size_t)ncol * G->maxT * es);
+    W.T = p.alloc<unsigned char>(t_entries(G, ncol) * es);
     // the FP32 sweeps' interleaved vectors: whole pairs of columns per group, at most two columns for each
     const size_t wide = (size_t)(prec == 1 ? 1 : 2) * ncol;
     W.zfac = p.alloc<unsigned char>(wide * G->F.nfac * es);
@@ -2015,7 +2040,7 @@ int gt_apply(gt_geometry* G, gt_operators* ops, int32_t kind, int32_t precision,
             GT_CUDA(cudaMemcpy(xi, h32.data(), h32.size() * sizeof(c32), cudaMemcpyHostToDevice));
         }
         if (kind == 0 || kind == 2) {
-            cx<R>* T = tmp.alloc<cx<R>>((size_t)n_cols * G->maxT);
+            cx<R>* T = tmp.alloc<cx<R>>(t_entries(G, n_cols));
             matvec<R>(G, ops, xi, nullptr, yo, n, n, n_cols, d_op, kind == 0 ? 0 : 2, T, st);
         } else {
             std::vector<int> gptr, gslot, gop, gpair, all(n_cols);
