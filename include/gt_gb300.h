@@ -171,7 +171,7 @@ int gt_operators_create_shared(gt_geometry* g, int32_t n_ops, const double* omeg
                                const double* zcap, const double* zbr, const double* table, const int32_t* factor_of,
                                gt_operators** out);
 /* As gt_operators_create_shared with flags.  GT_OPS_FP32_PANELS: keep only the FP32 copies of the factor panels
- * (column- and row-major, 16 bytes per entry instead of 48): the FP64 factor is made in temporary memory and
+ * (for either sweep in the order its tiles read it, 16 bytes per entry instead of 48): the FP64 factor is made in temporary memory and
  * freed once converted, no FP64 row-major copy is made.  Such operators serve precision 0 and 2 solves and FP32
  * applications; precision 1 and 3, FP64 preconditioner applications and gt_operators_derive on them return
  * GT_INVALID_ARGUMENT.  A stiff set (see gt_solve_opts.precision) keeps its FP64 panels regardless.  For hosts
