@@ -3,10 +3,10 @@
 //
 // Classical Gram-Schmidt with one conditional re-orthogonalisation (DGKS: a second pass when the norm fell
 // below 0.7 of the product's, peec.py:3156-3159).  Dot products are reduced per warp by shuffles, per block
-// through shared memory in FP64, and across blocks by a second FP64 pass over per-block partials (fixed
-// order: results are reproducible).  The Hessenberg column, its Givens rotations and the least-squares
-// right-hand side live on the device in FP64 (peec.py:3160-3184); so does the decision that a slot's cycle
-// has converged.
+// through shared memory in FP64, and across blocks in FP64 by the slot's last block to finish, over per-block
+// partials in a fixed order: results are reproducible.  The Hessenberg column, its Givens rotations and the
+// least-squares right-hand side live on the device in FP64 (peec.py:3160-3184); so does the decision that a
+// slot's cycle has converged.  A basis of the arithmetic's own type is stored unnormalised (vinv: 1 / norm).
 #include <type_traits>
 #include "kernels.h"
 #include "solver.h"
