@@ -1,8 +1,7 @@
 // Launch interfaces between the kernel files and the host driver (api.cu).
 #pragma once
 #include "common.cuh"
-
-#include <vector>
+#include "sweep_plan.h"
 
 namespace gt {
 
@@ -164,24 +163,6 @@ struct Groups {
 };
 
 // --- FP32 sweeps in one launch (sweep.cu)
-struct alignas(16) SwTask {
-    int r0, h;             // outputs r0 .. r0 + h: rows of the front (forward) or own columns (backward)
-    int k0, k1;            // inner indices: own columns (forward), front rows (backward)
-    int dep, need;         // counter to wait on and the finished tiles it has to show
-    int sig;               // counter to raise when done
-    int nown, own0, voff;  // the front's own count, first factor index and place among the update vectors
-    int64_t goff;          // forward: the front's first row in the source table; backward: its first boundary entry
-    int64_t off;           // first panel entry
-};
-struct SweepPlanHost {
-    std::vector<SwTask> tasks;          // forward, leaves to root, then backward, root to leaves
-    int nft = 0, nbt = 0, nsrc = 0;
-    int64_t src_rows = 0, ptotal = 0;
-    std::vector<int> src, bidx;
-    std::vector<int> hf, hb;            // outputs per tile of each front
-    std::vector<int64_t> offf, offb;    // first entry of each front's tiles
-    std::vector<int> level_f, level_b;  // tasks up to the end of each level, in the order they run
-};
 struct SweepPlan {
     const SwTask* tasks;
     int nft, nbt, nsrc;
@@ -191,10 +172,6 @@ struct SweepPlan {
     const int *hf, *hb;
     const int64_t *offf, *offb;
 };
-SweepPlanHost make_sweep_plan(int nfront, int nlev, const int64_t* level_ptr, const int64_t* order, const int64_t* own_start,
-                              const int64_t* nown, const int64_t* nbnd, const int64_t* bnd_ptr, const int64_t* bnd_idx,
-                              const int64_t* child_ptr, const int64_t* child_idx, const int64_t* cmap_ptr,
-                              const int64_t* cmap_idx, const int64_t* vec_off);
 // tasks t0 .. t1 of the plan for every column group; cnt: sweep_counters ints, zero before the first launch of a sweep and
 // the first of them (the ticket counter) before each.
 // s: [slot][nfac]; z, y, u: interleaved by group (2 columns a pair, pair0 pairs before a group); sd: [slot][nnode]
