@@ -55,11 +55,13 @@ struct Timeout : std::runtime_error {
     using std::runtime_error::runtime_error;
 };
 
-// after a call's kernels have finished: did a bounded wait of the L_p pass or of the sweeps give up?
-static void check_device_waits() {
-    const bool lp = lp_take_wait_timeouts() != 0, sweep = sweep_take_wait_timeouts() != 0;
-    if (lp) throw Timeout("a TMA load of the L_p product's FFT grid did not arrive within its wait limit");
-    if (sweep) throw Timeout("a wait inside the preconditioner's triangular sweeps ran out");
+static const char* const SWEEP_RAN_OUT = "a wait inside the preconditioner's triangular sweeps ran out";
+
+// after a call's kernels have finished: did a bounded wait of the L_p pass or of the sweeps (their count) give up?
+static void check_device_waits(unsigned int sweep) {
+    if (lp_take_wait_timeouts())
+        throw Timeout("a TMA load of the L_p product's FFT grid did not arrive within its wait limit");
+    if (sweep) throw Timeout(SWEEP_RAN_OUT);
 }
 
 // Device allocations owned by an object, freed together.
@@ -219,6 +221,7 @@ struct Workspace {
     // the FP32 sweeps: solutions interleaved by column group (zfac, uvec likewise), and the tiles' counters
     c32* yint = nullptr;
     int* cnt = nullptr;
+    unsigned int *gave_up = nullptr, *gave_up_host = nullptr;    // their waits that ran out in the present call (host: pinned)
     c64* partial = nullptr;
     // precision 3: the FP32 inner solve's preconditioner applied in FP64 (input, output and the sweeps' vectors)
     c64 *pr64 = nullptr, *pz64 = nullptr, *zfac64 = nullptr, *yfac64 = nullptr, *uvec64 = nullptr, *sd64 = nullptr;
@@ -238,6 +241,7 @@ struct Workspace {
     int* its_col = nullptr;
     ~Workspace() {
         if (flag_host) cudaFreeHost(flag_host);
+        if (gave_up_host) cudaFreeHost(gave_up_host);
         if (togo_host) cudaFreeHost(togo_host);
         for (cudaEvent_t e : togo_ev)
             if (e) cudaEventDestroy(e);
@@ -567,11 +571,12 @@ static void matvec(gt_geometry* G, gt_operators* ops, const cx<R>* x, const cx<R
 
 // the FP32 sweeps over all groups: one launch, or, with the profiler's level timing, one per elimination level
 static void sweep32(gt_geometry* G, const gt_operators* ops, const Groups& grp, const c32* s, c32* z, c32* y, c32* u, c32* sd,
-                    int* cnt, int nslot, cudaStream_t st) {
+                    int* cnt, unsigned int* gave_up, int nslot, cudaStream_t st) {
     Profiler* P = &G->prof;
     const double es = sizeof(c32), panel = (double)grp.ngroup * es * G->F.panel_total, nfac = (double)G->F.nfac;
     auto run = [&](int t0, int t1) {
-        launch_sweep(G->sweep, G->F, ops->panel32, ops->panel32_b, ops->dinv32, s, z, y, u, sd, grp, cnt, t0, t1, st);
+        launch_sweep(G->sweep, G->F, ops->panel32, ops->panel32_b, ops->dinv32, s, z, y, u, sd, grp, cnt, gave_up, t0,
+                     t1, st);
     };
     const int nt = G->sweep.nft + G->sweep.nbt;
     if (!P->on || !P->levels) {
@@ -641,12 +646,12 @@ static void sweep64(gt_geometry* G, const gt_operators* ops, const Groups& grp, 
     }
 }
 
-// out = M^-1 r for nslot slots whose vectors are ldr apart (inputs) and ldo apart (outputs).  yint and cnt are the FP32
-// sweeps' (null in FP64)
+// out = M^-1 r for nslot slots whose vectors are ldr apart (inputs) and ldo apart (outputs).  yint, cnt and gave_up are the
+// FP32 sweeps' (null in FP64)
 template <typename R>
 static void precond(gt_geometry* G, gt_operators* ops, const cx<R>* r, int64_t ldr, cx<R>* out, int64_t ldo, int nslot,
                     const int* slot_op, const Groups& grp, int gmax, cx<R>* zfac, cx<R>* yfac, cx<R>* uvec, cx<R>* sd,
-                    c32* yint, int* cnt, cudaStream_t st, const int* col_list = nullptr,
+                    c32* yint, int* cnt, unsigned int* gave_up, cudaStream_t st, const int* col_list = nullptr,
                     const double* rscale = nullptr) {
     constexpr bool f32 = sizeof(R) == 4;
     Profiler* P = &G->prof;
@@ -659,7 +664,7 @@ static void precond(gt_geometry* G, gt_operators* ops, const cx<R>* r, int64_t l
         launch_pc_node<R>(G->geo, r, ldr, yfac, nslot, slot_op, tab_of<R>(ops), col_list, f32 ? cnt : nullptr,
                           f32 ? sweep_counters(G->F.nfront, grp.ngroup) : 0, rscale, st);
     }
-    if constexpr (f32) sweep32(G, ops, grp, yfac, zfac, yint, uvec, sd, cnt, nslot, st);
+    if constexpr (f32) sweep32(G, ops, grp, yfac, zfac, yint, uvec, sd, cnt, gave_up, nslot, st);
     else sweep64(G, ops, grp, gmax, yfac, zfac, uvec, sd, nslot, st);
     if (ops->nlow) {
         // the derived stack's added branches: y -= W Minv U^T y (the coefficients in zfac, free after the sweeps)
@@ -735,6 +740,8 @@ static void lowrank_w(gt_geometry* G, const gt_operators* base, int nf, int k, c
     cx<R>* uv = tmp.alloc<cx<R>>((size_t)wide * std::max<int64_t>(G->F.vec_total, 1));
     c32* yv = f32 ? tmp.alloc<c32>((size_t)wide * nfac) : nullptr;
     int* cnt = f32 ? tmp.alloc<int>(sweep_counters(G->F.nfront, bc)) : nullptr;
+    unsigned int* gave_up = f32 ? tmp.alloc<unsigned int>(1) : nullptr;
+    if (f32) GT_CUDA(cudaMemsetAsync(gave_up, 0, sizeof(unsigned int), st));
     int* d_gptr = tmp.alloc<int>(bc + 1);
     int* d_gslot = tmp.alloc<int>(bc);
     int* d_gop = tmp.alloc<int>(bc);
@@ -758,8 +765,8 @@ static void lowrank_w(gt_geometry* G, const gt_operators* base, int nf, int k, c
         const Groups grp{(int)gop.size(), d_gptr, d_gslot, d_gop, d_gpair};
         if constexpr (f32) {
             GT_CUDA(cudaMemsetAsync(cnt, 0, sweep_counters(G->F.nfront, grp.ngroup) * sizeof(int), st));
-            launch_sweep(G->sweep, G->F, base->panel32, base->panel32_b, base->dinv32, sv, zv, yv, uv, wout, grp, cnt, 0,
-                         G->sweep.nft + G->sweep.nbt, st);
+            launch_sweep(G->sweep, G->F, base->panel32, base->panel32_b, base->dinv32, sv, zv, yv, uv, wout, grp, cnt, gave_up,
+                         0, G->sweep.nft + G->sweep.nbt, st);
         } else {
             const int nlev = (int)G->level_ptr.size() - 1;
             for (int h = 0; h < nlev; ++h)
@@ -771,6 +778,11 @@ static void lowrank_w(gt_geometry* G, const gt_operators* base, int nf, int k, c
                                     G->level_maxnf[h], G->level_maxnown[h], base->panel64_rm, zv, sv, wout, grp, gmax, st);
         }
         GT_CUDA(cudaStreamSynchronize(st));   // the group tables are reused by the next batch
+    }
+    if (f32) {
+        unsigned int h = 0;
+        GT_CUDA(cudaMemcpy(&h, gave_up, sizeof(h), cudaMemcpyDeviceToHost));
+        if (h) throw Timeout(SWEEP_RAN_OUT);
     }
 }
 
@@ -832,6 +844,7 @@ static void fill_ws(Workspace& W, gt_geometry* G, int ncol, int m, int prec, int
         W.yint = p.alloc<c32>(wide * G->F.nfac);
         W.cnt = p.alloc<int>(sweep_counters(G->F.nfront, ncol));
     }
+    W.gave_up = p.alloc<unsigned int>(1);
     // node-ordered s / y of the preconditioner: entries of nodes that are not kept stay zero
     W.sd = p.alloc<unsigned char>((size_t)ncol * G->F.nnode * es);
     if (!dry) GT_CUDA(cudaMemsetAsync(W.sd, 0, (size_t)ncol * G->F.nnode * es, st));
@@ -876,6 +889,7 @@ static void fill_ws(Workspace& W, gt_geometry* G, int ncol, int m, int prec, int
     W.done = p.alloc<int>(ncol);
     if (!dry) {
         GT_CUDA(cudaMemsetAsync(W.done, 0, ncol * sizeof(int), st));
+        GT_CUDA(cudaMallocHost(&W.gave_up_host, sizeof(unsigned int)));
         GT_CUDA(cudaMallocHost(&W.togo_host, (size_t)m * ncol * sizeof(double)));
         for (cudaEvent_t& e : W.togo_ev) GT_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
@@ -914,6 +928,7 @@ static int solve_impl(gt_geometry* G, gt_operators* ops, int ncol, const int* h_
     Profiler* P = &G->prof;
     GT_CUDA(cudaMemcpyAsync(W.col_op, h_col_op, ncol * sizeof(int), cudaMemcpyHostToDevice, st));
     GT_CUDA(cudaMemsetAsync(W.its_col, 0, ncol * sizeof(int), st));
+    GT_CUDA(cudaMemsetAsync(W.gave_up, 0, sizeof(unsigned int), st));
     norms64(G, W.b64, n, ncol, W.bnorm, st);
     if (o.use_guess) {
         // x holds the starting points: r = b - K x in FP64
@@ -949,12 +964,13 @@ static int solve_impl(gt_geometry* G, gt_operators* ops, int ncol, const int* h_
             if (pc64) {
                 launch_recast<double, float>(W.pr64, n, rin, ldr, list, n, nsl, rscale, st);
                 precond<double>(G, ops, W.pr64, n, W.pz64, n, nsl, W.slot_pc, g, gmax, W.zfac64, W.yfac64, W.uvec64,
-                                W.sd64, nullptr, nullptr, st, list);
+                                W.sd64, nullptr, nullptr, nullptr, st, list);
                 launch_recast<float, double>(out, n, W.pz64, n, list, n, nsl, nullptr, st);
                 return;
             }
         }
-        precond<R>(G, ops, rin, ldr, out, n, nsl, W.slot_pc, g, gmax, zfac, yfac, uvec, sd, W.yint, W.cnt, st, list, rscale);
+        precond<R>(G, ops, rin, ldr, out, n, nsl, W.slot_pc, g, gmax, zfac, yfac, uvec, sd, W.yint, W.cnt, W.gave_up, st, list,
+                   rscale);
     };
     std::vector<int> slot_col, slot_op, slot_pc, gptr, gslot, gop, gpair, act;
     auto upload_groups = [&](const std::vector<int>& slots) {
@@ -1184,6 +1200,20 @@ static int run_solve(gt_geometry* G, gt_operators* ops, int ncol, const int* col
     }
     if (o.precision != 0) throw Invalid("precision must be 0, 1, 2 or 3");
     return solve_impl<float>(G, ops, ncol, col_op, o, its, res, st);
+}
+
+// The end of a solve on st.  One whose waits ran out has left what it was given by then in the workspace, among it the basis
+// vectors that later solves take zero times: the workspace goes, and the next solve makes a new one.
+static void finish_solve(gt_geometry* G, cudaStream_t st) {
+    Workspace& W = *G->ws;
+    GT_CUDA(cudaMemcpyAsync(W.gave_up_host, W.gave_up, sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
+    GT_CUDA(cudaStreamSynchronize(st));
+    try {
+        check_device_waits(*W.gave_up_host);
+    } catch (const Timeout&) {
+        G->ws.reset();
+        throw;
+    }
 }
 
 // precision 0 becomes 3 when a column's factorisation is stiff and the FP64 sweeps fit its fronts
@@ -1941,8 +1971,7 @@ int gt_solve_device(gt_geometry* G, gt_operators* ops, int32_t n_cols, const int
         GT_CUDA(cudaMemcpyAsync(W.x64, x_device, (size_t)n_cols * G->geo.n * sizeof(c64), cudaMemcpyDeviceToDevice, st));
     int rc = run_solve(G, ops, n_cols, col_op, opts, its_out, resid_out, st);
     GT_CUDA(cudaMemcpyAsync(x_device, W.x64, (size_t)n_cols * G->geo.n * sizeof(c64), cudaMemcpyDeviceToDevice, st));
-    GT_CUDA(cudaStreamSynchronize(st));
-    check_device_waits();
+    finish_solve(G, st);
     if (rc != GT_OK) gt::set_error("GMRES did not converge for at least one column");
     return rc;
     GT_GUARD_END
@@ -1973,8 +2002,7 @@ int gt_solve(gt_geometry* G, gt_operators* ops, int32_t n_cols, const int32_t* c
     int rc = run_solve(G, ops, n_cols, col_op, opts, its_out, resid_out, st);
     launch_gather(G->d_c2d, nc, W.x64, G->geo.n, d_c, nc, n_cols, st);
     GT_CUDA(cudaMemcpyAsync(x_out, d_c, (size_t)n_cols * nc * sizeof(c64), cudaMemcpyDeviceToHost, st));
-    GT_CUDA(cudaStreamSynchronize(st));
-    check_device_waits();
+    finish_solve(G, st);
     if (rc != GT_OK) gt::set_error("GMRES did not converge for at least one column");
     return rc;
     GT_GUARD_END
@@ -2021,6 +2049,9 @@ int gt_apply(gt_geometry* G, gt_operators* ops, int32_t kind, int32_t precision,
     // kind 1 groups columns by factorisation: require them sorted
     for (int c = 1; c < n_cols; ++c)
         if (kind == 1 && h_pc[c] < h_pc[c - 1]) throw Invalid("preconditioner columns must be sorted by operator");
+    unsigned int* gave_up = tmp.alloc<unsigned int>(1);
+    unsigned int h_gave_up = 0;
+    GT_CUDA(cudaMemsetAsync(gave_up, 0, sizeof(unsigned int), st));
     auto run = [&](auto tag) {
         using R = decltype(tag);
         cx<R>* xi;
@@ -2060,7 +2091,7 @@ int gt_apply(gt_geometry* G, gt_operators* ops, int32_t kind, int32_t precision,
             int* cnt = f32 ? tmp.alloc<int>(sweep_counters(G->F.nfront, n_cols)) : nullptr;
             cx<R>* sdv = tmp.alloc<cx<R>>((size_t)n_cols * G->F.nnode);
             GT_CUDA(cudaMemsetAsync(sdv, 0, (size_t)n_cols * G->F.nnode * sizeof(cx<R>), st));
-            precond<R>(G, ops, xi, n, yo, n, n_cols, d_pc, grp, gmax, zf, yf, uv, sdv, yi, cnt, st);
+            precond<R>(G, ops, xi, n, yo, n, n_cols, d_pc, grp, gmax, zf, yf, uv, sdv, yi, cnt, gave_up, st);
         }
         if constexpr (sizeof(R) == 4) {
             std::vector<c32> h32((size_t)n_cols * n);
@@ -2075,8 +2106,9 @@ int gt_apply(gt_geometry* G, gt_operators* ops, int32_t kind, int32_t precision,
     else run(float{});
     launch_gather(G->d_c2d, nc, yout, n, d_c, nc, n_cols, st);
     GT_CUDA(cudaMemcpyAsync(y, d_c, (size_t)n_cols * nc * sizeof(c64), cudaMemcpyDeviceToHost, st));
+    GT_CUDA(cudaMemcpyAsync(&h_gave_up, gave_up, sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
     GT_CUDA(cudaStreamSynchronize(st));
-    check_device_waits();
+    check_device_waits(h_gave_up);
     return GT_OK;
     GT_GUARD_END
 }

@@ -173,13 +173,12 @@ struct SweepPlan {
     const int64_t *offf, *offb;
 };
 // tasks t0 .. t1 of the plan for every column group; cnt: sweep_counters ints, zero before the first launch of a sweep and
-// the first of them (the ticket counter) before each.
+// the first of them (the ticket counter) before each.  gave_up: counts the waits that ran out, in memory of the call's own
+// (a word that calls shared would end the others' waits, and be read and cleared by whichever came first).
 // s: [slot][nfac]; z, y, u: interleaved by group (2 columns a pair, pair0 pairs before a group); sd: [slot][nnode]
 inline int64_t sweep_counters(int nfront, int ngroup) { return 1 + 3 * (int64_t)nfront * ngroup; }
 void launch_sweep(const SweepPlan& S, const Fronts& F, const c32* pf, const c32* pb, const c32* dinv, const c32* s, c32* z,
-                  c32* y, c32* u, c32* sd, const Groups& G, int* cnt, int t0, int t1, cudaStream_t st);
-// waits of the sweep that gave up since the last call (and clears the count); read once the kernels are done
-unsigned int sweep_take_wait_timeouts();
+                  c32* y, c32* u, c32* sd, const Groups& G, int* cnt, unsigned int* gave_up, int t0, int t1, cudaStream_t st);
 // the solve panels: own blocks get a unit diagonal and zeros above it (pivot reciprocals to d64 / d32,
 // [op][nfac]); the FP32 sweeps' forward and backward tiles (pf, pb) and the FP64 row-major copy
 // the small fronts of a level: from assembly to the finished solve panels (small_front_smem bytes for the largest; r64 null:

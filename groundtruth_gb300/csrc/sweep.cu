@@ -27,6 +27,7 @@
 #include "kernels.h"
 
 #include <algorithm>
+#include <cstdlib>
 #include <map>
 #include <mutex>
 
@@ -40,6 +41,7 @@ constexpr int SW_STAGE_ENT = 1792;     // panel entries per stage (14 KB)
 constexpr int SW_XROWS = 256;          // inner rows staged at once (16 KB at 8 columns)
 constexpr int SW_HMAX = 128;
 constexpr long long SW_WAIT_CYCLES = 4000000000ll;       // two seconds
+constexpr long long SW_TEST_WAIT_CYCLES = 2000000ll;     // a millisecond, where a test makes a wait run out
 constexpr uint32_t SW_POLLS = 1u << 28;
 
 struct SwDesc {                        // one ring stage, written by the producer
@@ -62,8 +64,6 @@ struct alignas(16) SwShared {
 };
 static_assert(SW_XROWS * 4 >= 2 * SWT * 4, "the partial sums take the staged rows' place");
 
-__device__ unsigned int g_sweep_timeouts = 0;
-
 __device__ __forceinline__ uint32_t sw_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ bool sw_try(uint32_t bar, uint32_t parity) {
     uint32_t ok;
@@ -71,10 +71,10 @@ __device__ __forceinline__ bool sw_try(uint32_t bar, uint32_t parity) {
                  "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
-// a wait that gives up is counted, and everything after it goes on without its inputs: the launch ends and the
-// host reports GT_TIMEOUT
-__device__ __noinline__ void sw_gave_up() { atomicAdd(&g_sweep_timeouts, 1u); }
-__device__ __forceinline__ void sw_wait_bar(uint64_t* b, uint32_t parity) {
+// a wait that gives up is counted in the call's own word (gave_up), and everything after it goes on without its inputs: the
+// launch ends and the host reports GT_TIMEOUT
+__device__ __noinline__ void sw_gave_up(unsigned int* gave_up) { atomicAdd(gave_up, 1u); }
+__device__ __forceinline__ void sw_wait_bar(uint64_t* b, uint32_t parity, unsigned int* gave_up) {
     const uint32_t bar = sw_smem(b);
     if (sw_try(bar, parity)) return;
     const long long t0 = clock64();
@@ -82,25 +82,25 @@ __device__ __forceinline__ void sw_wait_bar(uint64_t* b, uint32_t parity) {
         if (sw_try(bar, parity)) return;
         if (clock64() - t0 > 2 * SW_WAIT_CYCLES) break;
     }
-    sw_gave_up();
+    sw_gave_up(gave_up);
 }
 __device__ __forceinline__ int sw_acquire(const int* p) {
     int v;
     asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ void sw_wait_count(const int* p, int need) {
+__device__ __forceinline__ void sw_wait_count(const int* p, int need, unsigned int* gave_up, long long limit) {
     if (sw_acquire(p) >= need) return;
     const long long t0 = clock64();
     for (uint32_t it = 0; it < SW_POLLS; ++it) {
         if (sw_acquire(p) >= need) return;
         if ((it & 63) == 63) {
-            if (*(volatile unsigned int*)&g_sweep_timeouts) return;      // someone gave up already
-            if (clock64() - t0 > SW_WAIT_CYCLES) break;
+            if (*(volatile unsigned int*)gave_up) return;        // someone of this call gave up already
+            if (clock64() - t0 > limit) break;
         }
         __nanosleep(32);
     }
-    sw_gave_up();
+    sw_gave_up(gave_up);
 }
 __device__ __forceinline__ void sw_sync() { asm volatile("bar.sync 1, %0;" ::"n"(SWT) : "memory"); }
 
@@ -158,6 +158,9 @@ struct SwArgs {
     int* cnt;                          // [counter][ngroup] finished tiles
     int* ticket;                       // this launch's ticket counter
     int t0, t1;                        // tickets of this launch
+    unsigned int* gave_up;             // the call's count of waits that ran out
+    long long wait;                    // the limit of the waits for tiles, in clock cycles
+    int surplus;                       // 0, except when a test makes the waits run out: tiles waited for that nobody finishes
 };
 
 // where the partial sum of row pair row2, entry e = row * NP + pair, stands: the entries of a row pair permuted by the row
@@ -307,7 +310,7 @@ __device__ void sw_task(const SwArgs& A, SwShared& sm, uint32_t& it, const SwDes
             sm.ext[tid + i * SWT] = make_float4(d.x, d.y, 0.f, 0.f);
         }
         if (nsrc) {
-            if (tid == 0) sw_wait_count(A.cnt + (int64_t)t.dep * ng + g, t.need);
+            if (tid == 0) sw_wait_count(A.cnt + (int64_t)t.dep * ng + g, t.need + A.surplus, A.gave_up, A.wait);
             sw_sync();
             sw_add_children<NP, HE>(A, nsrc, t.goff + t.r0, h, lo, sm.hrow[0], sm.hrow[1], u, sm.ext, tid);
             sw_add_children<NP, XE>(A, nsrc, t.goff + t.k0, xend - xbeg, 0, sm.xrow[0], sm.xrow[1], u, sm.x, tid);
@@ -317,7 +320,7 @@ __device__ void sw_task(const SwArgs& A, SwShared& sm, uint32_t& it, const SwDes
 #pragma unroll
         for (int i = 0; i < HE; ++i)
             if (rt + i * RS < h) sm.ext[tid + i * SWT].x = __int_as_float((int)A.iperm[t.own0 + t.r0 + rt + i * RS]);
-        if (tid == 0 && t.need > 0) sw_wait_count(A.cnt + (int64_t)t.dep * ng + g, t.need);
+        if (tid == 0 && t.need > 0) sw_wait_count(A.cnt + (int64_t)t.dep * ng + g, t.need + A.surplus, A.gave_up, A.wait);
         sw_sync();
         sw_stage_back<NP, XE>(z, y, xend - xbeg, t.nown - xbeg, sm.xrow[0], sm.x, tid);
     }
@@ -331,7 +334,7 @@ __device__ void sw_task(const SwArgs& A, SwShared& sm, uint32_t& it, const SwDes
     do {
         const int slot = it % SW_STAGES;
         const SwDesc& d = sm.desc[slot];
-        sw_wait_bar(&sm.full[slot], (it / SW_STAGES) & 1);
+        sw_wait_bar(&sm.full[slot], (it / SW_STAGES) & 1, A.gave_up);
         const int ka = d.ka, kb = d.kb;
         last = d.last;
         const float2* ring = sm.ring[slot];
@@ -443,7 +446,7 @@ __global__ void __launch_bounds__(SW_BLOCK, 4) sweep_kernel(SwArgs A) {
             int k = t.k0;
             do {
                 const int slot = it % SW_STAGES;
-                if (it >= SW_STAGES) sw_wait_bar(&sm.empty[slot], (it / SW_STAGES - 1) & 1);
+                if (it >= SW_STAGES) sw_wait_bar(&sm.empty[slot], (it / SW_STAGES - 1) & 1, A.gave_up);
                 SwDesc& d = sm.desc[slot];
                 const int e = min(t.k1, k + step);
                 d.f_dir = dir;
@@ -471,7 +474,7 @@ __global__ void __launch_bounds__(SW_BLOCK, 4) sweep_kernel(SwArgs A) {
     uint32_t it = 0;
     for (;;) {
         const int slot = it % SW_STAGES;
-        sw_wait_bar(&sm.full[slot], (it / SW_STAGES) & 1);
+        sw_wait_bar(&sm.full[slot], (it / SW_STAGES) & 1, A.gave_up);
         const SwDesc& d = sm.desc[slot];
         if (d.f_dir < 0) return;
         switch (A.G.pair0[d.g + 1] - A.G.pair0[d.g]) {
@@ -480,13 +483,6 @@ __global__ void __launch_bounds__(SW_BLOCK, 4) sweep_kernel(SwArgs A) {
             default: sw_task<4>(A, sm, it, d); break;
         }
     }
-}
-
-unsigned int sweep_take_wait_timeouts() {
-    unsigned int h = 0, zero_v = 0;
-    GT_CUDA(cudaMemcpyFromSymbol(&h, g_sweep_timeouts, sizeof(h)));
-    if (h) GT_CUDA(cudaMemcpyToSymbol(g_sweep_timeouts, &zero_v, sizeof(zero_v)));
-    return h;
 }
 
 // blocks of the sweep kernel the current device holds at once
@@ -507,7 +503,7 @@ static int resident_blocks() {
 }
 
 void launch_sweep(const SweepPlan& S, const Fronts& F, const c32* pf, const c32* pb, const c32* dinv, const c32* s, c32* z,
-                  c32* y, c32* u, c32* sd, const Groups& G, int* cnt, int t0, int t1, cudaStream_t st) {
+                  c32* y, c32* u, c32* sd, const Groups& G, int* cnt, unsigned int* gave_up, int t0, int t1, cudaStream_t st) {
     SwArgs A{};
     A.tasks = S.tasks;
     A.nft = S.nft;
@@ -534,6 +530,11 @@ void launch_sweep(const SweepPlan& S, const Fronts& F, const c32* pf, const c32*
     A.ticket = cnt;
     A.t0 = t0 * G.ngroup;
     A.t1 = t1 * G.ngroup;
+    const char* test = std::getenv("GT_SWEEP_TEST_SHORTFALL");
+    const bool shortfall = test && test[0] == '1';
+    A.gave_up = gave_up;
+    A.wait = shortfall ? SW_TEST_WAIT_CYCLES : SW_WAIT_CYCLES;
+    A.surplus = shortfall ? 1 : 0;
     const int64_t tickets = (int64_t)(t1 - t0) * G.ngroup;
     if (tickets <= 0) return;
     raise_smem((const void*)sweep_kernel, sizeof(SwShared));
