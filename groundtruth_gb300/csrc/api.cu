@@ -1167,7 +1167,9 @@ static int solve_impl(gt_geometry* G, gt_operators* ops, int ncol, const int* h_
         verified = false;
         GT_CUDA(cudaMemcpyAsync(h_rho.data(), W.rho, ncol * sizeof(double), cudaMemcpyDeviceToHost, st));
         GT_CUDA(cudaMemcpyAsync(its_slot.data(), S.its_total, ns * sizeof(int), cudaMemcpyDeviceToHost, st));
+        GT_CUDA(cudaMemcpyAsync(W.gave_up_host, W.gave_up, sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
         GT_CUDA(cudaStreamSynchronize(st));
+        if (*W.gave_up_host) break;                     // (the caller reports it)
         for (int s = 0; s < ns; ++s) h_its[slot_col[s]] = its_slot[s];
         P->flush(st);
     }

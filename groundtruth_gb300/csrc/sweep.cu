@@ -44,11 +44,10 @@ constexpr long long SW_WAIT_CYCLES = 4000000000ll;       // two seconds
 constexpr long long SW_TEST_WAIT_CYCLES = 2000000ll;     // a millisecond, where a test makes a wait run out
 constexpr uint32_t SW_POLLS = 1u << 28;
 
-struct SwDesc {                        // one ring stage, written by the producer
+struct SwDesc {                        // a task, written by the producer beside its first ring stage
     int f_dir;                         // 0 forward, 1 backward, -1 no more work
     int g;                             // column group
-    int ka, kb;                        // inner range of the stage
-    int first, last;
+    int step;                          // inner indices per stage
     SwTask t;
 };
 
@@ -61,6 +60,7 @@ struct alignas(16) SwShared {
     int hrow[2][SW_HMAX];              // forward: the outputs' sources
     SwDesc desc[SW_STAGES];
     uint64_t full[SW_STAGES], empty[SW_STAGES];
+    int quit;                          // a consumer has not got the next task: the block leaves
 };
 static_assert(SW_XROWS * 4 >= 2 * SWT * 4, "the partial sums take the staged rows' place");
 
@@ -71,18 +71,38 @@ __device__ __forceinline__ bool sw_try(uint32_t bar, uint32_t parity) {
                  "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
-// a wait that gives up is counted in the call's own word (gave_up), and everything after it goes on without its inputs: the
-// launch ends and the host reports GT_TIMEOUT
+// Waits are bounded.  One that gives up is counted in the call's own word (gave_up), which ends the call's other waits, and
+// the host reports GT_TIMEOUT.  What follows a wait that gave up stays in bounds and leads to the launch's end:
+//   for another tile's results (sw_wait_count)   the tile is made from what is there
+//   for a task's first stage (full)              its descriptor may not be there: sm.quit, which all of the block's consumers
+//                                                look at behind the task's second barrier, and leave
+//   for a further stage of a task (full)         the tile is made from what is there, the number of its stages being the
+//                                                task's; the consumers leave as they do without the next descriptor, which is
+//                                                not looked for: a thread that went on without a stage may be ahead by the
+//                                                whole ring, where a barrier's parity takes an old stage for the one it wants
+//   for a stage to be read (empty)               the producer stops, as it does before a stage whose last copy is not
+//                                                complete, and waits once more for its copies in flight before it leaves
 __device__ __noinline__ void sw_gave_up(unsigned int* gave_up) { atomicAdd(gave_up, 1u); }
-__device__ __forceinline__ void sw_wait_bar(uint64_t* b, uint32_t parity, unsigned int* gave_up) {
-    const uint32_t bar = sw_smem(b);
-    if (sw_try(bar, parity)) return;
+__device__ __noinline__ bool sw_wait_slow(uint32_t bar, uint32_t parity, unsigned int* gave_up, long long limit) {
     const long long t0 = clock64();
     for (uint32_t it = 0; it < SW_POLLS; ++it) {
-        if (sw_try(bar, parity)) return;
-        if (clock64() - t0 > 2 * SW_WAIT_CYCLES) break;
+        if (sw_try(bar, parity)) return true;
+        if ((it & 1023) == 1023 && *(volatile unsigned int*)gave_up) return false;
+        if (clock64() - t0 > 2 * limit) break;
     }
     sw_gave_up(gave_up);
+    return false;
+}
+__device__ __forceinline__ bool sw_wait_bar(uint64_t* b, uint32_t parity, unsigned int* gave_up, long long limit) {
+    const uint32_t bar = sw_smem(b);
+    return sw_try(bar, parity) || sw_wait_slow(bar, parity, gave_up, limit);
+}
+// a wait without a count and whatever the word says: the copies in flight of a block that leaves
+__device__ __noinline__ void sw_drain(uint64_t* b, uint32_t parity, long long limit) {
+    const uint32_t bar = sw_smem(b);
+    const long long t0 = clock64();
+    for (uint32_t it = 0; it < SW_POLLS; ++it)
+        if (sw_try(bar, parity) || clock64() - t0 > limit) return;
 }
 __device__ __forceinline__ int sw_acquire(const int* p) {
     int v;
@@ -159,8 +179,9 @@ struct SwArgs {
     int* ticket;                       // this launch's ticket counter
     int t0, t1;                        // tickets of this launch
     unsigned int* gave_up;             // the call's count of waits that ran out
-    long long wait;                    // the limit of the waits for tiles, in clock cycles
-    int surplus;                       // 0, except when a test makes the waits run out: tiles waited for that nobody finishes
+    long long wait;                    // the limit of the waits for tiles, in clock cycles; those for stages have twice as long
+    int surplus, missing;              // 0, except when a test makes waits run out: tiles that nobody finishes, bytes of a stage
+                                       // that no copy brings
 };
 
 // where the partial sum of row pair row2, entry e = row * NP + pair, stands: the entries of a row pair permuted by the row
@@ -267,11 +288,12 @@ __device__ __forceinline__ void sw_back_rows(const int* bidx, int own0, int nown
     }
 }
 
+// false: one of the consumers did not get here with the task.  bad: this thread went on without a stage
 template <int NP>
-__device__ void sw_task(const SwArgs& A, SwShared& sm, uint32_t& it, const SwDesc& d0) {
+__device__ bool sw_task(const SwArgs& A, SwShared& sm, uint32_t& it, const SwDesc& d0, bool& bad) {
     const int tid = threadIdx.x;
     const SwTask t = d0.t;
-    const int dir = d0.f_dir, g = d0.g, ng = A.G.ngroup;
+    const int dir = d0.f_dir, g = d0.g, step = d0.step, ng = A.G.ngroup;
     const int* gs = A.G.gslot + A.G.gptr[g];
     const int gc = A.G.gptr[g + 1] - A.G.gptr[g];
     const int64_t gb = A.G.pair0[g];                     // column pairs before this group's
@@ -314,6 +336,8 @@ __device__ void sw_task(const SwArgs& A, SwShared& sm, uint32_t& it, const SwDes
             sw_sync();
             sw_add_children<NP, HE>(A, nsrc, t.goff + t.r0, h, lo, sm.hrow[0], sm.hrow[1], u, sm.ext, tid);
             sw_add_children<NP, XE>(A, nsrc, t.goff + t.k0, xend - xbeg, 0, sm.xrow[0], sm.xrow[1], u, sm.x, tid);
+        } else {
+            sw_sync();
         }
     } else {
         sw_back_rows(A.bidx + t.goff, t.own0, t.nown, xbeg, xend - xbeg, sm.xrow[0], tid);
@@ -325,18 +349,17 @@ __device__ void sw_task(const SwArgs& A, SwShared& sm, uint32_t& it, const SwDes
         sw_stage_back<NP, XE>(z, y, xend - xbeg, t.nown - xbeg, sm.xrow[0], sm.x, tid);
     }
     sw_sync();
+    if (*(const volatile int*)&sm.quit) return false;
     uint64_t re[2][NP], im[2][NP];
 #pragma unroll
     for (int r = 0; r < 2; ++r)
 #pragma unroll
         for (int p = 0; p < NP; ++p) re[r][p] = im[r][p] = 0;
-    bool last;
+    int ka = t.k0;
     do {
         const int slot = it % SW_STAGES;
-        const SwDesc& d = sm.desc[slot];
-        sw_wait_bar(&sm.full[slot], (it / SW_STAGES) & 1, A.gave_up);
-        const int ka = d.ka, kb = d.kb;
-        last = d.last;
+        bad |= !sw_wait_bar(&sm.full[slot], (it / SW_STAGES) & 1, A.gave_up, A.wait);
+        const int kb = min(t.k1, ka + step);
         const float2* ring = sm.ring[slot];
         for (int k = ka; k < kb;) {
             if (k >= xend) {
@@ -371,10 +394,11 @@ __device__ void sw_task(const SwArgs& A, SwShared& sm, uint32_t& it, const SwDes
             k = e;
         }
         ++it;
+        ka = kb;
         __syncwarp();
         if ((tid & 31) == 0)
             asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sw_smem(&sm.empty[slot])) : "memory");
-    } while (!last);
+    } while (ka < t.k1);
     // the segments' partial sums meet in the staged rows' place
     sw_sync();
     if (act) {
@@ -409,6 +433,7 @@ __device__ void sw_task(const SwArgs& A, SwShared& sm, uint32_t& it, const SwDes
     // (the release carries the whole block's outputs, ordered before it by the barrier)
     if (tid == 0 && t.sig >= 0)
         asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(A.cnt + (int64_t)t.sig * ng + g) : "memory");
+    return true;
 }
 
 __global__ void __launch_bounds__(SW_BLOCK, 4) sweep_kernel(SwArgs A) {
@@ -416,6 +441,7 @@ __global__ void __launch_bounds__(SW_BLOCK, 4) sweep_kernel(SwArgs A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SwShared& sm = *reinterpret_cast<SwShared*>(smem_raw);
     if (threadIdx.x == 0) {
+        sm.quit = 0;
         for (int s = 0; s < SW_STAGES; ++s) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sw_smem(&sm.full[s])) : "memory");
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(sw_smem(&sm.empty[s])), "r"(SWW) : "memory");
@@ -428,7 +454,7 @@ __global__ void __launch_bounds__(SW_BLOCK, 4) sweep_kernel(SwArgs A) {
         if (threadIdx.x != SWT) return;
         // the producer: tickets in order, each task's panel run stage by stage
         uint32_t it = 0;
-        for (;;) {
+        for (bool go = true; go;) {
             const int tk = A.t0 + atomicAdd(A.ticket, 1);
             const bool done = tk >= A.t1;
             SwTask t{};
@@ -446,19 +472,24 @@ __global__ void __launch_bounds__(SW_BLOCK, 4) sweep_kernel(SwArgs A) {
             int k = t.k0;
             do {
                 const int slot = it % SW_STAGES;
-                if (it >= SW_STAGES) sw_wait_bar(&sm.empty[slot], (it / SW_STAGES - 1) & 1, A.gave_up);
-                SwDesc& d = sm.desc[slot];
+                if (it >= SW_STAGES) {
+                    const uint32_t prev = (it / SW_STAGES - 1) & 1;
+                    if (!sw_wait_bar(&sm.empty[slot], prev, A.gave_up, A.wait) || !sw_try(sw_smem(&sm.full[slot]), prev)) {
+                        go = false;
+                        break;
+                    }
+                }
                 const int e = min(t.k1, k + step);
-                d.f_dir = dir;
-                d.g = g;
-                d.ka = k;
-                d.kb = e;
-                d.first = k == t.k0;
-                d.last = e >= t.k1;
-                if (d.first) d.t = t;
+                if (k == t.k0) {
+                    SwDesc& d = sm.desc[slot];
+                    d.f_dir = dir;
+                    d.g = g;
+                    d.step = step;
+                    d.t = t;
+                }
                 const uint32_t bytes = (uint32_t)(e - k) * hp * sizeof(float2), bar = sw_smem(&sm.full[slot]);
                 if (bytes) {
-                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes + A.missing) : "memory");
                     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                                  ::"r"(sw_smem(sm.ring[slot])), "l"(src + (int64_t)(k - t.k0) * hp), "r"(bytes), "r"(bar)
                                  : "memory");
@@ -468,20 +499,31 @@ __global__ void __launch_bounds__(SW_BLOCK, 4) sweep_kernel(SwArgs A) {
                 ++it;
                 k = e;
             } while (k < t.k1);
-            if (done) return;
+            if (done) go = false;
         }
+        for (uint32_t q = it - min(it, (uint32_t)SW_STAGES); q < it; ++q)
+            sw_drain(&sm.full[q % SW_STAGES], (q / SW_STAGES) & 1, A.wait);
+        return;
     }
     uint32_t it = 0;
+    bool bad = false;
     for (;;) {
         const int slot = it % SW_STAGES;
-        sw_wait_bar(&sm.full[slot], (it / SW_STAGES) & 1, A.gave_up);
+        const bool here = __all_sync(0xffffffffu, !bad && sw_wait_bar(&sm.full[slot], (it / SW_STAGES) & 1, A.gave_up, A.wait));
         const SwDesc& d = sm.desc[slot];
-        if (d.f_dir < 0) return;
-        switch (A.G.pair0[d.g + 1] - A.G.pair0[d.g]) {
-            case 1: sw_task<1>(A, sm, it, d); break;
-            case 2: sw_task<2>(A, sm, it, d); break;
-            default: sw_task<4>(A, sm, it, d); break;
+        if (!here) sm.quit = 1;
+        if (!here || d.f_dir < 0) {                      // (the barriers of those that have a task)
+            sw_sync();
+            sw_sync();
+            return;
         }
+        bool go;
+        switch (A.G.pair0[d.g + 1] - A.G.pair0[d.g]) {
+            case 1: go = sw_task<1>(A, sm, it, d, bad); break;
+            case 2: go = sw_task<2>(A, sm, it, d, bad); break;
+            default: go = sw_task<4>(A, sm, it, d, bad); break;
+        }
+        if (!go) return;
     }
 }
 
@@ -531,10 +573,11 @@ void launch_sweep(const SweepPlan& S, const Fronts& F, const c32* pf, const c32*
     A.t0 = t0 * G.ngroup;
     A.t1 = t1 * G.ngroup;
     const char* test = std::getenv("GT_SWEEP_TEST_SHORTFALL");
-    const bool shortfall = test && test[0] == '1';
+    const bool shortfall = test && test[0] == '1', stages = test && test[0] == '2';
     A.gave_up = gave_up;
-    A.wait = shortfall ? SW_TEST_WAIT_CYCLES : SW_WAIT_CYCLES;
+    A.wait = shortfall || stages ? SW_TEST_WAIT_CYCLES : SW_WAIT_CYCLES;
     A.surplus = shortfall ? 1 : 0;
+    A.missing = stages ? 16 : 0;
     const int64_t tickets = (int64_t)(t1 - t0) * G.ngroup;
     if (tickets <= 0) return;
     raise_smem((const void*)sweep_kernel, sizeof(SwShared));

@@ -1,6 +1,7 @@
 """Waits of the FP32 sweeps (csrc/sweep.cu) that run out: told to wait a millisecond for a tile that nobody finishes
-(GT_SWEEP_TEST_SHORTFALL), every kind of call that runs the sweeps returns GT_TIMEOUT (RuntimeError here) by itself, and the
-calls after it on the same context are right.  Needs a GPU."""
+(GT_SWEEP_TEST_SHORTFALL=1) or for 16 bytes more than a panel stage's copy brings (=2), every kind of call that runs the
+sweeps returns GT_TIMEOUT (RuntimeError here) by itself, and the calls after it on the same context are right.  Needs a
+GPU."""
 import numpy as np
 import pytest
 
@@ -11,13 +12,16 @@ from test_gpu_small_fronts import _stack, rel
 pytestmark = pytest.mark.gpu
 
 
-def test_an_application_reports_it(monkeypatch):
+@pytest.mark.parametrize("short", ["1", "2"])
+@pytest.mark.parametrize("leaf", [1, 48, 2000])
+@pytest.mark.parametrize("cols", [1, 3, 17])
+def test_an_application_reports_it(short, leaf, cols, monkeypatch):
     b = synth.small_stack3()
-    st, _ = gs.from_board(b)
+    st = _stack(b, leaf)
     obj, k = st.factorise([float(b.freqs[0])])[0]
     rng = np.random.default_rng(3)
-    x = rng.standard_normal((3, st.handle.n_compact)) + 1j * rng.standard_normal((3, st.handle.n_compact))
-    monkeypatch.setenv("GT_SWEEP_TEST_SHORTFALL", "1")
+    x = rng.standard_normal((cols, st.handle.n_compact)) + 1j * rng.standard_normal((cols, st.handle.n_compact))
+    monkeypatch.setenv("GT_SWEEP_TEST_SHORTFALL", short)
     with pytest.raises(RuntimeError, match="triangular sweeps ran out"):
         native.apply(st.handle, obj, "precond", x, k, "fp32")
     # a call without sweeps, between the one that ran out and the next, has nothing to report
