@@ -55,13 +55,15 @@ struct Timeout : std::runtime_error {
     using std::runtime_error::runtime_error;
 };
 
+// The waits of a call's kernels that ran out, in memory of the call's own: of the FP32 sweeps, of pass C of the FP32 L_p
+// product.
+enum { SWEEP_WAITS, LP_WAITS, N_WAITS };
 static const char* const SWEEP_RAN_OUT = "a wait inside the preconditioner's triangular sweeps ran out";
 
-// after a call's kernels have finished: did a bounded wait of the L_p pass or of the sweeps (their count) give up?
-static void check_device_waits(unsigned int sweep) {
-    if (lp_take_wait_timeouts())
-        throw Timeout("a TMA load of the L_p product's FFT grid did not arrive within its wait limit");
-    if (sweep) throw Timeout(SWEEP_RAN_OUT);
+// after the call's kernels have finished: did one give up?
+static void check_waits(const unsigned int* gave_up) {
+    if (gave_up[LP_WAITS]) throw Timeout("a TMA load of the L_p product's FFT grid did not arrive within its wait limit");
+    if (gave_up[SWEEP_WAITS]) throw Timeout(SWEEP_RAN_OUT);
 }
 
 // Device allocations owned by an object, freed together.
@@ -221,7 +223,7 @@ struct Workspace {
     // the FP32 sweeps: solutions interleaved by column group (zfac, uvec likewise), and the tiles' counters
     c32* yint = nullptr;
     int* cnt = nullptr;
-    unsigned int *gave_up = nullptr, *gave_up_host = nullptr;    // their waits that ran out in the present call (host: pinned)
+    unsigned int *gave_up = nullptr, *gave_up_host = nullptr;    // the present call's waits that ran out (host: pinned)
     c64* partial = nullptr;
     // precision 3: the FP32 inner solve's preconditioner applied in FP64 (input, output and the sweeps' vectors)
     c64 *pr64 = nullptr, *pz64 = nullptr, *zfac64 = nullptr, *yfac64 = nullptr, *uvec64 = nullptr, *sd64 = nullptr;
@@ -485,7 +487,8 @@ static size_t t_entries(const gt_geometry* G, int ncol) {
 // System product out = K x (mode 0), rhs - K x (1), or the L_p product of the strips (2).
 template <typename R>
 static void matvec(gt_geometry* G, gt_operators* ops, const cx<R>* x, const cx<R>* rhs, cx<R>* out, int64_t ld, int64_t ldo,
-                   int ncol, const int* col_op, int mode, cx<R>* T, cudaStream_t st, const int* col_list = nullptr) {
+                   int ncol, const int* col_op, int mode, cx<R>* T, unsigned int* gave_up, cudaStream_t st,
+                   const int* col_list = nullptr) {
     Profiler* P = &G->prof;
     const cudaStream_t main = st;
     const bool fork = !P->on && side_by_side(G, ncol);
@@ -519,6 +522,7 @@ static void matvec(gt_geometry* G, gt_operators* ops, const cx<R>* x, const cx<R
         a.tw0 = tw0_of<R>(o);
         a.tw1 = tw1_of<R>(o);
         a.spec = spec_of<R>(o);
+        a.gave_up = gave_up + LP_WAITS;
         a.T = T + (fork && k ? (int64_t)ncol * G->maxT : 0);
         a.ldt = o.ld0;
         a.mask = G->geo.mask;
@@ -575,8 +579,8 @@ static void sweep32(gt_geometry* G, const gt_operators* ops, const Groups& grp, 
     Profiler* P = &G->prof;
     const double es = sizeof(c32), panel = (double)grp.ngroup * es * G->F.panel_total, nfac = (double)G->F.nfac;
     auto run = [&](int t0, int t1) {
-        launch_sweep(G->sweep, G->F, ops->panel32, ops->panel32_b, ops->dinv32, s, z, y, u, sd, grp, cnt, gave_up, t0,
-                     t1, st);
+        launch_sweep(G->sweep, G->F, ops->panel32, ops->panel32_b, ops->dinv32, s, z, y, u, sd, grp, cnt,
+                     gave_up + SWEEP_WAITS, t0, t1, st);
     };
     const int nt = G->sweep.nft + G->sweep.nbt;
     if (!P->on || !P->levels) {
@@ -844,7 +848,7 @@ static void fill_ws(Workspace& W, gt_geometry* G, int ncol, int m, int prec, int
         W.yint = p.alloc<c32>(wide * G->F.nfac);
         W.cnt = p.alloc<int>(sweep_counters(G->F.nfront, ncol));
     }
-    W.gave_up = p.alloc<unsigned int>(1);
+    W.gave_up = p.alloc<unsigned int>(N_WAITS);
     // node-ordered s / y of the preconditioner: entries of nodes that are not kept stay zero
     W.sd = p.alloc<unsigned char>((size_t)ncol * G->F.nnode * es);
     if (!dry) GT_CUDA(cudaMemsetAsync(W.sd, 0, (size_t)ncol * G->F.nnode * es, st));
@@ -889,7 +893,7 @@ static void fill_ws(Workspace& W, gt_geometry* G, int ncol, int m, int prec, int
     W.done = p.alloc<int>(ncol);
     if (!dry) {
         GT_CUDA(cudaMemsetAsync(W.done, 0, ncol * sizeof(int), st));
-        GT_CUDA(cudaMallocHost(&W.gave_up_host, sizeof(unsigned int)));
+        GT_CUDA(cudaMallocHost(&W.gave_up_host, N_WAITS * sizeof(unsigned int)));
         GT_CUDA(cudaMallocHost(&W.togo_host, (size_t)m * ncol * sizeof(double)));
         for (cudaEvent_t& e : W.togo_ev) GT_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
@@ -928,11 +932,11 @@ static int solve_impl(gt_geometry* G, gt_operators* ops, int ncol, const int* h_
     Profiler* P = &G->prof;
     GT_CUDA(cudaMemcpyAsync(W.col_op, h_col_op, ncol * sizeof(int), cudaMemcpyHostToDevice, st));
     GT_CUDA(cudaMemsetAsync(W.its_col, 0, ncol * sizeof(int), st));
-    GT_CUDA(cudaMemsetAsync(W.gave_up, 0, sizeof(unsigned int), st));
+    GT_CUDA(cudaMemsetAsync(W.gave_up, 0, N_WAITS * sizeof(unsigned int), st));
     norms64(G, W.b64, n, ncol, W.bnorm, st);
     if (o.use_guess) {
         // x holds the starting points: r = b - K x in FP64
-        matvec<double>(G, ops, W.x64, W.b64, W.r64, n, n, ncol, W.col_op, 1, W.T64, st);
+        matvec<double>(G, ops, W.x64, W.b64, W.r64, n, n, ncol, W.col_op, 1, W.T64, W.gave_up, st);
         norms64(G, W.r64, n, ncol, W.rho, st);
     } else {
         GT_CUDA(cudaMemsetAsync(W.x64, 0, (size_t)ncol * n * sizeof(c64), st));
@@ -989,7 +993,7 @@ static int solve_impl(gt_geometry* G, gt_operators* ops, int ncol, const int* h_
     std::vector<int> colact(ncol);
     // the true residual r = b - K x in FP64 (and its norms), which also restarts the GCR directions
     auto true_residual = [&]() {
-        matvec<double>(G, ops, W.x64, W.b64, W.r64, n, n, ncol, W.col_op, 1, W.T64, st);
+        matvec<double>(G, ops, W.x64, W.b64, W.r64, n, n, ncol, W.col_op, 1, W.T64, W.gave_up, st);
         {
             Scope sc(P, "norms", st, 16.0 * ncol * n);
             norms64(G, W.r64, n, ncol, W.rho, st);
@@ -1070,7 +1074,7 @@ static int solve_impl(gt_geometry* G, gt_operators* ops, int ncol, const int* h_
                 ldin = ldw = lds;
             }
             apply_pc(vin, ldin, narrow ? nullptr : S.inv_hn, z, na, grp, W.act);
-            matvec<R>(G, ops, z, nullptr, wj, n, ldw, na, W.slot_op, 0, T, st, W.act);
+            matvec<R>(G, ops, z, nullptr, wj, n, ldw, na, W.slot_op, 0, T, W.gave_up, st, W.act);
             // classical Gram-Schmidt: the dot products read the j+1 basis vectors and w; the update reads
             // them again, reads w and writes it
             {
@@ -1147,7 +1151,7 @@ static int solve_impl(gt_geometry* G, gt_operators* ops, int ncol, const int* h_
             GT_CUDA(cudaMemsetAsync(Pk, 0, (size_t)ldk * sizeof(c64), st));
             launch_to64<R>(Pk, n, z, n, W.slot_col, n, ns, st);
         }
-        matvec<double>(G, ops, Pk, nullptr, Qk, n, n, ns, W.col_op, 0, W.T64, st, W.slot_col);
+        matvec<double>(G, ops, Pk, nullptr, Qk, n, n, ns, W.col_op, 0, W.T64, W.gave_up, st, W.slot_col);
         {
             Scope sc(P, "gcr", st, 0.0);
             if (k > 0) {
@@ -1167,9 +1171,9 @@ static int solve_impl(gt_geometry* G, gt_operators* ops, int ncol, const int* h_
         verified = false;
         GT_CUDA(cudaMemcpyAsync(h_rho.data(), W.rho, ncol * sizeof(double), cudaMemcpyDeviceToHost, st));
         GT_CUDA(cudaMemcpyAsync(its_slot.data(), S.its_total, ns * sizeof(int), cudaMemcpyDeviceToHost, st));
-        GT_CUDA(cudaMemcpyAsync(W.gave_up_host, W.gave_up, sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
+        GT_CUDA(cudaMemcpyAsync(W.gave_up_host, W.gave_up, N_WAITS * sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
         GT_CUDA(cudaStreamSynchronize(st));
-        if (*W.gave_up_host) break;                     // (the caller reports it)
+        if (W.gave_up_host[SWEEP_WAITS] || W.gave_up_host[LP_WAITS]) break;      // (the caller reports it)
         for (int s = 0; s < ns; ++s) h_its[slot_col[s]] = its_slot[s];
         P->flush(st);
     }
@@ -1208,10 +1212,10 @@ static int run_solve(gt_geometry* G, gt_operators* ops, int ncol, const int* col
 // vectors that later solves take zero times: the workspace goes, and the next solve makes a new one.
 static void finish_solve(gt_geometry* G, cudaStream_t st) {
     Workspace& W = *G->ws;
-    GT_CUDA(cudaMemcpyAsync(W.gave_up_host, W.gave_up, sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
+    GT_CUDA(cudaMemcpyAsync(W.gave_up_host, W.gave_up, N_WAITS * sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
     GT_CUDA(cudaStreamSynchronize(st));
     try {
-        check_device_waits(*W.gave_up_host);
+        check_waits(W.gave_up_host);
     } catch (const Timeout&) {
         G->ws.reset();
         throw;
@@ -2051,9 +2055,9 @@ int gt_apply(gt_geometry* G, gt_operators* ops, int32_t kind, int32_t precision,
     // kind 1 groups columns by factorisation: require them sorted
     for (int c = 1; c < n_cols; ++c)
         if (kind == 1 && h_pc[c] < h_pc[c - 1]) throw Invalid("preconditioner columns must be sorted by operator");
-    unsigned int* gave_up = tmp.alloc<unsigned int>(1);
-    unsigned int h_gave_up = 0;
-    GT_CUDA(cudaMemsetAsync(gave_up, 0, sizeof(unsigned int), st));
+    unsigned int* gave_up = tmp.alloc<unsigned int>(N_WAITS);
+    unsigned int h_gave_up[N_WAITS] = {};
+    GT_CUDA(cudaMemsetAsync(gave_up, 0, sizeof(h_gave_up), st));
     auto run = [&](auto tag) {
         using R = decltype(tag);
         cx<R>* xi;
@@ -2074,7 +2078,7 @@ int gt_apply(gt_geometry* G, gt_operators* ops, int32_t kind, int32_t precision,
         }
         if (kind == 0 || kind == 2) {
             cx<R>* T = tmp.alloc<cx<R>>(t_entries(G, n_cols));
-            matvec<R>(G, ops, xi, nullptr, yo, n, n, n_cols, d_op, kind == 0 ? 0 : 2, T, st);
+            matvec<R>(G, ops, xi, nullptr, yo, n, n, n_cols, d_op, kind == 0 ? 0 : 2, T, gave_up, st);
         } else {
             std::vector<int> gptr, gslot, gop, gpair, all(n_cols);
             for (int c = 0; c < n_cols; ++c) all[c] = c;
@@ -2108,9 +2112,9 @@ int gt_apply(gt_geometry* G, gt_operators* ops, int32_t kind, int32_t precision,
     else run(float{});
     launch_gather(G->d_c2d, nc, yout, n, d_c, nc, n_cols, st);
     GT_CUDA(cudaMemcpyAsync(y, d_c, (size_t)n_cols * nc * sizeof(c64), cudaMemcpyDeviceToHost, st));
-    GT_CUDA(cudaMemcpyAsync(&h_gave_up, gave_up, sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
+    GT_CUDA(cudaMemcpyAsync(h_gave_up, gave_up, sizeof(h_gave_up), cudaMemcpyDeviceToHost, st));
     GT_CUDA(cudaStreamSynchronize(st));
-    check_device_waits(h_gave_up);
+    check_waits(h_gave_up);
     return GT_OK;
     GT_GUARD_END
 }

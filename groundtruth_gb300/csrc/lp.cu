@@ -600,8 +600,6 @@ constexpr size_t CT_SMEM = 1024 + (size_t)(CT_TILE_BYTES > RW_WARPS * WX_SLOTS *
 constexpr uint64_t CT_WAIT_NS = 1000000000ull;     // a tile not in after a second counts as lost
 constexpr uint32_t CT_SPIN_LIMIT = 1u << 26;        // and polls, should the timer not advance
 
-__device__ unsigned int g_lp_wait_timeouts = 0;   // TMA waits that gave up (read and cleared by the host)
-
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ uint64_t global_ns() {
@@ -636,10 +634,11 @@ __global__ void __launch_bounds__(CT_WARPS * 32, GT_RW_MINB) lp_pass_ct(const __
                                                                 const double* __restrict__ omega, const c64* __restrict__ zs,
                                                                 int mode, const int* __restrict__ col_list,
                                                                 const int* __restrict__ sheet_layer,
-                                                                uint32_t missing_bytes, uint64_t wait_ns) {
+                                                                uint32_t missing_bytes, uint64_t wait_ns,
+                                                                unsigned int* gave_up) {
     pdl_enter();
     // missing_bytes: 0, except when a test makes the wait run out (the barrier then expects bytes no load
-    // brings; the loads themselves are the usual two)
+    // brings; the loads themselves are the usual two).  gave_up: the call's count of threads whose wait ran out
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bar;
     // the 128-byte swizzle repeats every 1024 bytes: the tile starts on a 1024-byte boundary
@@ -690,7 +689,7 @@ __global__ void __launch_bounds__(CT_WARPS * 32, GT_RW_MINB) lp_pass_ct(const __
     }
     if (!mbar_wait_bounded(b, 0, wait_ns)) {
         // the tile did not arrive: record it and leave once the copies in flight have landed (or given up on)
-        if (threadIdx.x == 0) atomicAdd(&g_lp_wait_timeouts, 1u);
+        atomicAdd(gave_up, 1u);
         mbar_wait_bounded(b, 0, wait_ns);
         return;
     }
@@ -730,13 +729,6 @@ __global__ void __launch_bounds__(CT_WARPS * 32, GT_RW_MINB) lp_pass_ct(const __
                                     off_v + ((int64_t)layer * nx + ii) * ny, (int64_t)di * ny + dj, x + base, rhs ? rhs + base : nullptr,
                                     out + (int64_t)col * ldo, mask, w, z, mode);
     }
-}
-
-unsigned int lp_take_wait_timeouts() {
-    unsigned int h = 0, zero_v = 0;
-    GT_CUDA(cudaMemcpyFromSymbol(&h, g_lp_wait_timeouts, sizeof(h)));
-    if (h) GT_CUDA(cudaMemcpyToSymbol(g_lp_wait_timeouts, &zero_v, sizeof(zero_v)));
-    return h;
 }
 
 // Row passes for P a power of 8: the first stage of pass A reads the strip row straight from x, the last
@@ -1082,7 +1074,7 @@ static void launch_c(const LpArgs<R>& a, int rows, cudaStream_t st) {
             pdl_launch(lp_pass_ct, dim3(ceil_div(a.n0, 16), a.S, a.ncol), CT_WARPS * 32, CT_SMEM, st, 
                 m, a.x, a.rhs, a.out, a.ld, a.ldo, a.off, a.off_v, a.S, a.n0, a.n1, a.nx, a.ny, a.di, a.dj, a.tw1, a.mask,
                 a.col_op, a.omega, a.zs, a.mode, a.col_list, a.sheet_layer, shortfall ? 16u : 0u,
-                shortfall ? 1000000ull : CT_WAIT_NS);
+                shortfall ? 1000000ull : CT_WAIT_NS, a.gave_up);
             GT_LAUNCH_CHECK();
             return;
         }

@@ -63,3 +63,20 @@ def test_a_derived_set_made_by_the_fp32_sweeps_reports_it(monkeypatch):
     obj, k = dst.factorise([f])[0]
     x = np.ones(dst.handle.n_compact, complex)
     assert np.isfinite(native.apply(dst.handle, obj, "precond", x, k, "fp32")).all()
+
+
+def test_a_solve_whose_tile_loads_ran_out_reports_it_and_the_next_is_as_on_a_new_stack(monkeypatch):
+    """The same for pass C of the FP32 L_p product (GT_LP_TMA_TEST_SHORTFALL), on the smallest board that takes it."""
+    b = synth.slotted_pair(n_nets=1, n_freq=1)
+    f = float(b.freqs[0])
+
+    def solve(st, routes):
+        return st.solve_batch([f], [routes[0].rhs_top(f)], [routes[0].J()], tol=1e-9)[0]
+    st, routes = gs.from_board(b)
+    st.factorise([f])
+    monkeypatch.setenv("GT_LP_TMA_TEST_SHORTFALL", "1")
+    with pytest.raises(RuntimeError, match="did not arrive"):
+        solve(st, routes)
+    monkeypatch.delenv("GT_LP_TMA_TEST_SHORTFALL")
+    a, c = solve(st, routes), solve(*gs.from_board(b))
+    assert a[4] <= 1e-9 and a[2] == c[2] and np.array_equal(a[3], c[3])
