@@ -15,6 +15,7 @@
 // children's update vectors, eliminates its own rows and passes its boundary rows up), z /= D, root down
 // for L^T y = z (each front reads its ancestors' finished y).
 #include "kernels.h"
+#include "pivot.h"
 
 namespace gt {
 
@@ -62,27 +63,9 @@ struct FrontView {
     }
 };
 
-// 1 / d for a positive normal d: an FP32 seed of the mantissa and two Newton steps r += r (1 - d r) (within 2 ulp; the
-// compiler's division occupies the FP64 pipe, two operations a clock and SM, three times as long, on the pivots' chain)
-__device__ __forceinline__ double recip64(double d) {
-    const long long bits = __double_as_longlong(d);
-    const int e = (int)(bits >> 52) - 1023;
-    const double m = __longlong_as_double((bits & 0xfffffffffffffll) | 0x3ff0000000000000ll);      // in [1, 2)
-    double r = (double)(1.0f / (float)m);
-    r = __fma_rn(r, __fma_rn(-m, r, 1.0), r);
-    r = __fma_rn(r, __fma_rn(-m, r, 1.0), r);
-    return r * __longlong_as_double((long long)(1023 - e) << 52);
-}
-
 __device__ __forceinline__ c64 pivot_inverse(c64 d, int* status) {
-    double dd = d.re * d.re + d.im * d.im;
-    if (!(dd > 1e-300) || !isfinite(dd)) {
-        atomicOr(status, 1);
-        d = mk<double>(1e-150, 0.0);
-        dd = 1e-300;
-    }
-    const double r = recip64(dd);
-    return mk<double>(d.re * r, -d.im * r);
+    if (!pivot_recip(d.re, d.im)) atomicOr(status, 1);
+    return d;
 }
 
 __device__ __forceinline__ FrontView front_view(const Fronts& F, int f, int op, c64* panel, c64* upd) {
