@@ -145,8 +145,11 @@ __global__ void __launch_bounds__(128) moment_sum_kernel(const c64* __restrict__
 void launch_moment(const Geo& g, const c64* x, int64_t ld, int ncol, const SheetZ& zs, double d, c64* part, c64* m,
                    cudaStream_t st) {
     const int nb = mom_blocks(g);
-    moment_rows_kernel<<<dim3(nb, ncol), 256, 0, st>>>(g, x, ld, zs, d, part);
-    GT_LAUNCH_CHECK();
+    constexpr int MOST = 65535;                            // of a grid's second dimension
+    for (int c = 0; c < ncol; c += MOST) {
+        moment_rows_kernel<<<dim3(nb, std::min(MOST, ncol - c)), 256, 0, st>>>(g, x + c * ld, ld, zs, d, part + (int64_t)c * nb * 3);
+        GT_LAUNCH_CHECK();
+    }
     moment_sum_kernel<<<ncol, 128, 0, st>>>(part, nb, m);
     GT_LAUNCH_CHECK();
 }
