@@ -86,17 +86,15 @@ class MemoryBudget:
             self.cv.notify_all()
 
 
-def _column_bytes(job: BoardJob, restart: int, precision: str) -> int:
-    """Device bytes one more column adds to a solve: its workspace share and its dense right-hand side and
-    solution."""
+def _solve_bytes(job: BoardJob, n_cols: int, restart: int, precision: str) -> int:
+    """Device bytes of a solve of n_cols columns: its workspace and their dense right-hand sides and solutions."""
     h = job.stack.handle
-    one = native.memory(h, 1, restart, precision)["need"]
-    return int(native.memory(h, 2, restart, precision)["need"] - one + 2 * h.n_dense * 16)
+    return int(native.memory(h, n_cols, restart, precision)["need"] + n_cols * 2 * h.n_dense * 16)
 
 
 def _device_bytes(job: BoardJob, restart: int, precision: str) -> int:
     """What a board asks of the budget: its factorisations and all its columns at once."""
-    return int(job.stack.factorisation_bytes(len(job.freqs)) + len(job.cols) * _column_bytes(job, restart, precision))
+    return int(job.stack.factorisation_bytes(len(job.freqs)) + _solve_bytes(job, len(job.cols), restart, precision))
 
 
 def solve_board(job: BoardJob, stream=None, restart: int = 50, precision: str = "mixed", max_its: int = 4000,
@@ -120,7 +118,6 @@ def solve_board(job: BoardJob, stream=None, restart: int = 50, precision: str = 
         avail = int(avail_bytes if avail_bytes is not None else 0.9 * native.memory(st.handle, 1)["free"])
         nq = len(job.freqs)
         chunk = max(1, min(nq, int(0.5 * avail // max(st.factorisation_bytes(1), 1))))
-        per_col = _column_bytes(job, restart, precision)
         for q0 in range(0, nq, chunk):
             qs = list(range(q0, min(nq, q0 + chunk)))
             tf = time.perf_counter()
@@ -129,8 +126,9 @@ def solve_board(job: BoardJob, stream=None, restart: int = 50, precision: str = 
             obj = ops[0][0]
             prec = "mixed_pc64" if precision == "mixed" and getattr(obj, "stiff", False) else precision
             mine = [c for c, (_, q) in enumerate(job.cols) if q0 <= q < q0 + len(qs)]
-            room = max(avail - st.resident_bytes(len(qs)), per_col)
-            step = max(1, min(len(mine), int(room // per_col), st.columns_that_fit(len(mine), restart, prec)))
+            room = avail - st.resident_bytes(len(qs))
+            fit = native.most_columns(lambda n: _solve_bytes(job, n, restart, prec), room, len(mine))
+            step = max(1, min(fit, st.columns_that_fit(len(mine), restart, prec)))
             for c0 in range(0, len(mine), step):
                 sel = mine[c0: c0 + step]
                 m = len(sel)

@@ -477,6 +477,25 @@ def memory(geom: Geometry, n_cols: int, restart: int = 50, precision: str = "mix
     return dict(zip(("need", "held", "free", "total"), (x.value for x in v)))
 
 
+def most_columns(need, room: float, most: int) -> int:
+    """The largest number of columns, at most `most`, whose need(columns) bytes fit room; 0 when not even one's do.  need grows
+    with the columns, but not by the same for each (a solve's workspace holds grids for both orientations side by side up to
+    a size), so that no cost per column stands for it."""
+    if most < 1 or need(1) > room:
+        return 0
+    lo, hi = 1, 2
+    while hi <= most and need(hi) <= room:
+        lo, hi = hi, 2 * hi
+    hi = min(hi, most + 1)
+    while hi - lo > 1:
+        mid = (lo + hi) // 2
+        if need(mid) <= room:
+            lo = mid
+        else:
+            hi = mid
+    return lo
+
+
 def kernel_spectrum(n_axial: int, n_lateral: int, d: float, dz: float, P0: int, P1: int,
                     near: np.ndarray) -> np.ndarray:
     """The strip kernel's real spectrum quadrant (P0/2+1, P1/2+1) computed on the device (gt_kernel_spectrum);

@@ -71,14 +71,11 @@ class Server:
         self.streams = {name: torch.cuda.Stream() for name in self.geo}
         # columns per batch: every geometry keeps a workspace as wide as the widest batch it took, so the budget
         # holds max_cols columns of each geometry's workspace
-        one = per = 0
         for w in self.geo.values():
             w.stack.trim()                         # what the baselines left behind
-            o = native.memory(w.stack.handle, 1, restart)["need"]
-            one += o
-            per += max(native.memory(w.stack.handle, 2, restart)["need"] - o, 1)
-        fit = int((budget_bytes - one) // per) + 1
-        self.max_cols = max(1, min(fit, max_cols or fit))
+        fit = native.most_columns(lambda n: sum(native.memory(w.stack.handle, n, restart)["need"] for w in self.geo.values()),
+                                  budget_bytes, max_cols or 1 << 24)
+        self.max_cols = max(1, fit)
         for w in self.geo.values():          # every device solve of a geometry in batches of at most that
             w.max_cols = self.max_cols
         self.resident_bytes = sum(w.stack.resident_bytes(len(w.freqs)) for w in self.geo.values())

@@ -1119,13 +1119,13 @@ class PlaneStack:
         room = full["held"] + self.MEMORY_HEADROOM * full["free"]
         if full["need"] <= room:
             return ncol
-        one = native.memory(self.handle, 1, restart, precision)["need"]
-        per = (full["need"] - one) / max(ncol - 1, 1)
-        fit = int((room - one) // per) + 1 if room >= one else 0
+        def need(n):
+            return native.memory(self.handle, n, restart, precision)["need"]
+        fit = native.most_columns(need, room, ncol)
         if fit < 1:
-            raise MemoryError(f"a solve of one column needs {one / 2**30:.1f} GiB, "
+            raise MemoryError(f"a solve of one column needs {need(1) / 2**30:.1f} GiB, "
                               f"{room / 2**30:.1f} GiB are available on the device")
-        return min(fit, ncol)
+        return fit
 
     def _warm_start(self, ops, rhs: np.ndarray, guesses) -> Optional[np.ndarray]:
         """Starting points from guess vectors (peec.py:2570-2578): per column x0 = G c with c minimising

@@ -60,3 +60,30 @@ def test_a_sweep_wants_its_columns_sorted_by_frequency_group():
     col_key = np.array([0, 0, 3, 1])           # a column of group 1 after one of group 3 (two groups of two)
     with pytest.raises(ValueError, match="sorted"):
         native.solve_sweep(None, keys, [None] * 4, col_key, np.zeros((4, 3), complex), 1e-10, chunks=2)
+
+
+@pytest.mark.parametrize("one", [2 ** 18, 3 * 2 ** 18, 2 ** 20, 2 ** 20 + 1, 5 * 2 ** 20])
+@pytest.mark.parametrize("cols", [1, 2, 3, 7, 40])
+def test_a_board_asks_for_what_its_solve_allocates(one, cols, monkeypatch):
+    """Admission by the workspace's own size at the count of columns: its grids hold both orientations side by side while that is
+    no more than 2^20 entries each, so that the second column may cost nothing and the fifth all of its grid."""
+    side = 2 ** 20
+
+    def need(n):
+        return 1000 + 40 * n + 24 * max(n * one, min(2 * n * one, 2 * side))
+    monkeypatch.setattr(native, "memory", lambda g, n, *a, **k: {"need": need(n), "held": 0, "free": free[0], "total": 0})
+    free = [0]
+    st = SimpleNamespace(handle=SimpleNamespace(n_dense=7), factorisation_bytes=lambda n: 5 * n)
+    job = batch.BoardJob("b", st, [], [1e6, 1e7], 1e-6, [(0, 0)] * cols)
+    asked = batch._device_bytes(job, 50, "mixed")
+    assert asked == 10 + need(cols) + cols * 2 * 7 * 16
+    # what fits it: all the columns, and with a byte less one fewer
+    solve = lambda n: batch._solve_bytes(job, n, 50, "mixed")
+    assert native.most_columns(solve, solve(cols), 1000) == cols
+    assert native.most_columns(solve, solve(cols) - 1, 1000) == cols - 1
+    assert native.most_columns(solve, solve(cols), max(1, cols - 2)) == max(1, cols - 2)
+    # the solve's own gate, on the same sizes
+    whole = gs.PlaneStack.__new__(gs.PlaneStack)
+    whole.handle = st.handle
+    free[0] = need(cols) / gs.PlaneStack.MEMORY_HEADROOM * (1 + 1e-12)
+    assert whole.columns_that_fit(64) == cols
