@@ -2032,6 +2032,27 @@ int gt_memory(gt_geometry* G, int32_t n_cols, const gt_solve_opts* opts, int64_t
     GT_GUARD_END
 }
 
+int gt_operators_bytes(gt_geometry* G, int32_t n_ops, int32_t flags, int64_t* held, int64_t* making) {
+    GT_GUARD_BEGIN
+    if (flags & ~GT_OPS_FP32_PANELS) throw Invalid("unknown operator flags");
+    if (!G || n_ops < 1) throw Invalid("bad arguments");
+    const Geo& g = G->geo;
+    const Fronts& F = G->F;
+    const bool keep64 = !(flags & GT_OPS_FP32_PANELS);
+    const int64_t panel64 = F.panel_total * (int64_t)sizeof(c64);
+    // frequency, impedances and table; the panels (in FP64 by columns and by rows); the pivots
+    const int64_t own = sizeof(double) + (g.S + std::max(G->ntw, 1) + g.np + g.nbr) * (int64_t)sizeof(c64) +
+                        g.ntab * (int64_t)(sizeof(c64) + sizeof(c32)) + 2 * G->sweep.ptotal * (int64_t)sizeof(c32) +
+                        (keep64 ? 2 * panel64 : 0) + F.nfac * (int64_t)(sizeof(c64) + sizeof(c32));
+    // the Schur values, the update matrices and the large fronts' diagonal inverses; the FP64 factor that is not kept
+    const int64_t tmp = (F.nsv + std::max<int64_t>(F.upd_total, 1) + G->xtotal * FACTOR_BLOCK * FACTOR_BLOCK) *
+                            (int64_t)sizeof(c64) + (keep64 ? 0 : panel64);
+    if (held) *held = n_ops * own;
+    if (making) *making = n_ops * tmp;
+    return GT_OK;
+    GT_GUARD_END
+}
+
 int gt_apply(gt_geometry* G, gt_operators* ops, int32_t kind, int32_t precision, int32_t n_cols, const int32_t* col_op,
              const double* x, double* y, void* stream) {
     GT_GUARD_BEGIN

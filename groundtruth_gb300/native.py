@@ -128,6 +128,7 @@ def load():
                                        C.c_int32, DP]
     lib.gt_moment.argtypes = [P, C.c_int32, P, DP, C.c_double, DP, P]
     lib.gt_lp_product_noalloc.argtypes = [P, C.c_int32, P, P, P]
+    lib.gt_operators_bytes.argtypes = [P, C.c_int32, C.c_int32, C.POINTER(C.c_int64), C.POINTER(C.c_int64)]
     lib.gt_memory.argtypes = [P, C.c_int32, C.POINTER(SolveOpts), C.POINTER(C.c_int64), C.POINTER(C.c_int64),
                               C.POINTER(C.c_int64), C.POINTER(C.c_int64)]
     if lib.gt_device_count() < 1:
@@ -297,6 +298,13 @@ class Geometry:
         check(self.lib, self.lib.gt_moment(self.h, n_cols, P(x_ptr), _ptr(z, C.c_double), float(pitch),
                                            _ptr(m.view(np.float64), C.c_double), P(stream)), "gt_moment")
         return m
+
+    def operators_bytes(self, n_ops: int, fp32_panels: bool = False) -> tuple:
+        """gt_operators_bytes: (device bytes n_ops factorised operators hold, bytes besides while they are made)."""
+        v = [C.c_int64(0) for _ in range(2)]
+        check(self.lib, self.lib.gt_operators_bytes(self.h, int(n_ops), GT_OPS_FP32_PANELS if fp32_panels else 0,
+                                                    *(C.byref(x) for x in v)), "gt_operators_bytes")
+        return tuple(x.value for x in v)
 
     def profile(self, on: bool | None = None, levels: bool = False) -> dict:
         """Toggle (on=True/False: reset; levels: time each elimination level too) or read

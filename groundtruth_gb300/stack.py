@@ -1065,21 +1065,26 @@ class PlaneStack:
 
     MEMORY_HEADROOM = 0.9         # of the device's free memory a solve or a factorisation may take
 
-    def factorisation_bytes(self, n_fact: int) -> int:
-        """Device bytes of n_fact factorisations while they are made (gt_operators_create_ex): each one's panels in
-        FP64 and FP32, column- and row-major (with fp32_panels the FP32 pair kept and the FP64 factor in
-        temporary memory), its pivots and tables, and the Schur values and update matrices."""
+    def _operator_bytes(self, n_fact: int) -> tuple:
+        """(device bytes n_fact factorisations hold, bytes besides while they are made): the library's own count
+        (gt_operators_bytes), or without a device the panels' entries in each of their copies, the pivots and tables, and the
+        Schur values and update matrices."""
+        from . import native
+        if isinstance(self.handle, native.Geometry):
+            return self.handle.operators_bytes(n_fact, self.fp32_panels)
         sym = self.sym
-        panel = (16 + 8 + 8) if self.fp32_panels else (16 + 8 + 8 + 16)
-        per = sym.panel_total * panel + sym.n * (16 + 8) + self.n_table * (16 + 8)
-        made = self.sterm.shape[0] * 16 + max(sym.upd_total, 1) * 16
-        return int(n_fact * (per + made))
+        kept, made = (8 + 8, 16) if self.fp32_panels else (16 + 8 + 8 + 16, 0)
+        held = sym.panel_total * kept + sym.n * (16 + 8) + self.n_table * (16 + 8)
+        making = sym.panel_total * made + self.sterm.shape[0] * 16 + max(sym.upd_total, 1) * 16
+        return int(n_fact * held), int(n_fact * making)
+
+    def factorisation_bytes(self, n_fact: int) -> int:
+        """Device bytes of n_fact factorisations while they are made."""
+        return sum(self._operator_bytes(n_fact))
 
     def resident_bytes(self, n_fact: int) -> int:
         """Device bytes n_fact factorisations hold once made."""
-        sym = self.sym
-        panel = (8 + 8) if self.fp32_panels else (16 + 8 + 8 + 16)
-        return int(n_fact * (sym.panel_total * panel + sym.n * (16 + 8) + self.n_table * (16 + 8)))
+        return self._operator_bytes(n_fact)[0]
 
     def trim(self):
         """Free the device solve workspace of this stack (the next solve makes it again)."""

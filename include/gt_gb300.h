@@ -206,6 +206,11 @@ int gt_solve(gt_geometry* g, gt_operators* ops, int32_t n_cols, const int32_t* c
 int gt_memory(gt_geometry* g, int32_t n_cols, const gt_solve_opts* opts, int64_t* need, int64_t* held,
               int64_t* free_bytes, int64_t* total_bytes);
 
+/* Device memory of operators: *held the bytes that gt_operators_create_ex with these flags allocates for n_ops operators of
+ * their own factorisations and keeps, *making those of its temporaries besides.  (A stiff set keeps its FP64 panels whatever
+ * the flags: ask without GT_OPS_FP32_PANELS for it.)  Either pointer may be NULL. */
+int gt_operators_bytes(gt_geometry* g, int32_t n_ops, int32_t flags, int64_t* held, int64_t* making);
+
 /* The same with device-resident dense vectors: rhs_device / x_device are [n_cols*n_dense] complex128 in the
  * dense layout; nothing crosses to the host but the per-column scalars. */
 int gt_solve_device(gt_geometry* g, gt_operators* ops, int32_t n_cols, const int32_t* col_op,
