@@ -238,11 +238,7 @@ struct Workspace {
     int kmax = 0;
     c64 *gP = nullptr, *gQ = nullptr, *gbeta = nullptr, *galpha = nullptr, *gnu2 = nullptr;
     int* colact = nullptr;
-    int* flag_dev = nullptr;
-    int* flag_host = nullptr;
-    int* its_col = nullptr;
     ~Workspace() {
-        if (flag_host) cudaFreeHost(flag_host);
         if (gave_up_host) cudaFreeHost(gave_up_host);
         if (togo_host) cudaFreeHost(togo_host);
         for (cudaEvent_t e : togo_ev)
@@ -608,11 +604,11 @@ static void sweep64(gt_geometry* G, const gt_operators* ops, const Groups& grp, 
     const double es = sizeof(c64), panel = (double)grp.ngroup * es * G->F.panel_total, nfac = (double)G->F.nfac;
     const int nlev = (int)G->level_ptr.size() - 1;
     auto fwd = [&](int h, const Groups& g, cudaStream_t sk) {
-        launch_fwd_level<double>(G->F, G->d_order + G->level_ptr[h], (int)(G->level_ptr[h + 1] - G->level_ptr[h]),
+        launch_fwd_level(G->F, G->d_order + G->level_ptr[h], (int)(G->level_ptr[h + 1] - G->level_ptr[h]),
                                  G->level_maxnf[h], G->level_maxnown[h], ops->panel64, ops->dinv64, s, z, u, s, g, gmax, sk);
     };
     auto bwd = [&](int h, const Groups& g, cudaStream_t sk) {
-        launch_bwd_level<double>(G->F, G->d_order + G->level_ptr[h], (int)(G->level_ptr[h + 1] - G->level_ptr[h]),
+        launch_bwd_level(G->F, G->d_order + G->level_ptr[h], (int)(G->level_ptr[h + 1] - G->level_ptr[h]),
                                  G->level_maxnf[h], G->level_maxnown[h], ops->panel64_rm, z, s, sd, g, gmax, sk);
     };
     const bool levels = P->on && P->levels;
@@ -774,11 +770,11 @@ static void lowrank_w(gt_geometry* G, const gt_operators* base, int nf, int k, c
         } else {
             const int nlev = (int)G->level_ptr.size() - 1;
             for (int h = 0; h < nlev; ++h)
-                launch_fwd_level<R>(G->F, G->d_order + G->level_ptr[h], (int)(G->level_ptr[h + 1] - G->level_ptr[h]),
+                launch_fwd_level(G->F, G->d_order + G->level_ptr[h], (int)(G->level_ptr[h + 1] - G->level_ptr[h]),
                                     G->level_maxnf[h], G->level_maxnown[h], base->panel64, base->dinv64, sv, zv, uv, sv, grp,
                                     gmax, st);
             for (int h = nlev - 1; h >= 0; --h)
-                launch_bwd_level<R>(G->F, G->d_order + G->level_ptr[h], (int)(G->level_ptr[h + 1] - G->level_ptr[h]),
+                launch_bwd_level(G->F, G->d_order + G->level_ptr[h], (int)(G->level_ptr[h + 1] - G->level_ptr[h]),
                                     G->level_maxnf[h], G->level_maxnown[h], base->panel64_rm, zv, sv, wout, grp, gmax, st);
         }
         GT_CUDA(cudaStreamSynchronize(st));   // the group tables are reused by the next batch
@@ -904,10 +900,7 @@ static void fill_ws(Workspace& W, gt_geometry* G, int ncol, int m, int prec, int
     W.gnu2 = p.alloc<c64>(ncol);
     W.colact = p.alloc<int>(ncol);
     W.col_op = p.alloc<int>(ncol);
-    W.flag_dev = p.alloc<int>(1);
-    W.its_col = p.alloc<int>(ncol);
     if (dry) return;
-    GT_CUDA(cudaMallocHost(&W.flag_host, sizeof(int)));
     GT_CUDA(cudaMemsetAsync(W.V, 0, (size_t)ncol * (m + 1) * n * eb, st));
 }
 
@@ -928,10 +921,9 @@ static int solve_impl(gt_geometry* G, gt_operators* ops, int ncol, const int* h_
     Workspace& W = *G->ws;
     const int64_t n = G->geo.n;
     const int m = o.restart;
-    const int nch = nchunks(n), nchu = update_chunks(n);
+    const int nch = nchunks(n);
     Profiler* P = &G->prof;
     GT_CUDA(cudaMemcpyAsync(W.col_op, h_col_op, ncol * sizeof(int), cudaMemcpyHostToDevice, st));
-    GT_CUDA(cudaMemsetAsync(W.its_col, 0, ncol * sizeof(int), st));
     GT_CUDA(cudaMemsetAsync(W.gave_up, 0, N_WAITS * sizeof(unsigned int), st));
     norms64(G, W.b64, n, ncol, W.bnorm, st);
     if (o.use_guess) {

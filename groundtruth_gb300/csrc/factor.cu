@@ -21,12 +21,6 @@ namespace gt {
 
 // Complex multiply-accumulate as four explicit FMAs (acc += a u): written out, the
 // product and the sum round as separate operations (six instructions instead of four on the FP64 pipe).
-__device__ __forceinline__ void cfma(c32& acc, c32 a, c32 u) {
-    acc.re = __fmaf_rn(a.re, u.re, acc.re);
-    acc.re = __fmaf_rn(-a.im, u.im, acc.re);
-    acc.im = __fmaf_rn(a.re, u.im, acc.im);
-    acc.im = __fmaf_rn(a.im, u.re, acc.im);
-}
 __device__ __forceinline__ void cfma(c64& acc, c64 a, c64 u) {
     acc.re = __fma_rn(a.re, u.re, acc.re);
     acc.re = __fma_rn(-a.im, u.im, acc.re);
@@ -654,62 +648,41 @@ void launch_panel_convert(const Fronts& F, const SweepPlan& S, const int64_t* fr
 constexpr int LB = 8;
 constexpr int SOLVE_THREADS = 512;
 
-template <typename R>
-static void smem_attr(const void* fn, size_t bytes) { raise_smem(fn, bytes); }
-
-// two consecutive columns' entries of a k-major shared vector (one 16-byte load in FP32)
-__device__ __forceinline__ void lds2(const c32* p, c32& a, c32& b) {
-    const float4 t = *reinterpret_cast<const float4*>(p);
-    a = mk<float>(t.x, t.y);
-    b = mk<float>(t.z, t.w);
-}
-__device__ __forceinline__ void lds2(const c64* p, c64& a, c64& b) {
-    a = p[0];
-    b = p[1];
-}
-
 // acc[c] += a * x[c] over all GC columns of one k-major shared row x (unused columns hold zeros)
-template <typename R, int GC>
-__device__ __forceinline__ void mac_row(cx<R>* acc, cx<R> a, const cx<R>* x) {
+template <int GC>
+__device__ __forceinline__ void mac_row(c64* acc, c64 a, const c64* x) {
 #pragma unroll
-    for (int c2 = 0; c2 < GC / 2; ++c2) {
-        cx<R> u, v;
-        lds2(x + 2 * c2, u, v);
-        cfma(acc[2 * c2], a, u);
-        cfma(acc[2 * c2 + 1], a, v);
-    }
-    if constexpr (GC % 2 == 1) cfma(acc[GC - 1], a, x[GC - 1]);
+    for (int c = 0; c < GC; ++c) cfma(acc[c], a, x[c]);
 }
 
 // acc[c] += sum_{t < cnt} A[t * lda] x[t * xs + c]: A a strided run of panel elements (part of one row or
 // column of a front's panel), x the matching k-major shared rows.  The first LB elements were loaded into
 // l ahead of time (prefetch_run, issued before the shared rows were staged); LB loads in flight after that.
-template <typename R>
-__device__ __forceinline__ void prefetch_run(const cx<R>* __restrict__ A, int lda, int cnt, cx<R>* l) {
+__device__ __forceinline__ void prefetch_run(const c64* __restrict__ A, int lda, int cnt, c64* l) {
 #pragma unroll
-    for (int u = 0; u < LB; ++u) l[u] = u < cnt ? A[u * lda] : zero<R>();
+    for (int u = 0; u < LB; ++u) l[u] = u < cnt ? A[u * lda] : zero<double>();
 }
 
-template <typename R, int GC>
-__device__ __forceinline__ void sweep(const cx<R>* __restrict__ A, int lda, const cx<R>* x, int xs, int cnt,
-                                      const cx<R>* l0, cx<R>* acc) {
+template <int GC>
+__device__ __forceinline__ void sweep(const c64* __restrict__ A, int lda, const c64* x, int xs, int cnt,
+                                      const c64* l0, c64* acc) {
 #pragma unroll
     for (int u = 0; u < LB; ++u)
-        if (u < cnt) mac_row<R, GC>(acc, l0[u], x + u * xs);
+        if (u < cnt) mac_row<GC>(acc, l0[u], x + u * xs);
     A += LB * lda;
     x += LB * xs;
     int t = LB;
     for (; t + LB <= cnt; t += LB) {
-        cx<R> l[LB];
+        c64 l[LB];
 #pragma unroll
         for (int u = 0; u < LB; ++u) l[u] = A[u * lda];
 #pragma unroll
-        for (int u = 0; u < LB; ++u) mac_row<R, GC>(acc, l[u], x + u * xs);
+        for (int u = 0; u < LB; ++u) mac_row<GC>(acc, l[u], x + u * xs);
         A += LB * lda;
         x += LB * xs;
     }
     for (; t < cnt; ++t) {
-        mac_row<R, GC>(acc, *A, x);
+        mac_row<GC>(acc, *A, x);
         A += lda;
         x += xs;
     }
@@ -718,16 +691,16 @@ __device__ __forceinline__ void sweep(const cx<R>* __restrict__ A, int lda, cons
 // The forward rows of front f for a group: own rows of w (s in factor order plus the children's updates)
 // into ws (k-major, ldw = GC) and boundary rows r0 <= p < r1 into wt ([c][TR]).  Loads are issued four
 // at a time per thread ahead of their stores.
-template <typename R, int GC>
-__device__ __forceinline__ void fwd_gather(const Fronts& F, int f, const int* gs, int gc, const cx<R>* __restrict__ sf,
-                                           const cx<R>* __restrict__ uvec, cx<R>* ws, cx<R>* wt, int TR, int r0, int r1) {
+template <int GC>
+__device__ __forceinline__ void fwd_gather(const Fronts& F, int f, const int* gs, int gc, const c64* __restrict__ sf,
+                                           const c64* __restrict__ uvec, c64* ws, c64* wt, int TR, int r0, int r1) {
     const int nown = (int)F.nown[f];
     const int64_t own0 = F.own_start[f];
     const int tid = threadIdx.x, nth = blockDim.x;
     const int tot = gc * nown;
-    for (int q = tot + tid; q < GC * nown; q += nth) ws[(q % nown) * GC + q / nown] = zero<R>();
+    for (int q = tot + tid; q < GC * nown; q += nth) ws[(q % nown) * GC + q / nown] = zero<double>();
     for (int q0 = tid; q0 < tot; q0 += 4 * nth) {
-        cx<R> v[4];
+        c64 v[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const int q = min(q0 + u * nth, tot - 1), c = q / nown;
@@ -747,7 +720,7 @@ __device__ __forceinline__ void fwd_gather(const Fronts& F, int f, const int* gs
         const int64_t voff = F.vec_off[ch];
         for (int q0 = tid; q0 < tc; q0 += 4 * nth) {
             int p[4];
-            cx<R> v[4];
+            c64 v[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const int q = min(q0 + u * nth, tc - 1), c = q / nb, i = q - c * nb;
@@ -769,22 +742,22 @@ __device__ __forceinline__ void fwd_gather(const Fronts& F, int f, const int* gs
 
 // Forward assembly of a front split over several blocks, once per (front, group): w_own to wasm (factor
 // order), the children's updates of the boundary rows to the front's own update-vector slots.
-template <typename R, int GC>
+template <int GC>
 __global__ void __launch_bounds__(256) fwd_assemble_kernel(Fronts F, const int64_t* __restrict__ front_list,
-                                                           const cx<R>* sf, cx<R>* __restrict__ uvec, cx<R>* wasm,
+                                                           const c64* sf, c64* __restrict__ uvec, c64* wasm,
                                                            Groups G, int ldw, int TR) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    cx<R>* ws = reinterpret_cast<cx<R>*>(smem_raw);   // [k][GC]
-    cx<R>* wt = ws + GC * ldw;                      // [c][TR] boundary rows
+    c64* ws = reinterpret_cast<c64*>(smem_raw);   // [k][GC]
+    c64* wt = ws + GC * ldw;                      // [c][TR] boundary rows
     const int g = blockIdx.x % G.ngroup;
     const int f = (int)front_list[blockIdx.x / G.ngroup];
     const int* gs = G.gslot + G.gptr[g];
     const int gc = G.gptr[g + 1] - G.gptr[g];
     const int nown = (int)F.nown[f], nbnd = (int)F.nbnd[f], nf = nown + nbnd;
     const int64_t own0 = F.own_start[f];
-    for (int q = threadIdx.x; q < GC * TR; q += blockDim.x) wt[q] = zero<R>();
+    for (int q = threadIdx.x; q < GC * TR; q += blockDim.x) wt[q] = zero<double>();
     __syncthreads();
-    fwd_gather<R, GC>(F, f, gs, gc, sf, uvec, ws, wt, TR, nown, nf);
+    fwd_gather<GC>(F, f, gs, gc, sf, uvec, ws, wt, TR, nown, nf);
     for (int q = threadIdx.x; q < gc * nown; q += blockDim.x) {
         const int c = q / nown, r = q - c * nown;
         wasm[(int64_t)gs[c] * F.nfac + own0 + r] = ws[r * GC + c];
@@ -796,17 +769,17 @@ __global__ void __launch_bounds__(256) fwd_assemble_kernel(Fronts F, const int64
 }
 
 // pre: the front was assembled by fwd_assemble_kernel (own rows in wasm, boundary rows in uvec)
-template <typename R, int GC>
+template <int GC>
 __global__ void __launch_bounds__(SOLVE_THREADS, 2) fwd_gemv_kernel(Fronts F, const int64_t* __restrict__ front_list, int nblk,
-                                                                 int rt, int kseg, const cx<R>* __restrict__ panel,
-                                                                 const cx<R>* __restrict__ dinv, const cx<R>* sf,
-                                                                 cx<R>* __restrict__ z, cx<R>* __restrict__ uvec,
-                                                                 const cx<R>* wasm, Groups G, int ldw, int pre) {
+                                                                 int rt, int kseg, const c64* __restrict__ panel,
+                                                                 const c64* __restrict__ dinv, const c64* sf,
+                                                                 c64* __restrict__ z, c64* __restrict__ uvec,
+                                                                 const c64* wasm, Groups G, int ldw, int pre) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int TR = 32 * rt;
-    cx<R>* ws = reinterpret_cast<cx<R>*>(smem_raw);   // [k][GC] own rows of w
-    cx<R>* wt = ws + GC * ldw;                      // [c][TR] the block's boundary rows of w
-    cx<R>* red = wt + GC * TR;                      // [seg][c][TR] partial sums
+    c64* ws = reinterpret_cast<c64*>(smem_raw);   // [k][GC] own rows of w
+    c64* wt = ws + GC * ldw;                      // [c][TR] the block's boundary rows of w
+    c64* red = wt + GC * TR;                      // [seg][c][TR] partial sums
     const int b = blockIdx.x % nblk, rest = blockIdx.x / nblk;
     const int g = rest % G.ngroup;
     const int f = (int)front_list[rest / G.ngroup];
@@ -818,7 +791,7 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 2) fwd_gemv_kernel(Fronts F, co
     const int gc = G.gptr[g + 1] - G.gptr[g], op = G.op[g];
     const int64_t own0 = F.own_start[f];
     const int tid = threadIdx.x, nth = blockDim.x;
-    const cx<R>* __restrict__ P = panel + (int64_t)op * F.panel_total + F.panel_off[f];
+    const c64* __restrict__ P = panel + (int64_t)op * F.panel_total + F.panel_off[f];
     const int lane = tid & 31, warp = tid >> 5;
     const int tile = warp % rt, seg = warp / rt;
     const int rl = tile * 32 + lane, r = r0 + rl;
@@ -828,29 +801,29 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 2) fwd_gemv_kernel(Fronts F, co
     const int k0 = min(kmax, seg * ks), k1 = min(kmax, k0 + ks);
     const bool valid = r < r1;
     // lanes past the block's rows sweep its last row (results dropped)
-    const cx<R>* A = P + (int64_t)k0 * nf + min(r, r1 - 1);
+    const c64* A = P + (int64_t)k0 * nf + min(r, r1 - 1);
     if (pre) {
         for (int q = tid; q < GC * nown; q += nth) {
             const int c = q / nown, r = q - c * nown;
-            ws[r * GC + c] = c < gc ? wasm[(int64_t)gs[c] * F.nfac + own0 + r] : zero<R>();
+            ws[r * GC + c] = c < gc ? wasm[(int64_t)gs[c] * F.nfac + own0 + r] : zero<double>();
         }
         for (int q = tid; q < GC * TR; q += nth) {
             const int c = q / TR, rr = q - c * TR, row = r0 + rr;
             wt[q] = (c < gc && row >= nown && row < r1)
-                        ? uvec[(int64_t)gs[c] * F.vec_total + F.vec_off[f] + (row - nown)] : zero<R>();
+                        ? uvec[(int64_t)gs[c] * F.vec_total + F.vec_off[f] + (row - nown)] : zero<double>();
         }
         __syncthreads();
     } else {
-        for (int q = tid; q < GC * TR; q += nth) wt[q] = zero<R>();
+        for (int q = tid; q < GC * TR; q += nth) wt[q] = zero<double>();
         __syncthreads();
-        fwd_gather<R, GC>(F, f, gs, gc, sf, uvec, ws, wt, TR, r0, r1);
+        fwd_gather<GC>(F, f, gs, gc, sf, uvec, ws, wt, TR, r0, r1);
     }
-    cx<R> l0[LB];
-    prefetch_run<R>(A, nf, k1 - k0, l0);
-    cx<R> acc[GC];
+    c64 l0[LB];
+    prefetch_run(A, nf, k1 - k0, l0);
+    c64 acc[GC];
 #pragma unroll
-    for (int c = 0; c < GC; ++c) acc[c] = zero<R>();
-    sweep<R, GC>(A, nf, ws + k0 * GC, GC, k1 - k0, l0, acc);
+    for (int c = 0; c < GC; ++c) acc[c] = zero<double>();
+    sweep<GC>(A, nf, ws + k0 * GC, GC, k1 - k0, l0, acc);
     if (kseg > 1) {
 #pragma unroll
         for (int c = 0; c < GC; ++c)
@@ -859,7 +832,7 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 2) fwd_gemv_kernel(Fronts F, co
         for (int q = tid; q < gc * TR; q += nth) {
             const int c = q / TR, rr = q - c * TR;
             if (r0 + rr >= r1) continue;
-            cx<R> v = red[c * TR + rr];
+            c64 v = red[c * TR + rr];
             for (int sg = 1; sg < kseg; ++sg) v += red[(sg * GC + c) * TR + rr];
             const int row = r0 + rr;
             if (row < nown) z[(int64_t)gs[c] * F.nfac + own0 + row] = dinv[(int64_t)op * F.nfac + own0 + row] * v;
@@ -867,7 +840,7 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 2) fwd_gemv_kernel(Fronts F, co
         }
     } else if (valid) {
         if (r < nown) {
-            const cx<R> dv = dinv[(int64_t)op * F.nfac + own0 + r];
+            const c64 dv = dinv[(int64_t)op * F.nfac + own0 + r];
 #pragma unroll
             for (int c = 0; c < GC; ++c)
                 if (c < gc) z[(int64_t)gs[c] * F.nfac + own0 + r] = dv * acc[c];
@@ -879,16 +852,16 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 2) fwd_gemv_kernel(Fronts F, co
     }
 }
 
-template <typename R, int GC>
+template <int GC>
 __global__ void __launch_bounds__(SOLVE_THREADS, 2) bwd_gemv_kernel(Fronts F, const int64_t* __restrict__ front_list, int nblk,
                                                                  int ct, int iseg, int cw,
-                                                                 const cx<R>* __restrict__ panel_rm,
-                                                                 const cx<R>* __restrict__ z, cx<R>* __restrict__ y,
-                                                                 cx<R>* __restrict__ sd, Groups G, int ldv) {
+                                                                 const c64* __restrict__ panel_rm,
+                                                                 const c64* __restrict__ z, c64* __restrict__ y,
+                                                                 c64* __restrict__ sd, Groups G, int ldv) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int TC = cw * ct;       // a tile: cw columns, its warp's 32 / cw lane groups take alternate rows
-    cx<R>* v = reinterpret_cast<cx<R>*>(smem_raw);    // [i - kb0][GC]: rows kb0 .. nf of [z_own; y_bnd]
-    cx<R>* red = v + GC * ldv;                      // [seg][c][TC]
+    c64* v = reinterpret_cast<c64*>(smem_raw);    // [i - kb0][GC]: rows kb0 .. nf of [z_own; y_bnd]
+    c64* red = v + GC * ldv;                      // [seg][c][TC]
     const int b = blockIdx.x % nblk, rest = blockIdx.x / nblk;
     const int g = rest % G.ngroup;
     const int f = (int)front_list[rest / G.ngroup];
@@ -901,7 +874,7 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 2) bwd_gemv_kernel(Fronts F, co
     const int64_t own0 = F.own_start[f];
     const int64_t* bnd = F.bnd_idx + F.bnd_ptr[f];
     const int tid = threadIdx.x, nth = blockDim.x;
-    const cx<R>* __restrict__ P = panel_rm + (int64_t)op * F.panel_total + F.panel_off[f];   // (nf x nown) row-major
+    const c64* __restrict__ P = panel_rm + (int64_t)op * F.panel_total + F.panel_off[f];   // (nf x nown) row-major
     const int lane = tid & 31, warp = tid >> 5;
     const int nph = 32 / cw, ph = lane / cw;
     const int tile = warp % ct, seg = warp / ct;
@@ -913,13 +886,13 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 2) bwd_gemv_kernel(Fronts F, co
     const int cnt = max(0, (i1 - i0 - ph + nph - 1) / nph);
     const bool valid = k < kb1;
     // lanes past the block's columns sweep its last column (results dropped)
-    const cx<R>* A = P + (int64_t)(i0 + ph) * nown + min(k, kb1 - 1);
-    cx<R> l0[LB];
-    prefetch_run<R>(A, nph * nown, cnt, l0);
+    const c64* A = P + (int64_t)(i0 + ph) * nown + min(k, kb1 - 1);
+    c64 l0[LB];
+    prefetch_run(A, nph * nown, cnt, l0);
     const int nv = nf - kb0, tot = gc * nv;
     for (int q = gc * nv + tid; q < GC * nv; q += nth) {
         const int c = q / nv;
-        v[(q - c * nv) * GC + c] = zero<R>();
+        v[(q - c * nv) * GC + c] = zero<double>();
     }
     for (int q0 = tid; q0 < tot; q0 += 4 * nth) {
         int64_t src[4];
@@ -928,7 +901,7 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 2) bwd_gemv_kernel(Fronts F, co
             const int q = min(q0 + u * nth, tot - 1), c = q / nv, i = kb0 + (q - c * nv);
             src[u] = (int64_t)gs[c] * F.nfac + (i < nown ? own0 + i : bnd[i - nown]);
         }
-        cx<R> x[4];
+        c64 x[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const int q = min(q0 + u * nth, tot - 1), c = q / nv, i = kb0 + (q - c * nv);
@@ -941,10 +914,10 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 2) bwd_gemv_kernel(Fronts F, co
         }
     }
     __syncthreads();
-    cx<R> acc[GC];
+    c64 acc[GC];
 #pragma unroll
-    for (int c = 0; c < GC; ++c) acc[c] = zero<R>();
-    sweep<R, GC>(A, nph * nown, v + (i0 + ph - kb0) * GC, nph * GC, cnt, l0, acc);
+    for (int c = 0; c < GC; ++c) acc[c] = zero<double>();
+    sweep<GC>(A, nph * nown, v + (i0 + ph - kb0) * GC, nph * GC, cnt, l0, acc);
     if (nph == 2) {
 #pragma unroll
         for (int c = 0; c < GC; ++c) {
@@ -960,7 +933,7 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 2) bwd_gemv_kernel(Fronts F, co
         for (int q = tid; q < gc * TC; q += nth) {
             const int c = q / TC, kk = q - c * TC;
             if (kb0 + kk >= kb1) continue;
-            cx<R> s = red[c * TC + kk];
+            c64 s = red[c * TC + kk];
             for (int sg = 1; sg < iseg; ++sg) s += red[(sg * GC + c) * TC + kk];
             y[(int64_t)gs[c] * F.nfac + own0 + kb0 + kk] = s;
             sd[(int64_t)gs[c] * F.nnode + F.iperm[own0 + kb0 + kk]] = s;
@@ -995,9 +968,9 @@ static void solve_shape(int nfront_level, int ntile, int inner, int& per_blk, in
     }
 }
 
-template <typename R, int GC>
+template <int GC>
 static void fwd_level_gc(const Fronts& F, const int64_t* front_list, int nf_level, int max_nf, int max_nown,
-                         const cx<R>* panel, const cx<R>* dinv, const cx<R>* sf, cx<R>* z, cx<R>* uvec, cx<R>* wasm,
+                         const c64* panel, const c64* dinv, const c64* sf, c64* z, c64* uvec, c64* wasm,
                          const Groups& G, cudaStream_t st) {
     const int ntask = nf_level * G.ngroup;
     const int ntile = ceil_div(max_nf, 32);
@@ -1007,21 +980,21 @@ static void fwd_level_gc(const Fronts& F, const int64_t* front_list, int nf_leve
     const int pre = nblk > 1;
     if (pre) {
         const int TRa = std::max(max_nf - 1, 1);
-        const size_t sa = (size_t)GC * (ldw + TRa) * sizeof(cx<R>);
-        smem_attr<R>((const void*)fwd_assemble_kernel<R, GC>, sa);
-        fwd_assemble_kernel<R, GC><<<ntask, 256, sa, st>>>(F, front_list, sf, uvec, wasm, G, ldw, TRa);
+        const size_t sa = (size_t)GC * (ldw + TRa) * sizeof(c64);
+        raise_smem((const void*)fwd_assemble_kernel<GC>, sa);
+        fwd_assemble_kernel<GC><<<ntask, 256, sa, st>>>(F, front_list, sf, uvec, wasm, G, ldw, TRa);
         GT_LAUNCH_CHECK();
     }
-    const size_t sm = (size_t)GC * (ldw + 32 * rt + (kseg > 1 ? kseg * 32 * rt : 0)) * sizeof(cx<R>);
-    smem_attr<R>((const void*)fwd_gemv_kernel<R, GC>, sm);
-    fwd_gemv_kernel<R, GC><<<ntask * nblk, 32 * rt * kseg, sm, st>>>(F, front_list, nblk, rt, kseg, panel, dinv, sf, z, uvec,
+    const size_t sm = (size_t)GC * (ldw + 32 * rt + (kseg > 1 ? kseg * 32 * rt : 0)) * sizeof(c64);
+    raise_smem((const void*)fwd_gemv_kernel<GC>, sm);
+    fwd_gemv_kernel<GC><<<ntask * nblk, 32 * rt * kseg, sm, st>>>(F, front_list, nblk, rt, kseg, panel, dinv, sf, z, uvec,
                                                                 wasm, G, ldw, pre);
     GT_LAUNCH_CHECK();
 }
 
-template <typename R, int GC>
+template <int GC>
 static void bwd_level_gc(const Fronts& F, const int64_t* front_list, int nf_level, int max_nf, int max_nown,
-                         const cx<R>* panel_rm, const cx<R>* z, cx<R>* y, cx<R>* sd, const Groups& G, cudaStream_t st) {
+                         const c64* panel_rm, const c64* z, c64* y, c64* sd, const Groups& G, cudaStream_t st) {
     const int ntask = nf_level * G.ngroup;
     // tiles of 16 columns (two lane groups on alternate rows) where they waste fewer lanes than 32
     const int cw = ceil_div(max_nown, 16) * 16 - max_nown < ceil_div(max_nown, 32) * 32 - max_nown ? 16 : 32;
@@ -1029,42 +1002,37 @@ static void bwd_level_gc(const Fronts& F, const int64_t* front_list, int nf_leve
     int ct, iseg;
     solve_shape(nf_level, ntile, max_nf, ct, iseg);
     const int nblk = ceil_div(ntile, ct), ldv = std::max(max_nf, 1);
-    const size_t sm = (size_t)GC * (ldv + (iseg > 1 ? iseg * cw * ct : 0)) * sizeof(cx<R>);
-    smem_attr<R>((const void*)bwd_gemv_kernel<R, GC>, sm);
-    bwd_gemv_kernel<R, GC><<<ntask * nblk, 32 * ct * iseg, sm, st>>>(F, front_list, nblk, ct, iseg, cw, panel_rm, z, y, sd,
+    const size_t sm = (size_t)GC * (ldv + (iseg > 1 ? iseg * cw * ct : 0)) * sizeof(c64);
+    raise_smem((const void*)bwd_gemv_kernel<GC>, sm);
+    bwd_gemv_kernel<GC><<<ntask * nblk, 32 * ct * iseg, sm, st>>>(F, front_list, nblk, ct, iseg, cw, panel_rm, z, y, sd,
                                                                  G, ldv);
     GT_LAUNCH_CHECK();
 }
 
 // the column-group widths the sweep kernels are built for: a front's rows for GC columns are staged in shared
 // memory, so wide fronts take narrower groups (the panel is then read once per fewer columns)
-template <typename R>
 void launch_fwd_level(const Fronts& F, const int64_t* front_list, int nf_level, int max_nf, int max_nown,
-                      const cx<R>* panel, const cx<R>* dinv, const cx<R>* sf, cx<R>* z, cx<R>* uvec, cx<R>* wasm,
+                      const c64* panel, const c64* dinv, const c64* sf, c64* z, c64* uvec, c64* wasm,
                       const Groups& G, int gmax, cudaStream_t st) {
     switch (gmax) {
-        case 8: fwd_level_gc<R, 8>(F, front_list, nf_level, max_nf, max_nown, panel, dinv, sf, z, uvec, wasm, G, st); return;
-        case 4: fwd_level_gc<R, 4>(F, front_list, nf_level, max_nf, max_nown, panel, dinv, sf, z, uvec, wasm, G, st); return;
-        case 2: fwd_level_gc<R, 2>(F, front_list, nf_level, max_nf, max_nown, panel, dinv, sf, z, uvec, wasm, G, st); return;
-        case 1: fwd_level_gc<R, 1>(F, front_list, nf_level, max_nf, max_nown, panel, dinv, sf, z, uvec, wasm, G, st); return;
+        case 8: fwd_level_gc<8>(F, front_list, nf_level, max_nf, max_nown, panel, dinv, sf, z, uvec, wasm, G, st); return;
+        case 4: fwd_level_gc<4>(F, front_list, nf_level, max_nf, max_nown, panel, dinv, sf, z, uvec, wasm, G, st); return;
+        case 2: fwd_level_gc<2>(F, front_list, nf_level, max_nf, max_nown, panel, dinv, sf, z, uvec, wasm, G, st); return;
+        case 1: fwd_level_gc<1>(F, front_list, nf_level, max_nf, max_nown, panel, dinv, sf, z, uvec, wasm, G, st); return;
         default: throw CudaError{cudaErrorInvalidValue, "column group width must be 8, 4, 2 or 1"};
     }
 }
 
-template <typename R>
 void launch_bwd_level(const Fronts& F, const int64_t* front_list, int nf_level, int max_nf, int max_nown,
-                      const cx<R>* panel_rm, const cx<R>* z, cx<R>* y, cx<R>* sd, const Groups& G, int gmax,
+                      const c64* panel_rm, const c64* z, c64* y, c64* sd, const Groups& G, int gmax,
                       cudaStream_t st) {
     switch (gmax) {
-        case 8: bwd_level_gc<R, 8>(F, front_list, nf_level, max_nf, max_nown, panel_rm, z, y, sd, G, st); return;
-        case 4: bwd_level_gc<R, 4>(F, front_list, nf_level, max_nf, max_nown, panel_rm, z, y, sd, G, st); return;
-        case 2: bwd_level_gc<R, 2>(F, front_list, nf_level, max_nf, max_nown, panel_rm, z, y, sd, G, st); return;
-        case 1: bwd_level_gc<R, 1>(F, front_list, nf_level, max_nf, max_nown, panel_rm, z, y, sd, G, st); return;
+        case 8: bwd_level_gc<8>(F, front_list, nf_level, max_nf, max_nown, panel_rm, z, y, sd, G, st); return;
+        case 4: bwd_level_gc<4>(F, front_list, nf_level, max_nf, max_nown, panel_rm, z, y, sd, G, st); return;
+        case 2: bwd_level_gc<2>(F, front_list, nf_level, max_nf, max_nown, panel_rm, z, y, sd, G, st); return;
+        case 1: bwd_level_gc<1>(F, front_list, nf_level, max_nf, max_nown, panel_rm, z, y, sd, G, st); return;
         default: throw CudaError{cudaErrorInvalidValue, "column group width must be 8, 4, 2 or 1"};
     }
 }
-
-template void launch_fwd_level<double>(const Fronts&, const int64_t*, int, int, int, const c64*, const c64*, const c64*, c64*, c64*, c64*, const Groups&, int, cudaStream_t);
-template void launch_bwd_level<double>(const Fronts&, const int64_t*, int, int, int, const c64*, const c64*, c64*, c64*, const Groups&, int, cudaStream_t);
 
 }  // namespace gt

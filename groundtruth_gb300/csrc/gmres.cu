@@ -446,29 +446,6 @@ __global__ void init_state_kernel(GmresState s, const int* __restrict__ slot_col
     s.eta[slot] = fmax(inner_tol, need);
 }
 
-// x[col] += rho[col] * e[slot] (FP64 accumulation of the cycle's correction)
-template <typename R>
-__global__ void refine_kernel(c64* __restrict__ x, int64_t ldx, const cx<R>* __restrict__ e, int64_t lde,
-                              const int* __restrict__ slot_col, const double* __restrict__ rho, int64_t n) {
-    const int slot = blockIdx.y;
-    const int col = slot_col[slot];
-    const double f = rho[col];
-    const cx<R>* es = e + (int64_t)slot * lde;
-    c64* xc = x + (int64_t)col * ldx;
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x)
-        xc[q] += f * cvt<double>(es[q]);
-}
-
-__global__ void any_active_kernel(const int* __restrict__ active, int n, int* __restrict__ flag) {
-    __shared__ int any;
-    if (threadIdx.x == 0) any = 0;
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x)
-        if (active[i]) any = 1;
-    __syncthreads();
-    if (threadIdx.x == 0) *flag = any;
-}
-
 __global__ void sqrt_norms_kernel(const c64* __restrict__ nrm2, int ld, int n, double* __restrict__ out) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = sqrt(nrm2[(int64_t)i * ld].re);
@@ -563,17 +540,6 @@ void launch_init_state(const GmresState& s, const int* slot_col, const double* r
     init_state_kernel<<<ceil_div(s.nslot, 64), 64, 0, st>>>(s, slot_col, rho, bnorm, tol, inner_tol);
     GT_LAUNCH_CHECK();
 }
-template <typename R>
-void launch_refine(c64* x, int64_t ldx, const cx<R>* e, int64_t lde, const int* slot_col, const double* rho, int64_t n,
-                   int nslot, cudaStream_t st) {
-    int blocks = (int)std::min<int64_t>((n + 255) / 256, 1024);
-    refine_kernel<R><<<dim3(blocks, nslot), 256, 0, st>>>(x, ldx, e, lde, slot_col, rho, n);
-    GT_LAUNCH_CHECK();
-}
-void launch_any_active(const int* active, int n, int* flag, cudaStream_t st) {
-    any_active_kernel<<<1, 256, 0, st>>>(active, n, flag);
-    GT_LAUNCH_CHECK();
-}
 __global__ void sqrt_norms_active_kernel(const c64* __restrict__ nrm2, int ld, int n, const int* __restrict__ active,
                                          double* __restrict__ out) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -594,7 +560,5 @@ template void launch_scale<float, h16c>(const GmresStateT<float, h16c>&, int, in
 template void launch_init_cycle<float, c32>(const GmresStateT<float, c32>&, const c64*, int64_t, const int*, const double*, int64_t, cudaStream_t);
 template void launch_init_cycle<float, h16c>(const GmresStateT<float, h16c>&, const c64*, int64_t, const int*, const double*, int64_t, cudaStream_t);
 template void launch_init_cycle<double, c64>(const GmresStateT<double, c64>&, const c64*, int64_t, const int*, const double*, int64_t, cudaStream_t);
-template void launch_refine<float>(c64*, int64_t, const c32*, int64_t, const int*, const double*, int64_t, int, cudaStream_t);
-template void launch_refine<double>(c64*, int64_t, const c64*, int64_t, const int*, const double*, int64_t, int, cudaStream_t);
 
 }  // namespace gt

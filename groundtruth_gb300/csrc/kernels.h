@@ -205,13 +205,11 @@ void launch_panel_convert(const Fronts& F, const SweepPlan& S, const int64_t* fr
 // forward: own rows from s in factor order (sf), results to z (factor order) and the update vectors (wasm:
 // factor-ordered scratch for fronts assembled ahead of a split product, may be sf itself);
 // backward: reads z and the ancestors' y, writes y (factor order) and sd (node order)
-template <typename R>
 void launch_fwd_level(const Fronts& F, const int64_t* front_list, int nf_level, int max_nf, int max_nown,
-                      const cx<R>* panel, const cx<R>* dinv, const cx<R>* sf, cx<R>* z, cx<R>* uvec, cx<R>* wasm,
+                      const c64* panel, const c64* dinv, const c64* sf, c64* z, c64* uvec, c64* wasm,
                       const Groups& G, int gmax, cudaStream_t st);
-template <typename R>
 void launch_bwd_level(const Fronts& F, const int64_t* front_list, int nf_level, int max_nf, int max_nown,
-                      const cx<R>* panel_rm, const cx<R>* z, cx<R>* y, cx<R>* sd, const Groups& G, int gmax,
+                      const c64* panel_rm, const c64* z, c64* y, c64* sd, const Groups& G, int gmax,
                       cudaStream_t st);
 
 // --- low-rank branch update of a factorised Schur complement (woodbury.cu)

@@ -52,10 +52,6 @@ void launch_init_cycle(const GmresStateT<R, B>& s, const c64* r, int64_t ldr, co
                        int64_t n, cudaStream_t st);
 void launch_init_state(const GmresState& s, const int* slot_col, const double* rho, const double* bnorm, double tol,
                        double inner_tol, cudaStream_t st);
-template <typename R>
-void launch_refine(c64* x, int64_t ldx, const cx<R>* e, int64_t lde, const int* slot_col, const double* rho, int64_t n,
-                   int nslot, cudaStream_t st);
-void launch_any_active(const int* active, int n, int* flag, cudaStream_t st);
 // dst[slot_col[s]] = src[s] (precision R -> FP64), s < nslot
 template <typename R>
 void launch_to64(c64* dst, int64_t ldd, const cx<R>* src, int64_t lds, const int* slot_col, int64_t n, int nslot,

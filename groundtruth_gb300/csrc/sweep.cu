@@ -158,8 +158,8 @@ __device__ __forceinline__ void mac_row(uint64_t* re, uint64_t* im, float pr, fl
 }
 
 struct SwArgs {
-    const SwTask* tasks;               // nft forward tasks, then nbt backward ones
-    int nft, nbt;
+    const SwTask* tasks;               // nft forward tasks, then the backward ones
+    int nft;
     int nsrc;
     int64_t src_rows;
     const int* src;                    // [nsrc][src_rows] update-vector rows added into a front's rows (-1: none)
@@ -549,7 +549,6 @@ void launch_sweep(const SweepPlan& S, const Fronts& F, const c32* pf, const c32*
     SwArgs A{};
     A.tasks = S.tasks;
     A.nft = S.nft;
-    A.nbt = S.nbt;
     A.nsrc = S.nsrc;
     A.src_rows = S.src_rows;
     A.src = S.src;
