@@ -906,6 +906,11 @@ __global__ void __launch_bounds__(1024) lp_pass_c(const cx<R>* __restrict__ T, c
 // ------------------------------------------------------------------------------------------ launchers
 template <typename R> static int ldt_of(const LpArgs<R>& a) { return a.ldt > 0 ? a.ldt : a.n0; }
 template <typename R> static bool b8_fits(const LpArgs<R>& a);
+template <typename R> static bool rw_fits(const LpArgs<R>& a);
+// the column lengths that FP32 transforms by warps (launch_b)
+constexpr bool warp_column(int P) {
+    return P == 96 || P == 128 || P == 192 || P == 256 || P == 384 || P == 512 || P == 768 || P == 1024;
+}
 template <typename R>
 static void set_smem(const void* fn, size_t bytes) { raise_smem(fn, bytes); }
 
@@ -921,8 +926,9 @@ void lp_shapes(const LpArgs<R>& a, int* rows_out, int* bt_out) {
     const int per_col = b8_fits(a) ? teamB : a.S * teamB;
     while (bt > 1 && (bt * per_col > 512 * (b8_fits(a) ? 1 : 2) ||
                       nbuf * bt * a.S * srow(a.P0) * sizeof(cx<R>) > 160 * 1024)) bt /= 2;
-    *rows_out = rows;
-    *bt_out = bt;
+    // the passes by warps have shapes of their own
+    *rows_out = rw_fits(a) ? 1 : rows;
+    *bt_out = std::is_same<R, float>::value && warp_column(a.P0) ? 1 : bt;
 }
 
 // the specialised lengths; others run the runtime-length kernels
@@ -997,8 +1003,7 @@ static void launch_bg(const LpArgs<float>& a, cudaStream_t st) {
 template <typename R, int PB>
 static void launch_b(const LpArgs<R>& a, int bt, cudaStream_t st) {
     // FP32: warp transforms for the lengths of 32 A (every length P0 >= 2 n0 - 1 is even, so n0 <= P0 / 2)
-    constexpr bool warp = std::is_same<R, float>::value && (PB == 96 || PB == 128 || PB == 192 || PB == 256 || PB == 384 ||
-                                                            PB == 512 || PB == 768 || PB == 1024);
+    constexpr bool warp = std::is_same<R, float>::value && warp_column(PB);
     if constexpr (warp) {
         if constexpr (PB == 512) {
             if (a.S == 2) return launch_bw<2>(a, st);
