@@ -270,8 +270,8 @@ struct gt_geometry {
     int* d_xfirst = nullptr;           // the large fronts' first diagonal block among all of theirs
     int64_t xtotal = 0;
     // every large front (all levels), for the blocked selective inversion
+    InvertPlan invert;
     int64_t* d_bigfronts = nullptr;
-    int nbig = 0, bigmax_nf = 1, bigmax_nown = 1;
     int64_t n_compact = 0, n_strips = 0;
     int64_t* d_c2d = nullptr;
     int64_t* d_sterm_ptr = nullptr;
@@ -1562,15 +1562,10 @@ int gt_geometry_create(const gt_geometry_desc* d, gt_geometry** out) {
         }
         G->d_forder = p.upload(ord.data(), ord.size());
         std::vector<int64_t> big;
-        for (int f = 0; f < nf; ++f) {
-            const int nff = (int)(d->nown[f] + d->nbnd[f]);
-            if (xfirst[f] < 0) continue;
-            big.push_back(f);
-            G->bigmax_nf = std::max(G->bigmax_nf, nff);
-            G->bigmax_nown = std::max<int>(G->bigmax_nown, (int)d->nown[f]);
-        }
-        G->nbig = (int)big.size();
-        G->d_bigfronts = p.upload(big.data(), big.size());
+        for (int f = 0; f < nf; ++f)
+            if (xfirst[f] >= 0) big.push_back(f);
+        G->invert = make_invert_plan(std::move(big), d->nown, d->nbnd, FACTOR_BLOCK);
+        G->d_bigfronts = p.upload(G->invert.fronts.data(), G->invert.fronts.size());
         G->d_xfirst = p.upload(xfirst.data(), xfirst.size());
     }
     {
@@ -1766,12 +1761,11 @@ int gt_operators_create_ex(gt_geometry* G, int32_t n_ops, const double* omega, c
     }
     {
         Scope sc(P, "factor_invert_tiled", st);
-        launch_invert_tiled(F, G->d_bigfronts, G->nbig, G->bigmax_nf, G->bigmax_nown, O->panel64, xinv, G->d_xfirst, G->xtotal,
-                            n_ops, st);
+        launch_invert_tiled(F, G->d_bigfronts, G->invert, O->panel64, xinv, G->d_xfirst, G->xtotal, n_ops, st);
     }
     {
         Scope sc(P, "factor_convert", st);
-        launch_panel_convert(F, G->sweep, G->d_bigfronts, G->nbig, O->panel64, O->panel32, O->panel32_b, O->panel64_rm,
+        launch_panel_convert(F, G->sweep, G->d_bigfronts, (int)G->invert.fronts.size(), O->panel64, O->panel32, O->panel32_b, O->panel64_rm,
                              O->dinv64, O->dinv32, n_ops, st);
     }
     int h_status = 0;

@@ -579,21 +579,21 @@ __global__ void __launch_bounds__(256) inv_trail_kernel(Fronts F, const int64_t*
     }
 }
 
-void launch_invert_tiled(const Fronts& F, const int64_t* front_list, int nfront, int max_nf, int max_nown, c64* panel,
-                         const c64* xinv, const int* xfirst, int64_t xtotal, int nops, cudaStream_t st) {
-    if (nfront <= 0) return;
+void launch_invert_tiled(const Fronts& F, const int64_t* front_list, const InvertPlan& plan, c64* panel, const c64* xinv,
+                         const int* xfirst, int64_t xtotal, int nops, cudaStream_t st) {
     const DiagInv X{const_cast<c64*>(xinv), xfirst, xtotal};
-    for (int kb = 0; kb < max_nown; kb += FB) {
-        pdl_launch(inv_rows_kernel, dim3(kb / 32 + 1, nfront, nops), 256, 0, st, F, front_list, kb, panel, X);
+    for (size_t s = 0; s < plan.count.size(); ++s) {
+        const int kb = (int)s * FB, n = plan.count[s];
+        pdl_launch(inv_rows_kernel, dim3(kb / 32 + 1, n, nops), 256, 0, st, F, front_list, kb, panel, X);
         GT_LAUNCH_CHECK();
-        const int below = max_nf - kb - 1;
+        const int below = plan.max_nf[s] - kb - 1;
         if (below <= 0) continue;
         const int rt = ceil_div(below, FT);
         if (kb > 0) {
-            pdl_launch(inv_trail_kernel, dim3(rt * ceil_div(kb, FT), nfront, nops), 256, 0, st, F, front_list, kb, panel, 0);
+            pdl_launch(inv_trail_kernel, dim3(rt * ceil_div(kb, FT), n, nops), 256, 0, st, F, front_list, kb, panel, 0);
             GT_LAUNCH_CHECK();
         }
-        pdl_launch(inv_trail_kernel, dim3(rt, nfront, nops), 256, 0, st, F, front_list, kb, panel, 1);
+        pdl_launch(inv_trail_kernel, dim3(rt, n, nops), 256, 0, st, F, front_list, kb, panel, 1);
         GT_LAUNCH_CHECK();
     }
 }

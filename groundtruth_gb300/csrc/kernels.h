@@ -1,6 +1,7 @@
 // Launch interfaces between the kernel files and the host driver (api.cu).
 #pragma once
 #include "common.cuh"
+#include "invert_plan.h"
 #include "sweep_plan.h"
 
 namespace gt {
@@ -193,9 +194,10 @@ constexpr int FACTOR_BLOCK = 32;
 void launch_factor_tiled(const Fronts& F, const int64_t* front_list, int nf_level, int max_nf, int max_nown,
                          const c64* svals, c64* panel, c64* upd, c64* xinv, const int* xfirst, int64_t xtotal, int nops,
                          int* status, cudaStream_t st);
-// the listed (large) fronts' own blocks replaced by their inverses and the boundary rows by -L_bnd Linv_own, in place
-void launch_invert_tiled(const Fronts& F, const int64_t* front_list, int nfront, int max_nf, int max_nown, c64* panel,
-                         const c64* xinv, const int* xfirst, int64_t xtotal, int nops, cudaStream_t st);
+// the large fronts' own blocks replaced by their inverses and the boundary rows by -L_bnd Linv_own, in place (front_list: the
+// plan's fronts on the device)
+void launch_invert_tiled(const Fronts& F, const int64_t* front_list, const InvertPlan& plan, c64* panel, const c64* xinv,
+                         const int* xfirst, int64_t xtotal, int nops, cudaStream_t st);
 // their solve panels: unit diagonal (pivot reciprocals to d64 / d32, [op][nfac]), the FP32 sweeps' forward and backward
 // tiles (pf, pb) and the FP64 row-major copy
 void launch_panel_convert(const Fronts& F, const SweepPlan& S, const int64_t* front_list, int nfront, c64* p64, c32* pf, c32* pb,
