@@ -1927,7 +1927,7 @@ int gt_to_dense(gt_geometry* G, int32_t n_cols, const double* compact, void* den
     GT_GUARD_BEGIN
     cudaStream_t st = (cudaStream_t)stream;
     Pool tmp;
-    c64* d_in = tmp.upload(reinterpret_cast<const c64*>(compact), (size_t)n_cols * G->n_compact);
+    c64* d_in = tmp.upload(reinterpret_cast<const c64*>(compact), (size_t)n_cols * G->n_compact, st);
     GT_CUDA(cudaMemsetAsync(dense, 0, (size_t)n_cols * G->geo.n * sizeof(c64), st));
     launch_scatter(G->d_c2d, G->n_compact, d_in, G->n_compact, static_cast<c64*>(dense), G->geo.n, n_cols, st);
     GT_CUDA(cudaStreamSynchronize(st));
@@ -2049,22 +2049,25 @@ int gt_apply(gt_geometry* G, gt_operators* ops, int32_t kind, int32_t precision,
     cudaStream_t st = (cudaStream_t)stream;
     const int64_t n = G->geo.n, nc = G->n_compact;
     Pool tmp;
-    c64* d_c = tmp.upload(reinterpret_cast<const c64*>(x), (size_t)n_cols * nc);
+    c64* d_c = tmp.upload(reinterpret_cast<const c64*>(x), (size_t)n_cols * nc, st);
     c64* xin = tmp.alloc<c64>((size_t)n_cols * n);
     c64* yout = tmp.alloc<c64>((size_t)n_cols * n);
-    int* d_op = tmp.upload(col_op, n_cols);
     GT_CUDA(cudaMemsetAsync(xin, 0, (size_t)n_cols * n * sizeof(c64), st));
     GT_CUDA(cudaMemsetAsync(yout, 0, (size_t)n_cols * n * sizeof(c64), st));
     launch_scatter(G->d_c2d, nc, d_c, nc, xin, n, n_cols, st);
     std::vector<int> h_op(col_op, col_op + n_cols), h_pc(n_cols);
     for (int c = 0; c < n_cols; ++c) h_pc[c] = ops->fslot[h_op[c]];
-    int* d_pc = tmp.upload(h_pc.data(), n_cols);
     // kind 1 groups columns by factorisation: require them sorted
     for (int c = 1; c < n_cols; ++c)
         if (kind == 1 && h_pc[c] < h_pc[c - 1]) throw Invalid("preconditioner columns must be sorted by operator");
-    unsigned int* gave_up = tmp.alloc<unsigned int>(N_WAITS);
+    // the columns' operators and factorisations, and the count of FP32's waits that ran out
+    std::vector<int> h_tab(h_op);
+    h_tab.insert(h_tab.end(), h_pc.begin(), h_pc.end());
+    h_tab.resize(h_tab.size() + N_WAITS, 0);
+    int* d_op = tmp.upload(h_tab.data(), h_tab.size(), st);
+    int* d_pc = d_op + n_cols;
+    unsigned int* gave_up = reinterpret_cast<unsigned int*>(d_pc + n_cols);
     unsigned int h_gave_up[N_WAITS] = {};
-    GT_CUDA(cudaMemsetAsync(gave_up, 0, sizeof(h_gave_up), st));
     auto run = [&](auto tag) {
         using R = decltype(tag);
         cx<R>* xi;
@@ -2081,7 +2084,9 @@ int gt_apply(gt_geometry* G, gt_operators* ops, int32_t kind, int32_t precision,
             GT_CUDA(cudaMemcpy(hx.data(), xin, hx.size() * sizeof(c64), cudaMemcpyDeviceToHost));
             std::vector<c32> h32(hx.size());
             for (size_t i = 0; i < hx.size(); ++i) h32[i] = cvt<float>(hx[i]);
-            GT_CUDA(cudaMemcpy(xi, h32.data(), h32.size() * sizeof(c32), cudaMemcpyHostToDevice));
+            GT_CUDA(cudaMemcpyAsync(xi, h32.data(), h32.size() * sizeof(c32), cudaMemcpyHostToDevice, st));
+            GT_CUDA(cudaStreamSynchronize(st));          // h32 goes out of scope
+            GT_CUDA(cudaMemsetAsync(yo, 0, (size_t)n_cols * n * sizeof(c32), st));     // (kind 2 writes the strips only)
         }
         if (kind == 0 || kind == 2) {
             cx<R>* T = tmp.alloc<cx<R>>(t_entries(G, n_cols));
@@ -2091,10 +2096,11 @@ int gt_apply(gt_geometry* G, gt_operators* ops, int32_t kind, int32_t precision,
             for (int c = 0; c < n_cols; ++c) all[c] = c;
             const int gmax = group_max(G, sizeof(cx<R>));
             make_groups(all, h_pc, gmax, gptr, gslot, gop, gpair);
-            int* g0 = tmp.upload(gptr.data(), gptr.size());
-            int* g1 = tmp.upload(gslot.data(), gslot.size());
-            int* g2 = tmp.upload(gop.data(), gop.size());
-            Groups grp{(int)gop.size(), g0, g1, g2, tmp.upload(gpair.data(), gpair.size())};
+            int* g0 = tmp.upload(gptr.data(), gptr.size(), st);
+            int* g1 = tmp.upload(gslot.data(), gslot.size(), st);
+            int* g2 = tmp.upload(gop.data(), gop.size(), st);
+            Groups grp{(int)gop.size(), g0, g1, g2, tmp.upload(gpair.data(), gpair.size(), st)};
+            GT_CUDA(cudaStreamSynchronize(st));          // the group tables go out of scope
             constexpr bool f32 = sizeof(R) == 4;
             const size_t wide = (size_t)(f32 ? 2 : 1) * n_cols;
             cx<R>* zf = tmp.alloc<cx<R>>(wide * G->F.nfac);
@@ -2112,14 +2118,15 @@ int gt_apply(gt_geometry* G, gt_operators* ops, int32_t kind, int32_t precision,
             GT_CUDA(cudaMemcpy(h32.data(), yo, h32.size() * sizeof(c32), cudaMemcpyDeviceToHost));
             std::vector<c64> h64(h32.size());
             for (size_t i = 0; i < h32.size(); ++i) h64[i] = cvt<double>(h32[i]);
-            GT_CUDA(cudaMemcpy(yout, h64.data(), h64.size() * sizeof(c64), cudaMemcpyHostToDevice));
+            GT_CUDA(cudaMemcpyAsync(yout, h64.data(), h64.size() * sizeof(c64), cudaMemcpyHostToDevice, st));
+            GT_CUDA(cudaStreamSynchronize(st));          // h64 goes out of scope
         }
     };
     if (precision == 1) run(double{});
     else run(float{});
     launch_gather(G->d_c2d, nc, yout, n, d_c, nc, n_cols, st);
     GT_CUDA(cudaMemcpyAsync(y, d_c, (size_t)n_cols * nc * sizeof(c64), cudaMemcpyDeviceToHost, st));
-    GT_CUDA(cudaMemcpyAsync(h_gave_up, gave_up, sizeof(h_gave_up), cudaMemcpyDeviceToHost, st));
+    if (precision != 1) GT_CUDA(cudaMemcpyAsync(h_gave_up, gave_up, sizeof(h_gave_up), cudaMemcpyDeviceToHost, st));
     GT_CUDA(cudaStreamSynchronize(st));
     check_waits(h_gave_up);
     return GT_OK;
