@@ -388,8 +388,11 @@ __global__ void __launch_bounds__(BW_WARPS * 32, GT_BW_MINB) lp_pass_bw(int n0, 
 // multiply, one thread per pixel of a column, and back.  A block takes as many columns as give it about four warps.
 // The Stockham form of these lengths (lp_pass_b) moves every value through shared memory four times per transform under
 // block-wide barriers and spills: 103 us for six columns of a four-sheet 131 x 203 board at length 384.
-template <int A>
-__global__ void __launch_bounds__(256, 2) lp_pass_bg(int S, int n0, int P1, int ncol, int bt, const float* __restrict__ spec,
+// HELP: the warps from rw on have no rows, they help with the spectrum's column and the multiply where there are few columns.
+// One column took up to three times as long without them as in the Stockham form (four sheets of 120 x 64: 10.7 us, 30.2, now
+// 11.4; six of 250 x 64: 16.4, 51.6, 26.5), many are slower with the registers of their tests.
+template <int A, bool HELP>
+__global__ void __launch_bounds__(256, 2) lp_pass_bg(int S, int n0, int P1, int ncol, int bt, int rw, const float* __restrict__ spec,
                                                      const c32* __restrict__ tw, c32* __restrict__ T, int ldt) {
     pdl_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -397,11 +400,11 @@ __global__ void __launch_bounds__(256, 2) lp_pass_bg(int S, int n0, int P1, int 
     c32* Z = reinterpret_cast<c32*>(smem_raw);           // [row][k1 * 33 + k2], pixel k1 + A k2
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int c = blockIdx.x, b0 = blockIdx.y * bt, nb = min(bt, ncol - b0), nrow = nb * S;
-    c32* sx = Z + warp * RR * RS;
+    c32* sx = Z + warp * RR * RS;                        // (of a warp with rows)
     // the spectrum's column, [Q0][S S] padded to an odd stride: read from global memory by the pixels' threads, each S x S
     // block a strided run, it took 77 us of the same six columns, 43 so
     const int SS = S * S, KS = SS | 1;
-    float* Ks = reinterpret_cast<float*>(Z + (blockDim.x >> 5) * RR * RS);
+    float* Ks = reinterpret_cast<float*>(Z + (HELP ? rw : (int)(blockDim.x >> 5)) * RR * RS);
     {
         const float* Kc = spec + (int64_t)min(c, P1 - c) * Q0 * SS;
         for (int q = threadIdx.x; q < Q0 * SS; q += blockDim.x) {
@@ -418,7 +421,7 @@ __global__ void __launch_bounds__(256, 2) lp_pass_bg(int S, int n0, int P1, int 
         src[q] = T + (((int64_t)(b0 + min(b, nb - 1)) * S + (row - b * S)) * P1 + c) * ldt;
     }
     c32 u[32];
-    {
+    if (!HELP || (int)threadIdx.x < 32 * rw) {
         c32 v[RR][A];
 #pragma unroll
         for (int q = 0; q < RR; ++q)
@@ -428,10 +431,10 @@ __global__ void __launch_bounds__(256, 2) lp_pass_bg(int S, int n0, int P1, int 
                 v[q][r] = r < H && ok[q] && j < n0 ? src[q][j] : zero<float>();
             }
         fftw_fwd<float, A>(v, u, sx, tw);
-    }
-    if (lane < RR * A)
+        if (lane < RR * A)
 #pragma unroll
-        for (int k2 = 0; k2 < 32; ++k2) sx[lane * 33 + k2] = u[k2];
+            for (int k2 = 0; k2 < 32; ++k2) sx[lane * 33 + k2] = u[k2];
+    }
     __syncthreads();
     for (int idx = threadIdx.x; idx < nb * N; idx += blockDim.x) {
         const int b = idx / N, p = idx - b * N, k2 = p / A, k1 = p - k2 * A;
@@ -456,6 +459,7 @@ __global__ void __launch_bounds__(256, 2) lp_pass_bg(int S, int n0, int P1, int 
         }
     }
     __syncthreads();
+    if (HELP && (int)threadIdx.x >= 32 * rw) return;
     const int at = lane < RR * A ? lane : 0;
 #pragma unroll
     for (int k2 = 0; k2 < 32; ++k2) u[k2] = sx[at * 33 + k2];
@@ -992,11 +996,16 @@ template <int A>
 static void launch_bg(const LpArgs<float>& a, cudaStream_t st) {
     constexpr int RR = WarpFft<A>::RR;
     const int bt = std::max(1, std::min(a.ncol, (4 * RR + a.S - 1) / a.S));
-    const int warps = ceil_div(bt * a.S, RR);
-    const size_t sm = (size_t)warps * WarpFft<A>::SLOTS * sizeof(c32) + (size_t)(16 * A + 1) * ((a.S * a.S) | 1) * sizeof(float);
-    set_smem<float>((const void*)lp_pass_bg<A>, sm);
-    pdl_launch(lp_pass_bg<A>, dim3(a.P1, ceil_div(a.ncol, bt)), warps * 32, sm, st, a.S, a.n0, a.P1, a.ncol, bt, a.spec, a.tw0, a.T,
-                                                                          ldt_of(a));
+    const int rw = ceil_div(bt * a.S, RR);
+    // more warps than the rows need, up to eight: for a block that is alone on its SM, and for a few columns (in one block),
+    // where the warps of their rows would take the spectrum's column by more than a dozen loads a thread
+    const dim3 grid(a.P1, ceil_div(a.ncol, bt));
+    const int loads = ceil_div((int64_t)(16 * A + 1) * a.S * a.S, 12 * 32);
+    const int warps = grid.x * grid.y <= 2 * 152 ? 8 : grid.y == 1 ? std::max(rw, std::min(8, loads)) : rw;
+    const size_t sm = (size_t)rw * WarpFft<A>::SLOTS * sizeof(c32) + (size_t)(16 * A + 1) * ((a.S * a.S) | 1) * sizeof(float);
+    const auto kernel = warps > rw ? lp_pass_bg<A, true> : lp_pass_bg<A, false>;
+    set_smem<float>((const void*)kernel, sm);
+    pdl_launch(kernel, grid, warps * 32, sm, st, a.S, a.n0, a.P1, a.ncol, bt, rw, a.spec, a.tw0, a.T, ldt_of(a));
     GT_LAUNCH_CHECK();
 }
 
