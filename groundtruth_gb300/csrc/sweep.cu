@@ -203,8 +203,8 @@ __device__ __forceinline__ void sw_sources(const SwArgs& A, int nsrc, int64_t ro
 }
 
 // out += the children's updates of n rows (from row `from` on), in the children's order: the thread's entries tid + i SWT, i < N, each a column
-// pair p of row rt + i RS.  Two entries' values of two children are in flight together; four spill registers (1929 us per
-// application with 128 columns against 2608).
+// pair p of row rt + i RS.  Two entries' values of two children are in flight together; four spill registers, which
+// took an application with 128 columns 1.35 times as long.
 template <int NP, int N>
 __device__ __forceinline__ void sw_add_children(const SwArgs& A, int nsrc, int64_t row0, int n, int from, const int* rows0,
                                                 const int* rows1, const float4* u, float4* out, int tid) {
