@@ -968,15 +968,26 @@ static int solve_impl(gt_geometry* G, gt_operators* ops, int ncol, const int* h_
         precond<R>(G, ops, rin, ldr, out, n, nsl, W.slot_pc, g, gmax, zfac, yfac, uvec, sd, W.yint, W.cnt, W.gave_up, st, list,
                    rscale);
     };
-    std::vector<int> slot_col, slot_op, slot_pc, gptr, gslot, gop, gpair, act;
+    std::vector<int> slot_col, slot_op, slot_pc, act;
+    // the group tables, in three sets in turn: when one is made again, the host has seen the end of a step that was launched
+    // behind its last copies
+    struct Tables {
+        std::vector<int> slots, gptr, gslot, gop, gpair;
+    } tables[3];
+    int set = 0;
     auto upload_groups = [&](const std::vector<int>& slots) {
-        make_groups(slots, slot_pc, gmax, gptr, gslot, gop, gpair);
-        GT_CUDA(cudaMemcpyAsync(W.act, slots.data(), slots.size() * sizeof(int), cudaMemcpyHostToDevice, st));
-        GT_CUDA(cudaMemcpyAsync(W.g_ptr, gptr.data(), gptr.size() * sizeof(int), cudaMemcpyHostToDevice, st));
-        GT_CUDA(cudaMemcpyAsync(W.g_slot, gslot.data(), gslot.size() * sizeof(int), cudaMemcpyHostToDevice, st));
-        GT_CUDA(cudaMemcpyAsync(W.g_op, gop.data(), gop.size() * sizeof(int), cudaMemcpyHostToDevice, st));
-        GT_CUDA(cudaMemcpyAsync(W.g_pair, gpair.data(), gpair.size() * sizeof(int), cudaMemcpyHostToDevice, st));
-        return Groups{(int)gop.size(), W.g_ptr, W.g_slot, W.g_op, W.g_pair};
+        Tables& t = tables[set = (set + 1) % 3];
+        t.slots = slots;
+        make_groups(t.slots, slot_pc, gmax, t.gptr, t.gslot, t.gop, t.gpair);
+        auto put = [&](int* d, const std::vector<int>& h) {
+            GT_CUDA(cudaMemcpyAsync(d, h.data(), h.size() * sizeof(int), cudaMemcpyHostToDevice, st));
+        };
+        put(W.act, t.slots);
+        put(W.g_ptr, t.gptr);
+        put(W.g_slot, t.gslot);
+        put(W.g_op, t.gop);
+        put(W.g_pair, t.gpair);
+        return Groups{(int)t.gop.size(), W.g_ptr, W.g_slot, W.g_op, W.g_pair};
     };
     const int K = std::max(1, o.outer_k);
     const int64_t ldk = (int64_t)ncol * n;          // between GCR directions
