@@ -308,8 +308,8 @@ __device__ bool sw_task(const SwArgs& A, SwShared& sm, uint32_t& it, const SwDes
     // A thread's entries (of the staged rows and of the outputs) are one column pair of every RS-th row.  All that does not
     // depend on other tasks is fetched before their results are waited for: the rows' sources, the right-hand sides, what
     // the outputs need besides the product.  A tile's time is in these chains of loads (row index, then value), not in its
-    // product: fetched one entry after the other, after the wait, they made an application 708 us with 32 columns (534
-    // now), 2316 with 128 (1787), 393 with 6 on the stack (309), 77 and 56 with one column on small planes (49 and 38).
+    // product: fetched one entry after the other, after the wait, they made an application 708 us with 32 columns (529
+    // now), 2316 with 128 (1695), 393 with 6 on the stack (314), 77 and 56 with one column on small planes (49 and 38).
     constexpr int RS = SWT / NP, XE = SW_XROWS / RS, HE = SW_HMAX / RS;
     const int p = tid % NP, rt = tid / NP;
     const int c0 = 2 * p < gc ? gs[2 * p] : -1, c1 = 2 * p + 1 < gc ? gs[2 * p + 1] : -1;
@@ -348,8 +348,9 @@ __device__ bool sw_task(const SwArgs& A, SwShared& sm, uint32_t& it, const SwDes
         sw_sync();
         sw_stage_back<NP, XE>(z, y, xend - xbeg, t.nown - xbeg, sm.xrow[0], sm.x, tid);
     }
+    const int quit = *(const volatile int*)&sm.quit;     // (set before the first barrier, or not at all)
     sw_sync();
-    if (*(const volatile int*)&sm.quit) return false;
+    if (quit) return false;
     uint64_t re[2][NP], im[2][NP];
 #pragma unroll
     for (int r = 0; r < 2; ++r)
