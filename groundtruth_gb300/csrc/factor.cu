@@ -579,22 +579,32 @@ __global__ void __launch_bounds__(256) inv_trail_kernel(Fronts F, const int64_t*
     }
 }
 
+// the large fronts of all levels in a launch: they stand in the grid's second dimension, which ends at 65,535 (six planes of
+// 1024 x 1024 have 31,000 of them)
+template <typename L>
+static void in_parts(int nfront, L&& launch) {
+    constexpr int MOST = 65535;
+    for (int f = 0; f < nfront; f += MOST) launch(f, std::min(MOST, nfront - f));
+}
+
 void launch_invert_tiled(const Fronts& F, const int64_t* front_list, const InvertPlan& plan, c64* panel, const c64* xinv,
                          const int* xfirst, int64_t xtotal, int nops, cudaStream_t st) {
     const DiagInv X{const_cast<c64*>(xinv), xfirst, xtotal};
     for (size_t s = 0; s < plan.count.size(); ++s) {
-        const int kb = (int)s * FB, n = plan.count[s];
-        pdl_launch(inv_rows_kernel, dim3(kb / 32 + 1, n, nops), 256, 0, st, F, front_list, kb, panel, X);
-        GT_LAUNCH_CHECK();
-        const int below = plan.max_nf[s] - kb - 1;
-        if (below <= 0) continue;
-        const int rt = ceil_div(below, FT);
-        if (kb > 0) {
-            pdl_launch(inv_trail_kernel, dim3(rt * ceil_div(kb, FT), n, nops), 256, 0, st, F, front_list, kb, panel, 0);
+        const int kb = (int)s * FB;
+        const int below = plan.max_nf[s] - kb - 1, rt = ceil_div(std::max(below, 0), FT);
+        in_parts(plan.count[s], [&](int first, int n) {
+            const int64_t* fr = front_list + first;
+            pdl_launch(inv_rows_kernel, dim3(kb / 32 + 1, n, nops), 256, 0, st, F, fr, kb, panel, X);
             GT_LAUNCH_CHECK();
-        }
-        pdl_launch(inv_trail_kernel, dim3(rt, n, nops), 256, 0, st, F, front_list, kb, panel, 1);
-        GT_LAUNCH_CHECK();
+            if (below <= 0) return;
+            if (kb > 0) {
+                pdl_launch(inv_trail_kernel, dim3(rt * ceil_div(kb, FT), n, nops), 256, 0, st, F, fr, kb, panel, 0);
+                GT_LAUNCH_CHECK();
+            }
+            pdl_launch(inv_trail_kernel, dim3(rt, n, nops), 256, 0, st, F, fr, kb, panel, 1);
+            GT_LAUNCH_CHECK();
+        });
     }
 }
 
@@ -629,9 +639,10 @@ __global__ void panel_convert_kernel(Fronts F, SweepPlan S, const int64_t* __res
 
 void launch_panel_convert(const Fronts& F, const SweepPlan& S, const int64_t* front_list, int nfront, c64* p64, c32* pf, c32* pb,
                           c64* r64, c64* d64, c32* d32, int nops, cudaStream_t st) {
-    if (nfront <= 0) return;
-    pdl_launch(panel_convert_kernel, dim3(16, nfront, nops), 256, 0, st, F, S, front_list, p64, pf, pb, r64, d64, d32);
-    GT_LAUNCH_CHECK();
+    in_parts(nfront, [&](int first, int n) {
+        pdl_launch(panel_convert_kernel, dim3(16, n, nops), 256, 0, st, F, S, front_list + first, p64, pf, pb, r64, d64, d32);
+        GT_LAUNCH_CHECK();
+    });
 }
 
 // ------------------------------------------------------------------------------------------ solves
